@@ -37,9 +37,9 @@ _REF_DEFAULT = "/root/reference"
 
 def ref_dir() -> str | None:
     """The reference tree the checker compiles in place: HYPE_REF_DIR, else the recipe's
-    default location; None where neither exists (then only the restatement is built)."""
+    default location; None where neither holds its sources (then only the restatement is built)."""
     d = os.environ.get("HYPE_REF_DIR") or _REF_DEFAULT
-    return d if os.path.isdir(d) else None
+    return d if os.path.isdir(os.path.join(d, "3d")) else None
 
 
 def build(ref: str | None = None, quiet: bool = True) -> None:
