@@ -6,7 +6,9 @@
 // polynomial at the 2x2 Gauss points of every face, the central flux
 // c^2 (grad_L + grad_R) . n / 2 (pde.c:12-34), and SSPRK(4,3) with a fixed dt.
 //
-// Per RHS evaluation (rhs_function.c:12-345):
+// With the R4 polynomial (the program's setting) the scheme is linear with constant
+// coefficients, and a whole stage is one kernel over a 19-point star (k_ac_star below).
+// With CWENO4, per RHS evaluation (rhs_function.c:12-345):
 //   k_ac_ghost   u with 3 ghost layers: periodic wrap, or the adiabatic wall's odd
 //                mirror u_ghost = -u (rhs_function.c:43-131);
 //   k_ac_recon   per extended cell: the 33-point stencil, CWENO4 / R4 coefficients,
@@ -121,7 +123,7 @@ __device__ __forceinline__ void face_normal_grads(const double* c, double* __res
 
 // T[face][gp][extended cell]: the face-normal gradient (times h) at the 4 Gauss points
 // of the 6 faces; Gauss point q = 2 (t1 > 0) + (t2 > 0), (t1, t2) the remaining axes
-__global__ void __launch_bounds__(128) k_ac_recon(const double* __restrict__ G, double* __restrict__ T, Geo g, int linear) {
+__global__ void __launch_bounds__(128) k_ac_recon(const double* __restrict__ G, double* __restrict__ T, Geo g) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y - 1;
     const int k = blockIdx.z - 1;
@@ -153,7 +155,7 @@ __global__ void __launch_bounds__(128) k_ac_recon(const double* __restrict__ G, 
         for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int d = 0; d < 2; ++d) s[euler::SO(a, b, d)] = __ldg(p + (2 * a - 1) + (2 * b - 1) * sy + (2 * d - 1) * sz);
-    euler::cweno4<double>(s, linear != 0, cf);
+    euler::cweno4<double>(s, false, cf);
     const long long e = ext_index(g, i, j, k);
     face_normal_grads<0>(cf, T, g.NE, e);
     face_normal_grads<1>(cf, T, g.NE, e);
@@ -187,10 +189,9 @@ __device__ __forceinline__ void face_normal_grads_df(const df64* c, df64* __rest
     }
 }
 
-// k_ac_recon in double-float: the R4 / CWENO4 coefficients (euler_df64.cuh) and the 24 face-
+// k_ac_recon in double-float: the CWENO4 coefficients (euler_df64.cuh) and the 24 face-
 // normal gradients, kept as pairs for k_ac_faces_df
-__global__ void __launch_bounds__(128, 2) k_ac_recon_df(const df64* __restrict__ G, df64* __restrict__ T, Geo g,
-                                                        int linear) {
+__global__ void __launch_bounds__(128, 2) k_ac_recon_df(const df64* __restrict__ G, df64* __restrict__ T, Geo g) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y - 1;
     const int k = blockIdx.z - 1;
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(128, 2) k_ac_recon_df(const df64* __restrict__
         for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int d = 0; d < 2; ++d) s[euler::SO(a, b, d)] = p[(2 * a - 1) + (2 * b - 1) * sy + (2 * d - 1) * sz];
-    euler::cweno4_df(s, linear != 0, cf);
+    euler::cweno4_df(s, false, cf);
     const long long e = ext_index(g, i, j, k);
     face_normal_grads_df<0>(cf, T, g.NE, e);
     face_normal_grads_df<1>(cf, T, g.NE, e);
@@ -303,6 +304,96 @@ __global__ void __launch_bounds__(256) k_ac_update(const double* __restrict__ Fx
     }
 }
 
+// ---------------------------------------------------------------- the linear scheme as one star
+// With the R4 polynomial every step from u to the divergence is linear.  Averaged over the 2x2
+// Gauss points of a face (coordinates +-GPT, whose squares average to 1/12) the gradient
+// component normal to it keeps only the terms c_D + 0.6 c_DDD +- c_DD of face_normal_grads, all
+// of them along D, and the mean of the two sides' gradients differenced over the cell is
+//   (F_{i+1/2} - F_{i-1/2}) h / c^2 = 49/48 s1 + 1/24 s2 - 1/48 s3 - 25/12 w,  s_k = w_{i-k} + w_{i+k}
+// (R4's derivatives, reconstruction.c:90-108, the central flux pde.c:12-34), so a stage is
+//   out_u = a U_u + b W_u + c dt W_v,   out_v = a U_v + b W_v + c dt c^2 / h^2 (sum over x, y, z).
+// s1 is summed as differences to w (exact where the neighbours lie within a factor 2): the
+// second difference carries no rounding of the size of w, and what is left, s2 / 24 - s3 / 48 -
+// w / 24, enters scaled by 1/24.
+//
+// Bound: FP64 issue, 26 FP64 instructions per cell and stage against about 280 for the
+// polynomial form and its trace and flux arrays; a thread marches kz planes of its column with
+// the seven z values in registers and reads its x and y neighbours through L1.  The plane is
+// indexed flat, so no warp is left partly empty at the end of a row (its FP64 instructions cost
+// the same with one active lane as with 32).  200^3: 14.5 -> 1.82 ms per step (4.4 G cell-updates/s,
+// 73 % of the FP64 issue ceiling); 16^3: 120 -> 27 us.
+struct StarCoef {
+    double k0, k1, k2, k3;  // of w, sum of (w_k - w) over the six nearest, s2 and s3 summed over the axes
+    double cdt;             // c dt (0 for RHS-only calls)
+};
+constexpr int kStarThreads = 256;
+
+template <bool RHS_ONLY, bool WITH_U>
+__global__ void __launch_bounds__(kStarThreads) k_ac_star(const double* __restrict__ W, const double* __restrict__ U,
+                                                          double* __restrict__ out, Geo g, StarCoef kc, double a,
+                                                          double b, SourceArgs src, int kz) {
+    const int plane = g.nx * g.ny;
+    const int q = blockIdx.x * kStarThreads + threadIdx.x;
+    if (q >= plane) return;
+    const int i = q % g.nx, j = q / g.nx;
+    // offsets from the cell to its x and y neighbours at -3..-1, 1..3 (periodic wrap or the adiabatic
+    // wall's mirror) and, one bit each, the sign of a mirrored value
+    int off[12];
+    unsigned neg = 0;
+#pragma unroll
+    for (int o = 0; o < 6; ++o) {
+        const int d = o < 3 ? o - 3 : o - 2;
+        int f = 0;
+        off[o] = amap(i + d, g.nx, g.bc[0], g.bc[1], &f) - i;
+        neg |= (unsigned)f << o;
+        f = 0;
+        off[6 + o] = (amap(j + d, g.ny, g.bc[2], g.bc[3], &f) - j) * g.nx;
+        neg |= (unsigned)f << (6 + o);
+    }
+    auto signed_as = [](double v, unsigned f) {
+        return __hiloint2double(__double2hiint(v) ^ (int)(f << 31), __double2loint(v));
+    };
+    auto at_z = [&](int k) {
+        int f = 0;
+        const int m = amap(k, g.nz, g.bc[4], g.bc[5], &f);
+        return signed_as(__ldg(W + (long long)m * plane + q), (unsigned)f);
+    };
+    const int k0 = blockIdx.y * kz, k1 = min(k0 + kz, g.nz);
+    double z[7];
+#pragma unroll
+    for (int o = 0; o < 6; ++o) z[o + 1] = at_z(k0 + o - 3);
+    double dlo = z[4] - z[3];
+    for (int k = k0; k < k1; ++k) {
+#pragma unroll
+        for (int o = 0; o < 6; ++o) z[o] = z[o + 1];
+        z[6] = at_z(k + 3);
+        const long long cell = (long long)k * plane + q;
+        const double* p = W + cell;
+        double n[12];
+#pragma unroll
+        for (int o = 0; o < 12; ++o) n[o] = signed_as(__ldg(p + off[o]), (neg >> o) & 1u);
+        const double v = __ldg(W + g.N + cell);
+        const double w = z[3], dhi = z[4] - w;
+        const double t1 = ((n[2] - w) + (n[3] - w)) + ((n[8] - w) + (n[9] - w)) + (dhi - dlo);
+        const double s2 = (n[1] + n[4]) + (n[7] + n[10]) + (z[1] + z[5]);
+        const double s3 = (n[0] + n[5]) + (n[6] + n[11]) + (z[0] + z[6]);
+        dlo = dhi;
+        double div = fma(kc.k1, t1, fma(kc.k2, s2, fma(kc.k3, s3, kc.k0 * w)));
+        if (cell == src.rec_cell) *src.slot = w;
+        if (RHS_ONLY) {
+            if (cell == src.src_cell) div += src.src_val;
+            out[cell] = v;
+            out[g.N + cell] = div;
+        } else {
+            if (cell == src.src_cell) div = fma(kc.cdt, src.src_val, div);
+            const double bu = WITH_U ? fma(a, __ldg(U + cell), b * w) : w;
+            const double bv = WITH_U ? fma(a, __ldg(U + g.N + cell), b * v) : v;
+            out[cell] = fma(kc.cdt, v, bu);
+            out[g.N + cell] = bv + div;
+        }
+    }
+}
+
 __global__ void k_ac_aos2soa(const double* __restrict__ a, double* __restrict__ s, long long N) {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (q >= N) return;
@@ -328,15 +419,38 @@ struct hype_acoustic {
     cudaStream_t stream = nullptr;
     double *U = nullptr, *W = nullptr, *L = nullptr, *S = nullptr, *Gh = nullptr, *T = nullptr;
     double *Fx = nullptr, *Fy = nullptr, *Fz = nullptr, *aos = nullptr;
+    int nsm = 1;
     PointSource ps;
 };
+
+// One RK stage, out = a U + b W + (c dt) L(W) (or out = L(W)); t is the time of the RHS evaluation (the
+// point source's argument).  The star reads its neighbours from W: out must be another array.
+static int ac_star(hype_acoustic* s, const double* U, const double* W, double* out, Stage st, double dt, double t) {
+    const Geo& g = s->g;
+    const double cdt = st.rhs_only ? 0.0 : st.c * dt;
+    const double k = (st.rhs_only ? 1.0 : cdt) * (s->p.c * s->p.c) / (s->p.h * s->p.h);
+    // w appears as 49/48 (s1 - 2 w) + ... with 3 axes: -25/12 + 49/24 = -1/24 each
+    const StarCoef kc{-0.125 * k, (49.0 / 48.0) * k, k / 24.0, -k / 48.0, cdt};
+    // planes per thread: long columns re-read six planes less often, short ones fill the chip on small
+    // grids; 12 blocks per SM keep the last wave's share small
+    const unsigned bx = cdiv((long long)g.nx * g.ny, kStarThreads);
+    int kz = 16;
+    while (kz > 1 && (long long)bx * cdiv(g.nz, kz) < 12LL * s->nsm) kz /= 2;
+    const dim3 gr(bx, cdiv(g.nz, kz));
+    const SourceArgs src = source_args(s->ps, t);
+    if (st.rhs_only) k_ac_star<true, false><<<gr, kStarThreads, 0, s->stream>>>(W, U, out, g, kc, 0.0, 0.0, src, kz);
+    else if (st.a != 0.0) k_ac_star<false, true><<<gr, kStarThreads, 0, s->stream>>>(W, U, out, g, kc, st.a, st.b, src, kz);
+    else k_ac_star<false, false><<<gr, kStarThreads, 0, s->stream>>>(W, U, out, g, kc, 0.0, 1.0, src, kz);
+    HYPE_LAUNCHED(1);
+    return HYPE_OK;
+}
 
 static int ac_rhs(hype_acoustic* a, const double* Win) {
     const Geo& g = a->g;
     if (a->p.precision == HYPE_PREC_DF64) {
         k_ac_ghost<df64><<<dim3(cdiv(g.gx, 128), g.gy, g.nz + 2 * GW), 128, 0, a->stream>>>(Win, (df64*)a->Gh, g);
         k_ac_recon_df<<<dim3(cdiv(g.nx + 2, 32), cdiv(g.ny + 2, 4), g.nz + 2), dim3(32, 4), 0, a->stream>>>(
-            (const df64*)a->Gh, (df64*)a->T, g, a->p.recon == HYPE_RECON_LINEAR4);
+            (const df64*)a->Gh, (df64*)a->T, g);
         const double c2 = a->p.c * a->p.c;
         const dim3 bf(32, 4);
         const df64* T = (const df64*)a->T;
@@ -348,7 +462,7 @@ static int ac_rhs(hype_acoustic* a, const double* Win) {
     }
     k_ac_ghost<double><<<dim3(cdiv(g.gx, 128), g.gy, g.nz + 2 * GW), 128, 0, a->stream>>>(Win, a->Gh, g);
     k_ac_recon<<<dim3(cdiv(g.nx + 2, 32), cdiv(g.ny + 2, 4), g.nz + 2), dim3(32, 4), 0, a->stream>>>(
-        a->Gh, a->T, g, a->p.recon == HYPE_RECON_LINEAR4);
+        a->Gh, a->T, g);
     const double c2 = a->p.c * a->p.c;
     const dim3 bf(32, 4);
     k_ac_faces<0><<<dim3(cdiv(g.nx + 1, 32), cdiv(g.ny, 4), g.nz), bf, 0, a->stream>>>(a->T, a->Fx, g, c2);
@@ -365,6 +479,16 @@ static int ac_update(hype_acoustic* a, const double* U, const double* W, double*
         a->Fx, a->Fy, a->Fz, U, W, out, g, 1.0 / (a->p.h * a->p.h), st, dt, source_args(a->ps, t));
     HYPE_LAUNCHED(1);
     return HYPE_OK;
+}
+
+// One RK stage by the form the reconstruction takes: the star for the linear scheme in both precisions
+// (its FP64 sum costs less than the double-float polynomial form and rounds less: 256^3, ms per step,
+// polynomial FP64 29.7, polynomial double-float 10.1, star 3.62), or ghost fill, reconstruction, faces
+// and update (CWENO4).
+static int ac_stage(hype_acoustic* a, const double* U, const double* W, double* out, Stage st, double dt, double t) {
+    if (a->p.recon == HYPE_RECON_LINEAR4) return ac_star(a, U, W, out, st, dt, t);
+    const int rc = ac_rhs(a, W);
+    return rc ? rc : ac_update(a, U, W, out, st, dt, t);
 }
 
 extern "C" int hype_acoustic_create(const hype_acoustic_params* p, hype_acoustic** out) {
@@ -393,11 +517,16 @@ extern "C" int hype_acoustic_create(const hype_acoustic_params* p, hype_acoustic
     double** bufs[] = {&a->U, &a->W, &a->L, &a->S, &a->aos};
     for (auto b : bufs)
         if (ce == cudaSuccess) ce = cudaMalloc((void**)b, sN);
-    if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->Gh, sizeof(double) * (size_t)g.GN);
-    if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->T, sizeof(double) * NTR * (size_t)g.NE);
-    if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->Fx, sizeof(double) * (size_t)(p->nx + 1) * p->ny * p->nz);
-    if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->Fy, sizeof(double) * (size_t)p->nx * (p->ny + 1) * p->nz);
-    if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->Fz, sizeof(double) * (size_t)p->nx * p->ny * (p->nz + 1));
+    int dev = 0;
+    if (ce == cudaSuccess) ce = cudaGetDevice(&dev);
+    if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&a->nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (p->recon == HYPE_RECON_CWENO4) {  // the star keeps no ghosted copy, traces or face fluxes
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->Gh, sizeof(double) * (size_t)g.GN);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->T, sizeof(double) * NTR * (size_t)g.NE);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->Fx, sizeof(double) * (size_t)(p->nx + 1) * p->ny * p->nz);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->Fy, sizeof(double) * (size_t)p->nx * (p->ny + 1) * p->nz);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&a->Fz, sizeof(double) * (size_t)p->nx * p->ny * (p->nz + 1));
+    }
     if (ce != cudaSuccess) {
         set_last_error("hype_acoustic_create", ce);
         hype_acoustic_destroy(a);
@@ -450,8 +579,7 @@ extern "C" int hype_acoustic_download(hype_acoustic* a, double* U_aos) {
 extern "C" int hype_acoustic_rhs_t(hype_acoustic* a, double t, const double* U_aos, double* RHS_aos) {
     if (!a || !U_aos || !RHS_aos) return HYPE_ERR_ARG;
     int rc = ac_h2d(a, U_aos, a->S);
-    if (rc || (rc = ac_rhs(a, a->S))) return rc;
-    if ((rc = ac_update(a, a->S, a->S, a->L, Stage{0.0, 0.0, 0.0, 1}, 0.0, t))) return rc;
+    if (rc || (rc = ac_stage(a, a->S, a->S, a->L, Stage{0.0, 0.0, 0.0, 1}, 0.0, t))) return rc;
     return ac_d2h(a, a->L, RHS_aos);
 }
 
@@ -517,11 +645,12 @@ extern "C" int hype_acoustic_step(hype_acoustic* a, int nsteps, double t_final, 
         double dt = a->p.dt;
         if (t_final > 0.0 && t + dt > t_final) dt = t_final - t;
         int rc;
-        // u1 = u + dt/2 L(u); u2 = u1 + dt/2 L(u1); u3 = 2/3 u + u2/3 + dt/6 L(u2); u3 + dt/2 L(u3)
-        if ((rc = ac_rhs(a, a->U)) || (rc = ac_update(a, a->U, a->U, a->W, s12, dt, t + ct(0) * dt))) return rc;
-        if ((rc = ac_rhs(a, a->W)) || (rc = ac_update(a, a->U, a->W, a->W, s12, dt, t + ct(1) * dt))) return rc;
-        if ((rc = ac_rhs(a, a->W)) || (rc = ac_update(a, a->U, a->W, a->W, s3, dt, t + ct(2) * dt))) return rc;
-        if ((rc = ac_rhs(a, a->W)) || (rc = ac_update(a, a->U, a->W, a->U, s12, dt, t + ct(3) * dt))) return rc;
+        // u1 = u + dt/2 L(u); u2 = u1 + dt/2 L(u1); u3 = 2/3 u + u2/3 + dt/6 L(u2); u3 + dt/2 L(u3);
+        // no stage writes the array whose neighbours it reads
+        if ((rc = ac_stage(a, a->U, a->U, a->W, s12, dt, t + ct(0) * dt))) return rc;
+        if ((rc = ac_stage(a, a->U, a->W, a->L, s12, dt, t + ct(1) * dt))) return rc;
+        if ((rc = ac_stage(a, a->U, a->L, a->W, s3, dt, t + ct(2) * dt))) return rc;
+        if ((rc = ac_stage(a, a->U, a->W, a->U, s12, dt, t + ct(3) * dt))) return rc;
         t += dt;
     }
     HYPE_CK(cudaStreamSynchronize(a->stream));

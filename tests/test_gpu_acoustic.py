@@ -166,3 +166,33 @@ def test_df64_convergence_table_and_point_source(hype, oracle):
                                                                                       250.0, 100.0))
     print(f"acoustic df64 point source 100^3: receiver misfit {misfit:.3e}")
     assert misfit < 5e-3
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+@pytest.mark.parametrize("shape,bc", [((3, 3, 3), (4,) * 6), ((3, 4, 5), (0,) * 6), ((257, 3, 4), (4, 4, 0, 0, 4, 4)),
+                                      ((16, 16, 17), (0, 0, 4, 4, 0, 0)), ((31, 33, 40), (4,) * 6),
+                                      ((5, 7, 70), (0, 0, 4, 4, 4, 4))])
+def test_linear_star_edges(hype, oracle, shape, bc, precision):
+    """the one-kernel stage of the linear scheme at the edges of its plane blocks (256 cells) and
+    z columns (1..16 planes), against the checker: RHS and five steps with a source and a receiver.
+    RHS tolerance: the star sums terms of at most 13 |u| / h^2 with a rounding of 2^-53 each, the
+    checker its own polynomial terms alike, so 64 such roundings bound the difference."""
+    rng = np.random.default_rng(7)
+    U = rng.standard_normal(shape[::-1] + (2,))
+    h = 0.1
+    cfg = oracle.acoustic_cfg(shape, h, bc=bc)
+    s = hype.AcousticFV3D(*shape, h, 0.02, boundaries=bc, precision=precision)
+    R = s.RHSFunction(0.0, U)
+    Ro = oracle.acoustic_rhs(cfg, U)
+    assert np.array_equal(R[..., 0], U[..., 1])
+    assert np.abs(R - Ro).max() <= 64 * 2.0**-53 * 13 * np.abs(U).max() / h**2
+    src, rec = tuple(n // 2 for n in shape), (0, shape[1] - 1, shape[2] - 1)
+    s.set_point_source(src, 3.0, rec, 20)
+    s.set_state(U)
+    s.step(5)
+    with oracle.point_source(src, 3.0, rec) as S:
+        Uo, t, n = oracle.acoustic_run(cfg, U, 5, 0.02)
+    to, uo, cnt = S.trace()
+    assert rel(s.get_state(), Uo) <= 1e-12
+    tt, u, c = s.receiver_trace()
+    assert c == cnt == 20 and np.array_equal(tt, to) and np.abs(u - uo).max() <= 1e-12 * np.abs(U).max()
