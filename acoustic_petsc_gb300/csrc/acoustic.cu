@@ -21,6 +21,7 @@
 #include <math.h>
 #include <string.h>
 
+#include "cweno64.cuh"
 #include "euler_df64.cuh"
 #include "euler_kernels.cuh"
 #include "point_source.cuh"
@@ -155,7 +156,9 @@ __global__ void __launch_bounds__(128) k_ac_recon(const double* __restrict__ G, 
         for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int d = 0; d < 2; ++d) s[euler::SO(a, b, d)] = __ldg(p + (2 * a - 1) + (2 * b - 1) * sy + (2 * d - 1) * sz);
-    euler::cweno4<double>(s, false, cf);
+    euler::Poly64 poly;
+    euler::cweno4_64(s, poly);
+    euler::coeffs64(poly, cf);
     const long long e = ext_index(g, i, j, k);
     face_normal_grads<0>(cf, T, g.NE, e);
     face_normal_grads<1>(cf, T, g.NE, e);

@@ -1,15 +1,15 @@
 // euler.cu -- 3D Euler CWENO4 + Rusanov RHS and the SSPRK(4,3) stepper on sm_103a.
 //
-// Per RK stage three kernels run on the context's stream:
-//   recon  : one thread per cell of the extended box [-1,n]^3 that some face of an
-//            owned cell needs; ghost values come from the boundary index map
-//            (replaces DMGlobalToLocal + the BC sweeps of
-//            3d/weno4/Navier-Stokes-3D/rhs_function.c:41-181); writes the 24 face
-//            Gauss-point traces of each variable (rhs_function.c:185-274);
-//   faces  : one thread per face and direction; four Rusanov solves at the 2x2
-//            Gauss points, the weighted flux (rhs_function.c:276-417), the block
-//            max of the wave speed (atomicMax on the bit pattern: speeds are >= 0)
-//            and the admissibility flag (replaces MPI_Abort, pde.c:56-66);
+// Per RK stage four kernels run on the context's stream (FP64; the other forms alike):
+//   ghost  : the stage input with three ghost layers (replaces DMGlobalToLocal + the
+//            BC sweeps of 3d/weno4/Navier-Stokes-3D/rhs_function.c:41-181);
+//   recon  : one thread per variable and cell of the extended box [-1,n]^3 that some
+//            face of an owned cell needs; writes the 24 face Gauss-point traces
+//            (rhs_function.c:185-274);
+//   faces  : all three directions; one Riemann solve per thread, the weighted flux
+//            (rhs_function.c:276-417), the block max of the wave speed (atomicMax on
+//            the bit pattern: speeds are >= 0) and the admissibility flag (replaces
+//            MPI_Abort, pde.c:56-66);
 //   update : flux divergence (rhs_function.c:419-433) fused with the SSP stage
 //            combination; dt comes from device memory, so a whole step needs no
 //            host round trip.
@@ -24,6 +24,7 @@
 
 #include <vector>
 
+#include "cweno64.cuh"
 #include "euler_df64.cuh"
 #include "euler_kernels.cuh"
 #include "mlp_kernels.cuh"
@@ -290,13 +291,12 @@ __device__ __forceinline__ void store_first_order_g(const R* __restrict__ G, R* 
     }
 }
 
-// Reconstruction of every owned cell and of the first ghost layer (faces of the
-// domain boundary); the FP32 form checks admissibility in dynamic shared memory
+// FP32 reconstruction of every owned cell and of the first ghost layer (faces of the
+// domain boundary), admissibility checked in dynamic shared memory
 // (4 warps x 2 x NTR x 32 floats, launched only with the positivity fallback on).
-template <typename R>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
-    k_recon(const R* __restrict__ G, R* __restrict__ T, Geo g, int recon, int pad, double gm1,
-            unsigned long long* __restrict__ counters, double* __restrict__ C4 = nullptr, double c4_scale = 1.0) {
+__global__ void __launch_bounds__(128, 4)
+    k_recon_f32(const float* __restrict__ G, float* __restrict__ T, Geo g, int recon, int pad, double gm1,
+                unsigned long long* __restrict__ counters) {
     extern __shared__ float ck_dyn[];
     const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y - 1;
@@ -306,32 +306,80 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
     if (gi + gj + gk > 1) return;  // edge/corner ghosts feed no face of an owned cell
     const long long e = ext_index(g, i, j, k), ge = ghost_index(g, i, j, k);
     const int sy = g.gx, sz = g.gx * g.gy;
-    constexpr bool f32 = sizeof(R) == sizeof(float);
     TraceCheck ck{ck_dyn + threadIdx.y * (2 * NTR * 32) + threadIdx.x, (float)gm1, true};
-    TraceCheck* ckp = (f32 && pad) ? &ck : nullptr;
+    TraceCheck* ckp = pad ? &ck : nullptr;
 #pragma unroll 1
     for (int c = 0; c < NV; ++c) {
-        R s[33], cf[20];
-        gather33g<R>(G + (long long)c * g.GN + ge, sy, sz, s);
-        if (recon == HYPE_RECON_WENO3) weno3<R>(s, cf);
-        else cweno4<R>(s, recon == HYPE_RECON_LINEAR4, cf);
-        store_traces<R>(T, g, e, c, cf, ckp);
-        if (sizeof(R) == sizeof(double) && C4) {  // the R4 polynomial, whose gradients the viscous fluxes take
-            R r4[20];
-            if (recon == HYPE_RECON_LINEAR4) {
-#pragma unroll
-                for (int q = 0; q < 20; ++q) r4[q] = cf[q];
-            } else {
-                cweno4<R>(s, true, r4);
-            }
-#pragma unroll
-            for (int q = 0; q < 20; ++q) C4[((long long)c * 20 + q) * g.NE + e] = (double)r4[q] * c4_scale;
-        }
+        float s[33], cf[20];
+        gather33g<float>(G + (long long)c * g.GN + ge, sy, sz, s);
+        if (recon == HYPE_RECON_WENO3) weno3<float>(s, cf);
+        else cweno4<float>(s, recon == HYPE_RECON_LINEAR4, cf);
+        store_traces<float>(T, g, e, c, cf, ckp);
     }
-    if (pad && !(f32 ? ck.ok : traces_admissible<R>(T, g, e, gm1))) {
-        store_first_order_g<R>(G, T, g, ge, e);
+    if (pad && !ck.ok) {
+        store_first_order_g<float>(G, T, g, ge, e);
         if (!gi && !gj && !gk) atomicAdd(&counters[1], 1ull);
     }
+}
+
+// FP64 reconstruction of the same cells, one thread per variable and cell (blockIdx.y = variable), or,
+// with the positivity fallback (PAD), one per cell with the variables in turn.
+// Bound: FP64 issue (361 operations per variable with CWENO4; DRAM below 4 % of peak).  The cells are
+// indexed flat over the extended box: a warp of 32 x-neighbours per row left 11 % of the lanes idle at
+// nx + 2 = 258 and 44 % at 18, at the full cost of its FP64 instructions.  A variable per thread gives a
+// small grid five times the warps (16^3: 183 warps of one serial 2300-instruction thread each took
+// 87 us) and leaves no loop around the 190-register body.  kThreads is small so that few blocks spread
+// evenly over the SMs.
+constexpr int kReconThreads = 64;
+
+template <int RECON, bool PAD>
+__global__ void __launch_bounds__(kReconThreads)
+    k_recon64(const double* __restrict__ G, double* __restrict__ T, Geo g, double gm1,
+              unsigned long long* __restrict__ counters, double* __restrict__ C4) {
+    const unsigned e = blockIdx.x * (unsigned)kReconThreads + threadIdx.x;
+    if (e >= (unsigned)g.NE) return;
+    const unsigned row = e / (unsigned)g.ex, pl = row / (unsigned)g.ey;
+    const int i = (int)(e - row * (unsigned)g.ex) - 1, j = (int)(row - pl * (unsigned)g.ey) - 1, k = (int)pl - 1;
+    const int gi = (i < 0 || i >= g.nx), gj = (j < 0 || j >= g.ny), gk = (k < 0 || k >= g.nz);
+    if (gi + gj + gk > 1) return;  // edge/corner ghosts feed no face of an owned cell
+    const long long ge = ghost_index(g, i, j, k);
+    const int sy = g.gx, sz = g.gx * g.gy;
+    const int c0 = PAD ? 0 : blockIdx.y, c1 = PAD ? NV : c0 + 1;
+#pragma unroll 1
+    for (int c = c0; c < c1; ++c) {
+        double s[33];
+        gather33g<double>(G + (long long)c * g.GN + ge, sy, sz, s);
+        double* Tc = T + (long long)c * NTR * g.NE + e;
+        if constexpr (RECON == HYPE_RECON_WENO3) {
+            double cf[20];
+            weno3<double>(s, cf);
+            store_traces<double>(T, g, e, c, cf);
+        } else {
+            Poly64 poly;
+            if constexpr (RECON == HYPE_RECON_LINEAR4) r4_64(s, poly);
+            else cweno4_64(s, poly);
+            store_traces64(poly, Tc, g.NE);
+            if (RECON == HYPE_RECON_LINEAR4 && C4) store_grad_coeffs(poly, C4 + (long long)c * 20 * g.NE + e, g.NE);
+        }
+        if (RECON != HYPE_RECON_LINEAR4 && C4) {  // the viscous fluxes take the gradients of R4
+            Poly64 r4;
+            r4_64(s, r4);
+            store_grad_coeffs(r4, C4 + (long long)c * 20 * g.NE + e, g.NE);
+        }
+    }
+    if (PAD && !traces_admissible<double>(T, g, e, gm1)) {
+        store_first_order_g<double>(G, T, g, ge, e);
+        if (!gi && !gj && !gk) atomicAdd(&counters[1], 1ull);
+    }
+}
+
+static void launch_recon64(const Geo& g, const double* G, double* T, int recon, int pad, double gm1,
+                           unsigned long long* counters, double* C4, cudaStream_t st) {
+    const dim3 gr(cdiv(g.NE, kReconThreads), pad ? 1 : NV);
+    auto go = [&](auto kern) { kern<<<gr, kReconThreads, 0, st>>>(G, T, g, gm1, counters, C4); };
+    if (recon == HYPE_RECON_WENO3) pad ? go(k_recon64<HYPE_RECON_WENO3, true>) : go(k_recon64<HYPE_RECON_WENO3, false>);
+    else if (recon == HYPE_RECON_LINEAR4) pad ? go(k_recon64<HYPE_RECON_LINEAR4, true>) : go(k_recon64<HYPE_RECON_LINEAR4, false>);
+    else pad ? go(k_recon64<HYPE_RECON_CWENO4, true>) : go(k_recon64<HYPE_RECON_CWENO4, false>);
 }
 
 // HYPE_PREC_DF64: the per-variable reference value r_c of one stage, the stage input's
@@ -610,10 +658,18 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
             ck.ok = true;
 #pragma unroll 1
             for (int c = 0; c < NV; ++c) {
-                R s[33], cf[20];
+                R s[33];
                 gather33g<R>(G + (long long)c * g.GN + ge, sy, sz, s);
-                cweno4<R>(s, !full, cf);
-                store_traces<R>(T, g, e, c, cf, f32 ? &ck : nullptr);
+                if constexpr (f32) {
+                    R cf[20];
+                    cweno4<R>(s, !full, cf);
+                    store_traces<R>(T, g, e, c, cf, &ck);
+                } else {
+                    Poly64 poly;
+                    if (full) cweno4_64(s, poly);
+                    else r4_64(s, poly);
+                    store_traces64(poly, T + (long long)c * NTR * g.NE + e, g.NE);
+                }
             }
             if (f32 ? ck.ok : traces_admissible<R>(T, g, e, gm1)) break;
             if (full) {  // CWENO4 itself inadmissible: first order (when enabled)
@@ -786,8 +842,11 @@ __global__ void __launch_bounds__(128) k_features(const double* __restrict__ W, 
     for (int c = 0; c < NV; ++c) {
         double st[33], cf[20], cl[20], ta[8], tb[8];
         gather33<double, double>(W + (long long)c * g.N, c, g, m, st);
-        cweno4<double>(st, false, cf);
-        cweno4<double>(st, true, cl);
+        Poly64 poly;
+        cweno4_64(st, poly);
+        coeffs64(poly, cf);
+        r4_64(st, poly);
+        coeffs64(poly, cl);
         const double scale = mlp::var_scale<double>(c, rho, E) + 1e-30;
         double dd = 0.0;
         face_traces<double, 0>(cf, ta);
@@ -812,42 +871,6 @@ __global__ void __launch_bounds__(128) k_features(const double* __restrict__ W, 
 
 __device__ __forceinline__ void atomic_max_pos(unsigned long long* a, double v) {
     atomicMax(a, (unsigned long long)__double_as_longlong(v));
-}
-
-// The viscous fluxes of one face side at its 4 Gauss points, 0.125 F_v each, added to
-// av: NS = +1 for the low cell's high face, -1 for the high cell's low face.  The
-// traces come from T, the gradients from the cell's R4 coefficients (stored times 1/h).
-template <int D, int NS>
-__device__ __forceinline__ double visc_side(const double* __restrict__ T, const double* __restrict__ C4, const Geo& g,
-                                            long long e, double gamma, const Visc& vp, double* av) {
-    FaceGrad fg[NV][3];
-#pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        const double* p = C4 + (long long)c * 20 * g.NE + e;
-        fg[c][0] = face_grad<D, NS, 0>(p, g.NE);
-        fg[c][1] = face_grad<D, NS, 1>(p, g.NE);
-        fg[c][2] = face_grad<D, NS, 2>(p, g.NE);
-    }
-    constexpr int face = 2 * D + (NS > 0 ? 1 : 0);
-    double sv = 0.0;
-    auto at = [&](auto gpc) {
-        constexpr int gp = decltype(gpc)::value;
-        double Q[NV], G[NV][3], Fv[NV];
-#pragma unroll
-        for (int c = 0; c < NV; ++c) {
-            Q[c] = __ldg(T + ((long long)c * NTR + face * 4 + gp) * g.NE + e);
-#pragma unroll
-            for (int b = 0; b < 3; ++b) G[c][b] = fg_eval<gp>(fg[c][b]);
-        }
-        sv = fmax(sv, visc_flux<D>(Q, G, gamma - 1.0, vp.mu, vp.kc, vp.vmax, Fv));
-#pragma unroll
-        for (int c = 0; c < NV; ++c) av[c] = fma(0.125, Fv[c], av[c]);
-    };
-    at(std::integral_constant<int, 0>{});
-    at(std::integral_constant<int, 1>{});
-    at(std::integral_constant<int, 2>{});
-    at(std::integral_constant<int, 3>{});
-    return sv;
 }
 
 // Face fluxes of direction D.  Face index (i,j,k) is the face on the low side of
@@ -957,50 +980,40 @@ __global__ void __launch_bounds__(128) k_faces_df(const df64* __restrict__ T, do
     }
 }
 
-template <typename R, int D, int FLUX, bool VISC = false>
-__global__ void __launch_bounds__(128) k_faces(const R* __restrict__ T, double* __restrict__ F, Geo g, double gamma,
-                                               DevScalars* __restrict__ ds, int slot, const double* __restrict__ C4 = nullptr,
-                                               Visc vp = Visc{0.0, 0.0, 0.0, 0.0}) {
+// the FP32 face fluxes of direction D, one thread per face
+template <int D, int FLUX>
+__global__ void __launch_bounds__(128) k_faces_f32(const float* __restrict__ T, double* __restrict__ F, Geo g, double gamma,
+                                                   DevScalars* __restrict__ ds, int slot) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
     const int fx = g.nx + (D == 0), fy = g.ny + (D == 1);
-    double smax = 0.0, smaxv = 0.0;
+    double smax = 0.0;
     bool bad = false;
     const bool active = (i < fx && j < fy);
     if (active) {
         const long long eR = ext_index(g, i, j, k);
         const long long eL = ext_index(g, i - (D == 0), j - (D == 1), k - (D == 2));
-        R acc[NV];
+        float acc[NV];
 #pragma unroll
-        for (int c = 0; c < NV; ++c) acc[c] = R(0);
-        const R gm = (R)gamma, gm1 = (R)(gamma - 1.0);
+        for (int c = 0; c < NV; ++c) acc[c] = 0.0f;
+        const float gm = (float)gamma, gm1 = (float)(gamma - 1.0);
 #pragma unroll
         for (int gp = 0; gp < 4; ++gp) {
-            R QL[NV], QR[NV], fl[NV];
+            float QL[NV], QR[NV], fl[NV];
 #pragma unroll
             for (int c = 0; c < NV; ++c) {
                 QL[c] = T[((long long)c * NTR + (2 * D + 1) * 4 + gp) * g.NE + eL];
                 QR[c] = T[((long long)c * NTR + (2 * D) * 4 + gp) * g.NE + eR];
             }
             // Rusanov's 1/2 goes into the Gauss weight 1/4
-            const R s = FLUX == HYPE_FLUX_RUSANOV ? rusanov<R, D, false>(QL, QR, gm, gm1, fl, bad)
-                                                  : face_solver<R, D, FLUX>(QL, QR, gm, gm1, fl, bad);
+            float s;
+            if constexpr (FLUX == HYPE_FLUX_RUSANOV) s = rusanov<float, D, false>(QL, QR, gm, gm1, fl, bad);
+            else s = face_solver<float, D, FLUX>(QL, QR, gm, gm1, fl, bad);
             smax = fmax(smax, (double)s);
-            const R wq = FLUX == HYPE_FLUX_RUSANOV ? R(0.125) : R(0.25);
+            const float wq = FLUX == HYPE_FLUX_RUSANOV ? 0.125f : 0.25f;
 #pragma unroll
             for (int c = 0; c < NV; ++c) acc[c] += wq * fl[c];
-        }
-        if constexpr (VISC) {
-            // PDEViscRiemannSolver (Navier-Stokes-3D/pde.c:386-404): 0.5 (F_v(L) + F_v(R)) at
-            // each Gauss point, weight 0.25, added to the inviscid flux (rhs_function.c:310-316)
-            double av[NV];
-#pragma unroll
-            for (int c = 0; c < NV; ++c) av[c] = 0.0;
-            smaxv = visc_side<D, 1>((const double*)T, C4, g, eL, gamma, vp, av);
-            smaxv = fmax(smaxv, visc_side<D, -1>((const double*)T, C4, g, eR, gamma, vp, av));
-#pragma unroll
-            for (int c = 0; c < NV; ++c) acc[c] += (R)av[c];
         }
         const long long nf = (long long)fx * fy * (g.nz + (D == 2));
         const long long f = ((long long)k * fy + j) * fx + i;
@@ -1015,11 +1028,152 @@ __global__ void __launch_bounds__(128) k_faces(const R* __restrict__ T, double* 
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) smax = fmax(smax, __shfl_xor_sync(0xffffffffu, smax, o));
     if ((threadIdx.x & 31) == 0 && smax > 0.0) atomic_max_pos(&ds->smax_bits[slot], smax);
-    if constexpr (VISC) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) smaxv = fmax(smaxv, __shfl_xor_sync(0xffffffffu, smaxv, o));
-        if ((threadIdx.x & 31) == 0 && smaxv > 0.0) atomic_max_pos(&ds->smaxv_bits[slot], smaxv);
+}
+
+// The faces normal to D, indexed flat: face (i, j, k) is the low side of cell (i, j, k) and runs to n
+// along D.  Its number, its two cells in the trace array and the cell an inadmissible state is reported at.
+template <int D>
+struct FaceAt {
+    unsigned nf, f;
+    int i, j, k;
+    __device__ __forceinline__ FaceAt(const Geo& g, unsigned face) : f(face) {
+        const unsigned fx = g.nx + (D == 0), fy = g.ny + (D == 1), fz = g.nz + (D == 2);
+        nf = fx * fy * fz;
+        const unsigned row = f / fx, pl = row / fy;
+        i = (int)(f - row * fx);
+        j = (int)(row - pl * fy);
+        k = (int)pl;
     }
+    __device__ __forceinline__ long long hi(const Geo& g) const { return ext_index(g, i, j, k); }
+    __device__ __forceinline__ long long lo(const Geo& g) const {
+        return ext_index(g, i - (D == 0), j - (D == 1), k - (D == 2));
+    }
+    __device__ __forceinline__ void report(const Geo& g, DevScalars* ds) const {
+        const int ci = i < g.nx ? i : g.nx - 1, cj = j < g.ny ? j : g.ny - 1, ck = k < g.nz ? k : g.nz - 1;
+        atomicMin(&ds->bad, (unsigned long long)(((long long)ck * g.ny + cj) * g.nx + ci));
+    }
+};
+
+// the warp's maximum of a non-negative number, decided on the bit pattern
+__device__ __forceinline__ double warp_max_pos(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = max_pos(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+// The maximum only grows while a kernel runs: a warp whose value does not exceed what it reads leaves it
+// alone (one atomic per warp to one address would serialise millions of them).
+__device__ __forceinline__ void raise_max(unsigned long long* slot, double v) {
+    if (v > 0.0 && (unsigned long long)__double_as_longlong(v) > *(volatile unsigned long long*)slot) atomic_max_pos(slot, v);
+}
+
+// FP64 face fluxes, all three directions in one launch (blockIdx.y = direction).  A block is 32 faces x
+// the 4 Gauss points of the 2x2 rule, one point per warp: a quarter of the registers of a thread per face,
+// four times the warps on a small grid (16^3: three launches of one 16 us wave each), the traces of a warp
+// contiguous in x and the four fluxes summed through shared memory without FP64 instructions of their own.
+// Bound: FP64 issue (63 operations per Rusanov solve).
+template <int D, int FLUX>
+__device__ __forceinline__ void faces64(const double* __restrict__ T, double* __restrict__ F, const Geo& g, double gamma,
+                                        DevScalars* __restrict__ ds, int slot, double (*sh)[NV][32]) {
+    const int lane = threadIdx.x & 31, gp = threadIdx.x >> 5;
+    const FaceAt<D> at(g, blockIdx.x * 32u + lane);
+    if (blockIdx.x * 32u >= at.nf) return;  // the grid is as wide as the direction with the most faces
+    double smax = 0.0;
+    if (at.f < at.nf) {
+        const double* TL = T + ((2 * D + 1) * 4 + gp) * g.NE + at.lo(g);
+        const double* TR = T + (2 * D * 4 + gp) * g.NE + at.hi(g);
+        double QL[NV], QR[NV], fl[NV];
+#pragma unroll
+        for (int c = 0; c < NV; ++c) {
+            QL[c] = __ldg(TL + c * NTR * g.NE);
+            QR[c] = __ldg(TR + c * NTR * g.NE);
+        }
+        bool bad = false;
+        if constexpr (FLUX == HYPE_FLUX_RUSANOV) smax = rusanov64<D>(QL, QR, gamma, gamma - 1.0, fl, bad);
+        else smax = face_solver<double, D, FLUX>(QL, QR, gamma, gamma - 1.0, fl, bad);
+#pragma unroll
+        for (int c = 0; c < NV; ++c) sh[gp][c][lane] = fl[c];
+        if (bad) at.report(g, ds);
+    }
+    smax = warp_max_pos(smax);
+    if (lane == 0) raise_max(&ds->smax_bits[slot], smax);
+    __syncthreads();
+    // Rusanov's 1/2 goes into the Gauss weight 1/4
+    constexpr double wq = FLUX == HYPE_FLUX_RUSANOV ? 0.125 : 0.25;
+    for (int c = gp; c < NV; c += 4)
+        if (at.f < at.nf)
+            F[(long long)c * at.nf + at.f] = wq * ((sh[0][c][lane] + sh[1][c][lane]) + (sh[2][c][lane] + sh[3][c][lane]));
+}
+
+template <int FLUX>
+__global__ void __launch_bounds__(128) k_faces64(const double* __restrict__ T, double* __restrict__ Fx,
+                                                 double* __restrict__ Fy, double* __restrict__ Fz, Geo g, double gamma,
+                                                 DevScalars* __restrict__ ds, int slot) {
+    __shared__ double sh[4][NV][32];
+    if (blockIdx.y == 0) faces64<0, FLUX>(T, Fx, g, gamma, ds, slot, sh);
+    else if (blockIdx.y == 1) faces64<1, FLUX>(T, Fy, g, gamma, ds, slot, sh);
+    else faces64<2, FLUX>(T, Fz, g, gamma, ds, slot, sh);
+}
+
+// Navier-Stokes faces: the inviscid flux plus, at each Gauss point, half of both sides' viscous fluxes
+// (PDEViscRiemannSolver, Navier-Stokes-3D/pde.c:386-404; rhs_function.c:310-316).  One thread per face:
+// the gradients at a side's four points come from one set of 11 bilinear forms.  Bound: FP64 issue.
+template <int D, int FLUX>
+__device__ __forceinline__ void faces_visc64(const double* __restrict__ T, double* __restrict__ F, const Geo& g,
+                                             double gamma, DevScalars* __restrict__ ds, int slot,
+                                             const double* __restrict__ C4, const Visc& vp) {
+    constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
+    const FaceAt<D> at(g, blockIdx.x * 128u + threadIdx.x);
+    double smax = 0.0, smaxv = 0.0;
+    if (at.f < at.nf) {
+        const long long eR = at.hi(g), eL = at.lo(g);
+        double acc[NV], av[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int c = 0; c < NV; ++c) acc[c] = 0.0;
+        bool bad = false;
+        constexpr double wq = FLUX == HYPE_FLUX_RUSANOV ? 0.125 : 0.25;
+#pragma unroll
+        for (int gp = 0; gp < 4; ++gp) {
+            double QL[NV], QR[NV], fl[NV], s;
+#pragma unroll
+            for (int c = 0; c < NV; ++c) {
+                QL[c] = __ldg(T + ((long long)c * NTR + (2 * D + 1) * 4 + gp) * g.NE + eL);
+                QR[c] = __ldg(T + ((long long)c * NTR + (2 * D) * 4 + gp) * g.NE + eR);
+            }
+            if constexpr (FLUX == HYPE_FLUX_RUSANOV) s = rusanov64<D>(QL, QR, gamma, gamma - 1.0, fl, bad);
+            else s = face_solver<double, D, FLUX>(QL, QR, gamma, gamma - 1.0, fl, bad);
+            smax = max_pos(smax, s);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) acc[c] = fma(wq, fl[c], acc[c]);
+        }
+        const double kmu = vp.kc / vp.mu;
+        smaxv = visc_side64<D, 1>(T, C4, g.NE, eL, gamma - 1.0, kmu, av);
+        smaxv = vp.vmax * max_pos(smaxv, visc_side64<D, -1>(T, C4, g.NE, eR, gamma - 1.0, kmu, av));
+        // weight 1/4, both sides' mean, twice the gradients times h: mu / (16 h)
+        const double wv = -(1. / 16.) * vp.mu * vp.r1_h;
+        acc[1 + D] = fma(wv, av[0], acc[1 + D]);
+        acc[1 + T1] = fma(wv, av[1], acc[1 + T1]);
+        acc[1 + T2] = fma(wv, av[2], acc[1 + T2]);
+        acc[4] = fma(wv, av[3], acc[4]);
+#pragma unroll
+        for (int c = 0; c < NV; ++c) F[(long long)c * at.nf + at.f] = acc[c];
+        if (bad) at.report(g, ds);
+    }
+    smax = warp_max_pos(smax);
+    smaxv = warp_max_pos(smaxv);
+    if ((threadIdx.x & 31) == 0) {
+        raise_max(&ds->smax_bits[slot], smax);
+        raise_max(&ds->smaxv_bits[slot], smaxv);
+    }
+}
+
+template <int FLUX>
+__global__ void __launch_bounds__(128) k_faces_visc64(const double* __restrict__ T, double* __restrict__ Fx,
+                                                      double* __restrict__ Fy, double* __restrict__ Fz, Geo g, double gamma,
+                                                      DevScalars* __restrict__ ds, int slot, const double* __restrict__ C4,
+                                                      Visc vp) {
+    if (blockIdx.y == 0) faces_visc64<0, FLUX>(T, Fx, g, gamma, ds, slot, C4, vp);
+    else if (blockIdx.y == 1) faces_visc64<1, FLUX>(T, Fy, g, gamma, ds, slot, C4, vp);
+    else faces_visc64<2, FLUX>(T, Fz, g, gamma, ds, slot, C4, vp);
 }
 
 // stage combination: out = a*U + b*W + (c*dt)*L   (L = divergence of the face fluxes)
@@ -1051,42 +1205,40 @@ __device__ __forceinline__ double stage_value(const Stage& st, double cdt, doubl
     return __fma_rn(cdt, L, __fma_rn(st.b, w, __dmul_rn(st.a, u)));
 }
 
-// U, W and out may be one array (in-place stages), so they carry no __restrict__.
-// F32: the face fluxes hold FP32 values (the FP32 form); the divergence is formed in FP32
+// U, W and out may be one array (in-place stages), so they carry no __restrict__; a thread per cell and
+// variable (blockIdx.y) keeps the loads of one from waiting for the stores of another (16^3: 9.5 us with a
+// cell per thread).  F32: the face fluxes hold FP32 values (the FP32 form); the divergence is formed in FP32
+constexpr int kUpdateThreads = 128;
+
 template <bool F32 = false>
-__global__ void __launch_bounds__(256) k_update(const double* __restrict__ Fx, const double* __restrict__ Fy,
-                                                const double* __restrict__ Fz, const double* U,
-                                                const double* W, double* out, Geo g, double r1_h,
-                                                Stage st, const DevScalars* __restrict__ ds) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z;
-    if (i >= g.nx || j >= g.ny) return;
+__global__ void __launch_bounds__(kUpdateThreads) k_update(const double* __restrict__ Fx, const double* __restrict__ Fy,
+                                                           const double* __restrict__ Fz, const double* U,
+                                                           const double* W, double* out, Geo g, double r1_h,
+                                                           Stage st, const DevScalars* __restrict__ ds) {
+    const unsigned cell = blockIdx.x * (unsigned)kUpdateThreads + threadIdx.x;
+    if (cell >= (unsigned)g.N) return;
+    const unsigned row = cell / (unsigned)g.nx, k = row / (unsigned)g.ny;
+    const long long c = blockIdx.y;
     const long long nfx = (long long)(g.nx + 1) * g.ny * g.nz, nfy = (long long)g.nx * (g.ny + 1) * g.nz,
                     nfz = (long long)g.nx * g.ny * (g.nz + 1);
-    const long long ix = ((long long)k * g.ny + j) * (g.nx + 1) + i;
-    const long long iy = ((long long)k * (g.ny + 1) + j) * g.nx + i;
-    const long long iz = ((long long)k * g.ny + j) * g.nx + i;
-    const long long cell = iz;
+    Fx += c * nfx + cell + row;                    // (k ny + j) (nx + 1) + i
+    Fy += c * nfy + cell + k * (unsigned)g.nx;     // (k (ny + 1) + j) nx + i
+    Fz += c * nfz + cell;
     const double cdt = st.rhs_only ? 0.0 : st.c * ds->dt;
-#pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        double L;
-        if constexpr (F32) {
-            const float r1hf = (float)r1_h;
-            const float pxy = div_xy_f((float)Fx[c * nfx + ix + 1] - (float)Fx[c * nfx + ix],
-                                       (float)Fy[c * nfy + iy + g.nx] - (float)Fy[c * nfy + iy], r1hf);
-            L = df_f2d(div_z_f(pxy, (float)Fz[c * nfz + iz + (long long)g.nx * g.ny] - (float)Fz[c * nfz + iz], r1hf));
-        } else {
-            const double pxy =
-                div_xy(Fx[c * nfx + ix + 1] - Fx[c * nfx + ix], Fy[c * nfy + iy + g.nx] - Fy[c * nfy + iy], r1_h);
-            L = div_z(pxy, Fz[c * nfz + iz + (long long)g.nx * g.ny] - Fz[c * nfz + iz], r1_h);
-        }
-        const double u = (!st.rhs_only && st.a != 0.0) ? U[c * g.N + cell] : 0.0;
-        const double w = st.rhs_only ? 0.0 : W[c * g.N + cell];
-        out[c * g.N + cell] = stage_value(st, cdt, u, w, L);
+    const double u = (!st.rhs_only && st.a != 0.0) ? U[c * g.N + cell] : 0.0;
+    const double w = st.rhs_only ? 0.0 : W[c * g.N + cell];
+    double L;
+    if constexpr (F32) {
+        const float r1hf = (float)r1_h;
+        const float pxy = div_xy_f((float)Fx[1] - (float)Fx[0], (float)Fy[g.nx] - (float)Fy[0], r1hf);
+        L = df_f2d(div_z_f(pxy, (float)Fz[(long long)g.nx * g.ny] - (float)Fz[0], r1hf));
+    } else {
+        const double pxy = div_xy(Fx[1] - Fx[0], Fy[g.nx] - Fy[0], r1_h);
+        L = div_z(pxy, Fz[(long long)g.nx * g.ny] - Fz[0], r1_h);
     }
+    out[c * g.N + cell] = stage_value(st, cdt, u, w, L);
 }
+inline dim3 update_grid(const Geo& g) { return dim3(cdiv(g.N, kUpdateThreads), NV); }
 
 // ---------------------------------------------------------------- fused FP32 stage
 // One pass per RK stage for the FP32 reconstruction + Rusanov flux form: reconstruction of
@@ -1666,29 +1818,32 @@ static void prof_mark(hype_euler* e, int kind, bool start) {
     }
 }
 
-template <typename R, int FLUX, bool VISC = false>
-static void launch_faces_t(const Geo& g, const void* T, double* Fx, double* Fy, double* Fz, double gamma, DevScalars* ds,
-                           int slot, cudaStream_t st, const double* C4 = nullptr, Visc vp = Visc{0.0, 0.0, 0.0, 0.0}) {
-    const dim3 bf(32, 4);
-    const dim3 gx(cdiv(g.nx + 1, 32), cdiv(g.ny, 4), g.nz), gy(cdiv(g.nx, 32), cdiv(g.ny + 1, 4), g.nz),
-        gz(cdiv(g.nx, 32), cdiv(g.ny, 4), g.nz + 1);
-    k_faces<R, 0, FLUX, VISC><<<gx, bf, 0, st>>>((const R*)T, Fx, g, gamma, ds, slot, C4, vp);
-    k_faces<R, 1, FLUX, VISC><<<gy, bf, 0, st>>>((const R*)T, Fy, g, gamma, ds, slot, C4, vp);
-    k_faces<R, 2, FLUX, VISC><<<gz, bf, 0, st>>>((const R*)T, Fz, g, gamma, ds, slot, C4, vp);
+// the face-flux launches of one RHS (FP32 or FP64 traces), for the context's flux; vp: with viscosity
+template <int FLUX>
+static int launch_faces_t(const Geo& g, const void* T, double* Fx, double* Fy, double* Fz, double gamma, DevScalars* ds,
+                          int slot, bool f32, cudaStream_t st, const double* C4, const Visc* vp) {
+    if (f32) {
+        const dim3 bf(32, 4);
+        const dim3 gx(cdiv(g.nx + 1, 32), cdiv(g.ny, 4), g.nz), gy(cdiv(g.nx, 32), cdiv(g.ny + 1, 4), g.nz),
+            gz(cdiv(g.nx, 32), cdiv(g.ny, 4), g.nz + 1);
+        k_faces_f32<0, FLUX><<<gx, bf, 0, st>>>((const float*)T, Fx, g, gamma, ds, slot);
+        k_faces_f32<1, FLUX><<<gy, bf, 0, st>>>((const float*)T, Fy, g, gamma, ds, slot);
+        k_faces_f32<2, FLUX><<<gz, bf, 0, st>>>((const float*)T, Fz, g, gamma, ds, slot);
+        return 3;
+    }
+    const long long most = std::max({(long long)(g.nx + 1) * g.ny * g.nz, (long long)g.nx * (g.ny + 1) * g.nz,
+                                     (long long)g.nx * g.ny * (g.nz + 1)});
+    if (vp) k_faces_visc64<FLUX><<<dim3(cdiv(most, 128), 3), 128, 0, st>>>((const double*)T, Fx, Fy, Fz, g, gamma, ds, slot, C4, *vp);
+    else k_faces64<FLUX><<<dim3(cdiv(most, 32), 3), 128, 0, st>>>((const double*)T, Fx, Fy, Fz, g, gamma, ds, slot);
+    return 1;
 }
 
-// the three face-flux launches of one RHS, for the context's precision and flux
-static void launch_faces(const Geo& g, const void* T, double* Fx, double* Fy, double* Fz, double gamma, DevScalars* ds,
-                         int slot, bool f32, int flux, cudaStream_t st) {
-    if (f32) {
-        if (flux == HYPE_FLUX_HLLC) launch_faces_t<float, HYPE_FLUX_HLLC>(g, T, Fx, Fy, Fz, gamma, ds, slot, st);
-        else if (flux == HYPE_FLUX_ROTHLLC) launch_faces_t<float, HYPE_FLUX_ROTHLLC>(g, T, Fx, Fy, Fz, gamma, ds, slot, st);
-        else launch_faces_t<float, HYPE_FLUX_RUSANOV>(g, T, Fx, Fy, Fz, gamma, ds, slot, st);
-    } else {
-        if (flux == HYPE_FLUX_HLLC) launch_faces_t<double, HYPE_FLUX_HLLC>(g, T, Fx, Fy, Fz, gamma, ds, slot, st);
-        else if (flux == HYPE_FLUX_ROTHLLC) launch_faces_t<double, HYPE_FLUX_ROTHLLC>(g, T, Fx, Fy, Fz, gamma, ds, slot, st);
-        else launch_faces_t<double, HYPE_FLUX_RUSANOV>(g, T, Fx, Fy, Fz, gamma, ds, slot, st);
-    }
+static int launch_faces(const Geo& g, const void* T, double* Fx, double* Fy, double* Fz, double gamma, DevScalars* ds,
+                        int slot, bool f32, int flux, cudaStream_t st, const double* C4 = nullptr, const Visc* vp = nullptr) {
+    const auto go = flux == HYPE_FLUX_HLLC      ? launch_faces_t<HYPE_FLUX_HLLC>
+                    : flux == HYPE_FLUX_ROTHLLC ? launch_faces_t<HYPE_FLUX_ROTHLLC>
+                                                : launch_faces_t<HYPE_FLUX_RUSANOV>;
+    return go(g, T, Fx, Fy, Fz, gamma, ds, slot, f32, st, C4, vp);
 }
 
 static int launch_rhs(hype_euler* e, const double* Win, int slot) {
@@ -1727,12 +1882,12 @@ static int launch_rhs(hype_euler* e, const double* Win, int slot) {
             k_recon_df<false><<<gr, br, 0, e->stream>>>((const df64*)e->G, e->T, Win, g, rec, e->p.positivity, gm1,
                                                         e->mlp_cnt);
     } else if (f32) {
-        k_recon<float><<<gr, br, ck_bytes, e->stream>>>((const float*)e->G, (float*)e->T, g, rec, e->p.positivity, gm1,
-                                                        e->mlp_cnt);
+        k_recon_f32<<<gr, br, ck_bytes, e->stream>>>((const float*)e->G, (float*)e->T, g, rec, e->p.positivity, gm1,
+                                                     e->mlp_cnt);
     } else {
-        k_recon<double><<<gr, br, 0, e->stream>>>((const double*)e->G, (double*)e->T, g, rec, e->p.positivity, gm1,
-                                                  e->mlp_cnt, e->C4, 1.0 / e->p.h);
+        launch_recon64(g, (const double*)e->G, (double*)e->T, rec, e->p.positivity, gm1, e->mlp_cnt, e->C4, e->stream);
     }
+    int nk = 2;
     prof_mark(e, 0, false);
     prof_mark(e, 1, true);
     if (e->C4 && df) {
@@ -1748,14 +1903,12 @@ static int launch_rhs(hype_euler* e, const double* Win, int slot) {
         k_faces_df<0, true><<<fgx, bf, 0, e->stream>>>(Td, e->Fx, Win, g, e->p.gamma, e->ds, slot, C4, vp);
         k_faces_df<1, true><<<fgy, bf, 0, e->stream>>>(Td, e->Fy, Win, g, e->p.gamma, e->ds, slot, C4, vp);
         k_faces_df<2, true><<<fgz, bf, 0, e->stream>>>(Td, e->Fz, Win, g, e->p.gamma, e->ds, slot, C4, vp);
+        nk += 3;
     } else if (e->C4) {
         // Navier-Stokes: the inviscid flux plus the average of both sides' viscous fluxes
         const double mu = e->p.mu, g = e->p.gamma;
         const Visc vp{mu, e->p.cv * mu * g / e->p.prandtl, std::max((4. / 3.) * mu, g * mu / e->p.prandtl), 1.0 / e->p.h};
-        const auto lf = e->p.flux == HYPE_FLUX_HLLC      ? launch_faces_t<double, HYPE_FLUX_HLLC, true>
-                        : e->p.flux == HYPE_FLUX_ROTHLLC ? launch_faces_t<double, HYPE_FLUX_ROTHLLC, true>
-                                                         : launch_faces_t<double, HYPE_FLUX_RUSANOV, true>;
-        lf(e->g, e->T, e->Fx, e->Fy, e->Fz, e->p.gamma, e->ds, slot, e->stream, e->C4, vp);
+        nk += launch_faces(e->g, e->T, e->Fx, e->Fy, e->Fz, e->p.gamma, e->ds, slot, false, e->p.flux, e->stream, e->C4, &vp);
     } else if (df && e->p.flux == HYPE_FLUX_RUSANOV) {
         const dim3 bf(32, 4);
         const dim3 fgx(cdiv(g.nx + 1, 32), cdiv(g.ny, 4), g.nz), fgy(cdiv(g.nx, 32), cdiv(g.ny + 1, 4), g.nz),
@@ -1764,17 +1917,19 @@ static int launch_rhs(hype_euler* e, const double* Win, int slot) {
         k_faces_df<0><<<fgx, bf, 0, e->stream>>>(Td, e->Fx, Win, g, e->p.gamma, e->ds, slot);
         k_faces_df<1><<<fgy, bf, 0, e->stream>>>(Td, e->Fy, Win, g, e->p.gamma, e->ds, slot);
         k_faces_df<2><<<fgz, bf, 0, e->stream>>>(Td, e->Fz, Win, g, e->p.gamma, e->ds, slot);
+        nk += 3;
     } else {
-        launch_faces(e->g, e->T, e->Fx, e->Fy, e->Fz, e->p.gamma, e->ds, slot, f32, e->p.flux, e->stream);
+        nk += launch_faces(e->g, e->T, e->Fx, e->Fy, e->Fz, e->p.gamma, e->ds, slot, f32, e->p.flux, e->stream);
     }
     prof_mark(e, 1, false);
-    HYPE_LAUNCHED(4);
+    HYPE_LAUNCHED(nk - 1);  // the ghost fill is counted above
     return HYPE_OK;
 }
 
 static int launch_update(hype_euler* e, const double* U, const double* W, double* out, Stage st) {
     const Geo& g = e->g;
-    const dim3 b(32, 8), gr(cdiv(g.nx, 32), cdiv(g.ny, 8), g.nz);
+    const unsigned b = kUpdateThreads;
+    const dim3 gr = update_grid(g);
     prof_mark(e, 2, true);
     if (e->p.precision == HYPE_PREC_FP32)
         k_update<true><<<gr, b, 0, e->stream>>>(e->Fx, e->Fy, e->Fz, U, W, out, g, 1.0 / e->p.h, st, e->ds);
@@ -2431,19 +2586,20 @@ extern "C" int hype_euler_rhs_noalloc(const hype_euler_params* p, const double* 
         // dynamic shared memory, as in the context path
         const size_t ck_bytes = pad ? sizeof(float) * 4 * 2 * NTR * 32 : 0;
         k_ghost<float><<<ghost_grid(g), kGhostThreads, 0, s>>>(dU, (float*)G, g);
-        k_recon<float><<<gr, br, ck_bytes, s>>>((const float*)G, (float*)T, g, rec, pad, p->gamma - 1.0, counters);
+        k_recon_f32<<<gr, br, ck_bytes, s>>>((const float*)G, (float*)T, g, rec, pad, p->gamma - 1.0, counters);
     } else {
         k_ghost<double><<<ghost_grid(g), kGhostThreads, 0, s>>>(dU, (double*)G, g);
-        k_recon<double><<<gr, br, 0, s>>>((const double*)G, (double*)T, g, rec, pad, p->gamma - 1.0, counters);
+        launch_recon64(g, (const double*)G, (double*)T, rec, pad, p->gamma - 1.0, counters, nullptr, s);
     }
-    launch_faces(g, T, Fx, Fy, Fz, p->gamma, ds, 4, p->precision == HYPE_PREC_FP32, p->flux, s);
+    const int nfk = launch_faces(g, T, Fx, Fy, Fz, p->gamma, ds, 4, p->precision == HYPE_PREC_FP32, p->flux, s);
     const Stage st{0.0, 0.0, 0.0, 1};
-    const dim3 bu(32, 8), gu(cdiv(g.nx, 32), cdiv(g.ny, 8), g.nz);
+    const unsigned bu = kUpdateThreads;
+    const dim3 gu = update_grid(g);
     if (p->precision == HYPE_PREC_FP32)
         k_update<true><<<gu, bu, 0, s>>>(Fx, Fy, Fz, nullptr, nullptr, dRHS, g, 1.0 / p->h, st, ds);
     else
         k_update<false><<<gu, bu, 0, s>>>(Fx, Fy, Fz, nullptr, nullptr, dRHS, g, 1.0 / p->h, st, ds);
-    HYPE_LAUNCHED(7);
+    HYPE_LAUNCHED(4 + nfk);
     if (dt_out) {
         unsigned long long w[2];
         HYPE_CK(cudaMemcpyAsync(&w[0], &ds->smax_bits[4], sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));

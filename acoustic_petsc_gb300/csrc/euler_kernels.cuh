@@ -8,7 +8,8 @@
 // 24 face-Gauss-point traces per variable come from an even/odd split of the
 // polynomial at the symmetric Gauss points (about 40 operations per direction
 // instead of 8 full 20-term evaluations), and the arithmetic type R is a
-// template parameter (double: the FP64 path; float: the FP32 recon/flux form).
+// template parameter (float: the FP32 recon/flux form; double: WENO3 and the
+// HLLC family; CWENO4, R4 and Rusanov in FP64 are in cweno64.cuh).
 #pragma once
 
 #include "df64.cuh"
@@ -54,25 +55,61 @@ __host__ __device__ __forceinline__ double recip_wide(double x) {
 #endif
 }
 
-// 1/x for the face solvers: the approximate FP32 reciprocal (rcp.approx, ~1 ulp of FP32)
-// of x's leading bits, refined by two Newton steps r <- r + r (1 - x r) in FP64 (the
-// relative error squares at each: 2^-23, 2^-46, then FP64 rounding), four FP64 operations
-// against the longer correctly rounded division; the bits move between the formats on the
-// integer pipe.  x outside [2^-126, 2^126) in magnitude, zero or not finite: the division.
+// 1/x: the approximate FP32 reciprocal r of x's significand (relative error e0 below 2^-22), rescaled on
+// the integer pipe, and r (1 + e + e^2) with e = 1 - x r formed by one FMA: the remaining e^3 is far
+// below the FP64 rounding.  Biased exponent outside [2, 2044]: the division.
+__device__ __forceinline__ double recip3(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x);
+    const unsigned ex = (hi >> 20) & 0x7FFu;
+    if (ex - 2u > 2042u) return 1.0 / x;
+    const float mf = __uint_as_float((hi & 0x80000000u) | (127u << 23) | ((hi & 0xFFFFFu) << 3));
+    float rf;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(mf));
+    // rf in (1/2, 1] in magnitude: its exponent and significand move into place without a special case
+    const unsigned rb = __float_as_uint(rf);
+    const unsigned mag = rb & 0x7FFFFFFFu;
+    const double r = __hiloint2double(
+        (int)((rb & 0x80000000u) | ((mag >> 3) + ((896u + 1023u - ex) << 20))), (int)(mag << 29));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+// sqrt(x) for x > 0: with y the approximate FP32 reciprocal root of x rebased to [1, 4) and g = x y,
+// e = 1 - g y, sqrt(x) = g (1 + e/2 + 3 e^2/8 + O(e^3)), e below 2^-21.  Biased exponent outside
+// [2, 2044], or x negative, zero or NaN: sqrt().
+__device__ __forceinline__ double sqrt3(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x);
+    const unsigned ex = hi >> 20;  // with the sign: a negative x fails the range test
+    if (ex - 2u > 2042u) return sqrt(x);
+    const unsigned odd = (ex & 1u) ^ 1u;  // x = m 4^q, m in [1, 4): 2 q = ex - 1023 - odd
+    const float mf = __uint_as_float(((127u + odd) << 23) | ((hi & 0xFFFFFu) << 3));
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(mf));
+    const unsigned yb = __float_as_uint(yf);
+    const int q = ((int)ex - 1023 - (int)odd) / 2;
+    const double y = __hiloint2double((int)((yb >> 3) + ((896u << 20) - ((unsigned)q << 20))), (int)(yb << 29));
+    const double g = x * y;
+    const double e = fma(-g, y, 1.0);
+    return fma(g, e * fma(0.375, e, 0.5), g);
+}
+
+// x >= lo for a positive lo, as the floating comparison decides it (false for NaN), on the bit pattern
+__device__ __forceinline__ bool at_least(double x, double lo) {
+    const long long b = __double_as_longlong(x);
+    return b >= __double_as_longlong(lo) && b <= 0x7FF0000000000000ll;
+}
+// the larger of two non-negative numbers as fmax and (a < b) ? b : a decide it, on the bit patterns: a NaN
+// in b leaves a
+__device__ __forceinline__ double max_pos(double a, double b) {
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return (y > x && y <= 0x7FF0000000000000ll) ? b : a;
+}
+
+// 1/x in the working precision of a face solver
 template <typename R>
 __device__ __forceinline__ R recip(R x) {
-    if (sizeof(R) != sizeof(double)) return (R)rcp_fast((float)x);
-    const double xd = (double)x;
-    const unsigned hi = (unsigned)__double2hiint(xd);
-    const unsigned ex = (hi >> 20) & 0x7FFu;
-    if (ex - 897u > 251u) return R(1.0 / xd);
-    const float xf = __uint_as_float((hi & 0x80000000u) | ((ex - 896u) << 23) | ((hi & 0xFFFFFu) << 3));
-    float rf;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(xf));
-    double r = df_f2d(rf);
-    r = fma(r, fma(-xd, r, 1.0), r);
-    r = fma(r, fma(-xd, r, 1.0), r);
-    return (R)r;
+    if constexpr (sizeof(R) == sizeof(double)) return recip3(x);
+    else return rcp_fast(x);
 }
 
 constexpr int NV = 5;
@@ -115,12 +152,12 @@ struct Weights;
 
 
 
-// CWENO4 coefficients (20) of one variable from its 33-point stencil.
+// CWENO4 coefficients (20) of one variable from its 33-point stencil (R = float; the FP64 form is
+// cweno64.cuh's).
 // linear: the R4 polynomial (the limit in which all nonlinear weights equal the linear ones).
 //
 // The mathematics is the reference's weno() (3d/weno4/Viscous-Multiphase-Fourth-Order/
-// reconstruction.c:38-259); the operation count is cut for the FP64 pipe, which bounds
-// this kernel on GB300, with every value still formed in the working precision:
+// reconstruction.c:38-259), with every value formed in the working precision:
 //  * per axis the differences a = u(+1) - u(-1), b = u(+2) - u(-2) and the sum
 //    u(-1) + u(+1) serve the R4 first/second/third derivatives (:90-108) and the
 //    centred R3 derivatives (:123-140);
@@ -133,8 +170,7 @@ struct Weights;
 //    evaluated per coefficient as (w4/g4) c4 + sum_k (w_k - (w4/g4) g_k) c_k, one
 //    weighted sum instead of a linear and a nonlinear one.
 template <typename R>
-__host__ __device__ __forceinline__ void cweno4(const R* __restrict__ s, bool linear, R* __restrict__ cf,
-                                                R* wdev = nullptr) {
+__host__ __device__ __forceinline__ void cweno4(const R* __restrict__ s, bool linear, R* __restrict__ cf) {
     const R u0 = s[0];
     const R h = R(0.5), q = R(0.25);
     R d4[3], dd4[3], ddd4[3], c1[3];
@@ -173,7 +209,6 @@ __host__ __device__ __forceinline__ void cweno4(const R* __restrict__ s, bool li
         }
         cf[7] = cx[0]; cf[8] = cx[1]; cf[9] = cx[2];
         cf[13] = aab[0]; cf[14] = abb[0]; cf[15] = aab[1]; cf[16] = abb[1]; cf[17] = aab[2]; cf[18] = abb[2]; cf[19] = xyz;
-        if (wdev) *wdev = R(0);
         return;
     }
     const R r13_3 = R(13. / 3.), r7_6 = R(7. / 6.);
@@ -229,12 +264,6 @@ __host__ __device__ __forceinline__ void cweno4(const R* __restrict__ s, bool li
     Weights<R>::compute(IS4, IS0, IS3, gH, g0, gs, w4, w0, ws);
     // 1/gammaHi as a constant: a product, not a division
     const R wr = w4 * R(1.0 / 0.85);
-    if (wdev) {  // largest departure of a nonlinear weight from its linear value (indicator labels)
-        R d = fmax(fabs(w4 - gH), fabs(w0 - g0));
-#pragma unroll
-        for (int m = 0; m < 6; ++m) d = fmax(d, fabs(ws[m] - gs));
-        *wdev = d;
-    }
     // weights of the lower-order stencils' values in the combination: w_k - wr g_k
     const R o0 = w0 - wr * g0;
     R os[6];
@@ -259,53 +288,6 @@ __host__ __device__ __forceinline__ void cweno4(const R* __restrict__ s, bool li
     cf[13] = wr * aab[0]; cf[14] = wr * abb[0]; cf[15] = wr * aab[1]; cf[16] = wr * abb[1];
     cf[17] = wr * aab[2]; cf[18] = wr * abb[2]; cf[19] = wr * xyz;
 }
-
-// w = gamma / (IS + eps)^4, normalised.  FP64: the eight reciprocals 1/(IS + eps)^2
-// come from one reciprocal of their product (prefix products, then back-substitution:
-// 21 multiplications instead of 7 more reciprocals); a product outside the normal
-// range (IS beyond ~1e36) takes the plain reciprocals instead.  Reciprocals by recip_wide
-// (within an ulp of the division, on a fraction of its FP64 instructions).
-template <>
-struct Weights<double> {
-    __host__ __device__ __forceinline__ static void compute(double IS4, double IS0, const double* IS3, double gH, double g0, double gs,
-                                                   double& w4, double& w0, double* ws) {
-        double q[8], P[8], r[8];
-        q[0] = IS4 + 1.0e-12;
-        q[1] = IS0 + 1.0e-12;
-#pragma unroll
-        for (int m = 0; m < 6; ++m) q[2 + m] = IS3[m] + 1.0e-12;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) q[k] *= q[k];
-        P[0] = q[0];
-#pragma unroll
-        for (int k = 1; k < 8; ++k) P[k] = P[k - 1] * q[k];
-        if (P[7] > 1.0e-290 && P[7] < 1.0e290) {
-            double inv = recip_wide(P[7]);
-#pragma unroll
-            for (int k = 7; k > 0; --k) {
-                r[k] = inv * P[k - 1];
-                inv *= q[k];
-            }
-            r[0] = inv;
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) r[k] = recip_wide(q[k]);
-        }
-        w4 = gH * (r[0] * r[0]);
-        w0 = g0 * (r[1] * r[1]);
-        double total = w4 + w0;
-#pragma unroll
-        for (int m = 0; m < 6; ++m) {
-            ws[m] = gs * (r[2 + m] * r[2 + m]);
-            total += ws[m];
-        }
-        const double rt = recip_wide(total);
-        w4 *= rt;
-        w0 *= rt;
-#pragma unroll
-        for (int m = 0; m < 6; ++m) ws[m] *= rt;
-    }
-};
 
 // FP32: (1e-12)^4 underflows, so the weights are formed from ratios to the
 // smallest (IS + eps), which is the same normalised quantity.
@@ -495,131 +477,6 @@ __device__ __forceinline__ R rusanov(const R* QL, const R* QR, R gamma, R gm1, R
         F[c] = HALF ? R(0.5) * f : f;
     }
     return s;
-}
-
-// ---------------------------------------------------------------- viscous fluxes
-// The gradient of a cell's R4 polynomial on one of its faces (normal axis D, side
-// NS = +1 for the high face x_D = +1/2, -1 for the low face) is, in the two
-// tangential coordinates, g(t1, t2) = P + Q t1 + R t2 + S t1 t2 once the squares
-// t1^2 = t2^2 = GPT^2 of the 2x2 Gauss points are folded into P (the gradient of
-// evaluate_grad, Navier-Stokes-3D/reconstruction.c:24-35, at the face points of
-// rhs_function.c:224-270).  Built once per face side from the coefficients, it costs
-// 3 FMAs per Gauss point.  The tangential axes are the two other axes in increasing
-// order, as for the traces.
-struct FaceGrad {
-    double p, q, r, s;
-};
-
-// adds c k x^EX y^EY z^EZ to f
-template <int D, int NS, int EX, int EY, int EZ>
-__device__ __forceinline__ void fg_term(FaceGrad& f, double c, double k) {
-    constexpr int eD = D == 0 ? EX : (D == 1 ? EY : EZ);
-    constexpr int e1 = D == 0 ? EY : EX, e2 = D == 2 ? EY : EZ;
-    constexpr double n = 0.5 * NS;
-    constexpr double nf = eD == 0 ? 1.0 : (eD == 1 ? n : n * n);
-    if constexpr (e1 == 2 || e2 == 2) f.p = fma(c, k * (nf * G2), f.p);
-    else if constexpr (e1 == 0 && e2 == 0) f.p = fma(c, k * nf, f.p);
-    else if constexpr (e1 == 1 && e2 == 0) f.q = fma(c, k * nf, f.q);
-    else if constexpr (e1 == 0 && e2 == 1) f.r = fma(c, k * nf, f.r);
-    else f.s = fma(c, k * nf, f.s);
-}
-
-// component B of the gradient of the 20-term polynomial whose coefficient q is at p[q * st]
-template <int D, int NS, int B>
-__device__ __forceinline__ FaceGrad face_grad(const double* __restrict__ p, long long st) {
-    auto C = [&](int q) { return __ldg(p + q * st); };
-    FaceGrad f{0.0, 0.0, 0.0, 0.0};
-    if constexpr (B == 0) {  // d/dx
-        fg_term<D, NS, 0, 0, 0>(f, C(1), 1.0);
-        fg_term<D, NS, 1, 0, 0>(f, C(4), 2.0);
-        fg_term<D, NS, 0, 1, 0>(f, C(7), 1.0);
-        fg_term<D, NS, 0, 0, 1>(f, C(9), 1.0);
-        const double c10 = C(10), c14 = C(14), c18 = C(18);
-        fg_term<D, NS, 2, 0, 0>(f, c10, 3.0);
-        fg_term<D, NS, 0, 0, 0>(f, c10, -R3_20);
-        fg_term<D, NS, 1, 1, 0>(f, C(13), 2.0);
-        fg_term<D, NS, 0, 2, 0>(f, c14, 1.0);
-        fg_term<D, NS, 0, 0, 0>(f, c14, -R1_12);
-        fg_term<D, NS, 1, 0, 1>(f, C(17), 2.0);
-        fg_term<D, NS, 0, 0, 2>(f, c18, 1.0);
-        fg_term<D, NS, 0, 0, 0>(f, c18, -R1_12);
-        fg_term<D, NS, 0, 1, 1>(f, C(19), 1.0);
-    } else if constexpr (B == 1) {  // d/dy
-        fg_term<D, NS, 0, 0, 0>(f, C(2), 1.0);
-        fg_term<D, NS, 0, 1, 0>(f, C(5), 2.0);
-        fg_term<D, NS, 1, 0, 0>(f, C(7), 1.0);
-        fg_term<D, NS, 0, 0, 1>(f, C(8), 1.0);
-        const double c11 = C(11), c13 = C(13), c16 = C(16);
-        fg_term<D, NS, 0, 2, 0>(f, c11, 3.0);
-        fg_term<D, NS, 0, 0, 0>(f, c11, -R3_20);
-        fg_term<D, NS, 2, 0, 0>(f, c13, 1.0);
-        fg_term<D, NS, 0, 0, 0>(f, c13, -R1_12);
-        fg_term<D, NS, 1, 1, 0>(f, C(14), 2.0);
-        fg_term<D, NS, 0, 1, 1>(f, C(15), 2.0);
-        fg_term<D, NS, 0, 0, 2>(f, c16, 1.0);
-        fg_term<D, NS, 0, 0, 0>(f, c16, -R1_12);
-        fg_term<D, NS, 1, 0, 1>(f, C(19), 1.0);
-    } else {  // d/dz
-        fg_term<D, NS, 0, 0, 0>(f, C(3), 1.0);
-        fg_term<D, NS, 0, 0, 1>(f, C(6), 2.0);
-        fg_term<D, NS, 0, 1, 0>(f, C(8), 1.0);
-        fg_term<D, NS, 1, 0, 0>(f, C(9), 1.0);
-        const double c12 = C(12), c15 = C(15), c17 = C(17);
-        fg_term<D, NS, 0, 0, 2>(f, c12, 3.0);
-        fg_term<D, NS, 0, 0, 0>(f, c12, -R3_20);
-        fg_term<D, NS, 0, 2, 0>(f, c15, 1.0);
-        fg_term<D, NS, 0, 0, 0>(f, c15, -R1_12);
-        fg_term<D, NS, 0, 1, 1>(f, C(16), 2.0);
-        fg_term<D, NS, 2, 0, 0>(f, c17, 1.0);
-        fg_term<D, NS, 0, 0, 0>(f, c17, -R1_12);
-        fg_term<D, NS, 1, 0, 1>(f, C(18), 2.0);
-        fg_term<D, NS, 1, 1, 0>(f, C(19), 1.0);
-    }
-    return f;
-}
-
-// the value at Gauss point gp (t1 = -/+GPT for gp & 2, t2 = -/+GPT for gp & 1)
-template <int GP>
-__device__ __forceinline__ double fg_eval(const FaceGrad& f) {
-    constexpr double s1 = (GP & 2) ? GPT : -GPT, s2 = (GP & 1) ? GPT : -GPT;
-    return fma(f.s, s1 * s2, fma(f.r, s2, fma(f.q, s1, f.p)));
-}
-
-// PDEViscFlux (3d/weno4/Navier-Stokes-3D/pde.c:90-162) across a face of normal axis D:
-// Newtonian stress with Stokes' hypothesis and Fourier heat flux k = Cv mu gamma / Pr,
-// with the program's velocity gradients u_x = (rho u)_x - u rho_x / rho (:118-130);
-// returns the viscous speed max(4 mu / (3 rho), gamma mu / (Pr rho))
-template <int D>
-__device__ __forceinline__ double visc_flux(const double* Q, const double (*G)[3], double gm1, double mu, double kc,
-                                            double vmax, double* F) {
-    // kc = cv mu gamma / Pr (heat conductivity), vmax = max(4 mu / 3, gamma mu / Pr); the
-    // divisions by rho of the reference's expressions are products with 1/rho here
-    const double irho = 1.0 / Q[0];
-    const double u = irho * Q[1], v = irho * Q[2], w = irho * Q[3];
-    const double rhou = Q[1], rhov = Q[2], rhow = Q[3], e = Q[4];
-    const double m2 = rhou * rhou + rhov * rhov + rhow * rhow;
-    double vg[3][3], T[3];  // vg[a][b]: d(velocity a)/d(x_b)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-        const double rb = G[0][b] * irho;
-        vg[0][b] = G[1][b] - u * rb;
-        vg[1][b] = G[2][b] - v * rb;
-        vg[2][b] = G[3][b] - w * rb;
-        T[b] = (-gm1 * rb * irho) * (e - 0.5 * m2 * irho) +
-               (gm1 * irho) * (G[4][b] - (rhou * G[1][b] + rhov * G[2][b] + rhow * G[3][b]) * irho +
-                               0.5 * m2 * rb * irho);
-    }
-    const double div_v = -(2.0 / 3.0) * mu * (vg[0][0] + vg[1][1] + vg[2][2]);
-    const double tdd = div_v + 2.0 * mu * vg[D][D];                  // tau_DD
-    const double t0 = D == 0 ? tdd : mu * (vg[0][D] + vg[D][0]);     // tau_xD
-    const double t1 = D == 1 ? tdd : mu * (vg[1][D] + vg[D][1]);     // tau_yD
-    const double t2 = D == 2 ? tdd : mu * (vg[2][D] + vg[D][2]);     // tau_zD
-    F[0] = 0.0;
-    F[1] = -t0;
-    F[2] = -t1;
-    F[3] = -t2;
-    F[4] = -(u * t0 + v * t1 + w * t2 + kc * T[D]);
-    return vmax * irho;
 }
 
 // ---------------------------------------------------------------- HLLC family
@@ -822,10 +679,9 @@ __device__ __forceinline__ R rot_hllc(const R* QL, const R* QR, R nx, R ny, R nz
     return fmax(s1, fmax(s2, s3));
 }
 
-// numerical flux selected by the context (HYPE_FLUX_*) across an axis face of normal D
+// the HLLC family's flux selected by the context (HYPE_FLUX_*) across an axis face of normal D
 template <typename R, int D, int FLUX>
 __device__ __forceinline__ R face_solver(const R* QL, const R* QR, R gamma, R gm1, R* F, bool& bad) {
-    if (FLUX == HYPE_FLUX_RUSANOV) return rusanov<R, D>(QL, QR, gamma, gm1, F, bad);
     const R nx = R(D == 0), ny = R(D == 1), nz = R(D == 2);
     if (FLUX == HYPE_FLUX_HLLC) return hllc<R>(QL, QR, nx, ny, nz, gamma, gm1, F, bad);
     return rot_hllc<R>(QL, QR, nx, ny, nz, gamma, gm1, F, bad);

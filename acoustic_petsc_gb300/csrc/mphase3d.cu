@@ -26,13 +26,11 @@
 #include <algorithm>
 #include <vector>
 
-#include "euler_kernels.cuh"
+#include "cweno64.cuh"
 
 namespace hype {
 namespace mp3d {
 
-using euler::cweno4;
-using euler::face_traces;
 using euler::NTR;
 using euler::S1;
 using euler::SO;
@@ -355,17 +353,10 @@ __device__ __forceinline__ void gather33(const double* __restrict__ p, int sy, i
             for (int d = 0; d < 2; ++d) s[SO(a, b, d)] = __ldg(p + (2 * a - 1) + (2 * b - 1) * sy + (2 * d - 1) * sz);
 }
 
-__device__ __forceinline__ void store_traces6(double* __restrict__ T, const Geo& g, long long e, int c, const double* cf) {
-    double tr[8];
+__device__ __forceinline__ void store_traces6(double* __restrict__ T, const Geo& g, long long e, int c,
+                                              const euler::Poly64& poly) {
     double* Tc = T + (long long)c * NTR * g.NE + e;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        if (d == 0) face_traces<double, 0>(cf, tr);
-        else if (d == 1) face_traces<double, 1>(cf, tr);
-        else face_traces<double, 2>(cf, tr);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) Tc[(long long)(8 * d + q) * g.NE] = tr[q];
-    }
+    euler::store_traces64(poly, Tc, g.NE);
 }
 
 // T[c][face*4+gp][extended cell]; the cells the faces of owned cells need (at most one
@@ -387,34 +378,41 @@ __global__ void __launch_bounds__(128) k_m3_recon(const double* __restrict__ G, 
     bool fail = false;
     {  // density: the node check and its traces
         double s[33], cf[20];
+        euler::Poly64 poly;
         gather33(G + 0 * g.GN + ge, sy, sz, s);
-        cweno4<double>(s, false, cf);
+        euler::cweno4_64(s, poly);
+        euler::coeffs64(poly, cf);
         fail |= rho_fails(cf);
-        store_traces6(T, g, e_, 0, cf);
+        store_traces6(T, g, e_, 0, poly);
     }
     {  // volume fraction: coefficients kept for the pressure check
         double s[33], cf[20];
+        euler::Poly64 poly;
         gather33(G + 5 * g.GN + ge, sy, sz, s);
-        cweno4<double>(s, false, cf);
+        euler::cweno4_64(s, poly);
         if (stiff) {
+            euler::coeffs64(poly, cf);
 #pragma unroll
             for (int q = 0; q < 20; ++q) ph[q * 128] = cf[q];
         }
-        store_traces6(T, g, e_, 5, cf);
+        store_traces6(T, g, e_, 5, poly);
     }
     {  // pressure
         double s[33], cf[20];
+        euler::Poly64 poly;
         gather33(G + 4 * g.GN + ge, sy, sz, s);
-        cweno4<double>(s, false, cf);
+        euler::cweno4_64(s, poly);
+        euler::coeffs64(poly, cf);
         fail |= prs_fails(cf, ph, e, stiff);
-        store_traces6(T, g, e_, 4, cf);
+        store_traces6(T, g, e_, 4, poly);
     }
 #pragma unroll 1
     for (int c = 1; c < 4; ++c) {
-        double s[33], cf[20];
+        double s[33];
+        euler::Poly64 poly;
         gather33(G + c * g.GN + ge, sy, sz, s);
-        cweno4<double>(s, false, cf);
-        store_traces6(T, g, e_, c, cf);
+        euler::cweno4_64(s, poly);
+        store_traces6(T, g, e_, c, poly);
     }
     if (fail) {  // first order: every trace is the cell value (rhs_function.c:302-306)
 #pragma unroll 1
