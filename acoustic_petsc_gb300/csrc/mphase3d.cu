@@ -14,11 +14,10 @@
 //   k_m3_ghost   conservative SoA -> primitive with 3 ghost layers (boundary maps per
 //                axis: periodic, transmissive copy, reflective mirror with the normal
 //                velocity negated, rhs_function.c:98-230);
-//   k_m3_recon   per extended cell: CWENO4 of the 6 primitive variables, the 33-node
-//                density / pressure check (node values from compile-time monomials),
-//                the 24 face traces per variable (or the cell values on failure);
-//   k_m3_faces   per face: 4 Gauss points of the rotated HLLC flux (7 components),
-//                wave-speed maxima;
+//   k_m3_recon   per extended cell and variable: CWENO4, the 24 face traces, and the 33-node check of
+//                density and pressure (a bound on the polynomial first, node values where it fails);
+//   k_m3_first_order  the cell values as traces where a node failed;
+//   k_m3_faces   per face and Gauss point: the rotated HLLC flux (7 components), wave-speed maxima;
 //   k_m3_update  RHS with the phi term, fused with the SSP stage combination.
 #include <cuda_runtime.h>
 #include <string.h>
@@ -50,7 +49,16 @@ struct Geo {
 
 struct Eos {
     double g1, p1, g2, p2, mu1, mu2;
+    // formed once on the host: g1 - 1, g2 - g1, (g1 - 1)(g2 - 1) and its reciprocal, and g p / (g - 1) of
+    // the second gas and of the difference first - second
+    double g1m, dg, k, rk, c2, dc;
+    int stiff;
 };
+
+inline Eos make_eos(double g1, double p1, double g2, double p2, double mu1, double mu2) {
+    const double c1 = g1 * p1 / (g1 - 1.0), c2 = g2 * p2 / (g2 - 1.0), k = (g1 - 1.0) * (g2 - 1.0);
+    return Eos{g1, p1, g2, p2, mu1, mu2, g1 - 1.0, g2 - g1, k, 1.0 / k, c2, c1 - c2, p1 != 0.0 || p2 != 0.0};
+}
 
 struct DevScalars {
     unsigned long long smax_bits[6];   // [0..3] stages, [4] RHS-only calls
@@ -61,163 +69,221 @@ struct DevScalars {
 };
 
 // ---------------------------------------------------------------- EOS (pde.c:9-45)
-__device__ __forceinline__ double mix_g(const Eos& e, double phi) {
-    return 1.0 + (e.g1 - 1.0) * (e.g2 - 1.0) / ((1.0 - phi) * (e.g1 - 1.0) + phi * (e.g2 - 1.0));
-}
-__device__ __forceinline__ double mix_pinf(const Eos& e, double g, double phi) {
-    // with no stiffness in either gas both terms vanish, and so does the product: no divisions
-    if (e.p1 == 0.0 && e.p2 == 0.0) return 0.0;
-    return ((g - 1.0) / g) * (e.g1 * e.p1 * phi / (e.g1 - 1.0) + e.g2 * e.p2 * (1.0 - phi) / (e.g2 - 1.0));
+// With d = (1 - phi)(g1 - 1) + phi (g2 - 1), linear in phi, and k = (g1 - 1)(g2 - 1):
+//   gamma - 1 = k / d, 1 / (gamma - 1) = d / k, and gamma P_inf / (gamma - 1) = c1 phi + c2 (1 - phi), c = g p / (g - 1),
+// so a state costs one reciprocal.
+__device__ __forceinline__ double mix_d(const Eos& e, double phi) { return fma(phi, e.dg, e.g1m); }
+__device__ __forceinline__ double mix_c(const Eos& e, double phi) { return fma(phi, e.dc, e.c2); }
+// P_inf = (gamma - 1) / gamma (c1 phi + c2 (1 - phi)), 0 with no stiffness in either gas
+__device__ __forceinline__ double mix_pinf(const Eos& e, double phi) {
+    return e.stiff ? e.k / (mix_d(e, phi) + e.k) * mix_c(e, phi) : 0.0;
 }
 __device__ __forceinline__ void cons2prim(const Eos& e, const double* Q, double* V) {
-    const double g = mix_g(e, Q[5]);
-    const double P_inf = mix_pinf(e, g, Q[5]);
-    const double temp = 1.0 / Q[0];
+    const double gm1 = e.k * euler::recip(mix_d(e, Q[5]));
+    const double ir = euler::recip(Q[0]);
+    double pe = fma(-0.5 * ir, fma(Q[3], Q[3], fma(Q[2], Q[2], Q[1] * Q[1])), Q[4]);
+    if (e.stiff) pe -= mix_c(e, Q[5]);
     V[0] = Q[0];
-    V[1] = Q[1] * temp;
-    V[2] = Q[2] * temp;
-    V[3] = Q[3] * temp;
-    V[4] = (g - 1.0) * (Q[4] - 0.5 * temp * (Q[1] * Q[1] + Q[2] * Q[2] + Q[3] * Q[3])) - g * P_inf;
+    V[1] = Q[1] * ir;
+    V[2] = Q[2] * ir;
+    V[3] = Q[3] * ir;
+    V[4] = gm1 * pe;
     V[5] = Q[5];
 }
 
-// One side of a face: the primitive trace and what PDEConsFluxPrim / PDEPrim2Cons derive
-// from it that does not depend on the normal (pde.c:142-202, 27-45): mixture gamma and
-// P_inf, total energy, sound speed.  Computed once per trace instead of once per HLLC
-// evaluation (the rotated solver makes three).
+// One side of a Gauss point: the primitive trace, E + p and the sound speed (PDEConsFluxPrim, PDEPrim2Cons:
+// pde.c:142-202, 27-45)
 struct Side {
-    double rho, u, v, w, p, phi, E, a, irho;
+    double rho, u, v, w, p, phi, H, a;
 };
 
 __device__ __forceinline__ Side make_side(const Eos& e, const double* V, bool& bad) {
     Side s;
     s.rho = V[0]; s.u = V[1]; s.v = V[2]; s.w = V[3]; s.p = V[4]; s.phi = V[5];
-    const double g = mix_g(e, s.phi);
-    const double P_inf = mix_pinf(e, g, s.phi);
-    s.E = 0.5 * s.rho * (s.u * s.u + s.v * s.v + s.w * s.w) + (s.p + g * P_inf) / (g - 1.0);
-    if (s.rho < RHO_FLOOR || (s.p + P_inf) < PRS_FLOOR) bad = true;
-    s.irho = euler::recip(s.rho);
-    s.a = sqrt(g * (s.p + P_inf) * s.irho);
+    const double d = mix_d(e, s.phi);
+    const double gm1 = e.k * euler::recip(d);
+    double gp = fma(gm1, s.p, s.p);                  // gamma (p + P_inf)
+    double pe = fma(d * e.rk, s.p, s.p);             // p + (p + gamma P_inf) / (gamma - 1)
+    if (e.stiff) {
+        const double c = mix_c(e, s.phi);
+        gp = fma(gm1, c, gp);
+        pe += c;
+        bad |= gp < PRS_FLOOR * (1.0 + gm1);
+    } else {
+        bad |= s.p < PRS_FLOOR;
+    }
+    bad |= s.rho < RHO_FLOOR;
+    s.H = fma(0.5 * s.rho, fma(s.w, s.w, fma(s.v, s.v, s.u * s.u)), pe);
+    s.a = euler::sqrt3(gp * euler::recip(s.rho));
     return s;
 }
 
-// PDEHLLCRiemannSolver (pde.c:273-379) for a unit normal n, 7 flux components.  The
-// reference builds the star-state velocity from (S_star, u.t1, u.t2) in its Miller-Colella
-// frame M = [n; t1; t2] and the inverse of M (pde.c:290-323); since M^-1 M u = u, that
-// velocity is u + (S_star - u.n) c with c the first column of M^-1, (t1 x t2) / det M.
-// The frame's t2z of the first branch (pde.c:302) is not the one of n x t1, so M is not
-// orthonormal and c is not n: c is formed from the reference's t1, t2 as they are.
-__device__ __forceinline__ double hllc7(const Side& L, const Side& R, double nx, double ny, double nz, double* Flux) {
-    const double un_L = L.u * nx + L.v * ny + L.w * nz, un_R = R.u * nx + R.v * ny + R.w * nz;
-    const double S_L = fmin(un_R - R.a, un_L - L.a);
-    const double S_R = fmax(un_L + L.a, un_R + R.a);
-    const double S_star = (R.p - L.p + L.rho * un_L * (S_L - un_L) - R.rho * un_R * (S_R - un_R)) *
-                          euler::recip(L.rho * (S_L - un_L) - R.rho * (S_R - un_R));
-    // the reference's branch order (pde.c:368-376); with S_L == 0 and S_star >= 0 it leaves
-    // the flux unset, here zero
-    const int sel = (S_L > 0.0) ? 0 : (S_star >= 0.0 && S_L < 0.0) ? 1 : (S_star < 0.0 && S_R >= 0.0) ? 2
-                                : (S_R < 0.0) ? 3 : 4;
-    if (sel == 4) {
-#pragma unroll
-        for (int i = 0; i < MF; ++i) Flux[i] = 0.0;
-        return fmax(fabs(un_L) + L.a, fabs(un_R) + R.a);
-    }
-    const bool left = sel <= 1;
-    const Side& K = left ? L : R;
-    const double un = left ? un_L : un_R;
-    // the side's flux (PDEConsFluxPrim) and, for the star states, S (Q* - Q)
-    double F[MF];
-    F[0] = K.rho * un;
-    F[1] = K.rho * K.u * un + K.p * nx;
-    F[2] = K.rho * K.v * un + K.p * ny;
-    F[3] = K.rho * K.w * un + K.p * nz;
-    F[4] = (K.E + K.p) * un;
-    F[5] = K.phi * un;
-    F[6] = un;
-    if (sel == 1 || sel == 2) {
-        // the frame of pde.c:290-312 and the first column of its inverse
-        double t1x, t1y, t1z, t2x, t2y, t2z;
-        if (fabs(ny + nz) > fabs(ny - nz)) {
-            const double il = rsqrt(2.0 * (1.0 + nz * (ny - nx) + nx * ny));
-            t1x = (ny + nz) * il; t1y = (nz - nx) * il; t1z = -(nx + ny) * il;
-            t2x = (nx * (nz - ny) - ny * ny - nz * nz) * il;
-            t2y = (ny * (nx + nz) + nx * nx + nz * nz) * il;
-            t2z = (nz * (nx - nz) - nx * nx - ny * ny) * il;
-        } else {
-            const double il = rsqrt(2.0 * (1.0 - nx * ny - nx * nz - ny * nz));
-            t1x = (ny - nz) * il; t1y = (nz - nx) * il; t1z = (nx - ny) * il;
-            t2x = (nx * (ny + nz) - ny * ny - nz * nz) * il;
-            t2y = (ny * (nx + nz) - nx * nx - nz * nz) * il;
-            t2z = (nz * (nx + ny) - nx * nx - ny * ny) * il;
-        }
-        const double cx = t1y * t2z - t1z * t2y, cy = t1z * t2x - t1x * t2z, cz = t1x * t2y - t1y * t2x;
-        const double idet = euler::recip(nx * cx + ny * cy + nz * cz);
-        const double S = left ? S_L : S_R;
-        const double isd = euler::recip(S - S_star);
-        const double q0 = K.rho * (S - un) * isd;
-        const double dn = (S_star - un) * idet;
-        const double Qs[MV] = {q0, q0 * (K.u + dn * cx), q0 * (K.v + dn * cy), q0 * (K.w + dn * cz),
-                               q0 * ((K.E * K.irho) + (S_star - un) * (S_star + K.p * K.irho * euler::recip(S - un))),
-                               K.phi * (S - un) * isd};
-        const double Q[MV] = {K.rho, K.rho * K.u, K.rho * K.v, K.rho * K.w, K.E, K.phi};
-#pragma unroll
-        for (int i = 0; i < MV; ++i) F[i] = F[i] + S * (Qs[i] - Q[i]);
-        F[6] = un + S * (((S - un) * isd) - 1.0);
-    }
-#pragma unroll
-    for (int i = 0; i < MF; ++i) Flux[i] = F[i];
-    return fmax(fabs(un_L) + L.a, fabs(un_R) + R.a);
+// comparisons of a number with zero as the floating ones decide them (false for NaN), on the bit pattern
+__device__ __forceinline__ bool above0(double x) {
+    const long long b = __double_as_longlong(x);
+    return b > 0 && b <= 0x7FF0000000000000ll;
+}
+__device__ __forceinline__ bool below0(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    return b > 0x8000000000000000ull && b <= 0xFFF0000000000000ull;
+}
+__device__ __forceinline__ bool from0(double x) {  // x >= 0
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    return b <= 0x7FF0000000000000ull || b == 0x8000000000000000ull;
+}
+__device__ __forceinline__ bool abs_above(double x, double y) {  // |x| > |y|, neither NaN
+    return (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) > (__double_as_longlong(y) & 0x7FFFFFFFFFFFFFFFll);
+}
+__device__ __forceinline__ double neg_if(bool c, double x) {
+    return __hiloint2double(__double2hiint(x) ^ (c ? 0x80000000 : 0), __double2loint(x));
 }
 
-// PDErotHLLCRiemannSolver (pde.c:383-440): HLLC along the velocity-jump direction n1 and
-// its two Miller-Colella tangents, weighted by their projections on the face normal
-__device__ __forceinline__ double rot_hllc7(const Side& L, const Side& R, double nx, double ny, double nz, double* Flux) {
+// What the three HLLC solves of a Gauss point add up to.  With un the normal velocity of the side K that the
+// solve selects, e = S_star - un, z = e / (S - S_star) (so that the star state's density factor
+// (S - un) / (S - S_star) is 1 + z) and Y = S e rho (1 + z), the flux of PDEHLLCRiemannSolver
+// (pde.c:273-379) is, per component,
+//   rho m, rho u m + p n + Y c, (E + p) m + Y S_star, phi m, m,     m = un + S z
+// (z = Y = 0 outside the star region).  Everything that multiplies m depends on the side alone, so the
+// solves' weighted m are summed per side and the components formed once.
+struct HllcSum {
+    double mL, mR, px, py, pz, en;
+};
+
+// The selection of pde.c:368-376 (0 left, 1 left star, 2 right star, 3 right): with S_L == 0 and
+// S_star >= 0 the program leaves the flux unset, here zero (4)
+__device__ __forceinline__ int hllc_select(double SL, double SR, double Ss) {
+    return above0(SL) ? 0 : (from0(Ss) && below0(SL)) ? 1 : (below0(Ss) && from0(SR)) ? 2 : below0(SR) ? 3 : 4;
+}
+
+// The momentum of one solve along the unit normal n, weight wt: wt (p n + Y c).  The program builds the
+// star velocity from (S_star, u.t1, u.t2) in its Miller-Colella frame M = [n; t1; t2] and the inverse of M
+// (pde.c:290-323), which is u + e c with c the first column of M^-1.  Where |ny + nz| <= |ny - nz| the frame
+// is orthonormal and c = n.  In the other branch its t2z (pde.c:302) differs from that of n x t1 by
+// nz (ny - nz) il, and with q2 = (ny + nz)^2 + (nz - nx)^2 + (nx + ny)^2 = 1 / il^2 and d = nz (ny - nz),
+// t1 x t2 / det = (q2 n + d (nz - nx, -(ny + nz), 0)) / (q2 + d (nx (nz - nx) - ny (ny + nz))).
+__device__ __forceinline__ void hllc_momentum(double nx, double ny, double nz, double wt, double p, double Y, HllcSum& h) {
+    double pn = p + Y;
+    const double s = ny + nz, d = ny - nz;
+    if (abs_above(s, d)) {
+        const double b = nz - nx;
+        const double q2 = fma(2.0 * nz, ny - nx, fma(2.0 * nx, ny, 2.0));
+        const double dz = nz * d;
+        const double Yr = Y * euler::recip(fma(dz, fma(nx, b, -ny * s), q2));
+        pn = fma(q2, Yr, p);
+        const double g = wt * (dz * Yr);
+        h.px = fma(g, b, h.px);
+        h.py = fma(-g, s, h.py);
+    }
+    pn *= wt;
+    h.px = fma(pn, nx, h.px);
+    h.py = fma(pn, ny, h.py);
+    h.pz = fma(pn, nz, h.pz);
+}
+
+// One solve of weight wt along a normal of any direction: adds to h, returns the wave speed
+__device__ __forceinline__ double hllc_general(const Side& L, const Side& R, double nx, double ny, double nz, double wt,
+                                               HllcSum& h) {
+    const double unL = fma(L.w, nz, fma(L.v, ny, L.u * nx)), unR = fma(R.w, nz, fma(R.v, ny, R.u * nx));
+    const double SL = fmin(unR - R.a, unL - L.a), SR = fmax(unL + L.a, unR + R.a);
+    const double rL = L.rho * (SL - unL), rR = R.rho * (SR - unR);
+    const double Ss = fma(-rR, unR, fma(rL, unL, R.p - L.p)) * euler::recip(rL - rR);
+    const int sel = hllc_select(SL, SR, Ss);
+    if (sel != 4) {
+        const bool left = sel <= 1;
+        const double un = left ? unL : unR, p = left ? L.p : R.p;
+        double m = un, Y = 0.0;
+        if (sel == 1 || sel == 2) {
+            const double S = left ? SL : SR, e = Ss - un;
+            const double z = e * euler::recip(S - Ss);
+            m = fma(S, z, un);
+            Y = (S * e) * fma(left ? L.rho : R.rho, z, left ? L.rho : R.rho);
+            h.en = fma(wt * Y, Ss, h.en);
+        }
+        if (left) h.mL = fma(wt, m, h.mL);
+        else h.mR = fma(wt, m, h.mR);
+        hllc_momentum(nx, ny, nz, wt, p, Y, h);
+    }
+    return euler::max_pos(fabs(unL) + L.a, fabs(unR) + R.a);
+}
+
+// PDErotHLLCRiemannSolver (pde.c:383-440) across an axis face of normal D: HLLC along the velocity-jump
+// direction n1 and its two Miller-Colella tangents, weighted by their projections on the face normal.  The
+// tangents are perpendicular to the jump, so both sides have one normal velocity un there: the acoustic
+// speeds are un -+ amax and S_star - un, and with it z and rho (1 + z), is the same for both tangents.
+// Without a jump n1 is the face normal, the tangents' weights are exactly zero and only their wave
+// speeds count.  About 260 FP64 operations (three general solves: about 800).
+template <int D>
+__device__ __forceinline__ double rot_hllc7(const Side& L, const Side& R, double* Flux) {
     const double du = R.u - L.u, dv = R.v - L.v, dw = R.w - L.w;
-    const double dq2 = du * du + dv * dv + dw * dw;
-    double n1x, n1y, n1z;
-    if (dq2 < 1.0E-20) {  // |du| < 1e-10 (pde.c:391)
-        n1x = nx; n1y = ny; n1z = nz;
+    const double dq2 = fma(dw, dw, fma(dv, dv, du * du));
+    const bool still = dq2 < 1.0E-20;  // |du| < 1e-10 (pde.c:391)
+    double nx = D == 0 ? 1.0 : 0.0, ny = D == 1 ? 1.0 : 0.0, nz = D == 2 ? 1.0 : 0.0, a1 = 1.0;
+    if (!still) {
+        const double idq = euler::rsqrt3(dq2);
+        const bool flip = __double2hiint(D == 0 ? du : D == 1 ? dv : dw) < 0;
+        const double sg = neg_if(flip, idq);
+        nx = du * sg; ny = dv * sg; nz = dw * sg;
+        a1 = D == 0 ? nx : D == 1 ? ny : nz;
+    }
+    // t1 and t2 = n1 x t1 of pde.c:402-424
+    const double s = ny + nz, d = ny - nz, b = nz - nx;
+    double t1x, t1y, t1z;
+    if (abs_above(s, d)) {
+        const double il = euler::rsqrt3(fma(2.0 * nz, ny - nx, fma(2.0 * nx, ny, 2.0)));
+        t1x = s * il; t1y = b * il; t1z = -(nx + ny) * il;
     } else {
-        const double idq = rsqrt(dq2);
-        n1x = du * idq; n1y = dv * idq; n1z = dw * idq;
+        const double il = euler::rsqrt3(fma(-2.0 * nz, nx + ny, fma(-2.0 * nx, ny, 2.0)));
+        t1x = d * il; t1y = b * il; t1z = (nx - ny) * il;
     }
-    double a1 = n1x * nx + n1y * ny + n1z * nz;
-    if (a1 < 0.0) {
-        n1x = -n1x; n1y = -n1y; n1z = -n1z; a1 = -a1;
-    }
-    double t1x, t1y, t1z, t2x, t2y, t2z;
-    if (fabs(n1y + n1z) > fabs(n1y - n1z)) {
-        const double il = rsqrt(2.0 * (1.0 + n1z * (n1y - n1x) + n1x * n1y));
-        t1x = (n1y + n1z) * il; t1y = (n1z - n1x) * il; t1z = -(n1x + n1y) * il;
-        t2x = (n1x * (n1z - n1y) - n1y * n1y - n1z * n1z) * il;
-        t2y = (n1y * (n1x + n1z) + n1x * n1x + n1z * n1z) * il;
-        t2z = (n1z * (n1x - n1y) - n1x * n1x - n1y * n1y) * il;
+    double t2x = fma(ny, t1z, -nz * t1y), t2y = fma(nz, t1x, -nx * t1z), t2z = fma(nx, t1y, -ny * t1x);
+    HllcSum h{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    double smax = hllc_general(L, R, nx, ny, nz, a1, h);
+    if (still) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const double tx = q ? t2x : t1x, ty = q ? t2y : t1y, tz = q ? t2z : t1z;
+            const double unL = fma(L.w, tz, fma(L.v, ty, L.u * tx)), unR = fma(R.w, tz, fma(R.v, ty, R.u * tx));
+            smax = euler::max_pos(smax, euler::max_pos(fabs(unL) + L.a, fabs(unR) + R.a));
+        }
     } else {
-        const double il = rsqrt(2.0 * (1.0 - n1x * n1y - n1x * n1z - n1y * n1z));
-        t1x = (n1y - n1z) * il; t1y = (n1z - n1x) * il; t1z = (n1x - n1y) * il;
-        t2x = (n1x * (n1y + n1z) - n1y * n1y - n1z * n1z) * il;
-        t2y = (n1y * (n1x + n1z) - n1x * n1x - n1z * n1z) * il;
-        t2z = (n1z * (n1x + n1y) - n1x * n1x - n1y * n1y) * il;
-    }
-    double a2 = t1x * nx + t1y * ny + t1z * nz;
-    if (a2 < 0.0) {
-        t1x = -t1x; t1y = -t1y; t1z = -t1z; a2 = -a2;
-    }
-    double a3 = t2x * nx + t2y * ny + t2z * nz;
-    if (a3 < 0.0) {
-        t2x = -t2x; t2y = -t2y; t2z = -t2z; a3 = -a3;
-    }
-    double F1[MF];
-    const double s1 = hllc7(L, R, n1x, n1y, n1z, F1);
+        const double am = euler::max_pos(L.a, R.a);
+        const double e = (L.p - R.p) * euler::recip((L.rho + R.rho) * am);  // S_star - un
+        const double zL = -e * euler::recip(am + e), zR = e * euler::recip(am - e);
+        const double yL = e * fma(L.rho, zL, L.rho), yR = e * fma(R.rho, zR, R.rho);
 #pragma unroll
-    for (int c = 0; c < MF; ++c) Flux[c] = a1 * F1[c];
-    const double s2 = hllc7(L, R, t1x, t1y, t1z, F1);
-#pragma unroll
-    for (int c = 0; c < MF; ++c) Flux[c] += a2 * F1[c];
-    const double s3 = hllc7(L, R, t2x, t2y, t2z, F1);
-#pragma unroll
-    for (int c = 0; c < MF; ++c) Flux[c] += a3 * F1[c];
-    return fmax(s1, fmax(s2, s3));
+        for (int q = 0; q < 2; ++q) {
+            double tx = q ? t2x : t1x, ty = q ? t2y : t1y, tz = q ? t2z : t1z;
+            double wt = D == 0 ? tx : D == 1 ? ty : tz;
+            const bool flip = below0(wt);
+            wt = neg_if(flip, wt);
+            tx = neg_if(flip, tx); ty = neg_if(flip, ty); tz = neg_if(flip, tz);
+            const double un = fma(L.w, tz, fma(L.v, ty, L.u * tx));
+            const double SL = un - am, SR = un + am, Ss = un + e;
+            const int sel = hllc_select(SL, SR, Ss);
+            smax = euler::max_pos(smax, fabs(un) + am);
+            if (sel == 4) continue;
+            const bool left = sel <= 1;
+            double m = un, Y = 0.0;
+            if (sel == 1 || sel == 2) {
+                const double S = left ? SL : SR;
+                m = fma(S, left ? zL : zR, un);
+                Y = S * (left ? yL : yR);
+                h.en = fma(wt * Y, Ss, h.en);
+            }
+            if (left) h.mL = fma(wt, m, h.mL);
+            else h.mR = fma(wt, m, h.mR);
+            hllc_momentum(tx, ty, tz, wt, left ? L.p : R.p, Y, h);
+        }
+    }
+    const double qL = L.rho * h.mL, qR = R.rho * h.mR;
+    Flux[0] = qL + qR;
+    Flux[1] = fma(L.u, qL, fma(R.u, qR, h.px));
+    Flux[2] = fma(L.v, qL, fma(R.v, qR, h.py));
+    Flux[3] = fma(L.w, qL, fma(R.w, qR, h.pz));
+    Flux[4] = fma(L.H, h.mL, fma(R.H, h.mR, h.en));
+    Flux[5] = fma(L.phi, h.mL, R.phi * h.mR);
+    Flux[6] = h.mL + h.mR;
+    return smax;
 }
 
 // ---------------------------------------------------------------- admissibility nodes
@@ -281,22 +347,38 @@ __device__ __forceinline__ bool rho_fails(const double* c) {
     }
 }
 
-// true when some node has p + P_inf(phi) < floor; phi's coefficients at ph[q * 128]
+// true when some node has p + P_inf(phi) < floor; phi's polynomial at ph[q * st] (read only with stiffness)
 template <int M = 0>
-__device__ __forceinline__ bool prs_fails(const double* cp, const double* ph, const Eos& e, bool stiff) {
+__device__ __forceinline__ bool prs_fails(const double* cp, const double* ph, int st, const Eos& e) {
     if constexpr (M == 33) {
         return false;
     } else {
         double pinf = 0.0;
-        if (stiff) {
+        if (e.stiff) {
             double cphi[20];
 #pragma unroll
-            for (int q = 0; q < 20; ++q) cphi[q] = ph[q * 128];
-            const double phi = node_value<M>(cphi);
-            pinf = mix_pinf(e, mix_g(e, phi), phi);
+            for (int q = 0; q < 20; ++q) cphi[q] = ph[q * st];
+            pinf = mix_pinf(e, node_value<M>(cphi));
         }
-        return (node_value<M>(cp) + pinf < PRS_FLOOR) | prs_fails<M + 1>(cp, ph, e, stiff);
+        return (node_value<M>(cp) + pinf < PRS_FLOOR) | prs_fails<M + 1>(cp, ph, st, e);
     }
+}
+
+// How far a polynomial can be from its cell value at any of the 33 nodes: the basis functions are at most
+// 1/2 (linear), 1/6 (square), 1/4 (cross), 1/20 (cubic), 1/12 (mixed) and 1/8 there.
+__device__ __forceinline__ double spread(const euler::Poly64& p) {
+    const double l = (fabs(p.lin[0]) + fabs(p.lin[1])) + fabs(p.lin[2]);
+    const double q = (fabs(p.sq[0]) + fabs(p.sq[1])) + fabs(p.sq[2]);
+    const double x = (fabs(p.cr[0]) + fabs(p.cr[1])) + fabs(p.cr[2]);
+    const double c = (fabs(p.ddd[0]) + fabs(p.ddd[1])) + fabs(p.ddd[2]);
+    const double m = ((fabs(p.aab[0]) + fabs(p.abb[0])) + (fabs(p.aab[1]) + fabs(p.abb[1]))) + (fabs(p.aab[2]) + fabs(p.abb[2]));
+    const double r = fma(1. / 64., fabs(p.xyz), fma(1. / 48., m, 0.05 * c));
+    return fma(fabs(p.wr), r, fma(0.125, x, fma(1. / 12., q, 0.25 * l)));
+}
+// no node can be below a floor of 1e-12: 21 operations decide what 33 node values (300) would, except in
+// cells near the floor; the margin 1e-9 covers the rounding of either
+__device__ __forceinline__ bool surely_above(const euler::Poly64& p) {
+    return fma(1.0 - 1.0e-9, p.u0, -spread(p)) > 2.0e-12;
 }
 
 // ---------------------------------------------------------------- kernels
@@ -307,14 +389,28 @@ __device__ __forceinline__ long long ext_index(const Geo& g, int i, int j, int k
     return ((long long)(k + 1) * g.ey + (j + 1)) * g.ex + (i + 1);
 }
 
-__global__ void __launch_bounds__(128) k_m3_ghost(const double* __restrict__ U, double* __restrict__ G, Geo g, Eos e) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x - GW;
-    const int j = blockIdx.y - GW, k = blockIdx.z - GW;
-    if (i >= g.nx + GW) return;
+// The cells of every kernel are indexed flat: rows of 32 x-neighbours left a third of the lanes of a
+// 42-wide box without a cell.
+constexpr int kGhostThreads = 128, kReconThreads = 64, kUpdateThreads = 128;
+
+struct Box3 {
+    int i, j, k;
+    __device__ __forceinline__ Box3(unsigned q, int nx, int ny) {
+        const unsigned row = q / (unsigned)nx, pl = row / (unsigned)ny;
+        i = (int)(q - row * (unsigned)nx);
+        j = (int)(row - pl * (unsigned)ny);
+        k = (int)pl;
+    }
+};
+
+__global__ void __launch_bounds__(kGhostThreads) k_m3_ghost(const double* __restrict__ U, double* __restrict__ G, Geo g, Eos e) {
+    const unsigned dst = blockIdx.x * (unsigned)kGhostThreads + threadIdx.x;
+    if (dst >= (unsigned)g.GN) return;
+    const Box3 b(dst, g.gx, g.gy);
     int fi = 0, fj = 0, fk = 0;
-    const int mi = bmap(i, g.nx, g.bc[0], g.bc[1], &fi);
-    const int mj = bmap(j, g.ny, g.bc[2], g.bc[3], &fj);
-    const int mk = bmap(k, g.nz, g.bc[4], g.bc[5], &fk);
+    const int mi = bmap(b.i - GW, g.nx, g.bc[0], g.bc[1], &fi);
+    const int mj = bmap(b.j - GW, g.ny, g.bc[2], g.bc[3], &fj);
+    const int mk = bmap(b.k - GW, g.nz, g.bc[4], g.bc[5], &fk);
     const long long src = ((long long)mk * g.ny + mj) * g.nx + mi;
     double Q[MV], V[MV];
 #pragma unroll
@@ -323,7 +419,6 @@ __global__ void __launch_bounds__(128) k_m3_ghost(const double* __restrict__ U, 
     if (fi) V[1] = -V[1];
     if (fj) V[2] = -V[2];
     if (fk) V[3] = -V[3];
-    const long long dst = ghost_index(g, i, j, k);
 #pragma unroll
     for (int c = 0; c < MV; ++c) G[c * g.GN + dst] = V[c];
 }
@@ -353,137 +448,151 @@ __device__ __forceinline__ void gather33(const double* __restrict__ p, int sy, i
             for (int d = 0; d < 2; ++d) s[SO(a, b, d)] = __ldg(p + (2 * a - 1) + (2 * b - 1) * sy + (2 * d - 1) * sz);
 }
 
-__device__ __forceinline__ void store_traces6(double* __restrict__ T, const Geo& g, long long e, int c,
-                                              const euler::Poly64& poly) {
-    double* Tc = T + (long long)c * NTR * g.NE + e;
-    euler::store_traces64(poly, Tc, g.NE);
-}
-
-// T[c][face*4+gp][extended cell]; the cells the faces of owned cells need (at most one
-// coordinate outside the grid)
-__global__ void __launch_bounds__(128) k_m3_recon(const double* __restrict__ G, double* __restrict__ T, Geo g, Eos e,
-                                                  DevScalars* __restrict__ ds) {
-    __shared__ double sphi[20 * 128];  // phi's coefficients, [q][thread]
-    const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y - 1;
-    const int k = blockIdx.z - 1;
-    if (i > g.nx || j > g.ny) return;
+// T[c][face*4+gp][extended cell]; the cells the faces of owned cells need (at most one coordinate outside
+// the grid).  One thread per cell and variable (blockIdx.y), as the single-gas reconstruction: a cell's six
+// variables in turn left a 40 x 40 x 100 grid less than four waves of 2300-instruction threads.  Density and
+// pressure are checked at the nodes; with stiffness the pressure check needs phi's polynomial, so that thread
+// does phi first (blockIdx.y = 4: phi and p).  A failing cell is marked and its traces replaced by
+// k_m3_first_order, since its variables are in different threads.
+// Bound: FP64 issue (361 operations per variable, 21 per check).
+__global__ void __launch_bounds__(kReconThreads) k_m3_recon(const double* __restrict__ G, double* __restrict__ T, Geo g, Eos e,
+                                                            unsigned char* __restrict__ fail) {
+    __shared__ double sphi[20 * kReconThreads];  // phi's coefficients, [q][thread]
+    const unsigned e_ = blockIdx.x * (unsigned)kReconThreads + threadIdx.x;
+    if (e_ >= (unsigned)g.NE) return;
+    const Box3 b(e_, g.ex, g.ey);
+    const int i = b.i - 1, j = b.j - 1, k = b.k - 1;
     const int outside = (i < 0 || i >= g.nx) + (j < 0 || j >= g.ny) + (k < 0 || k >= g.nz);
     if (outside > 1) return;
-    const long long e_ = ext_index(g, i, j, k), ge = ghost_index(g, i, j, k);
+    const long long ge = ghost_index(g, i, j, k);
     const int sy = g.gx, sz = g.gx * g.gy;
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    double* ph = sphi + tid;
-    const bool stiff = e.p1 != 0.0 || e.p2 != 0.0;
-    bool fail = false;
-    {  // density: the node check and its traces
-        double s[33], cf[20];
-        euler::Poly64 poly;
-        gather33(G + 0 * g.GN + ge, sy, sz, s);
-        euler::cweno4_64(s, poly);
-        euler::coeffs64(poly, cf);
-        fail |= rho_fails(cf);
-        store_traces6(T, g, e_, 0, poly);
-    }
-    {  // volume fraction: coefficients kept for the pressure check
-        double s[33], cf[20];
-        euler::Poly64 poly;
-        gather33(G + 5 * g.GN + ge, sy, sz, s);
-        euler::cweno4_64(s, poly);
-        if (stiff) {
-            euler::coeffs64(poly, cf);
-#pragma unroll
-            for (int q = 0; q < 20; ++q) ph[q * 128] = cf[q];
-        }
-        store_traces6(T, g, e_, 5, poly);
-    }
-    {  // pressure
-        double s[33], cf[20];
-        euler::Poly64 poly;
-        gather33(G + 4 * g.GN + ge, sy, sz, s);
-        euler::cweno4_64(s, poly);
-        euler::coeffs64(poly, cf);
-        fail |= prs_fails(cf, ph, e, stiff);
-        store_traces6(T, g, e_, 4, poly);
-    }
+    double* ph = sphi + threadIdx.x;
+    const int last = blockIdx.y;  // 0..3, then p; without stiffness phi is a sixth row of blocks
+    bool phi_above = true;
 #pragma unroll 1
-    for (int c = 1; c < 4; ++c) {
+    for (int c = (e.stiff && last == 4) ? 5 : last;; c = last) {
         double s[33];
         euler::Poly64 poly;
         gather33(G + c * g.GN + ge, sy, sz, s);
         euler::cweno4_64(s, poly);
-        store_traces6(T, g, e_, c, poly);
-    }
-    if (fail) {  // first order: every trace is the cell value (rhs_function.c:302-306)
-#pragma unroll 1
-        for (int c = 0; c < MV; ++c) {
-            const double v = G[c * g.GN + ge];
+        euler::store_traces64(poly, T + (long long)c * NTR * g.NE + e_, g.NE);
+        if (c != last) {
+            // P_inf >= 0 wherever 0 <= phi <= 1
+            const double sp = spread(poly);
+            phi_above = poly.u0 - sp >= 0.0 && poly.u0 + sp <= 1.0 && e.p1 >= 0.0 && e.p2 >= 0.0;
+            if (!phi_above) {
+                double cf[20];
+                euler::coeffs64(poly, cf);
 #pragma unroll
-            for (int q = 0; q < NTR; ++q) T[((long long)c * NTR + q) * g.NE + e_] = v;
+                for (int q = 0; q < 20; ++q) ph[q * kReconThreads] = cf[q];
+            }
+            continue;
         }
-        if (outside == 0) atomicAdd(&ds->fallback, 1ull);
+        if (c == 0 || c == 4) {
+            if (!(surely_above(poly) && phi_above)) {
+                double cf[20];
+                euler::coeffs64(poly, cf);
+                if (phi_above && e.stiff && c == 4) {  // phi's polynomial was not kept: form it again
+                    double sf[33];
+                    euler::Poly64 pf;
+                    gather33(G + 5 * g.GN + ge, sy, sz, sf);
+                    euler::cweno4_64(sf, pf);
+                    double cp[20];
+                    euler::coeffs64(pf, cp);
+#pragma unroll
+                    for (int q = 0; q < 20; ++q) ph[q * kReconThreads] = cp[q];
+                }
+                if (c == 0 ? rho_fails(cf) : prs_fails(cf, ph, kReconThreads, e)) fail[e_] = 1;
+            }
+        }
+        break;
     }
 }
 
-__device__ __forceinline__ void atomic_max_pos(unsigned long long* a, double v) {
-    atomicMax(a, (unsigned long long)__double_as_longlong(v));
+// first order where a node was inadmissible: every trace is the cell value (rhs_function.c:302-306)
+__global__ void __launch_bounds__(128) k_m3_first_order(const double* __restrict__ G, double* __restrict__ T, Geo g,
+                                                        unsigned char* __restrict__ fail, DevScalars* __restrict__ ds) {
+    const unsigned e_ = blockIdx.x * 128u + threadIdx.x;
+    if (e_ >= (unsigned)g.NE || !fail[e_]) return;
+    fail[e_] = 0;
+    const Box3 b(e_, g.ex, g.ey);
+    const int i = b.i - 1, j = b.j - 1, k = b.k - 1;
+    const long long ge = ghost_index(g, i, j, k);
+#pragma unroll 1
+    for (int c = 0; c < MV; ++c) {
+        const double v = G[c * g.GN + ge];
+#pragma unroll
+        for (int q = 0; q < NTR; ++q) T[((long long)c * NTR + q) * g.NE + e_] = v;
+    }
+    if (i >= 0 && i < g.nx && j >= 0 && j < g.ny && k >= 0 && k < g.nz) atomicAdd(&ds->fallback, 1ull);
 }
 
-// faces normal to D: the low cell's face 2D+1 against the high cell's face 2D
+// The maximum only grows while a kernel runs: a warp that does not exceed what it reads leaves it alone
+__device__ __forceinline__ void raise_max(unsigned long long* a, double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    if (v > 0.0 && b > *(volatile unsigned long long*)a) atomicMax(a, b);
+}
+
+// Faces normal to D: the low cell's face 2D+1 against the high cell's face 2D.  All three directions in one
+// launch (blockIdx.y); a block is 32 faces, indexed flat, x the 4 Gauss points, one point per warp, summed
+// through shared memory.  Bound: FP64 issue.  With one thread per face, its four points in turn, and three
+// general solves per point the three face launches of a 40 x 40 x 100 RHS took 3.9 ms of 5.6; a whole RHS
+// and stage now takes 1.9 ms (22.5 -> 7.5 ms per step).
 template <int D>
-__global__ void __launch_bounds__(128) k_m3_faces(const double* __restrict__ T, double* __restrict__ F, Geo g, Eos e,
-                                                  DevScalars* __restrict__ ds, int slot) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z;
-    const int fx = g.nx + (D == 0), fy = g.ny + (D == 1);
-    const bool visc = e.mu1 != 0.0 || e.mu2 != 0.0;
+__device__ __forceinline__ void faces(const double* __restrict__ T, double* __restrict__ F, const Geo& g, const Eos& e,
+                                      DevScalars* __restrict__ ds, int slot, double (*sh)[MF][32]) {
+    const int lane = threadIdx.x & 31, gp = threadIdx.x >> 5;
+    const unsigned f = blockIdx.x * 32u + lane;
+    const unsigned fx = g.nx + (D == 0), fy = g.ny + (D == 1), nf = fx * fy * (g.nz + (D == 2));
+    if (blockIdx.x * 32u >= nf) return;  // the grid is as wide as the direction with the most faces
     double smax = 0.0, smaxv = 0.0;
-    bool bad = false;
-    if (i < fx && j < fy) {
-        const long long eR = ext_index(g, i, j, k);
-        const long long eL = ext_index(g, i - (D == 0), j - (D == 1), k - (D == 2));
-        double acc[MF];
+    if (f < nf) {
+        const Box3 b(f, (int)fx, (int)fy);
+        const double* TL = T + ((2 * D + 1) * 4 + gp) * g.NE + ext_index(g, b.i - (D == 0), b.j - (D == 1), b.k - (D == 2));
+        const double* TR = T + (2 * D * 4 + gp) * g.NE + ext_index(g, b.i, b.j, b.k);
+        double VL[MV], VR[MV], fc[MF];
 #pragma unroll
-        for (int c = 0; c < MF; ++c) acc[c] = 0.0;
-#pragma unroll 1
-        for (int gp = 0; gp < 4; ++gp) {
-            double VL[MV], VR[MV], fc[MF];
-#pragma unroll
-            for (int c = 0; c < MV; ++c) {
-                VL[c] = __ldg(T + ((long long)c * NTR + (2 * D + 1) * 4 + gp) * g.NE + eL);
-                VR[c] = __ldg(T + ((long long)c * NTR + (2 * D) * 4 + gp) * g.NE + eR);
-            }
-            const Side SL = make_side(e, VL, bad), SR = make_side(e, VR, bad);
-            const double s = rot_hllc7(SL, SR, D == 0 ? 1.0 : 0.0, D == 1 ? 1.0 : 0.0, D == 2 ? 1.0 : 0.0, fc);
-            smax = fmax(smax, s);
-            if (visc) {  // PDEViscFluxPrim's speed (4/3) mu / rho on both sides
-                const double r4_3 = 4. / 3;
-                const double svl = r4_3 * (VL[5] * e.mu1 + (1.0 - VL[5]) * e.mu2) / VL[0];
-                const double svr = r4_3 * (VR[5] * e.mu1 + (1.0 - VR[5]) * e.mu2) / VR[0];
-                smaxv = fmax(smaxv, fmax(svl, svr));
-            }
-#pragma unroll
-            for (int c = 0; c < MF; ++c) acc[c] += 0.25 * fc[c];
+        for (int c = 0; c < MV; ++c) {
+            VL[c] = __ldg(TL + c * NTR * g.NE);
+            VR[c] = __ldg(TR + c * NTR * g.NE);
         }
-        const long long nf = (long long)fx * fy * (g.nz + (D == 2));
-        const long long f = ((long long)k * fy + j) * fx + i;
+        bool bad = false;
+        const Side SL = make_side(e, VL, bad), SR = make_side(e, VR, bad);
+        smax = rot_hllc7<D>(SL, SR, fc);
+        if (e.mu1 != 0.0 || e.mu2 != 0.0) {  // PDEViscFluxPrim's speed (4/3) mu / rho on both sides
+            const double r4_3 = 4. / 3;
+            const double svl = r4_3 * (VL[5] * e.mu1 + (1.0 - VL[5]) * e.mu2) / VL[0];
+            const double svr = r4_3 * (VR[5] * e.mu1 + (1.0 - VR[5]) * e.mu2) / VR[0];
+            smaxv = fmax(0.0, fmax(svl, svr));
+        }
 #pragma unroll
-        for (int c = 0; c < MF; ++c) F[c * nf + f] = acc[c];
+        for (int c = 0; c < MF; ++c) sh[gp][c][lane] = fc[c];
         if (bad) {
-            const int ci = i < g.nx ? i : g.nx - 1, cj = j < g.ny ? j : g.ny - 1, ck = k < g.nz ? k : g.nz - 1;
+            const int ci = min(b.i, g.nx - 1), cj = min(b.j, g.ny - 1), ck = min(b.k, g.nz - 1);
             atomicMin(&ds->bad, (unsigned long long)(((long long)ck * g.ny + cj) * g.nx + ci));
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        smax = fmax(smax, __shfl_xor_sync(0xffffffffu, smax, o));
-        smaxv = fmax(smaxv, __shfl_xor_sync(0xffffffffu, smaxv, o));
+        smax = euler::max_pos(smax, __shfl_xor_sync(0xffffffffu, smax, o));
+        smaxv = euler::max_pos(smaxv, __shfl_xor_sync(0xffffffffu, smaxv, o));
     }
-    if ((threadIdx.x & 31) == 0) {
-        if (smax > 0.0) atomic_max_pos(&ds->smax_bits[slot], smax);
-        if (smaxv > 0.0) atomic_max_pos(&ds->smaxv_bits[slot], smaxv);
+    if (lane == 0) {
+        raise_max(&ds->smax_bits[slot], smax);
+        raise_max(&ds->smaxv_bits[slot], smaxv);
     }
+    __syncthreads();
+    for (int c = gp; c < MF; c += 4)
+        if (f < nf)
+            F[(long long)c * nf + f] = 0.25 * ((sh[0][c][lane] + sh[1][c][lane]) + (sh[2][c][lane] + sh[3][c][lane]));
+}
+
+__global__ void __launch_bounds__(128) k_m3_faces(const double* __restrict__ T, double* __restrict__ Fx, double* __restrict__ Fy,
+                                                  double* __restrict__ Fz, Geo g, Eos e, DevScalars* __restrict__ ds, int slot) {
+    __shared__ double sh[4][MF][32];
+    if (blockIdx.y == 0) faces<0>(T, Fx, g, e, ds, slot, sh);
+    else if (blockIdx.y == 1) faces<1>(T, Fy, g, e, ds, slot, sh);
+    else faces<2>(T, Fz, g, e, ds, slot, sh);
 }
 
 struct Stage {
@@ -494,42 +603,33 @@ struct Stage {
 // RHS (rhs_function.c:507-552) and the stage combination; Win: the stage input, whose
 // volume fraction multiplies the normal-velocity flux in the phi equation
 // Win, U, W and out may be one array (in-place stages), so they carry no __restrict__
-__global__ void __launch_bounds__(256) k_m3_update(const double* __restrict__ Fx, const double* __restrict__ Fy,
-                                                   const double* __restrict__ Fz, const double* Win,
-                                                   const double* U, const double* W,
-                                                   double* out, Geo g, double r1_h, Stage st,
-                                                   const DevScalars* __restrict__ ds) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z;
-    if (i >= g.nx || j >= g.ny) return;
+__global__ void __launch_bounds__(kUpdateThreads) k_m3_update(const double* __restrict__ Fx, const double* __restrict__ Fy,
+                                                              const double* __restrict__ Fz, const double* Win,
+                                                              const double* U, const double* W,
+                                                              double* out, Geo g, double r1_h, Stage st,
+                                                              const DevScalars* __restrict__ ds) {
+    const unsigned cell = blockIdx.x * (unsigned)kUpdateThreads + threadIdx.x;
+    if (cell >= (unsigned)g.N) return;
+    const unsigned row = cell / (unsigned)g.nx, k = row / (unsigned)g.ny;
+    const int c = blockIdx.y;
     const long long nfx = (long long)(g.nx + 1) * g.ny * g.nz, nfy = (long long)g.nx * (g.ny + 1) * g.nz,
                     nfz = (long long)g.nx * g.ny * (g.nz + 1);
-    const long long ix = ((long long)k * g.ny + j) * (g.nx + 1) + i;
-    const long long iy = ((long long)k * (g.ny + 1) + j) * g.nx + i;
-    const long long cell = ((long long)k * g.ny + j) * g.nx + i, iz = cell;
-    const long long sxy = (long long)g.nx * g.ny;
-    const double phi = Win[5 * g.N + cell];
+    const long long ix = cell + row, iy = cell + k * (unsigned)g.nx, iz = cell, sxy = (long long)g.nx * g.ny;
     const double cdt = st.rhs_only ? 0.0 : st.c * ds->dt;
-    double L[MV];
-#pragma unroll
-    for (int c = 0; c < 5; ++c)
-        L[c] = -r1_h * (Fx[c * nfx + ix + 1] - Fx[c * nfx + ix]) - r1_h * (Fy[c * nfy + iy + g.nx] - Fy[c * nfy + iy]) -
-               r1_h * (Fz[c * nfz + iz + sxy] - Fz[c * nfz + iz]);
-    L[5] = -r1_h * ((Fx[5 * nfx + ix + 1] - phi * Fx[6 * nfx + ix + 1]) - (Fx[5 * nfx + ix] - phi * Fx[6 * nfx + ix])) -
-           r1_h * ((Fy[5 * nfy + iy + g.nx] - phi * Fy[6 * nfy + iy + g.nx]) - (Fy[5 * nfy + iy] - phi * Fy[6 * nfy + iy])) -
-           r1_h * ((Fz[5 * nfz + iz + sxy] - phi * Fz[6 * nfz + iz + sxy]) - (Fz[5 * nfz + iz] - phi * Fz[6 * nfz + iz]));
-#pragma unroll
-    for (int c = 0; c < MV; ++c) {
-        double v;
-        if (st.rhs_only) {
-            v = L[c];
-        } else {
-            v = W[c * g.N + cell] + cdt * L[c];
-            if (st.a != 0.0) v = st.a * U[c * g.N + cell] + st.b * W[c * g.N + cell] + cdt * L[c];
-        }
-        out[c * g.N + cell] = v;
+    // the flux difference of component q over the three directions
+    auto div = [&](int q) {
+        return ((Fx[q * nfx + ix + 1] - Fx[q * nfx + ix]) + (Fy[q * nfy + iy + g.nx] - Fy[q * nfy + iy])) +
+               (Fz[q * nfz + iz + sxy] - Fz[q * nfz + iz]);
+    };
+    double L = div(c);
+    if (c == 5) L = fma(-Win[5 * g.N + cell], div(6), L);
+    L *= -r1_h;
+    double v = L;
+    if (!st.rhs_only) {
+        v = W[c * g.N + cell] + cdt * L;
+        if (st.a != 0.0) v = st.a * U[c * g.N + cell] + st.b * W[c * g.N + cell] + cdt * L;
     }
+    out[c * g.N + cell] = v;
 }
 
 // dt = (1/3) CFL h / (s_max + 2 s_visc / h) (rhs_function.c:559)
@@ -585,26 +685,26 @@ struct hype_mp3d {
     cudaStream_t stream = nullptr;
     double *U = nullptr, *W = nullptr, *S = nullptr, *L = nullptr, *G = nullptr, *T = nullptr;
     double *Fx = nullptr, *Fy = nullptr, *Fz = nullptr, *aos = nullptr;
+    unsigned char* fail = nullptr;  // per extended cell: first order in this RHS; zero between RHS calls
     DevScalars* ds = nullptr;
     DevScalars* hs = nullptr;
 };
 
 static int m3_rhs(hype_mp3d* m, const double* Win, int slot) {
     const Geo& g = m->g;
-    k_m3_ghost<<<dim3(cdiv(g.gx, 128), g.gy, g.nz + 2 * GW), 128, 0, m->stream>>>(Win, m->G, g, m->e);
-    k_m3_recon<<<dim3(cdiv(g.nx + 2, 32), cdiv(g.ny + 2, 4), g.nz + 2), dim3(32, 4), 0, m->stream>>>(m->G, m->T, g,
-                                                                                                     m->e, m->ds);
-    const dim3 bf(32, 4);
-    k_m3_faces<0><<<dim3(cdiv(g.nx + 1, 32), cdiv(g.ny, 4), g.nz), bf, 0, m->stream>>>(m->T, m->Fx, g, m->e, m->ds, slot);
-    k_m3_faces<1><<<dim3(cdiv(g.nx, 32), cdiv(g.ny + 1, 4), g.nz), bf, 0, m->stream>>>(m->T, m->Fy, g, m->e, m->ds, slot);
-    k_m3_faces<2><<<dim3(cdiv(g.nx, 32), cdiv(g.ny, 4), g.nz + 1), bf, 0, m->stream>>>(m->T, m->Fz, g, m->e, m->ds, slot);
-    HYPE_LAUNCHED(5);
+    k_m3_ghost<<<cdiv(g.GN, kGhostThreads), kGhostThreads, 0, m->stream>>>(Win, m->G, g, m->e);
+    k_m3_recon<<<dim3(cdiv(g.NE, kReconThreads), m->e.stiff ? 5 : 6), kReconThreads, 0, m->stream>>>(m->G, m->T, g, m->e, m->fail);
+    k_m3_first_order<<<cdiv(g.NE, 128), 128, 0, m->stream>>>(m->G, m->T, g, m->fail, m->ds);
+    const long long most = std::max({(long long)(g.nx + 1) * g.ny * g.nz, (long long)g.nx * (g.ny + 1) * g.nz,
+                                     (long long)g.nx * g.ny * (g.nz + 1)});
+    k_m3_faces<<<dim3(cdiv(most, 32), 3), 128, 0, m->stream>>>(m->T, m->Fx, m->Fy, m->Fz, g, m->e, m->ds, slot);
+    HYPE_LAUNCHED(4);
     return HYPE_OK;
 }
 
 static int m3_update(hype_mp3d* m, const double* Win, const double* U, const double* W, double* out, Stage st) {
     const Geo& g = m->g;
-    k_m3_update<<<dim3(cdiv(g.nx, 32), cdiv(g.ny, 8), g.nz), dim3(32, 8), 0, m->stream>>>(
+    k_m3_update<<<dim3(cdiv(g.N, kUpdateThreads), MV), kUpdateThreads, 0, m->stream>>>(
         m->Fx, m->Fy, m->Fz, Win, U, W, out, g, 1.0 / m->p.h, st, m->ds);
     HYPE_LAUNCHED(1);
     return HYPE_OK;
@@ -622,7 +722,7 @@ extern "C" int hype_mp3d_create(const hype_mp3d_params* p, hype_mp3d** out) {
     if (p->dt_mode < HYPE_DT_MONITOR || p->dt_mode > HYPE_DT_FIXED) return HYPE_ERR_ARG;
     hype_mp3d* m = new hype_mp3d();
     m->p = *p;
-    m->e = Eos{p->g1, p->p1, p->g2, p->p2, p->mu1, p->mu2};
+    m->e = make_eos(p->g1, p->p1, p->g2, p->p2, p->mu1, p->mu2);
     Geo& g = m->g;
     g.nx = p->nx; g.ny = p->ny; g.nz = p->nz;
     for (int f = 0; f < 6; ++f) g.bc[f] = p->bc[f];
@@ -642,6 +742,8 @@ extern "C" int hype_mp3d_create(const hype_mp3d_params* p, hype_mp3d** out) {
     al(&m->Fx, sizeof(double) * MF * (size_t)(g.nx + 1) * g.ny * g.nz);
     al(&m->Fy, sizeof(double) * MF * (size_t)g.nx * (g.ny + 1) * g.nz);
     al(&m->Fz, sizeof(double) * MF * (size_t)g.nx * g.ny * (g.nz + 1));
+    if (ce == cudaSuccess) ce = cudaMalloc((void**)&m->fail, (size_t)g.NE);
+    if (ce == cudaSuccess) ce = cudaMemset(m->fail, 0, (size_t)g.NE);
     if (ce == cudaSuccess) ce = cudaMalloc((void**)&m->ds, sizeof(DevScalars));
     if (ce == cudaSuccess) ce = cudaMallocHost((void**)&m->hs, sizeof(DevScalars));
     if (ce == cudaSuccess) {
@@ -663,7 +765,7 @@ extern "C" void hype_mp3d_destroy(hype_mp3d* m) {
     if (!m) return;
     if (m->stream) cudaStreamSynchronize(m->stream);
     cudaFree(m->U); cudaFree(m->W); cudaFree(m->S); cudaFree(m->L); cudaFree(m->aos); cudaFree(m->G); cudaFree(m->T);
-    cudaFree(m->Fx); cudaFree(m->Fy); cudaFree(m->Fz); cudaFree(m->ds);
+    cudaFree(m->Fx); cudaFree(m->Fy); cudaFree(m->Fz); cudaFree(m->fail); cudaFree(m->ds);
     if (m->hs) cudaFreeHost(m->hs);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
