@@ -24,7 +24,7 @@
 
 #include <vector>
 
-#include "cweno64.cuh"
+#include "cweno_fix.cuh"
 #include "euler_df64.cuh"
 #include "euler_kernels.cuh"
 #include "mlp_kernels.cuh"
@@ -324,16 +324,18 @@ __global__ void __launch_bounds__(128, 4)
 
 // FP64 reconstruction of the same cells, one thread per variable and cell (blockIdx.y = variable), or,
 // with the positivity fallback (PAD), one per cell with the variables in turn.
-// Bound: FP64 issue (361 operations per variable with CWENO4; DRAM below 4 % of peak).  The cells are
-// indexed flat over the extended box: a warp of 32 x-neighbours per row left 11 % of the lanes idle at
-// nx + 2 = 258 and 44 % at 18, at the full cost of its FP64 instructions.  A variable per thread gives a
-// small grid five times the warps (16^3: 183 warps of one serial 2300-instruction thread each took
-// 87 us) and leaves no loop around the 190-register body.  kThreads is small so that few blocks spread
-// evenly over the SMs.
+// CWENO4 and R4 run on the integer pipe (cweno_fix.cuh); stencils it does not apply to, and WENO3, in FP64.
+// The cells are indexed flat over the extended box: a warp of 32 x-neighbours per row left 11 % of the lanes
+// idle at nx + 2 = 258 and 44 % at 18.  A variable per thread gives a small grid five times the warps (16^3:
+// 183 warps of one serial 2300-instruction thread each took 87 us).  kReconThreads is small so that few blocks
+// spread evenly over the SMs.  Bound: the ALU's half-rate integer issue (2600 instructions per warp, 5100
+// cycles) beside 67 FP64 ones (4300); 16 warps per SM (128 registers, 360 bytes spilled) let one warp's FP64
+// weights overlap another's integer phase: 256^3, four stages 89.7 ms at 240 registers, 85.1 at 168, 80.3 at
+// 128, 85.2 at 96; all in FP64 237.7.
 constexpr int kReconThreads = 64;
 
 template <int RECON, bool PAD>
-__global__ void __launch_bounds__(kReconThreads)
+__global__ void __launch_bounds__(kReconThreads, 8)
     k_recon64(const double* __restrict__ G, double* __restrict__ T, Geo g, double gm1,
               unsigned long long* __restrict__ counters, double* __restrict__ C4) {
     const unsigned e = blockIdx.x * (unsigned)kReconThreads + threadIdx.x;
@@ -355,11 +357,17 @@ __global__ void __launch_bounds__(kReconThreads)
             weno3<double>(s, cf);
             store_traces<double>(T, g, e, c, cf);
         } else {
-            Poly64 poly;
-            if constexpr (RECON == HYPE_RECON_LINEAR4) r4_64(s, poly);
-            else cweno4_64(s, poly);
-            store_traces64(poly, Tc, g.NE);
-            if (RECON == HYPE_RECON_LINEAR4 && C4) store_grad_coeffs(poly, C4 + (long long)c * 20 * g.NE + e, g.NE);
+            constexpr bool linear = RECON == HYPE_RECON_LINEAR4;
+            PolyFix fix;
+            if (recon_fix<linear>(s, c == 0 || c == 4, Tc, g.NE, fix)) {
+                if (linear && C4) store_grad_coeffs(fix, C4 + (long long)c * 20 * g.NE + e, g.NE);
+            } else {
+                Poly64 poly;
+                if constexpr (linear) r4_64(s, poly);
+                else cweno4_64(s, poly);
+                store_traces64(poly, Tc, g.NE);
+                if (linear && C4) store_grad_coeffs(poly, C4 + (long long)c * 20 * g.NE + e, g.NE);
+            }
         }
         if (RECON != HYPE_RECON_LINEAR4 && C4) {  // the viscous fluxes take the gradients of R4
             Poly64 r4;

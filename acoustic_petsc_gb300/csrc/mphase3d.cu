@@ -25,7 +25,7 @@
 #include <algorithm>
 #include <vector>
 
-#include "cweno64.cuh"
+#include "cweno_fix.cuh"
 
 namespace hype {
 namespace mp3d {
@@ -454,8 +454,8 @@ __device__ __forceinline__ void gather33(const double* __restrict__ p, int sy, i
 // pressure are checked at the nodes; with stiffness the pressure check needs phi's polynomial, so that thread
 // does phi first (blockIdx.y = 4: phi and p).  A failing cell is marked and its traces replaced by
 // k_m3_first_order, since its variables are in different threads.
-// Bound: FP64 issue (361 operations per variable, 21 per check).
-__global__ void __launch_bounds__(kReconThreads) k_m3_recon(const double* __restrict__ G, double* __restrict__ T, Geo g, Eos e,
+// Bound: integer issue beside 67 FP64 operations, as the single-gas reconstruction (cweno_fix.cuh).
+__global__ void __launch_bounds__(kReconThreads, 8) k_m3_recon(const double* __restrict__ G, double* __restrict__ T, Geo g, Eos e,
                                                             unsigned char* __restrict__ fail) {
     __shared__ double sphi[20 * kReconThreads];  // phi's coefficients, [q][thread]
     const unsigned e_ = blockIdx.x * (unsigned)kReconThreads + threadIdx.x;
@@ -471,41 +471,49 @@ __global__ void __launch_bounds__(kReconThreads) k_m3_recon(const double* __rest
     bool phi_above = true;
 #pragma unroll 1
     for (int c = (e.stiff && last == 4) ? 5 : last;; c = last) {
+        const bool check = c == 0 || c == 4;
         double s[33];
-        euler::Poly64 poly;
         gather33(G + c * g.GN + ge, sy, sz, s);
-        euler::cweno4_64(s, poly);
-        euler::store_traces64(poly, T + (long long)c * NTR * g.NE + e_, g.NE);
-        if (c != last) {
-            // P_inf >= 0 wherever 0 <= phi <= 1
-            const double sp = spread(poly);
-            phi_above = poly.u0 - sp >= 0.0 && poly.u0 + sp <= 1.0 && e.p1 >= 0.0 && e.p2 >= 0.0;
-            if (!phi_above) {
-                double cf[20];
-                euler::coeffs64(poly, cf);
-#pragma unroll
-                for (int q = 0; q < 20; ++q) ph[q * kReconThreads] = cf[q];
+        double* Tc = T + (long long)c * NTR * g.NE + e_;
+        euler::PolyFix fix;
+        const bool fixed = euler::recon_fix<false>(s, check, Tc, g.NE, fix);
+        bool fp64 = !fixed;  // whether the FP64 polynomial is needed
+        if (fixed) {
+            if (c != last) {  // phi: P_inf >= 0 wherever 0 <= phi <= 1
+                const double u = euler::from_fixed(fix.u0, fix.top), sp = euler::from_fixed((long long)euler::spread_fix(fix), fix.top);
+                fp64 = !(phi_above = u - sp >= 0.0 && u + sp <= 1.0 && e.p1 >= 0.0 && e.p2 >= 0.0);
+            } else if (check) {
+                fp64 = !(phi_above && euler::surely_above(fix, 2.0e-12));
             }
-            continue;
         }
-        if (c == 0 || c == 4) {
-            if (!(surely_above(poly) && phi_above)) {
+        if (fp64) {
+            euler::Poly64 poly;
+            euler::cweno4_64(s, poly);
+            if (!fixed) euler::store_traces64(poly, Tc, g.NE);
+            if (c != last) {
+                const double sp = spread(poly);
+                phi_above = poly.u0 - sp >= 0.0 && poly.u0 + sp <= 1.0 && e.p1 >= 0.0 && e.p2 >= 0.0;
+            }
+            if (c != last || (check && !(phi_above && surely_above(poly)))) {
                 double cf[20];
                 euler::coeffs64(poly, cf);
-                if (phi_above && e.stiff && c == 4) {  // phi's polynomial was not kept: form it again
-                    double sf[33];
-                    euler::Poly64 pf;
-                    gather33(G + 5 * g.GN + ge, sy, sz, sf);
-                    euler::cweno4_64(sf, pf);
-                    double cp[20];
-                    euler::coeffs64(pf, cp);
+                if (c != last) {
 #pragma unroll
-                    for (int q = 0; q < 20; ++q) ph[q * kReconThreads] = cp[q];
+                    for (int q = 0; q < 20; ++q) ph[q * kReconThreads] = cf[q];
+                } else {
+                    if (e.stiff && c == 4 && phi_above) {  // phi's polynomial was not kept: form it again
+                        double sf[33], cp[20];
+                        gather33(G + 5 * g.GN + ge, sy, sz, sf);
+                        euler::cweno4_64(sf, poly);
+                        euler::coeffs64(poly, cp);
+#pragma unroll
+                        for (int q = 0; q < 20; ++q) ph[q * kReconThreads] = cp[q];
+                    }
+                    if (c == 0 ? rho_fails(cf) : prs_fails(cf, ph, kReconThreads, e)) fail[e_] = 1;
                 }
-                if (c == 0 ? rho_fails(cf) : prs_fails(cf, ph, kReconThreads, e)) fail[e_] = 1;
             }
         }
-        break;
+        if (c == last) break;
     }
 }
 

@@ -6,6 +6,7 @@ import os
 import numpy as np
 import pytest
 
+from acoustic_petsc_gb300 import _lib as L
 from conftest import GOLDEN
 
 pytestmark = pytest.mark.gpu
@@ -327,3 +328,40 @@ def test_graph_replayed_steps_equal_launched_steps(hype, precision, flux):
     assert np.array_equal(Ug, Ue) and tg == te and dg == de
     assert np.array_equal(Ug2, Ue2) and tg2 == te2 and dg2 == de2
     assert lg == le > 0
+
+
+@pytest.mark.parametrize("kind", ["exact", "shock", "zeros", "wide", "huge"])
+@pytest.mark.parametrize("recon", ["cweno4", "linear4"])
+def test_fixed_point_reconstruction_edges(hype, oracle, kind, recon):
+    """the integer form of the FP64 reconstruction where its scaling matters: a uniform state (its RHS is zero up to
+    the fluxes' rounding), density jumps beyond the factor 8 that sends a cell to the FP64 form, momenta that are
+    zero, 250 orders of magnitude below the density, and a state scaled by 1e30.  Tolerance: the RHS differs from the
+    checker's by rounding, a few 1e-16 of the fluxes' size times 6 faces / h, below 1e-12 of F / h."""
+    n, h = 9, 0.1
+    rng = np.random.default_rng(11)
+    U = np.zeros((n, n, n, 5))
+    U[..., 0] = 1.0
+    U[..., 4] = 2.5
+    if kind == "shock":
+        U[:, :, 4:, 0] = 9.5
+        U[..., 1:4] = 0.2 * (rng.random((n, n, n, 3)) - 0.5)
+        U[..., 4] += rng.random((n, n, n))
+    elif kind in ("wide", "huge"):
+        U[..., 0] += 0.2 * rng.random((n, n, n))
+        U[..., 4] += 0.3 * rng.random((n, n, n))
+        U[..., 1:4] = (1e-250 if kind == "wide" else 0.1) * (rng.random((n, n, n, 3)) - 0.5)
+        if kind == "huge":
+            U *= 1e30
+    elif kind == "zeros":
+        U[..., 0] += 0.2 * rng.random((n, n, n))
+    code = L.RECON_CWENO4 if recon == "cweno4" else L.RECON_LINEAR4
+    cfg = oracle.euler_cfg(n, h, cfl=0.4, recon=code)
+    R, _, rc = oracle.euler_rhs(cfg, U)[:3]
+    s = hype.EulerSolver(hype.AppCtx(N_x=n, N_y=n, N_z=n, h=h, CFL=0.4, recon=code))
+    if rc != 0:  # R4 overshoots the density jump below zero: refused by both
+        with pytest.raises(hype.HypeError):
+            s.RHSFunction(0.0, U)
+        return
+    R_g = s.RHSFunction(0.0, U)
+    size = np.abs(U).max() * 10.0 / h
+    assert np.abs(R_g - R).max() <= 1e-12 * size
