@@ -23,6 +23,7 @@
 #pragma once
 
 #include "euler_kernels.cuh"
+#include "fixed.cuh"
 
 namespace hype {
 namespace euler {
@@ -358,7 +359,7 @@ __device__ __forceinline__ double visc_side64(const double* __restrict__ T, cons
         const double* Tq = T + (face * 4 + q) * NE + e;
         const double rho = __ldg(Tq), md = __ldg(Tq + (1 + D) * NTR * NE), m1 = __ldg(Tq + (1 + T1) * NTR * NE),
                      m2 = __ldg(Tq + (1 + T2) * NTR * NE), E = __ldg(Tq + 4 * NTR * NE);
-        const double ir = recip3(rho);
+        const double ir = recip_fix(rho);
         const double u = md * ir, v = m1 * ir, w = m2 * ir;
         const double em = fma(-w, m2, fma(-v, m1, fma(-u, md, E)));  // E - |m|^2 / rho
         const double rd = gr[0][q] * ir, r1 = gr[1][q] * ir, r2 = gr[2][q] * ir;

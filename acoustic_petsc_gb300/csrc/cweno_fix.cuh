@@ -1,110 +1,31 @@
-// cweno_fix.cuh -- the CWENO4 / R4 reconstruction of one FP64 variable on the integer pipe.
+// cweno_fix.cuh -- the CWENO4 / R4 reconstruction of one FP64 variable and the Rusanov flux's side states on the
+// integer pipe.
 //
-// The mathematics is cweno64.cuh's.  What bounds that form is FP64 issue: a warp instruction holds the
-// FP64 pipe for 64 cycles of its scheduler, a 64-bit integer addition for 2 and a 64 x 64 bit product's
-// upper half for 17 (measured).  A stencil is therefore taken to 64-bit fixed point, scaled by the largest
-// magnitude in it (units of 2^-58 of its power of two, 64 times finer than that number's last FP64 place):
+// The mathematics is cweno64.cuh's.  What bounds that form is FP64 issue (fixed.cuh).  A stencil is therefore
+// taken to 64-bit fixed point, scaled by the largest magnitude in it (units of 2^-58 of its power of two, 64
+// times finer than that number's last FP64 place):
 //  * the differences are integer subtractions, exact for values within 2^-6 of the largest;
-//  * the smoothness indicators are sums of exact 128-bit products, rounded once.  With dp, dm the
-//    third differences of the one-sided stencils (s2 - D) and c2 = u_ab+ + u_ab-, the indicators of the
-//    one-sided stencils differ from the centred one's by dp (8 dp - 3 A + 13 D) and aab (aab +- 2 c2)
-//    terms: 34 products for all eight, and the cancellation in them is harmless because it is exact;
-//  * the nonlinear weights (two powers, nine reciprocals) stay in FP64: 67 operations;
+//  * the smoothness indicators are sums of exact 128-bit products.  With dp, dm the third differences of the
+//    one-sided stencils (s2 - D) and c2 = u_ab+ + u_ab-, the indicators of the one-sided stencils differ from
+//    the centred one's by dp (8 dp - 3 A + 13 D) and aab (aab +- 2 c2) terms: 37 products for all eight, and
+//    the cancellation in them is harmless because it is exact; eps enters through the one they share;
+//  * the nonlinear weights are significands with an exponent: one reciprocal and two squarings per indicator;
 //  * the weights sum to one, so the combination is R4's centred values plus two corrections per term,
 //    o_+ dp, o_- dm and (o_+ - o_-) aab;
-//  * the traces are sums of integers with products by fixed-point constants, rounded to FP64 once.
+//  * the traces are sums of integers with products by fixed-point constants, rounded to FP64 once by the
+//    conversion instruction (the FP64 pipe's only work here).
+// About 4300 instructions a warp and variable against 361 FP64 ones of 64 cycles.  At 256^3, four stages: all in
+// FP64 237.7 ms; integers with the weights in FP64 (67 operations) 80.3; that with products of 32-bit halves
+// 76.7; integer weights 73; conversions by instruction 66.4; eps added once 63.0.
 // Errors: 2^-57 of the stencil's largest magnitude, where the FP64 form has a few 2^-53.  A cell whose own
 // value is more than 8 times below the largest of its stencil (a strong shock in density, energy or
 // pressure) or whose stencil is not finite keeps the FP64 form, whose error there is relative to the cell.
 #pragma once
 
-#include <string.h>
-
 #include "cweno64.cuh"
 
 namespace hype {
 namespace euler {
-
-typedef unsigned long long u64;
-typedef long long i64;
-typedef unsigned __int128 u128;
-typedef __int128 i128;
-
-__host__ __device__ __forceinline__ u64 umulhi(u64 a, u64 b) {
-#ifdef __CUDA_ARCH__
-    return __umul64hi(a, b);
-#else
-    return (u64)(((u128)a * b) >> 64);
-#endif
-}
-__host__ __device__ __forceinline__ int clz64(u64 x) {  // x != 0
-#ifdef __CUDA_ARCH__
-    return __clzll((i64)x);
-#else
-    return __builtin_clzll(x);
-#endif
-}
-__host__ __device__ __forceinline__ i64 bits_of(double x) {
-#ifdef __CUDA_ARCH__
-    return __double_as_longlong(x);
-#else
-    i64 b;
-    memcpy(&b, &x, 8);
-    return b;
-#endif
-}
-__host__ __device__ __forceinline__ double from_bits(u64 b) {
-#ifdef __CUDA_ARCH__
-    return __longlong_as_double((i64)b);
-#else
-    double x;
-    memcpy(&x, &b, 8);
-    return x;
-#endif
-}
-__host__ __device__ __forceinline__ u128 sqr(i64 a) { return (u128)((i128)a * a); }
-__host__ __device__ __forceinline__ i128 prod(i64 a, i64 b) { return (i128)a * b; }
-
-// x * c / 2^64 for an unsigned multiplier, rounded to the nearest
-__host__ __device__ __forceinline__ i64 scale_u(i64 x, u64 c) {
-    return (i64)(umulhi((u64)x, c) - (x < 0 ? c : 0ull));
-}
-
-// a finite double with biased exponent e <= top as an integer: 2^(52 + SHIFT) stands for 2^(top - 1023)
-template <int SHIFT>
-__host__ __device__ __forceinline__ i64 to_fixed(i64 b, int top) {
-    const int e = (int)(b >> 52) & 0x7FF;
-    const u64 m = ((b & 0xFFFFFFFFFFFFFll) | 0x10000000000000ll) << SHIFT;
-    const int sh = top - e;
-    const i64 v = (i64)(m >> (sh < 63 ? sh : 63));
-    const i64 s = b >> 63;
-    return (v ^ s) - s;
-}
-// v * 2^(top - 1023 - 58) rounded to the nearest double; the result's exponent is in range by the clamp of top
-__host__ __device__ __forceinline__ double from_fixed(i64 v, int top) {
-    const i64 s = v >> 63;
-    const u64 m = (u64)((v ^ s) - s);
-    if (m == 0) return 0.0;
-    const int c = clz64(m);
-    const u64 t = m << c;
-    const u64 r = (t >> 11) + ((t >> 10) & 1);
-    return from_bits(((u64)(s & 1) << 63) | (((u64)(top + 5 - c - 1) << 52) + r));
-}
-// J * 2^e2 rounded to a double (0 for 0)
-__host__ __device__ __forceinline__ double from_u128(u128 J, int e2) {
-    u64 hi = (u64)(J >> 64), lo = (u64)J;
-    int n = 0;
-    if (hi == 0) {
-        hi = lo;
-        lo = 0;
-        n = 64;
-    }
-    if (hi == 0) return 0.0;
-    const int c = clz64(hi);
-    const u64 t = (hi << c) | ((lo >> 1) >> (63 - c));
-    const u64 r = (t >> 11) + ((t >> 10) & 1);
-    return from_bits(((u64)(1023 + 127 - n - c + e2 - 1) << 52) + r);
-}
 
 // The stencil in fixed point and what the traces need of it (units: 2^(top - 1023 - 58)); doubled differences
 // as in Poly64, and cr2 twice its cr
@@ -167,118 +88,114 @@ __host__ __device__ __forceinline__ void poly_fix(const double* __restrict__ s, 
         }
         return;
     }
-    // 24 times cweno64.cuh's indicators, in units of 2^(top - 1023 - 55) squared: three bits fewer keep every
-    // sum below 2^127
-    u128 J1 = 0, m = 0, DD = 0, J[6];
-    i128 sA = 0;
+    // 24 times cweno64.cuh's indicators, in units of 2^(t - 1023 - 55) squared, t = max(top, 1000): three bits
+    // fewer keep every sum below 2^127, and below 2^-23 the differences' 2^-78 is far finer than their
+    // comparison with eps = 1e-12 can tell.  eps enters all of them through J1.
+    const int t = top > 1000 ? top : 1000;
+    const int sh = t - top + 3 < 63 ? t - top + 3 : 63;
+    Sum128 J1, m{0, 0}, DD{0, 0}, sA{0, 0}, J[6];
+    {
+        const int x = -97 - 2 * (t - 1023 - 55);  // 24 * 4e-12 = em 2^x, x <= 59
+        constexpr u64 em = 15211807202738752818ull;
+        J1 = x > 0 ? Sum128{em >> (64 - x), em << x} : Sum128{0, (x > -64 ? em >> -x : 0) | 1};
+    }
+    Split x3[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const i64 a_ = A[a] >> 3, d_ = D[a] >> 3, x = p.cr2[a] >> 3, q = p.ddd[a] >> 3;
-        J1 += 24 * sqr(a_) + 104 * sqr(d_) + 7 * sqr(x);
-        DD += sqr(q);
-        sA += prod(q, a_);
-        const i64 f = dp[a] >> 3, g = dm[a] >> 3;
-        J[2 * a] = (u128)(16 * prod(f, 8 * f - 3 * a_ + 13 * d_));
-        J[2 * a + 1] = (u128)(16 * prod(g, 8 * g + 3 * a_ + 13 * d_));
+        const i64 a_ = A[a] >> sh, d_ = D[a] >> sh, x = p.cr2[a] >> sh, q = p.ddd[a] >> sh;
+        const Split as = split(a_), qs = split(q);
+        x3[a] = split(x);
+        J1 = J1 + times128(split(24 * a_), as) + times128(split(13 * d_), split(8 * d_)) + times128(split(7 * x), x3[a]);
+        DD = DD + square128(qs);
+        sA = sA + times128(split(8 * q), as);
+        const i64 f = dp[a] >> sh, g = dm[a] >> sh, w = 13 * d_, v = 3 * a_;
+        const Sum128 P = times128(split(8 * f), split(8 * f + (w - v))), Q = times128(split(8 * g), split(8 * g + (w + v)));
+        J[2 * a] = P + P;
+        J[2 * a + 1] = Q + Q;
     }
 #pragma unroll
     for (int P = 0; P < 3; ++P) {
         const int a = P == 1 ? 1 : 0, b = P == 0 ? 1 : 2;
-        const i64 x = p.cr2[P] >> 3, f = p.aab[P] >> 3, g = p.abb[P] >> 3;
-        const u128 ff = sqr(f), gg = sqr(g);
-        const i128 fx = 2 * prod(f, x), gx = 2 * prod(g, x);
-        m += ff + gg;
-        J[2 * a] += 7 * (ff + (u128)fx);
-        J[2 * a + 1] += 7 * (ff - (u128)fx);
-        J[2 * b] += 7 * (gg + (u128)gx);
-        J[2 * b + 1] += 7 * (gg - (u128)gx);
+        const i64 x = 2 * (p.cr2[P] >> sh), f = p.aab[P] >> sh, g = p.abb[P] >> sh;
+        const Split f7 = split(7 * f), g7 = split(7 * g);
+        m = m + square128(split(f)) + square128(split(g));
+        J[2 * a] = J[2 * a] + times128(f7, split(f + x));
+        J[2 * a + 1] = J[2 * a + 1] + times128(f7, split(f - x));
+        J[2 * b] = J[2 * b] + times128(g7, split(g + x));
+        J[2 * b + 1] = J[2 * b + 1] + times128(g7, split(g - x));
     }
-    const int e2 = 2 * (top - 1023 - 55);
-    constexpr double eps = 24 * 4.0e-12;
-    double is[8];
-    is[1] = from_u128(J1, e2) + eps;
+    // The nonlinear weights g_k / (IS_k + eps)^4: with IS + eps = m 2^x normalised and y = 2^127 / m, the fourth
+    // power y4 = y^4 2^-192 is in [2^60, 2^64) and what the weights share is taken out by the smallest x.
+    u64 y4[8];
+    int x[8], xm = 1 << 20;
+    auto power = [&](int k, Sum128 v) {
+        const Norm n = norm128(v);
+        u64 y = recip64(n.m);
+        y = umulhi(y, y);
+        y4[k] = umulhi(y, y);
+        x[k] = n.x;
+        xm = n.x < xm ? n.x : xm;
+    };
+    power(1, J1);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) is[2 + k] = from_u128(J1 + J[k], e2) + eps;
+    for (int k = 0; k < 6; ++k) power(2 + k, J1 + J[k]);
     {
         // + 28.2 m + 26.7 DD - 8 sA + 61/32 xyz^2
-        const u128 xx = sqr(p.xyz >> 3);
-        auto part = [](u128 x, u64 c) { return (u128)(u64)(x >> 64) * c + umulhi((u64)x, c); };  // x c / 2^64
-        u128 v4 = J1 + 28 * m + part(m, 3689348814741910323ull) + 27 * DD - part(DD, 5534023222112865485ull) -
-                  (u128)(8 * sA) + 2 * xx - ((3 * xx) >> 5);
-        is[0] = from_u128(v4, e2) + eps;
+        const Sum128 xx = square128(split(p.xyz >> sh)), x3 = scale128(xx, 3);
+        const Sum128 x32{x3.hi >> 5, (x3.lo >> 5) | (x3.hi << 59)};
+        power(0, (J1 + scale128(m, 28) + part128(m, 3689348814741910323ull)) +
+                     (scale128(DD, 27) - part128(DD, 5534023222112865485ull)) + (xx + xx - x32) - sA);
     }
-    // weights, as cweno64.cuh forms them
-    constexpr double g0 = (1.0 - 0.85) * 0.85, gs = (1. / 6.) * (1 - 0.85) * (1 - 0.85);
-    double r[8];
+    u64 low = 0;  // an eighth of the one-sided stencils' sum
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-#ifdef __CUDA_ARCH__
-        r[k] = recip3(is[k]);
-#else
-        r[k] = 1.0 / is[k];
-#endif
-        r[k] *= r[k];
-        r[k] *= r[k];
-    }
-    const double low = ((r[2] + r[3]) + (r[4] + r[5])) + (r[6] + r[7]);
-    const double tot = fma(gs, low, fma(g0, r[1], 0.85 * r[0]));
-#ifdef __CUDA_ARCH__
-    const double rt = recip3(tot);
-#else
-    const double rt = 1.0 / tot;
-#endif
-    const double wr = r[0] * rt, sc = gs * rt, sub = gs * wr;
-    p.wr = (u64)to_fixed<10>(bits_of(wr), 1024);
-    i64 o[6];  // w_k - wr g_k of the one-sided stencils, 2^61 for one
+    for (int k = 2; k < 8; ++k) low += shift_by(y4[k] >> 3, 4 * (x[k] - xm));
+    // gammaHi = gammaLo = 0.85: g = 0.85, 0.1275, and 0.00375 of each one-sided stencil
+    const u64 tot = umulhi(shift_by(y4[0], 4 * (x[0] - xm)), 15679732462653118874ull) + umulhi(shift_by(y4[1], 4 * (x[1] - xm)), 2351959869397967831ull) +
+                    umulhi(low, 553402322211286548ull);
+    const int z = clz64(tot);
+    const u64 rt = recip64(tot << z), rs = umulhi(rt, 17708874310761169551ull);  // 0.00375 2^8 times it
+    p.wr = shift_by(umulhi(y4[0], rt), 4 * (x[0] - xm) + 2 - z);
+    const u64 sub = umulhi(p.wr, 138350580552821637ull);  // 0.0075
+    i64 o[6];  // w_k - wr g_k of the one-sided stencils, 2^62 for one
 #pragma unroll
-    for (int k = 0; k < 6; ++k) o[k] = to_fixed<10>(bits_of(fma(sc, r[2 + k], -sub)), 1024);
-    // x o, o in units of 2^-61
-    auto times = [](i64 x, i64 w) { return (i64)((prod(x, w) + ((i128)1 << 60)) >> 61); };
+    for (int k = 0; k < 6; ++k) o[k] = (i64)(shift_by(umulhi(y4[2 + k], rs), 4 * (x[2 + k] - xm) + 9 - z) - sub);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const i64 f = times(dp[a], o[2 * a]), g = times(dm[a], o[2 * a + 1]);
+        const i64 f = times62(split(dp[a]), split(o[2 * a])), g = times62(split(dm[a]), split(o[2 * a + 1]));
         p.lin[a] = A[a] - f + g;
         p.sq[a] = D[a] + f + g;
     }
 #pragma unroll
     for (int P = 0; P < 3; ++P) {
         const int a = P == 1 ? 1 : 0, b = P == 0 ? 1 : 2;
-        p.cr2[P] += times(p.aab[P], o[2 * a] - o[2 * a + 1]) + times(p.abb[P], o[2 * b] - o[2 * b + 1]);
+        p.cr2[P] += times62(split(p.aab[P]), split(o[2 * a] - o[2 * a + 1])) +
+                    times62(split(p.abb[P]), split(o[2 * b] - o[2 * b + 1]));
     }
-}
-
-// x c, c in units of 2^-(64 + SH), rounded
-template <int SH>
-__host__ __device__ __forceinline__ i64 scaled(i64 x, u64 c) {
-    return (scale_u(x, c) + (1ll << (SH - 1))) >> SH;
 }
 
 // the 24 face traces, numbered as store_traces64 numbers them: put(q, value)
 template <class Put>
 __host__ __device__ __forceinline__ void traces_fix(const PolyFix& p, Put put) {
-    constexpr u64 kG2 = 5325116328314171392ull, kG8 = 5325116328314171392ull;  // GPT/2 2^65, GPT/8 2^67
-    constexpr u64 k12 = 6148914691236517205ull, k48 = 6148914691236517205ull;  // 2^66/12, 2^68/48
-    constexpr u64 k23 = 12297829382473034411ull;                          // 2^64 2/3
-    constexpr u64 kwt = 16567028576977422108ull, kwm = 14200310208837790379ull;  // 2^64 times 2^5 GPT 7/72 and 2^6 GPT/24
-    // w4/gammaHi times 1/24 (2^67 for one), GPT 7/72 (2^67), GPT/24 (2^68) and 1/192 (2^70)
-    const u64 w23 = umulhi(p.wr, k23) << 2;
-    const u64 wn = w23, wo = w23, wt = umulhi(p.wr, kwt) << 1, wm = umulhi(p.wr, kwm) << 1;
+    // 2^64 times GPT/2, GPT/8, 1/12, 1/48; and 8 times 1/24, GPT 7/72, GPT/24, 1/192 for wr's 2^61
+    constexpr i64 kG2 = 2662558164157085696ll, kG8 = 665639541039271424ll, k12 = 1537228672809129301ll, k48 = 384307168202282325ll;
+    const Split wn = split((i64)umulhi(p.wr, 6148914691236517205ull)), wt = split((i64)umulhi(p.wr, 4141757144244355527ull)),
+                wm = split((i64)umulhi(p.wr, 1775038776104723797ull)), wo = split((i64)umulhi(p.wr, 768614336404564651ull));
     i64 tan[3], odd[3], even[3], cg[3], cc[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        tan[a] = scaled<1>(p.lin[a], kG2) - scaled<3>(p.ddd[a], wt);
-        odd[a] = ((p.lin[a] + 2) >> 2) - scaled<3>(p.ddd[a], wn);
-        even[a] = p.u0 + scaled<2>(p.sq[a], k12);
-        cg[a] = scaled<3>(p.cr2[a], kG8);
-        cc[a] = scaled<4>(p.cr2[a], k48);
+        tan[a] = scaled(p.lin[a], split(kG2)) - scaled(p.ddd[a], wt);
+        odd[a] = ((p.lin[a] + 2) >> 2) - scaled(p.ddd[a], wn);
+        even[a] = p.u0 + scaled(p.sq[a], split(k12));
+        cg[a] = scaled(p.cr2[a], split(kG8));
+        cc[a] = scaled(p.cr2[a], split(k48));
     }
-    const i64 o12 = scaled<6>(p.xyz, wo);
+    const i64 o12 = scaled(p.xyz, wo);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const int t1 = d == 0 ? 1 : 0, t2 = d == 2 ? 1 : 2;
         const i64 m1 = d < t1 ? p.aab[pair_of(d, t1)] : p.abb[pair_of(d, t1)];
         const i64 m2 = d < t2 ? p.aab[pair_of(d, t2)] : p.abb[pair_of(d, t2)];
-        const i64 E1 = tan[t1] + scaled<4>(m1, wm), E2 = tan[t2] + scaled<4>(m2, wm);
+        const i64 E1 = tan[t1] + scaled(m1, wm), E2 = tan[t2] + scaled(m2, wm);
         const i64 c1 = cg[pair_of(d, t1)], c2 = cg[pair_of(d, t2)], c12 = cc[pair_of(t1, t2)];
 #pragma unroll
         for (int sn = 0; sn < 2; ++sn) {
@@ -335,6 +252,82 @@ __device__ __forceinline__ bool recon_fix(const double* __restrict__ s, bool str
     poly_fix<LINEAR>(s, top, p);
     traces_fix(p, [&](int q, double v) { T[q * st] = v; });
     return true;
+}
+
+// ---------------------------------------------------------------- Rusanov
+
+// One side of an axis face on the integer pipe: normal velocity, pressure and |u_n| + c from the conserved
+// trace (rho, normal, two tangential momenta, E), each to 2^-59 before its rounding to FP64.  Numbers are
+// 64-bit significands with an exponent; only sums align.  18 FP64 operations (a reciprocal, a root, 9 products
+// and sums) become about 290 integer ones, a third of their issue time.  False (the caller takes the FP64
+// form, which also decides on the floors) for a density below 2^-45, a pressure below 2^-38 or not positive,
+// and anything not finite or beyond 2^200.
+__host__ __device__ __forceinline__ bool side_fix(double rho, double mn, double m1, double m2, double E, double gamma, double gm1,
+                                                  double& un, double& p, double& sp) {
+    constexpr u64 FRAC = 0xFFFFFFFFFFFFFull, ONE = 0x10000000000000ull;
+    const u64 br = (u64)bits_of(rho), be = (u64)bits_of(E), b0 = (u64)bits_of(mn), b1 = (u64)bits_of(m1), b2 = (u64)bits_of(m2);
+    const int xr = (int)(br >> 52), xe = (int)(be >> 52);  // with the sign: a negative one fails the tests
+    const int x0 = (int)(b0 >> 52) & 0x7FF, x1 = (int)(b1 >> 52) & 0x7FF, x2 = (int)(b2 >> 52) & 0x7FF;
+    const int xm = x0 > x1 ? (x0 > x2 ? x0 : x2) : (x1 > x2 ? x1 : x2);
+    if ((unsigned)(xr - (1023 - 45)) > 245u || (unsigned)(xe - (1023 - 100)) > 300u || xm > 1223) return false;
+    const int er = xr - 1023, ee = xe - 1023, em = xm - 1023;
+    const u64 y = recip64(((br & FRAC) | ONE) << 11);  // 1/rho = y 2^(-64 - er)
+    // |m|^2 = s 2^(2 em - 58), |m|^2 / (2 rho) = k 2^(2 em - er - 59)
+    const u64 q0 = shift_by(((b0 & FRAC) | ONE) << 9, xm - x0), q1 = shift_by(((b1 & FRAC) | ONE) << 9, xm - x1),
+              q2 = shift_by(((b2 & FRAC) | ONE) << 9, xm - x2);
+    u64 k = umulhi(umulhi(q0, q0) + umulhi(q1, q1) + umulhi(q2, q2), y);
+    const int d = 2 * em - er - ee + 2;  // to E's unit 2^(ee - 61)
+    if (d > 0 && (d > 30 || (k >> (62 - d)))) return false;
+    k = shift_by(k, -d);
+    const i64 P0 = (i64)((((be & FRAC) | ONE) << 9) - k);
+    if (P0 <= 0) return false;
+    const int c0 = clz64((u64)P0);
+    const u64 bg = (u64)bits_of(gm1), ba = (u64)bits_of(gamma);
+    u64 q = umulhi((u64)P0 << c0, ((bg & FRAC) | ONE) << 11);
+    const int u0 = (int)((q >> 63) ^ 1);
+    q <<= u0;
+    const int xp = ee - 60 - c0 + ((int)(bg >> 52) - 1023) - u0;  // p = q 2^xp
+    if (xp < -38 - 63) return false;
+    p = pack(q, xp);
+    // c^2 = w 2^x
+    u64 w = umulhi(umulhi(q, y), ((ba & FRAC) | ONE) << 11);
+    int x = xp - er + ((int)(ba >> 52) - 1023) + 1;
+    const int c1 = clz64(w);
+    w <<= c1;
+    x -= c1;
+    w >>= x & 1;
+    x += x & 1;
+    const u64 C = sqrt64(w);  // c = C 2^(x/2 - 31)
+    // |u_n| = U 2^(e0 - er - 63)
+    const u64 U = x0 ? umulhi(((b0 & FRAC) | ONE) << 11, y) : 0;
+    const int u1 = (int)((U >> 63) ^ 1), e0 = x0 - 1023;
+    un = from_bits((x0 ? (u64)bits_of(pack(U << u1, e0 - er - 63 - u1)) : 0ull) | (b0 & 0x8000000000000000ull));
+    const int xu = e0 - er - 62, xc = x / 2 - 31, xs = xu > xc ? xu : xc;
+    const u64 S = shift_by(U >> 1, xs - xu) + shift_by(C, xs - xc);
+    const int c2 = clz64(S);
+    sp = pack(S << c2, xs - c2);
+    return true;
+}
+
+// rusanov64 with both sides' velocity, pressure and wave speed from the integer pipe: 22 FP64 operations
+template <int D>
+__device__ __forceinline__ double rusanov_fix(const double* __restrict__ QL, const double* __restrict__ QR, double gamma,
+                                              double gm1, double* __restrict__ F, bool& bad) {
+    constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
+    double un[2], p[2], sp[2];
+    if (!(side_fix(QL[0], QL[1 + D], QL[1 + T1], QL[1 + T2], QL[4], gamma, gm1, un[0], p[0], sp[0]) &&
+          side_fix(QR[0], QR[1 + D], QR[1 + T1], QR[1 + T2], QR[4], gamma, gm1, un[1], p[1], sp[1])))
+        return rusanov64<D>(QL, QR, gamma, gm1, F, bad);
+    const double s = max_pos(sp[0], sp[1]);
+    double f[NV];
+    f[0] = QL[1 + D] + QR[1 + D];
+    const double ps = p[0] + p[1];
+#pragma unroll
+    for (int i = 1; i < 4; ++i) f[i] = i == 1 + D ? fma(QR[i], un[1], fma(QL[i], un[0], ps)) : fma(QR[i], un[1], QL[i] * un[0]);
+    f[4] = fma(QR[4] + p[1], un[1], (QL[4] + p[0]) * un[0]);
+#pragma unroll
+    for (int c = 0; c < NV; ++c) F[c] = fma(-s, QR[c] - QL[c], f[c]);
+    return s;
 }
 
 }  // namespace euler

@@ -328,14 +328,13 @@ __global__ void __launch_bounds__(128, 4)
 // The cells are indexed flat over the extended box: a warp of 32 x-neighbours per row left 11 % of the lanes
 // idle at nx + 2 = 258 and 44 % at 18.  A variable per thread gives a small grid five times the warps (16^3:
 // 183 warps of one serial 2300-instruction thread each took 87 us).  kReconThreads is small so that few blocks
-// spread evenly over the SMs.  Bound: the ALU's half-rate integer issue (2600 instructions per warp, 5100
-// cycles) beside 67 FP64 ones (4300); 16 warps per SM (128 registers, 360 bytes spilled) let one warp's FP64
-// weights overlap another's integer phase: 256^3, four stages 89.7 ms at 240 registers, 85.1 at 168, 80.3 at
-// 128, 85.2 at 96; all in FP64 237.7.
+// spread evenly over the SMs.  Bound: integer issue and its latencies (4300 instructions a warp, half of the
+// issue slots taken).  256^3, four stages: 66.4 ms at 168 registers (10 warps per SM), 67.5 with six blocks, 70.2
+// at 128 registers with 360 bytes spilled; all in FP64 237.7.
 constexpr int kReconThreads = 64;
 
 template <int RECON, bool PAD>
-__global__ void __launch_bounds__(kReconThreads, 8)
+__global__ void __launch_bounds__(kReconThreads, 5)
     k_recon64(const double* __restrict__ G, double* __restrict__ T, Geo g, double gm1,
               unsigned long long* __restrict__ counters, double* __restrict__ C4) {
     const unsigned e = blockIdx.x * (unsigned)kReconThreads + threadIdx.x;
@@ -1077,8 +1076,9 @@ __device__ __forceinline__ void raise_max(unsigned long long* slot, double v) {
 // FP64 face fluxes, all three directions in one launch (blockIdx.y = direction).  A block is 32 faces x
 // the 4 Gauss points of the 2x2 rule, one point per warp: a quarter of the registers of a thread per face,
 // four times the warps on a small grid (16^3: three launches of one 16 us wave each), the traces of a warp
-// contiguous in x and the four fluxes summed through shared memory without FP64 instructions of their own.
-// Bound: FP64 issue (63 operations per Rusanov solve).
+// contiguous in x and the four fluxes summed through shared memory.
+// Bound: FP64 issue still, 30 operations per Rusanov solve with the side states on the integer pipe (about 1000
+// integer instructions beside them): 256^3, four stages 97.1 -> 42.9 ms.
 template <int D, int FLUX>
 __device__ __forceinline__ void faces64(const double* __restrict__ T, double* __restrict__ F, const Geo& g, double gamma,
                                         DevScalars* __restrict__ ds, int slot, double (*sh)[NV][32]) {
@@ -1096,7 +1096,7 @@ __device__ __forceinline__ void faces64(const double* __restrict__ T, double* __
             QR[c] = __ldg(TR + c * NTR * g.NE);
         }
         bool bad = false;
-        if constexpr (FLUX == HYPE_FLUX_RUSANOV) smax = rusanov64<D>(QL, QR, gamma, gamma - 1.0, fl, bad);
+        if constexpr (FLUX == HYPE_FLUX_RUSANOV) smax = rusanov_fix<D>(QL, QR, gamma, gamma - 1.0, fl, bad);
         else smax = face_solver<double, D, FLUX>(QL, QR, gamma, gamma - 1.0, fl, bad);
 #pragma unroll
         for (int c = 0; c < NV; ++c) sh[gp][c][lane] = fl[c];
@@ -1147,7 +1147,7 @@ __device__ __forceinline__ void faces_visc64(const double* __restrict__ T, doubl
                 QL[c] = __ldg(T + ((long long)c * NTR + (2 * D + 1) * 4 + gp) * g.NE + eL);
                 QR[c] = __ldg(T + ((long long)c * NTR + (2 * D) * 4 + gp) * g.NE + eR);
             }
-            if constexpr (FLUX == HYPE_FLUX_RUSANOV) s = rusanov64<D>(QL, QR, gamma, gamma - 1.0, fl, bad);
+            if constexpr (FLUX == HYPE_FLUX_RUSANOV) s = rusanov_fix<D>(QL, QR, gamma, gamma - 1.0, fl, bad);
             else s = face_solver<double, D, FLUX>(QL, QR, gamma, gamma - 1.0, fl, bad);
             smax = max_pos(smax, s);
 #pragma unroll

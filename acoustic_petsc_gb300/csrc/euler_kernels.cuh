@@ -93,22 +93,6 @@ __device__ __forceinline__ double sqrt3(double x) {
     return fma(g, e * fma(0.375, e, 0.5), g);
 }
 
-// 1/sqrt(x) for x > 0: with y and e = 1 - x y^2 as in sqrt3, y (1 + e/2 + 3 e^2/8)
-__device__ __forceinline__ double rsqrt3(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x);
-    const unsigned ex = hi >> 20;
-    if (ex - 2u > 2042u) return rsqrt(x);
-    const unsigned odd = (ex & 1u) ^ 1u;
-    const float mf = __uint_as_float(((127u + odd) << 23) | ((hi & 0xFFFFFu) << 3));
-    float yf;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(mf));
-    const unsigned yb = __float_as_uint(yf);
-    const int q = ((int)ex - 1023 - (int)odd) / 2;
-    const double y = __hiloint2double((int)((yb >> 3) + ((896u << 20) - ((unsigned)q << 20))), (int)(yb << 29));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y, e * fma(0.375, e, 0.5), y);
-}
-
 // x >= lo for a positive lo, as the floating comparison decides it (false for NaN), on the bit pattern
 __device__ __forceinline__ bool at_least(double x, double lo) {
     const long long b = __double_as_longlong(x);

@@ -79,8 +79,8 @@ __device__ __forceinline__ double mix_pinf(const Eos& e, double phi) {
     return e.stiff ? e.k / (mix_d(e, phi) + e.k) * mix_c(e, phi) : 0.0;
 }
 __device__ __forceinline__ void cons2prim(const Eos& e, const double* Q, double* V) {
-    const double gm1 = e.k * euler::recip(mix_d(e, Q[5]));
-    const double ir = euler::recip(Q[0]);
+    const double gm1 = e.k * euler::recip_fix(mix_d(e, Q[5]));
+    const double ir = euler::recip_fix(Q[0]);
     double pe = fma(-0.5 * ir, fma(Q[3], Q[3], fma(Q[2], Q[2], Q[1] * Q[1])), Q[4]);
     if (e.stiff) pe -= mix_c(e, Q[5]);
     V[0] = Q[0];
@@ -101,7 +101,7 @@ __device__ __forceinline__ Side make_side(const Eos& e, const double* V, bool& b
     Side s;
     s.rho = V[0]; s.u = V[1]; s.v = V[2]; s.w = V[3]; s.p = V[4]; s.phi = V[5];
     const double d = mix_d(e, s.phi);
-    const double gm1 = e.k * euler::recip(d);
+    const double gm1 = e.k * euler::recip_fix(d);
     double gp = fma(gm1, s.p, s.p);                  // gamma (p + P_inf)
     double pe = fma(d * e.rk, s.p, s.p);             // p + (p + gamma P_inf) / (gamma - 1)
     if (e.stiff) {
@@ -114,7 +114,7 @@ __device__ __forceinline__ Side make_side(const Eos& e, const double* V, bool& b
     }
     bad |= s.rho < RHO_FLOOR;
     s.H = fma(0.5 * s.rho, fma(s.w, s.w, fma(s.v, s.v, s.u * s.u)), pe);
-    s.a = euler::sqrt3(gp * euler::recip(s.rho));
+    s.a = euler::sqrt_fix(gp * euler::recip_fix(s.rho));
     return s;
 }
 
@@ -168,7 +168,7 @@ __device__ __forceinline__ void hllc_momentum(double nx, double ny, double nz, d
         const double b = nz - nx;
         const double q2 = fma(2.0 * nz, ny - nx, fma(2.0 * nx, ny, 2.0));
         const double dz = nz * d;
-        const double Yr = Y * euler::recip(fma(dz, fma(nx, b, -ny * s), q2));
+        const double Yr = Y * euler::recip_fix(fma(dz, fma(nx, b, -ny * s), q2));
         pn = fma(q2, Yr, p);
         const double g = wt * (dz * Yr);
         h.px = fma(g, b, h.px);
@@ -186,7 +186,7 @@ __device__ __forceinline__ double hllc_general(const Side& L, const Side& R, dou
     const double unL = fma(L.w, nz, fma(L.v, ny, L.u * nx)), unR = fma(R.w, nz, fma(R.v, ny, R.u * nx));
     const double SL = fmin(unR - R.a, unL - L.a), SR = fmax(unL + L.a, unR + R.a);
     const double rL = L.rho * (SL - unL), rR = R.rho * (SR - unR);
-    const double Ss = fma(-rR, unR, fma(rL, unL, R.p - L.p)) * euler::recip(rL - rR);
+    const double Ss = fma(-rR, unR, fma(rL, unL, R.p - L.p)) * euler::recip_fix(rL - rR);
     const int sel = hllc_select(SL, SR, Ss);
     if (sel != 4) {
         const bool left = sel <= 1;
@@ -194,7 +194,7 @@ __device__ __forceinline__ double hllc_general(const Side& L, const Side& R, dou
         double m = un, Y = 0.0;
         if (sel == 1 || sel == 2) {
             const double S = left ? SL : SR, e = Ss - un;
-            const double z = e * euler::recip(S - Ss);
+            const double z = e * euler::recip_fix(S - Ss);
             m = fma(S, z, un);
             Y = (S * e) * fma(left ? L.rho : R.rho, z, left ? L.rho : R.rho);
             h.en = fma(wt * Y, Ss, h.en);
@@ -219,22 +219,22 @@ __device__ __forceinline__ double rot_hllc7(const Side& L, const Side& R, double
     const bool still = dq2 < 1.0E-20;  // |du| < 1e-10 (pde.c:391)
     double nx = D == 0 ? 1.0 : 0.0, ny = D == 1 ? 1.0 : 0.0, nz = D == 2 ? 1.0 : 0.0, a1 = 1.0;
     if (!still) {
-        const double idq = euler::rsqrt3(dq2);
+        const double idq = euler::rsqrt_fix(dq2);
         const bool flip = __double2hiint(D == 0 ? du : D == 1 ? dv : dw) < 0;
         const double sg = neg_if(flip, idq);
         nx = du * sg; ny = dv * sg; nz = dw * sg;
         a1 = D == 0 ? nx : D == 1 ? ny : nz;
     }
     // t1 and t2 = n1 x t1 of pde.c:402-424
-    const double s = ny + nz, d = ny - nz, b = nz - nx;
-    double t1x, t1y, t1z;
-    if (abs_above(s, d)) {
-        const double il = euler::rsqrt3(fma(2.0 * nz, ny - nx, fma(2.0 * nx, ny, 2.0)));
-        t1x = s * il; t1y = b * il; t1z = -(nx + ny) * il;
-    } else {
-        const double il = euler::rsqrt3(fma(-2.0 * nz, nx + ny, fma(-2.0 * nx, ny, 2.0)));
-        t1x = d * il; t1y = b * il; t1z = (nx - ny) * il;
+    double t1x = ny + nz, t1y = nz - nx, t1z = -(nx + ny);
+    if (const double d = ny - nz; !abs_above(t1x, d)) {
+        t1x = d;
+        t1z = nx - ny;
     }
+    const double il = euler::rsqrt_fix(fma(t1z, t1z, fma(t1y, t1y, t1x * t1x)));
+    t1x *= il;
+    t1y *= il;
+    t1z *= il;
     double t2x = fma(ny, t1z, -nz * t1y), t2y = fma(nz, t1x, -nx * t1z), t2z = fma(nx, t1y, -ny * t1x);
     HllcSum h{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     double smax = hllc_general(L, R, nx, ny, nz, a1, h);
@@ -247,8 +247,8 @@ __device__ __forceinline__ double rot_hllc7(const Side& L, const Side& R, double
         }
     } else {
         const double am = euler::max_pos(L.a, R.a);
-        const double e = (L.p - R.p) * euler::recip((L.rho + R.rho) * am);  // S_star - un
-        const double zL = -e * euler::recip(am + e), zR = e * euler::recip(am - e);
+        const double e = (L.p - R.p) * euler::recip_fix((L.rho + R.rho) * am);  // S_star - un
+        const double zL = -e * euler::recip_fix(am + e), zR = e * euler::recip_fix(am - e);
         const double yL = e * fma(L.rho, zL, L.rho), yR = e * fma(R.rho, zR, R.rho);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -454,8 +454,8 @@ __device__ __forceinline__ void gather33(const double* __restrict__ p, int sy, i
 // pressure are checked at the nodes; with stiffness the pressure check needs phi's polynomial, so that thread
 // does phi first (blockIdx.y = 4: phi and p).  A failing cell is marked and its traces replaced by
 // k_m3_first_order, since its variables are in different threads.
-// Bound: integer issue beside 67 FP64 operations, as the single-gas reconstruction (cweno_fix.cuh).
-__global__ void __launch_bounds__(kReconThreads, 8) k_m3_recon(const double* __restrict__ G, double* __restrict__ T, Geo g, Eos e,
+// Bound: integer issue, as the single-gas reconstruction (cweno_fix.cuh).
+__global__ void __launch_bounds__(kReconThreads, 5) k_m3_recon(const double* __restrict__ G, double* __restrict__ T, Geo g, Eos e,
                                                             unsigned char* __restrict__ fail) {
     __shared__ double sphi[20 * kReconThreads];  // phi's coefficients, [q][thread]
     const unsigned e_ = blockIdx.x * (unsigned)kReconThreads + threadIdx.x;
@@ -545,7 +545,8 @@ __device__ __forceinline__ void raise_max(unsigned long long* a, double v) {
 // launch (blockIdx.y); a block is 32 faces, indexed flat, x the 4 Gauss points, one point per warp, summed
 // through shared memory.  Bound: FP64 issue.  With one thread per face, its four points in turn, and three
 // general solves per point the three face launches of a 40 x 40 x 100 RHS took 3.9 ms of 5.6; a whole RHS
-// and stage now takes 1.9 ms (22.5 -> 7.5 ms per step).
+// and stage then took 1.9 ms (22.5 -> 7.5 ms per step); with reciprocals and roots on the integer pipe the
+// faces are 0.83 ms (4.4 ms per step).
 template <int D>
 __device__ __forceinline__ void faces(const double* __restrict__ T, double* __restrict__ F, const Geo& g, const Eos& e,
                                       DevScalars* __restrict__ ds, int slot, double (*sh)[MF][32]) {
