@@ -259,5 +259,51 @@ __host__ __device__ __forceinline__ double rsqrt_fix(double x) {
     return pack(rsqrt64(significand(b) >> odd), -95 - (X + odd) / 2);
 }
 
+
+// a / b and sqrt(x) correctly rounded, as the division and the root of IEEE arithmetic are, for code whose
+// results must not change: the quotient or root to 2^-58, then its last place decided by the exact remainder
+// at the midpoint (of which 64 bits suffice).  About 70 instructions each.
+__host__ __device__ __forceinline__ double div_rn(double a, double b) {
+    const u64 ba = (u64)bits_of(a), bb = (u64)bits_of(b);
+    const int ea = (int)(ba >> 52) & 0x7FF, eb = (int)(bb >> 52) & 0x7FF;
+    const u64 sign = (ba ^ bb) & 0x8000000000000000ull;
+    const bool zero = (ba << 1) == 0;
+    const int e = ea - eb + 1023;
+    // normal operands, a quotient safely normal
+    if ((unsigned)(eb - 1) > 2045u || (!zero && ((unsigned)(ea - 1) > 2045u || (unsigned)(e - 2) > 2042u))) return a / b;
+    const u64 ma = significand(ba) >> 11, mb = significand(bb) >> 11;
+    u64 q = umulhi(ma << 11, recip64(mb << 11));  // 2^63 for one
+    const int up = (int)((q >> 63) ^ 1);          // below one
+    q <<= up;
+    u64 n = q >> 11;
+    if ((i64)((ma << (53 + up)) - (2 * n + 1) * mb) > 0) ++n;
+    return from_bits(sign | (zero ? 0 : ((u64)(e - up - 1) << 52) + n));
+}
+__host__ __device__ __forceinline__ double sqrt_rn(double x) {
+    const u64 b = (u64)bits_of(x);
+    const int ex = (int)(b >> 52);  // with the sign
+    if ((unsigned)(ex - 2) > 2040u) return sqrt(x);
+    const int X = ex - 1023 - 63, odd = X & 1;
+    const u64 m = significand(b) >> odd;  // x = m 2^(X + odd), m in [2^62, 2^64)
+    u64 n = sqrt64(m) >> 10;              // 2^21 sqrt(m), 53 bits
+    // sqrt(m) 2^22 against 2 n + 1: m 2^44 - (2 n + 1)^2
+    if ((i64)((m << 44) - (2 * n + 1) * (2 * n + 1)) > 0) ++n;
+    return from_bits(((u64)((X + odd) / 2 - 21 + 52 + 1023 - 1) << 52) + n);
+}
+
+// the exact conversion float -> double and the rounded one back, which the FP64 pipe would do at its rate
+__device__ __forceinline__ double widen_fix(float x) {
+    const unsigned b = __float_as_uint(x), ex = (b >> 23) & 0xFFu;
+    if (ex - 1u > 253u && (b << 1)) return (double)x;  // subnormal, infinite or NaN
+    return __hiloint2double((int)((b & 0x80000000u) | (ex ? (((b & 0x7FFFFFFFu) >> 3) + (896u << 20)) : 0u)), (int)(b << 29));
+}
+__device__ __forceinline__ float narrow_fix(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), ex = (hi >> 20) & 0x7FFu;
+    if (ex - 897u > 253u) return (float)x;  // the result is not a normal float
+    const unsigned f = (hi & 0x80000000u) | ((((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29));
+    const unsigned r = lo & 0x1FFFFFFFu;
+    return __uint_as_float(f + (r > 0x10000000u || (r == 0x10000000u && (f & 1u)) ? 1u : 0u));
+}
+
 }  // namespace euler
 }  // namespace hype

@@ -16,6 +16,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <type_traits>
 #include <vector>
 
 #include "mphase2d_dev.cuh"
@@ -38,36 +39,132 @@ __global__ void k_mp_prim(const double* __restrict__ U, double* __restrict__ P, 
     for (int c = 0; c < nv; ++c) P[c * N + q] = V[c];
 }
 
+// FP64 reconstruction, one thread per variable (blockIdx.y) and cell, the cells indexed flat over the extended
+// box; k_mp_pad then checks the cells and puts the minmod traces where a node is inadmissible, since a cell's
+// variables are in different threads.  Bound: FP64 issue.  A cell's variables in turn (38 k cells at 301 x 122)
+// left two to three serial warps per scheduler, and a third of the time with one: 301 x 122, one RHS 291 us; with
+// a variable per thread, divisions on the integer pipe and shared trace products 149 + 13.
+constexpr int kCellThreads = 64;
+
+__device__ __forceinline__ bool ext_cell(const Geo& g, unsigned q, int& i, int& j) {  // false: a corner, feeds no face
+    const unsigned row = q / (unsigned)(g.nx + 2);
+    i = (int)(q - row * (unsigned)(g.nx + 2)) - 1;
+    j = (int)row - 1;
+    return !((i < 0 || i >= g.nx) && (j < 0 || j >= g.ny));
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(kCellThreads) k_mp_recon64(const double* __restrict__ P, double* __restrict__ T, Geo g) {
+    const unsigned q = blockIdx.x * (unsigned)kCellThreads + threadIdx.x;
+    int i, j;
+    if (q >= (unsigned)g.NE || !ext_cell(g, q, i, j)) return;
+    CellMap cm;
+    cell_map(g, i, j, cm);
+    const int c = blockIdx.y;
+    double cf[NDOF], v[8];
+    mp_coeffs<double, MODEL>(P, g, cm, c, cf, false);
+    face_values<double>(cf, v);
+    double* Tc = T + (long long)c * 8 * g.NE + cm.e;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) Tc[(long long)k * g.NE] = v[k];
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(kCellThreads) k_mp_pad(const double* __restrict__ P, double* __restrict__ T, Geo g, Eos e,
+                                                         DevScalars* __restrict__ ds) {
+    constexpr int NV = MODEL == HYPE_MP_DI4 ? 5 : 6;
+    const unsigned q = blockIdx.x * (unsigned)kCellThreads + threadIdx.x;
+    int i, j;
+    if (q >= (unsigned)g.NE || !ext_cell(g, q, i, j)) return;
+    bool ok = true;
+#pragma unroll 1
+    for (int k = 0; k < 8; ++k) {
+        double V[NV];
+#pragma unroll
+        for (int c = 0; c < NV; ++c) V[c] = T[((long long)c * 8 + k) * g.NE + q];
+        ok = ok && pad_ok<double>(e, V);
+    }
+    if (ok) return;
+    if (i >= 0 && i < g.nx && j >= 0 && j < g.ny) atomicAdd(&ds->fallback, 1ull);
+    CellMap cm;
+    cell_map(g, i, j, cm);
+    mp_cell_fallback<double, MODEL, double>(P, T, g, cm);
+}
+
+// FP64 face fluxes, both directions in one launch (blockIdx.y): a block is 32 faces, indexed flat, x the two
+// Gauss points, one per warp, summed through shared memory in the reference's order.  Bound: FP64 issue; 301 x 122:
+// 241 us as a thread per face and a launch per direction with FP64 divisions, here 122.
+template <int MODEL, int D>
+__device__ __forceinline__ void faces64(const double* __restrict__ T, double* __restrict__ F, const Geo& g, const Eos& e,
+                                        DevScalars* __restrict__ ds, int slot, double (*sh)[32]) {
+    constexpr int NV = MODEL == HYPE_MP_DI4 ? 5 : 6;
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+    const unsigned f = blockIdx.x * 32u + lane, fx = g.nx + (D == 0), nf = fx * (g.ny + (D == 1));
+    if (blockIdx.x * 32u >= nf) return;  // the grid is as wide as the direction with more faces
+    double smax = 0.0, fl[MAXV + 1];
+    if (f < nf) {
+        const int j = (int)(f / fx), i = (int)(f - (unsigned)j * fx);
+        const long long eR = (long long)(j + 1) * (g.nx + 2) + (i + 1);
+        const long long eL = eR - (D == 0 ? 1 : (g.nx + 2));
+        double VL[NV], VR[NV];
+#pragma unroll
+        for (int c = 0; c < NV; ++c) {
+            VL[c] = __ldg(T + ((long long)c * 8 + (2 * D + 1) * 2 + q) * g.NE + eL);
+            VR[c] = __ldg(T + ((long long)c * 8 + (2 * D) * 2 + q) * g.NE + eR);
+        }
+        bool bad = false;
+        smax = fmax(0.0, rot_hllc2<double, MODEL>(e, VL, VR, D == 0, D == 1, fl, bad));
+        if (bad) atomicMin(&ds->bad, (unsigned long long)((long long)(j < g.ny ? j : g.ny - 1) * g.nx + (i < g.nx ? i : g.nx - 1)));
+        if (q == 1) {
+#pragma unroll
+            for (int c = 0; c <= NV; ++c) sh[c][lane] = fl[c];
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) smax = fmax(smax, __shfl_xor_sync(0xffffffffu, smax, o));
+    if (lane == 0 && smax > 0.0) atomicMax(&ds->smax_bits[slot], (unsigned long long)__double_as_longlong(smax));
+    __syncthreads();
+    if (q == 0 && f < nf) {
+#pragma unroll
+        for (int c = 0; c <= NV; ++c) F[(long long)c * nf + f] = 0.5 * fl[c] + 0.5 * sh[c][lane];
+    }
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(64) k_mp_faces64(const double* __restrict__ T, double* __restrict__ Fx, double* __restrict__ Fy,
+                                                   Geo g, Eos e, DevScalars* __restrict__ ds, int slot) {
+    __shared__ double sh[MAXV + 1][32];
+    if (blockIdx.y == 0) faces64<MODEL, 0>(T, Fx, g, e, ds, slot, sh);
+    else faces64<MODEL, 1>(T, Fy, g, e, ds, slot, sh);
+}
+
 // Win, X, Y and out may be one array (in-place stages), so they carry no __restrict__
-__global__ void __launch_bounds__(256) k_mp_update(const double* __restrict__ F, const double* __restrict__ G,
+// one thread per variable (blockIdx.y) and cell, indexed flat; the last variable also reads a of Win in the cell
+// it alone writes
+__global__ void __launch_bounds__(128) k_mp_update(const double* __restrict__ F, const double* __restrict__ G,
                                                    const double* Win, const double* X,
                                                    const double* Y, double* out, Geo g,
                                                    double r1_h, Stage st, const DevScalars* __restrict__ ds) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.nx || j >= g.ny) return;
-    const int nv = g.nv, ia = nv - 1;
+    const unsigned cell = blockIdx.x * 128u + threadIdx.x;
+    if (cell >= (unsigned)g.N) return;
+    const int c = blockIdx.y;
     const long long nfx = (long long)(g.nx + 1) * g.ny, nfy = (long long)g.nx * (g.ny + 1);
-    const long long fxl = (long long)j * (g.nx + 1) + i, fyl = (long long)j * g.nx + i;
-    const long long cell = (long long)j * g.nx + i;
-    const double a = Win[ia * g.N + cell];
-    const double cdt = st.rhs_only ? 0.0 : st.c * ds->dt / st.d;
-    for (int c = 0; c < nv; ++c) {
-        double L;
-        if (c == ia)
-            L = -r1_h * ((F[c * nfx + fxl + 1] - a * F[(c + 1) * nfx + fxl + 1]) - (F[c * nfx + fxl] - a * F[(c + 1) * nfx + fxl])) -
-                r1_h * ((G[c * nfy + fyl + g.nx] - a * G[(c + 1) * nfy + fyl + g.nx]) - (G[c * nfy + fyl] - a * G[(c + 1) * nfy + fyl]));
-        else
-            L = -r1_h * (F[c * nfx + fxl + 1] - F[c * nfx + fxl]) - r1_h * (G[c * nfy + fyl + g.nx] - G[c * nfy + fyl]);
-        double v;
-        if (st.rhs_only) {
-            v = L;
-        } else {
-            v = st.a * X[c * g.N + cell] + cdt * L;
-            if (st.b != 0.0) v += st.b * Y[c * g.N + cell];
-        }
-        out[c * g.N + cell] = v;
+    F += c * nfx + cell + cell / (unsigned)g.nx;  // j (nx + 1) + i
+    G += c * nfy + cell;
+    const double cdt = st.rhs_only ? 0.0 : quot(st.c * ds->dt, st.d);
+    double L;
+    if (c == g.nv - 1) {
+        const double a = Win[c * g.N + cell];
+        L = -r1_h * ((F[1] - a * F[nfx + 1]) - (F[0] - a * F[nfx])) - r1_h * ((G[g.nx] - a * G[nfy + g.nx]) - (G[0] - a * G[nfy]));
+    } else {
+        L = -r1_h * (F[1] - F[0]) - r1_h * (G[g.nx] - G[0]);
     }
+    double v = L;
+    if (!st.rhs_only) {
+        v = st.a * X[c * g.N + cell] + cdt * L;
+        if (st.b != 0.0) v += st.b * Y[c * g.N + cell];
+    }
+    out[c * g.N + cell] = v;
 }
 
 __global__ void k_mp_axpby(const double* __restrict__ X, const double* __restrict__ Y, double* __restrict__ out, double a,
@@ -139,8 +236,6 @@ struct hype_mp2d {
 
 static int mp_rhs(hype_mp2d* m, const double* Win, int slot) {
     const Geo& g = m->g;
-    const dim3 br(32, 4), gr(cdiv(g.nx + 2, 32), cdiv(g.ny + 2, 4));
-    const dim3 gx(cdiv(g.nx + 1, 32), cdiv(g.ny, 4)), gy(cdiv(g.nx, 32), cdiv(g.ny + 1, 4));
     const bool f32 = m->p.precision == HYPE_PREC_FP32;
     const bool learned = m->p.recon == HYPE_RECON_LEARNED;
     if (learned && !m->mlp) return HYPE_ERR_ARG;  // hype_mp2d_set_mlp first
@@ -148,39 +243,42 @@ static int mp_rhs(hype_mp2d* m, const double* Win, int slot) {
     // gate scored once per step: on the step's first stage (slot 0) and on RHS-only calls (slot 11)
     const bool per_step = learned && m->gate_per_step != 0;
     const GateStep gs{per_step, per_step && (slot == 0 || slot == 11), m->gate, m->gate_wide};
-#define MP_LAUNCH(R, M)                                                                                        \
-    do {                                                                                                       \
-        if (gs.on)                                                                                             \
-            launch_gated_recon<R, M, double>(m->P, (R*)m->T, g, m->e, m->ds, m->mlp, m->logit_thr, m->flagged, \
-                                             gs, m->stream);                                                   \
-        else if (learned)                                                                                      \
-            k_mp_recon_learned<R, M><<<gr, br, 0, m->stream>>>(m->P, (R*)m->T, g, m->e, m->ds, m->mlp,         \
-                                                               m->logit_thr, m->flagged);                      \
-        else                                                                                                   \
-            k_mp_recon<R, M><<<gr, br, 0, m->stream>>>(m->P, (R*)m->T, g, m->e, m->ds);                        \
-        k_mp_faces<R, M, 0><<<gx, br, 0, m->stream>>>((const R*)m->T, m->F, g, m->e, m->ds, slot);             \
-        k_mp_faces<R, M, 1><<<gy, br, 0, m->stream>>>((const R*)m->T, Gf, g, m->e, m->ds, slot);               \
-    } while (0)
+    int nk = 4;
     if (f32) {  // the FP32 form lives in mphase2d_f32.cu (compiled with FMA contraction)
         launch_rhs_f32(m->e.model, learned, Win, m->Pf, m->T, (float*)m->F, (float*)Gf, g, m->e, m->ds, slot, m->mlp,
                        m->logit_thr, m->flagged, gs, m->stream);
     } else {
-        k_mp_prim<<<cdiv(g.N, 256), 256, 0, m->stream>>>(Win, m->P, m->e, g.N, g.nv);
-        if (m->e.model == HYPE_MP_DI4) MP_LAUNCH(double, HYPE_MP_DI4);
-        else MP_LAUNCH(double, HYPE_MP_KAPILA5);
+        k_mp_prim<<<cdiv(g.N, kCellThreads), kCellThreads, 0, m->stream>>>(Win, m->P, m->e, g.N, g.nv);
+        auto go = [&](auto model) {
+            constexpr int M = decltype(model)::value;
+            double* T = (double*)m->T;
+            const unsigned cells = cdiv(g.NE, kCellThreads);
+            if (gs.on) {
+                launch_gated_recon<double, M, double>(m->P, T, g, m->e, m->ds, m->mlp, m->logit_thr, m->flagged, gs, m->stream);
+            } else if (learned) {
+                k_mp_recon_learned<double, M><<<dim3(cdiv(g.nx + 2, 32), cdiv(g.ny + 2, 4)), dim3(32, 4), 0, m->stream>>>(
+                    m->P, T, g, m->e, m->ds, m->mlp, m->logit_thr, m->flagged);
+            } else {
+                k_mp_recon64<M><<<dim3(cells, g.nv), kCellThreads, 0, m->stream>>>(m->P, T, g);
+                k_mp_pad<M><<<cells, kCellThreads, 0, m->stream>>>(m->P, T, g, m->e, m->ds);
+            }
+            const long long nfx = (long long)(g.nx + 1) * g.ny, nfy = (long long)g.nx * (g.ny + 1);
+            k_mp_faces64<M><<<dim3(cdiv(nfx > nfy ? nfx : nfy, 32), 2), 64, 0, m->stream>>>(T, m->F, Gf, g, m->e, m->ds, slot);
+        };
+        if (m->e.model == HYPE_MP_DI4) go(std::integral_constant<int, HYPE_MP_DI4>{});
+        else go(std::integral_constant<int, HYPE_MP_KAPILA5>{});
+        nk = learned ? 3 : 4;
     }
-#undef MP_LAUNCH
-    HYPE_LAUNCHED(4 + (gs.score ? 2 : 0));
+    HYPE_LAUNCHED(nk + (gs.score ? 2 : 0));
     return HYPE_OK;
 }
 
 static int mp_update(hype_mp2d* m, const double* Win, const double* X, const double* Y, double* out, Stage st) {
     const Geo& g = m->g;
-    const dim3 b(32, 8), gr(cdiv(g.nx, 32), cdiv(g.ny, 8));
     if (m->p.precision == HYPE_PREC_FP32)  // FP32 face fluxes (mphase2d_f32.cu)
         launch_update_f32((const float*)m->F, (const float*)m->G, Win, X, Y, out, g, 1.0 / m->p.h, st, m->ds, m->stream);
     else
-        k_mp_update<<<gr, b, 0, m->stream>>>(m->F, m->G, Win, X, Y, out, g, 1.0 / m->p.h, st, m->ds);
+        k_mp_update<<<dim3(cdiv(g.N, 128), g.nv), 128, 0, m->stream>>>(m->F, m->G, Win, X, Y, out, g, 1.0 / m->p.h, st, m->ds);
     HYPE_LAUNCHED(1);
     return HYPE_OK;
 }

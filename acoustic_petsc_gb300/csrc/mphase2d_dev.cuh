@@ -32,12 +32,6 @@ struct DevScalars {
     unsigned long long fallback;  // owned cells reconstructed with the minmod fallback
 };
 
-__device__ __forceinline__ double node_x(int q) {
-    return q < 2 ? 0.5 : q < 4 ? -0.5 : (q == 4 || q == 6) ? -0.28867513459481287 : 0.28867513459481287;
-}
-__device__ __forceinline__ double node_y(int q) {
-    return q < 4 ? ((q & 1) ? 0.28867513459481287 : -0.28867513459481287) : (q < 6 ? -0.5 : 0.5);
-}
 // face f (0 -x, 1 +x, 2 -y, 3 +y), Gauss point q (0: -g, 1: +g)
 __device__ __forceinline__ double face_x(int f, int q) {
     const double g = q ? 0.28867513459481287 : -0.28867513459481287;
@@ -81,31 +75,37 @@ __device__ __forceinline__ PT ldp(const PT* __restrict__ P, const Geo& g, const 
     return v;
 }
 
-// one cell: 2D CWENO4 (or its optimal-weight R4 limit) of every primitive variable,
-// its 8 face traces; returns whether the 8 admissibility nodes pass (rhs_function.c:173-250)
-template <typename R, int MODEL, typename PT>
-__device__ __forceinline__ bool mp_cell_recon(const PT* __restrict__ P, R* __restrict__ T, const Geo& g, const Eos& e,
-                                              const CellMap& cm, bool linear) {
-    constexpr int NV = MODEL == HYPE_MP_DI4 ? 5 : 6;
-    R VN[8][NV];
-#pragma unroll 1
-    for (int c = 0; c < NV; ++c) {
-        auto ld = [&](int oi, int oj) -> R { return (R)ldp<MODEL>(P, g, cm, c, oi, oj); };
-        R ux[5], uy[5], cf[NDOF];
+// The polynomial at the 8 face points (trace 2 f + q), each value summed in basis order as the reference's loop
+// sums it.  FP64: a product is formed once for the points that differ in its sign, partial sums are shared, and
+// the two basis functions that are exactly zero at the points of a face (+-GP^2 = 1/12) are left out: 82
+// operations for the 144 of eight separate sums, the same values.  FP32 (compiled with contraction): FMAs.
+template <typename R>
+__device__ __forceinline__ void face_values(const R* cf, R* out) {
+    if constexpr (sizeof(R) == sizeof(double)) {
+        constexpr double g = 0.28867513459481287;
+        static_assert(g * g - 1. / 12. == 0.0, "the square basis functions vanish at the Gauss points");
 #pragma unroll
-        for (int o = 0; o < 5; ++o) {
-            ux[o] = ld(o - 2, 0);
-            uy[o] = ld(0, o - 2);
+        for (int d = 0; d < 2; ++d) {  // faces along x, then along y
+            const double hx = d == 0 ? 0.5 : g, hy = d == 0 ? g : 0.5;
+            const double p1 = cf[1] * hx, p2 = cf[2] * hy, ps = cf[3 + d] * (0.5 * 0.5 - 1. / 12.), p5 = cf[5] * (hx * hy),
+                         p6 = cf[6] * (hx * (hx * hx - 3. / 20.)), p7 = cf[7] * (hy * (hy * hy - 3. / 20.)),
+                         pm = cf[8 + d] * (g * (0.5 * 0.5 - 1. / 12.));
+#pragma unroll
+            for (int sx = 0; sx < 2; ++sx) {
+                const double a = sx ? cf[0] + p1 : cf[0] - p1;
+#pragma unroll
+                for (int sy = 0; sy < 2; ++sy) {
+                    double v = sy ? a + p2 : a - p2;
+                    v += ps;
+                    v = sx == sy ? v + p5 : v - p5;
+                    v = sx ? v + p6 : v - p6;
+                    v = sy ? v + p7 : v - p7;
+                    v = (d == 0 ? sy : sx) ? v + pm : v - pm;
+                    out[d == 0 ? 2 * sx + sy : 4 + 2 * sy + sx] = v;
+                }
+            }
         }
-        cweno2d<R>(ux[2], ux, uy, ld(1, 1), ld(1, -1), ld(-1, 1), ld(-1, -1), cf, linear);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            R v = R(0);
-#pragma unroll
-            for (int k = 0; k < NDOF; ++k) v += cf[k] * R(basis2(node_x(q), node_y(q), k));
-            VN[q][c] = v;
-        }
-        R* Tc = T + (long long)c * 8 * g.NE + cm.e;
+    } else {
 #pragma unroll
         for (int f = 0; f < 4; ++f)
 #pragma unroll
@@ -113,8 +113,42 @@ __device__ __forceinline__ bool mp_cell_recon(const PT* __restrict__ P, R* __res
                 R v = R(0);
 #pragma unroll
                 for (int k = 0; k < NDOF; ++k) v += cf[k] * R(basis2(face_x(f, q), face_y(f, q), k));
-                Tc[(long long)(f * 2 + q) * g.NE] = v;
+                out[2 * f + q] = v;
             }
+    }
+}
+
+// the polynomial of primitive variable c in one cell
+template <typename R, int MODEL, typename PT>
+__device__ __forceinline__ void mp_coeffs(const PT* __restrict__ P, const Geo& g, const CellMap& cm, int c, R* cf, bool linear) {
+    auto ld = [&](int oi, int oj) -> R { return (R)ldp<MODEL>(P, g, cm, c, oi, oj); };
+    R ux[5], uy[5];
+#pragma unroll
+    for (int o = 0; o < 5; ++o) {
+        ux[o] = ld(o - 2, 0);
+        uy[o] = ld(0, o - 2);
+    }
+    cweno2d<R>(ux[2], ux, uy, ld(1, 1), ld(1, -1), ld(-1, 1), ld(-1, -1), cf, linear);
+}
+
+// one cell: 2D CWENO4 (or its optimal-weight R4 limit) of every primitive variable,
+// its 8 face traces; returns whether the 8 admissibility nodes pass (rhs_function.c:173-250)
+template <typename R, int MODEL, typename PT>
+__device__ __forceinline__ bool mp_cell_recon(const PT* __restrict__ P, R* __restrict__ T, const Geo& g, const Eos& e,
+                                              const CellMap& cm, bool linear) {
+    constexpr int NV = MODEL == HYPE_MP_DI4 ? 5 : 6;
+    R VN[8][NV];  // the admissibility nodes are the face points
+#pragma unroll 1
+    for (int c = 0; c < NV; ++c) {
+        R cf[NDOF], v[8];
+        mp_coeffs<R, MODEL>(P, g, cm, c, cf, linear);
+        face_values<R>(cf, v);
+        R* Tc = T + (long long)c * 8 * g.NE + cm.e;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            VN[q][c] = v[q];
+            Tc[(long long)q * g.NE] = v[q];
+        }
     }
     bool ok = true;
 #pragma unroll

@@ -12,6 +12,7 @@
 // p_inf = 6e8 Pa cancels catastrophically in FP32).
 #pragma once
 
+#include "fixed.cuh"
 #include "hype_common.cuh"
 
 namespace hype {
@@ -55,6 +56,20 @@ __host__ __device__ inline double basis2(double x, double y, int n) {
         case 9: return x * (y * y - 1. / 12.);
         default: return 0.0;
     }
+}
+
+// a / b and sqrt(a) as the reference rounds them.  FP64: the same correctly rounded values from the integer pipe
+// (fixed.cuh); FP64 issue bounds these kernels, and the compiler's FP64 division and root are sequences of about
+// ten FP64 instructions each, in a face solve more than everything else together.
+template <typename R>
+__device__ __forceinline__ R quot(R a, R b) {
+    if constexpr (sizeof(R) == sizeof(double)) return euler::div_rn(a, b);
+    else return a / b;
+}
+template <typename R>
+__device__ __forceinline__ R root(R a) {
+    if constexpr (sizeof(R) == sizeof(double)) return euler::sqrt_rn(a);
+    else return sqrt(a);
 }
 
 template <typename R>
@@ -139,7 +154,7 @@ __device__ __forceinline__ void cweno2d(R u0, const R* ux, const R* uy, R upp, R
         IS3[i] = X[i] * X[i] + Y[i] * Y[i] + r13_3 * (XX[i] * XX[i] + YY[i] * YY[i]) + r7_6 * XY[i] * XY[i];
     R w4, w3[5];
     Cw2Weights<R>::compute(IS4, IS3, gH, g3, w4, w3);
-    const R wr = w4 / gH;
+    const R wr = quot(w4, gH);
     const R* Q[5] = {X, Y, XX, YY, XY};
     const R R4[5] = {xR4, yR4, xxR4, yyR4, xyR4};
     cf[0] = u0;
@@ -160,16 +175,16 @@ template <>
 struct Cw2Weights<double> {
     __device__ __forceinline__ static void compute(double IS4, const double* IS3, double gH, const double* g3, double& w4,
                                                    double* w3) {
-        w4 = gH / (pow4(IS4 + 1.0e-12));
+        w4 = quot(gH, pow4(IS4 + 1.0e-12));
         double sum = w4;
 #pragma unroll
         for (int i = 0; i < 5; ++i) {
-            w3[i] = g3[i] / (pow4(IS3[i] + 1.0e-12));
+            w3[i] = quot(g3[i], pow4(IS3[i] + 1.0e-12));
             sum += w3[i];
         }
-        w4 = w4 / sum;
+        w4 = quot(w4, sum);
 #pragma unroll
-        for (int i = 0; i < 5; ++i) w3[i] = w3[i] / sum;
+        for (int i = 0; i < 5; ++i) w3[i] = quot(w3[i], sum);
     }
 };
 
@@ -201,12 +216,12 @@ struct Cw2Weights<float> {
 // mixture ratio of specific heats and stiffness (FP64)
 __device__ __forceinline__ void mix(const Eos& e, double a, double& g, double& pi) {
     if (e.model == HYPE_MP_DI4) {  // pde.c:11-12, a = phi
-        g = 1.0 + (e.g1 - 1.0) * (e.g2 - 1.0) / ((1.0 - a) * (e.g1 - 1.0) + a * (e.g2 - 1.0));
-        pi = ((g - 1.0) / g) * (e.g1 * e.p1 * a / (e.g1 - 1.0) + e.g2 * e.p2 * (1.0 - a) / (e.g2 - 1.0));
+        g = 1.0 + quot((e.g1 - 1.0) * (e.g2 - 1.0), (1.0 - a) * (e.g1 - 1.0) + a * (e.g2 - 1.0));
+        pi = quot(g - 1.0, g) * (quot(e.g1 * e.p1 * a, e.g1 - 1.0) + quot(e.g2 * e.p2 * (1.0 - a), e.g2 - 1.0));
     } else {  // kapila_5eqn.c:18-19, a = alpha_1
         const double a2 = 1.0 - a;
-        g = 1.0 + ((e.g1 - 1.0) * (e.g2 - 1.0)) / ((e.g2 - 1.0) * a + (e.g1 - 1.0) * a2);
-        pi = ((g - 1.0) / g) * (e.g1 * e.p1 * a / (e.g1 - 1.0) + e.g2 * e.p2 * a2 / (e.g2 - 1.0));
+        g = 1.0 + quot((e.g1 - 1.0) * (e.g2 - 1.0), (e.g2 - 1.0) * a + (e.g1 - 1.0) * a2);
+        pi = quot(g - 1.0, g) * (quot(e.g1 * e.p1 * a, e.g1 - 1.0) + quot(e.g2 * e.p2 * a2, e.g2 - 1.0));
     }
 }
 
@@ -236,7 +251,7 @@ __device__ __forceinline__ void cons2prim(const Eos& e, const double* Q, double*
     if (e.model == HYPE_MP_DI4) {
         const double phi = Q[4];
         mix(e, phi, g, pi);
-        const double irho = 1.0 / Q[0];
+        const double irho = quot(1.0, Q[0]);
         V[0] = Q[0];
         V[1] = irho * Q[1];
         V[2] = irho * Q[2];
@@ -246,9 +261,9 @@ __device__ __forceinline__ void cons2prim(const Eos& e, const double* Q, double*
         const double a1 = Q[5];
         mix(e, a1, g, pi);
         const double rho = Q[0] + Q[1];
-        const double u = Q[2] / rho, v = Q[3] / rho;
-        V[0] = Q[0] / a1;
-        V[1] = Q[1] / (1.0 - a1);
+        const double u = quot(Q[2], rho), v = quot(Q[3], rho);
+        V[0] = quot(Q[0], a1);
+        V[1] = quot(Q[1], 1.0 - a1);
         V[2] = u;
         V[3] = v;
         V[4] = (g - 1.0) * (Q[4] - 0.5 * rho * (u * u + v * v)) - g * pi;
@@ -295,14 +310,14 @@ __device__ __forceinline__ bool pad_ok(const Eos& e, const R* V) {
 template <typename R, int MODEL>
 __device__ __forceinline__ void prim2cons(const R* V, R g, R pi, R* Q) {
     if (MODEL == HYPE_MP_DI4) {
-        const R en = (V[3] + g * pi) / (g - R(1.0));
+        const R en = quot(V[3] + g * pi, g - R(1.0));
         const R k = R(0.5) * V[0] * (V[1] * V[1] + V[2] * V[2]);
         Q[0] = V[0]; Q[1] = V[0] * V[1]; Q[2] = V[0] * V[2]; Q[3] = k + en; Q[4] = V[4];
     } else {
         const R a1 = V[5], a2 = R(1.0) - a1;
         const R rho = a1 * V[0] + a2 * V[1];
         Q[0] = a1 * V[0]; Q[1] = a2 * V[1]; Q[2] = rho * V[2]; Q[3] = rho * V[3];
-        Q[4] = (V[4] + g * pi) / (g - R(1.0)) + R(0.5) * rho * (V[2] * V[2] + V[3] * V[3]);
+        Q[4] = quot(V[4] + g * pi, g - R(1.0)) + R(0.5) * rho * (V[2] * V[2] + V[3] * V[3]);
         Q[5] = a1;
     }
 }
@@ -329,8 +344,8 @@ __device__ __forceinline__ void make_side2(const R* V, R g, R pi, Side2<R>& s, b
         u = V[2]; v = V[3]; p = V[4];
     }
     bad |= (s.rho < R(1.0e-14)) || ((p + pi) < R(1.0e-12)) || !(s.rho == s.rho);
-    s.c = sqrt(g * (p + pi) / s.rho);
-    s.Eh = (p + g * pi) / (g - R(1.0)) + R(0.5) * s.rho * u * u + R(0.5) * s.rho * v * v;
+    s.c = root(quot(g * (p + pi), s.rho));
+    s.Eh = quot(p + g * pi, g - R(1.0)) + R(0.5) * s.rho * u * u + R(0.5) * s.rho * v * v;
 }
 
 // physical flux of a primitive state along (nx, ny) and its wave speed (PDEFluxPrim, pde.c:62-97);
@@ -387,7 +402,7 @@ __device__ __forceinline__ R hllc2(const R* VL, const R* VR, const Side2<R>& sL,
     const R SL = (a1 < b1) ? a1 : b1;
     const R a2 = unL + cL, b2 = unR + cR;
     const R SR = (a2 < b2) ? b2 : a2;
-    const R Ss = (PR - PL + rL * unL * (SL - unL) - rR * unR * (SR - unR)) / (rL * (SL - unL) - rR * (SR - unR));
+    const R Ss = quot(PR - PL + rL * unL * (SL - unL) - rR * unR * (SR - unR), rL * (SL - unL) - rR * (SR - unR));
     FL[NV] = unL;
     FR[NV] = unR;
     // only the star state of the selected side is needed
@@ -405,24 +420,24 @@ __device__ __forceinline__ R hllc2(const R* VL, const R* VR, const Side2<R>& sL,
         const R* Fk = left ? FL : FR;
         R Us[MAXV];
         if (MODEL == HYPE_MP_DI4) {
-            Us[0] = rk * (Sk - unk) / (Sk - Ss);
+            Us[0] = quot(rk * (Sk - unk), Sk - Ss);
             Us[1] = Us[0] * (Ss * nx - utk * ny);
             Us[2] = Us[0] * (Ss * ny + utk * nx);
-            Us[3] = Us[0] * ((Ek / rk) + (Ss - unk) * (Ss + Pk / (rk * (Sk - unk))));
-            Us[4] = Vk[4] * (Sk - unk) / (Sk - Ss);
+            Us[3] = Us[0] * (quot(Ek, rk) + (Ss - unk) * (Ss + quot(Pk, rk * (Sk - unk))));
+            Us[4] = quot(Vk[4] * (Sk - unk), Sk - Ss);
         } else {
-            const R f = (Sk - unk) / (Sk - Ss);
+            const R f = quot(Sk - unk, Sk - Ss);
             const R rs = rk * f;
             Us[0] = Qk[0] * f;
             Us[1] = Qk[1] * f;
             Us[2] = rs * (Ss * nx - utk * ny);
             Us[3] = rs * (Ss * ny + utk * nx);
-            Us[4] = rs * ((Ek / rk) + (Ss - unk) * (Ss + Pk / (rk * (Sk - unk))));
+            Us[4] = rs * (quot(Ek, rk) + (Ss - unk) * (Ss + quot(Pk, rk * (Sk - unk))));
             Us[5] = Vk[5] * f;
         }
 #pragma unroll
         for (int i = 0; i < NV; ++i) Flux[i] = Fk[i] + Sk * (Us[i] - Qk[i]);
-        Flux[NV] = unk + Sk * (((Sk - unk) / (Sk - Ss)) - R(1.0));
+        Flux[NV] = unk + Sk * (quot(Sk - unk, Sk - Ss) - R(1.0));
     }
     return (sl < sr) ? sr : sl;
 }
@@ -433,14 +448,14 @@ __device__ __forceinline__ R rot_hllc2(const Eos& e, const R* VL, const R* VR, R
     constexpr int NV = MODEL == HYPE_MP_DI4 ? 5 : 6;
     constexpr int IU = MODEL == HYPE_MP_DI4 ? 1 : 2;
     const R du = VR[IU] - VL[IU], dv = VR[IU + 1] - VL[IU + 1];
-    const R dq = sqrt(du * du + dv * dv);
+    const R dq = root(du * du + dv * dv);
     R n1x, n1y;
     if (dq < R(1.0E-10)) {
         n1x = nx;
         n1y = ny;
     } else {
-        n1x = du / dq;
-        n1y = dv / dq;
+        n1x = quot(du, dq);
+        n1y = quot(dv, dq);
     }
     R a1 = n1x * nx + n1y * ny;
     if (a1 < R(0)) {
