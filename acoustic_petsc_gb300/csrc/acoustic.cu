@@ -315,18 +315,18 @@ __global__ void __launch_bounds__(256) k_ac_update(const double* __restrict__ Fx
 //   (F_{i+1/2} - F_{i-1/2}) h / c^2 = 49/48 s1 + 1/24 s2 - 1/48 s3 - 25/12 w,  s_k = w_{i-k} + w_{i+k}
 // (R4's derivatives, reconstruction.c:90-108, the central flux pde.c:12-34), so a stage is
 //   out_u = a U_u + b W_u + c dt W_v,   out_v = a U_v + b W_v + c dt c^2 / h^2 (sum over x, y, z).
-// s1 is summed as differences to w (exact where the neighbours lie within a factor 2): the
-// second difference carries no rounding of the size of w, and what is left, s2 / 24 - s3 / 48 -
-// w / 24, enters scaled by 1/24.
+// In units of k / 48 the sum is 49 (s1 - 6 w) + 2 s2 - s3 - 6 w over the six, twice six and three directions:
+// integer coefficients, so it is formed exactly on the 19 values in fixed point (fixed.cuh; units of 2^-56 of the
+// largest one's power of two, exact for values within 2^-4 of it) and rounded once.  Stencils that are not
+// finite or beyond 2^877 take the same sum in FP64, differences to w first.
 //
-// Bound: FP64 issue, 26 FP64 instructions per cell and stage against about 280 for the
-// polynomial form and its trace and flux arrays; a thread marches kz planes of its column with
-// the seven z values in registers and reads its x and y neighbours through L1.  The plane is
-// indexed flat, so no warp is left partly empty at the end of a row (its FP64 instructions cost
-// the same with one active lane as with 32).  200^3: 14.5 -> 1.82 ms per step (4.4 G cell-updates/s,
-// 73 % of the FP64 issue ceiling); 16^3: 120 -> 27 us.
+// Bound: what the integer pipe (about 400 instructions a cell) and the FP64 pipe (5 to 9 operations) leave each
+// other; all in FP64 the star was 26 to 30 operations and the polynomial form about 280 with its trace and flux
+// arrays.  A thread marches kz planes of its column with the seven z values in registers and reads its x and y
+// neighbours through L1.  The plane is indexed flat, so no warp is left partly empty at the end of a row.
+// 200^3, a step: polynomial form 14.5 ms, star in FP64 1.82, here 0.90.
 struct StarCoef {
-    double k0, k1, k2, k3;  // of w, sum of (w_k - w) over the six nearest, s2 and s3 summed over the axes
+    double k;    // the stage's c dt c^2 / h^2 over 48
     double cdt;             // c dt (0 for RHS-only calls)
 };
 constexpr int kStarThreads = 256;
@@ -365,7 +365,6 @@ __global__ void __launch_bounds__(kStarThreads) k_ac_star(const double* __restri
     double z[7];
 #pragma unroll
     for (int o = 0; o < 6; ++o) z[o + 1] = at_z(k0 + o - 3);
-    double dlo = z[4] - z[3];
     for (int k = k0; k < k1; ++k) {
 #pragma unroll
         for (int o = 0; o < 6; ++o) z[o] = z[o + 1];
@@ -376,23 +375,42 @@ __global__ void __launch_bounds__(kStarThreads) k_ac_star(const double* __restri
 #pragma unroll
         for (int o = 0; o < 12; ++o) n[o] = signed_as(__ldg(p + off[o]), (neg >> o) & 1u);
         const double v = __ldg(W + g.N + cell);
-        const double w = z[3], dhi = z[4] - w;
-        const double t1 = ((n[2] - w) + (n[3] - w)) + ((n[8] - w) + (n[9] - w)) + (dhi - dlo);
-        const double s2 = (n[1] + n[4]) + (n[7] + n[10]) + (z[1] + z[5]);
-        const double s3 = (n[0] + n[5]) + (n[6] + n[11]) + (z[0] + z[6]);
-        dlo = dhi;
-        double div = fma(kc.k1, t1, fma(kc.k2, s2, fma(kc.k3, s3, kc.k0 * w)));
+        const double w = z[3];
+        double sum;  // 49 t1 + 2 s2 - s3 - 6 w
+        int top = 64;  // results stay normal numbers
+        auto widest = [&](double x) { top = max(top, (__double2hiint(x) >> 20) & 0x7FF); };
+#pragma unroll
+        for (int o = 0; o < 12; ++o) widest(n[o]);
+#pragma unroll
+        for (int o = 0; o < 7; ++o) widest(z[o]);
+        if (top <= 1900) {
+            using euler::i64;
+            auto fx = [&](double x) { return euler::to_fixed<4>(euler::bits_of(x), top); };
+            const i64 iw = fx(w);
+            const i64 t1 = (fx(n[2]) + fx(n[3])) + (fx(n[8]) + fx(n[9])) + (fx(z[2]) + fx(z[4])) - 6 * iw;
+            const i64 s2 = (fx(n[1]) + fx(n[4])) + (fx(n[7]) + fx(n[10])) + (fx(z[1]) + fx(z[5]));
+            const i64 s3 = (fx(n[0]) + fx(n[5])) + (fx(n[6]) + fx(n[11])) + (fx(z[0]) + fx(z[6]));
+            sum = fma(49.0, __ll2double_rn(t1), __ll2double_rn(2 * s2 - s3 - 6 * iw));
+            const int hi = __double2hiint(sum), lo = __double2loint(sum);
+            sum = __hiloint2double(hi + ((hi << 1) | lo ? (top - 1023 - 56) << 20 : 0), lo);
+        } else {
+            const double t1 = ((n[2] - w) + (n[3] - w)) + ((n[8] - w) + (n[9] - w)) + ((z[4] - w) + (z[2] - w));
+            const double s2 = (n[1] + n[4]) + (n[7] + n[10]) + (z[1] + z[5]);
+            const double s3 = (n[0] + n[5]) + (n[6] + n[11]) + (z[0] + z[6]);
+            sum = fma(49.0, t1, fma(2.0, s2, fma(-6.0, w, -s3)));
+        }
         if (cell == src.rec_cell) *src.slot = w;
         if (RHS_ONLY) {
+            double div = kc.k * sum;
             if (cell == src.src_cell) div += src.src_val;
             out[cell] = v;
             out[g.N + cell] = div;
         } else {
-            if (cell == src.src_cell) div = fma(kc.cdt, src.src_val, div);
             const double bu = WITH_U ? fma(a, __ldg(U + cell), b * w) : w;
-            const double bv = WITH_U ? fma(a, __ldg(U + g.N + cell), b * v) : v;
+            double bv = WITH_U ? fma(a, __ldg(U + g.N + cell), b * v) : v;
+            if (cell == src.src_cell) bv = fma(kc.cdt, src.src_val, bv);
             out[cell] = fma(kc.cdt, v, bu);
-            out[g.N + cell] = bv + div;
+            out[g.N + cell] = fma(kc.k, sum, bv);
         }
     }
 }
@@ -433,7 +451,7 @@ static int ac_star(hype_acoustic* s, const double* U, const double* W, double* o
     const double cdt = st.rhs_only ? 0.0 : st.c * dt;
     const double k = (st.rhs_only ? 1.0 : cdt) * (s->p.c * s->p.c) / (s->p.h * s->p.h);
     // w appears as 49/48 (s1 - 2 w) + ... with 3 axes: -25/12 + 49/24 = -1/24 each
-    const StarCoef kc{-0.125 * k, (49.0 / 48.0) * k, k / 24.0, -k / 48.0, cdt};
+    const StarCoef kc{k / 48.0, cdt};
     // planes per thread: long columns re-read six planes less often, short ones fill the chip on small
     // grids; 12 blocks per SM keep the last wave's share small
     const unsigned bx = cdiv((long long)g.nx * g.ny, kStarThreads);

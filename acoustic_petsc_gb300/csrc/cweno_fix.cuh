@@ -35,9 +35,9 @@ struct PolyFix {
     int top;
 };
 
-// the largest biased exponent of the stencil, not below 2^-400 (smaller numbers become zero)
+// the largest biased exponent of the stencil, not below 2^-959 (so that every result is a normal number)
 __host__ __device__ __forceinline__ int stencil_top(const double* __restrict__ s) {
-    int top = 623;
+    int top = 64;
 #pragma unroll
     for (int i = 0; i < 33; ++i) {
         const int e = (int)(bits_of(s[i]) >> 52) & 0x7FF;
@@ -45,10 +45,10 @@ __host__ __device__ __forceinline__ int stencil_top(const double* __restrict__ s
     }
     return top;
 }
-// whether the fixed-point form applies: finite, no overflow of the indicators, and (strict) the cell's own
+// whether the fixed-point form applies: finite, results in range, and (strict) the cell's own
 // value within a factor 8 of the largest
 __host__ __device__ __forceinline__ bool fix_applies(double u0, int top, bool strict) {
-    return top <= 1423 && !(strict && (((int)(bits_of(u0) >> 52) & 0x7FF) < top - 3));
+    return top <= 2000 && !(strict && (((int)(bits_of(u0) >> 52) & 0x7FF) < top - 3));
 }
 
 template <bool LINEAR>

@@ -196,3 +196,26 @@ def test_linear_star_edges(hype, oracle, shape, bc, precision):
     assert rel(s.get_state(), Uo) <= 1e-12
     tt, u, c = s.receiver_trace()
     assert c == cnt == 20 and np.array_equal(tt, to) and np.abs(u - uo).max() <= 1e-12 * np.abs(U).max()
+
+
+@pytest.mark.parametrize("n", [(7, 5, 6), (33, 3, 4)], ids=str)
+@pytest.mark.parametrize("scale", [1.0, 1e-270, 1e290], ids=["one", "tiny", "huge"])
+def test_star_scales_and_zeros(hype, n, scale):
+    """the star's fixed-point sum over ordinary and tiny numbers, numbers that take its FP64 form, and exact zeros,
+    against numpy's 64-bit star.  Tolerance: a few roundings of the terms' size, 1e-14 of their coefficients' sum
+    12.5 / h^2 times the largest value."""
+    rng = np.random.default_rng(5)
+    U = np.zeros((n[2], n[1], n[0], 2))
+    U[..., 0] = scale * rng.standard_normal(U.shape[:-1])
+    U[0, :, :, 0] = 0.0
+    h, dt = 0.5, 1e-3
+    s = hype.AcousticFV3D(*n, h, dt, boundaries=(0,) * 6)
+    R = s.RHSFunction(0.0, U)
+    u = U[..., 0] / scale
+    ref = np.zeros_like(u)
+    for ax in range(3):
+        s1, s2, s3 = (np.roll(u, k, ax) + np.roll(u, -k, ax) for k in (1, 2, 3))
+        ref += 49 / 48 * s1 + s2 / 24 - s3 / 48 - 25 / 12 * u
+    ref /= h * h
+    assert np.abs(R[..., 1] / scale - ref).max() <= 1e-14 * 12.5 / (h * h) * np.abs(u).max()
+    assert not R[..., 0].any()
