@@ -317,7 +317,7 @@ static int sw_d2h(hype_acoustic2d* a, const double* soa, double* aos) {
     const long long N = a->g.N;
     k_sw_soa2aos<<<cdiv(N, 256), 256, 0, a->stream>>>(soa, a->aos, N);
     HYPE_LAUNCHED(1);
-    HYPE_CK(cudaMemcpyAsync(aos, a->aos, sizeof(double) * 2 * N, cudaMemcpyDeviceToHost, a->stream));
+    HYPE_CK(copy_to_host(aos, a->aos, sizeof(double) * 2 * N, a->stream));
     HYPE_CK(cudaStreamSynchronize(a->stream));
     return HYPE_OK;
 }

@@ -2166,7 +2166,7 @@ static int d2h_aos(hype_euler* e, const double* soa, double* aos) {
     const long long n = e->g.N * NV;
     k_soa_to_aos<<<cdiv(n, 256), 256, 0, e->stream>>>(soa, e->stage_aos, e->g.N);
     HYPE_LAUNCHED(1);
-    HYPE_CK(cudaMemcpyAsync(aos, e->stage_aos, sizeof(double) * n, cudaMemcpyDeviceToHost, e->stream));
+    HYPE_CK(copy_to_host(aos, e->stage_aos, sizeof(double) * n, e->stream));
     return HYPE_OK;
 }
 

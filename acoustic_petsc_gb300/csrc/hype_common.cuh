@@ -15,6 +15,10 @@ void set_last_error(const char* where, cudaError_t e);
 // process-wide kernel launch counter (hype_launch_count)
 void count_launch(long long n = 1);
 
+// device -> pageable host memory, asynchronously as cudaMemcpyAsync: the destination's pages are made present
+// first, while the work queued on the stream runs (capi.cu)
+cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t stream);
+
 #define HYPE_CK(call)                                        \
     do {                                                     \
         cudaError_t e__ = (call);                            \

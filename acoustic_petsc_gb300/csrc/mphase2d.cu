@@ -358,7 +358,7 @@ static int mp_d2h(hype_mp2d* m, const double* soa, double* aos) {
     const long long n = m->g.N * m->g.nv;
     k_soa2aos<<<cdiv(n, 256), 256, 0, m->stream>>>(soa, m->stage_aos, m->g.N, m->g.nv);
     HYPE_LAUNCHED(1);
-    HYPE_CK(cudaMemcpyAsync(aos, m->stage_aos, sizeof(double) * n, cudaMemcpyDeviceToHost, m->stream));
+    HYPE_CK(copy_to_host(aos, m->stage_aos, sizeof(double) * n, m->stream));
     return HYPE_OK;
 }
 

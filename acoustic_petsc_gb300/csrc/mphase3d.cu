@@ -798,7 +798,7 @@ static int m3_d2h(hype_mp3d* m, const double* soa, double* aos) {
     const long long N = m->g.N;
     k_m3_soa2aos<<<cdiv(N * MV, 256), 256, 0, m->stream>>>(soa, m->aos, N);
     HYPE_LAUNCHED(1);
-    HYPE_CK(cudaMemcpyAsync(aos, m->aos, sizeof(double) * MV * N, cudaMemcpyDeviceToHost, m->stream));
+    HYPE_CK(copy_to_host(aos, m->aos, sizeof(double) * MV * N, m->stream));
     HYPE_CK(cudaStreamSynchronize(m->stream));
     return HYPE_OK;
 }

@@ -584,7 +584,7 @@ static int pc_d2h(hype_pc2d* m, const double* soa, double* aos) {
     const long long N = m->g.N;
     k_pc_soa2aos<<<cdiv(N * KV, 256), 256, 0, m->stream>>>(soa, m->aos, N);
     HYPE_LAUNCHED(1);
-    HYPE_CK(cudaMemcpyAsync(aos, m->aos, sizeof(double) * KV * N, cudaMemcpyDeviceToHost, m->stream));
+    HYPE_CK(copy_to_host(aos, m->aos, sizeof(double) * KV * N, m->stream));
     HYPE_CK(cudaStreamSynchronize(m->stream));
     return HYPE_OK;
 }
