@@ -274,110 +274,94 @@ __device__ __forceinline__ double rusanov64(const double* __restrict__ QL, const
 }
 
 // ---------------------------------------------------------------- viscous fluxes
-// The R4 differences that a cell's gradients need, kept for the face kernel: A, D, 2 u_ab (xy, yz, xz),
-// ddd, then aab and abb by pair, xyz (r4_64's lin, sq, cr, ddd, aab/abb, xyz)
-constexpr int NGC = 19;
+// The R4 differences that a cell's gradients need, kept for the face kernel in fixed point (units of
+// 2^(top - 1023 - 58)): A, D, 4 u_ab (xy, yz, xz), ddd, then aab and abb by pair, xyz, and top (r4_64's lin, sq,
+// twice its cr, ddd, aab/abb, xyz)
+constexpr int NGC = 20;
 
 __device__ __forceinline__ void store_grad_coeffs(const Poly64& p, double* __restrict__ C, long long st) {
+    const double v[19] = {p.lin[0], p.lin[1], p.lin[2], p.sq[0], p.sq[1], p.sq[2], 2.0 * p.cr[0], 2.0 * p.cr[1], 2.0 * p.cr[2],
+                          p.ddd[0], p.ddd[1], p.ddd[2], p.aab[0], p.abb[0], p.aab[1], p.abb[1], p.aab[2], p.abb[2], p.xyz};
+    int top = 64;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        C[a * st] = p.lin[a];
-        C[(3 + a) * st] = p.sq[a];
-        C[(6 + a) * st] = p.cr[a];
-        C[(9 + a) * st] = p.ddd[a];
-        C[(12 + 2 * a) * st] = p.aab[a];
-        C[(13 + 2 * a) * st] = p.abb[a];
-    }
-    C[18 * st] = p.xyz;
+    for (int q = 0; q < 19; ++q) top = max(top, (__double2hiint(v[q]) >> 20) & 0x7FF);
+#pragma unroll
+    for (int q = 0; q < 19; ++q) C[q * st] = __longlong_as_double(to_fixed<6>(bits_of(v[q]), top));
+    C[19 * st] = __longlong_as_double(top);
 }
 
-// Twice the derivative along axis B (times h) of the R4 polynomial at the 4 Gauss points of the face
-// x_D = NS/2: the gradient of evaluate_grad (Navier-Stokes-3D/reconstruction.c:24-35) is bilinear there,
-// P + Q t1 + R t2 + S t1 t2, with the squares t1^2 = t2^2 = 1/12 folded in, and its four values take two
-// levels of sums.  out[2 (t1 > 0) + (t2 > 0)].
+// Twice the derivative along axis B (times h) of the R4 polynomial at Gauss point gp = 2 (t1 > 0) + (t2 > 0) of
+// the face x_D = NS/2: the gradient of evaluate_grad (Navier-Stokes-3D/reconstruction.c:24-35) is bilinear
+// there, P + Q t1 + R t2 + S t1 t2, with the squares t1^2 = t2^2 = 1/12 folded in.  On the integer pipe, the
+// conversion included: the 22 forms of a face at its four points were 340 of its 810 FP64 operations.
 template <int D, int NS, int B>
-__device__ __forceinline__ void face_grads64(const double* __restrict__ C, long long st, double* __restrict__ out) {
+__device__ __forceinline__ double face_grad64(const double* __restrict__ C, long long st, int gp) {
     constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
-    auto ld = [&](int q) { return __ldg(C + q * st); };
+    constexpr i64 kG2 = 2662558164157085696ll, kG8 = 665639541039271424ll;                // 2^64 times GPT/2 and GPT/8
+    constexpr i64 k6 = 3074457345618258603ll, k12 = 1537228672809129301ll, k48 = 384307168202282325ll;  // 1/6, 1/12, 1/48
+    auto ld = [&](int q) { return (i64)__double_as_longlong(__ldg(C + q * st)); };
     auto lin = [&](int a) { return ld(a); };
     auto sq = [&](int a) { return ld(3 + a); };
-    auto cr = [&](int a, int b) { return ld(6 + pair_of(a, b)); };
+    auto cr2 = [&](int a, int b) { return ld(6 + pair_of(a, b)); };
     auto cube = [&](int a) { return ld(9 + a); };
     auto sqlin = [&](int a, int b) { return ld((a < b ? 12 : 13) + 2 * pair_of(a, b)); };  // of x_a^2 x_b
-    constexpr double ns = NS;
-    double P, Q, R, S;
+    auto toward = [&](i64 a, i64 b) { return NS > 0 ? a + b : a - b; };
+    const int top = (int)ld(19);
+    i64 P, Q, R, S;
     if constexpr (B == D) {
-        P = fma(-1. / 12., cube(D), fma(ns, sq(D), lin(D)));
-        Q = fma(ns * 0.5 * GPT, sqlin(D, T1), GPT * cr(D, T1));
-        R = fma(ns * 0.5 * GPT, sqlin(D, T2), GPT * cr(D, T2));
-        S = (1. / 48.) * ld(18);
+        P = toward(lin(D), sq(D)) - scaled(cube(D), split(k12));
+        Q = scaled(toward(cr2(D, T1), sqlin(D, T1)), split(kG2));
+        R = scaled(toward(cr2(D, T2), sqlin(D, T2)), split(kG2));
+        S = scaled(ld(18), split(k48));
     } else {
         constexpr int O = B == T1 ? T2 : T1;
-        P = fma(1. / 12., sqlin(D, B), fma(ns * 0.5, cr(D, B), fma(-1. / 6., cube(B), lin(B))));
-        const double q = fma(ns * 0.5 * GPT, sqlin(B, D), (2.0 * GPT) * sq(B));
-        const double r = fma(ns * 0.125 * GPT, ld(18), GPT * cr(B, O));
+        P = toward(lin(B) - scaled(cube(B), split(k6)) + scaled(sqlin(D, B), split(k12)), (cr2(D, B) + 2) >> 2);
+        // 2 GPT sq +- GPT/2 sqlin, GPT/2 cr2 +- GPT/8 xyz
+        const i64 q = toward(4 * scaled(sq(B), split(kG2)), scaled(sqlin(B, D), split(kG2)));
+        const i64 r = toward(scaled(cr2(B, O), split(kG2)), scaled(ld(18), split(kG8)));
         Q = B == T1 ? q : r;
         R = B == T1 ? r : q;
-        S = (1. / 12.) * sqlin(B, O);
+        S = scaled(sqlin(B, O), split(k12));
     }
-    const double a = P - Q, b = P + Q, c = R - S, d = R + S;
-    out[0] = a - c;
-    out[1] = a + c;
-    out[2] = b - d;
-    out[3] = b + d;
+    const i64 n1 = (gp & 2) ? 0 : -1, n2 = (gp & 1) ? 0 : -1;  // all ones where the coordinate is negative
+    const i64 RS = R + ((S ^ n1) - n1);
+    return double_of(P + ((Q ^ n1) - n1) + ((RS ^ n2) - n2), top);
 }
 
-// The viscous fluxes (PDEViscFlux, Navier-Stokes-3D/pde.c:90-162) of one face side at its 4 Gauss points,
-// summed and divided by mu/(2 h): Newtonian stress with Stokes' hypothesis and Fourier heat flux, with the
-// program's velocity gradients u_x = (rho u)_x - u rho_x / rho (:118-130).  Adds the momentum components
-// along D, T1, T2 and the energy's to av; kmu = k / mu; returns the largest 1 / rho.  Only the 11
-// gradient components that enter the flux along D are formed.
+// The viscous fluxes (PDEViscFlux, Navier-Stokes-3D/pde.c:90-162) of one face side at Gauss point gp, divided by
+// mu/(2 h): Newtonian stress with Stokes' hypothesis and Fourier heat flux, with the program's velocity
+// gradients u_x = (rho u)_x - u rho_x / rho (:118-130).  Adds the momentum components along D, T1, T2 and the
+// energy's to av; Q is the side's trace, kmu = k / mu; returns 1 / rho.  Only the 11 gradient components that
+// enter the flux along D are formed.
 template <int D, int NS>
-__device__ __forceinline__ double visc_side64(const double* __restrict__ T, const double* __restrict__ C4, long long NE,
-                                              long long e, double gm1, double kmu, double* av) {
+__device__ __forceinline__ double visc_point64(const double* __restrict__ Q, const double* __restrict__ C4, long long NE,
+                                               int gp, double gm1, double kmu, double* av) {
     constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
-    double gr[3][4], gd[3][4], gn[2][4], gt[2][4], ge[4];  // rho along D, T1, T2; m_D likewise; m_T along D and its own axis; E
     const long long cs = 20 * NE;
-    face_grads64<D, NS, D>(C4 + e, NE, gr[0]);
-    face_grads64<D, NS, T1>(C4 + e, NE, gr[1]);
-    face_grads64<D, NS, T2>(C4 + e, NE, gr[2]);
-    const double* Cd = C4 + (1 + D) * cs + e;
-    const double* C1 = C4 + (1 + T1) * cs + e;
-    const double* C2 = C4 + (1 + T2) * cs + e;
-    face_grads64<D, NS, D>(Cd, NE, gd[0]);
-    face_grads64<D, NS, T1>(Cd, NE, gd[1]);
-    face_grads64<D, NS, T2>(Cd, NE, gd[2]);
-    face_grads64<D, NS, D>(C1, NE, gn[0]);
-    face_grads64<D, NS, T1>(C1, NE, gt[0]);
-    face_grads64<D, NS, D>(C2, NE, gn[1]);
-    face_grads64<D, NS, T2>(C2, NE, gt[1]);
-    face_grads64<D, NS, D>(C4 + 4 * cs + e, NE, ge);
-    constexpr int face = 2 * D + (NS > 0 ? 1 : 0);
-    double imax = 0.0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const double* Tq = T + (face * 4 + q) * NE + e;
-        const double rho = __ldg(Tq), md = __ldg(Tq + (1 + D) * NTR * NE), m1 = __ldg(Tq + (1 + T1) * NTR * NE),
-                     m2 = __ldg(Tq + (1 + T2) * NTR * NE), E = __ldg(Tq + 4 * NTR * NE);
-        const double ir = recip_fix(rho);
-        const double u = md * ir, v = m1 * ir, w = m2 * ir;
-        const double em = fma(-w, m2, fma(-v, m1, fma(-u, md, E)));  // E - |m|^2 / rho
-        const double rd = gr[0][q] * ir, r1 = gr[1][q] * ir, r2 = gr[2][q] * ir;
-        const double ud = fma(-u, rd, gd[0][q]), u1 = fma(-u, r1, gd[1][q]), u2 = fma(-u, r2, gd[2][q]);
-        const double vd = fma(-v, rd, gn[0][q]), v1 = fma(-v, r1, gt[0][q]);
-        const double wd = fma(-w, rd, gn[1][q]), w2 = fma(-w, r2, gt[1][q]);
-        // the temperature gradient (times c_v) of pde.c:118-130, regrouped:
-        // (gamma - 1)/rho (E_D - u.m_D - rho_D/rho (E - |m|^2 / rho))
-        const double um = fma(w, gn[1][q], fma(v, gn[0][q], u * gd[0][q]));
-        const double td = fma(-rd, em, ge[q] - um) * (gm1 * ir);
-        const double tn = fma(-2. / 3., (ud + v1) + w2, 2.0 * ud), t1 = u1 + vd, t2 = u2 + wd;
-        av[0] += tn;
-        av[1] += t1;
-        av[2] += t2;
-        av[3] += fma(kmu, td, fma(w, t2, fma(v, t1, u * tn)));
-        imax = max_pos(imax, ir);
-    }
-    return imax;
+    const double* Cd = C4 + (1 + D) * cs;
+    const double* C1 = C4 + (1 + T1) * cs;
+    const double* C2 = C4 + (1 + T2) * cs;
+    const double rho = Q[0], md = Q[1 + D], m1 = Q[1 + T1], m2 = Q[1 + T2], E = Q[4];
+    const double ir = recip_fix(rho);
+    const double u = md * ir, v = m1 * ir, w = m2 * ir;
+    const double em = fma(-w, m2, fma(-v, m1, fma(-u, md, E)));  // E - |m|^2 / rho
+    const double rd = face_grad64<D, NS, D>(C4, NE, gp) * ir, r1 = face_grad64<D, NS, T1>(C4, NE, gp) * ir,
+                 r2 = face_grad64<D, NS, T2>(C4, NE, gp) * ir;
+    const double gd = face_grad64<D, NS, D>(Cd, NE, gp), g1 = face_grad64<D, NS, D>(C1, NE, gp), g2 = face_grad64<D, NS, D>(C2, NE, gp);
+    const double ud = fma(-u, rd, gd), u1 = fma(-u, r1, face_grad64<D, NS, T1>(Cd, NE, gp)),
+                 u2 = fma(-u, r2, face_grad64<D, NS, T2>(Cd, NE, gp));
+    const double vd = fma(-v, rd, g1), v1 = fma(-v, r1, face_grad64<D, NS, T1>(C1, NE, gp));
+    const double wd = fma(-w, rd, g2), w2 = fma(-w, r2, face_grad64<D, NS, T2>(C2, NE, gp));
+    // the temperature gradient (times c_v) of pde.c:118-130, regrouped:
+    // (gamma - 1)/rho (E_D - u.m_D - rho_D/rho (E - |m|^2 / rho))
+    const double um = fma(w, g2, fma(v, g1, u * gd));
+    const double td = fma(-rd, em, face_grad64<D, NS, D>(C4 + 4 * cs, NE, gp) - um) * (gm1 * ir);
+    const double tn = fma(-2. / 3., (ud + v1) + w2, 2.0 * ud), t1 = u1 + vd, t2 = u2 + wd;
+    av[0] += tn;
+    av[1] += t1;
+    av[2] += t2;
+    av[3] += fma(kmu, td, fma(w, t2, fma(v, t1, u * tn)));
+    return ir;
 }
 
 }  // namespace euler

@@ -230,16 +230,18 @@ __device__ __forceinline__ bool surely_above(const PolyFix& p, double lo) {
 
 // the R4 differences that the viscous fluxes take, as the Poly64 form of store_grad_coeffs stores them
 __device__ __forceinline__ void store_grad_coeffs(const PolyFix& p, double* __restrict__ C, long long st) {
+    auto put = [&](int q, i64 v) { C[q * st] = __longlong_as_double(v); };
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        C[a * st] = from_fixed(p.lin[a], p.top);
-        C[(3 + a) * st] = from_fixed(p.sq[a], p.top);
-        C[(6 + a) * st] = from_fixed(p.cr2[a], p.top - 1);
-        C[(9 + a) * st] = from_fixed(p.ddd[a], p.top);
-        C[(12 + 2 * a) * st] = from_fixed(p.aab[a], p.top);
-        C[(13 + 2 * a) * st] = from_fixed(p.abb[a], p.top);
+        put(a, p.lin[a]);
+        put(3 + a, p.sq[a]);
+        put(6 + a, p.cr2[a]);
+        put(9 + a, p.ddd[a]);
+        put(12 + 2 * a, p.aab[a]);
+        put(13 + 2 * a, p.abb[a]);
     }
-    C[18 * st] = from_fixed(p.xyz, p.top);
+    put(18, p.xyz);
+    put(19, p.top);
 }
 
 // the 24 traces of one variable's stencil, trace q at T[q * st], and with the fixed-point form not applying

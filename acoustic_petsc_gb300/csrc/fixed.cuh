@@ -233,6 +233,12 @@ __host__ __device__ __forceinline__ u64 shift_by(u64 v, int s) {
 __host__ __device__ __forceinline__ double pack(u64 m, int x) {
     return from_bits(((u64)(x + 63 + 1023 - 1) << 52) + ((m >> 11) + ((m >> 10) & 1)));
 }
+// from_fixed on the integer pipe, for kernels that FP64 issue bounds
+__host__ __device__ __forceinline__ double double_of(i64 v, int top) {
+    const u64 s = (u64)(v >> 63), m = ((u64)v ^ s) - s;
+    const int c = clz64(m | 1);
+    return from_bits((s & 0x8000000000000000ull) | (m ? (u64)bits_of(pack(m << c, top - 1023 - 58 - c)) : 0ull));
+}
 // 1/x, sqrt(x) and 1/sqrt(x) on the integer pipe (about 36, 45 and 45 instructions) for kernels that FP64 issue
 // bounds: 3, 5 and 5 FP64 operations of 64 cycles each.  Rounded from 2^-59; the ranges of recip3 and sqrt3.
 __host__ __device__ __forceinline__ u64 significand(u64 b) { return ((b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 11; }
@@ -303,6 +309,34 @@ __device__ __forceinline__ float narrow_fix(double x) {
     const unsigned f = (hi & 0x80000000u) | ((((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29));
     const unsigned r = lo & 0x1FFFFFFFu;
     return __uint_as_float(f + (r > 0x10000000u || (r == 0x10000000u && (f & 1u)) ? 1u : 0u));
+}
+
+// in FP64, as a call: inlined it would be predicated, and its operations issued for nothing
+static __device__ __noinline__ double sum_differences_fp64(double a1, double a0, double b1, double b0, double c1, double c0) {
+    return ((a1 - a0) + (b1 - b0)) + (c1 - c0);
+}
+// (a1 - a0) + (b1 - b0) + (c1 - c0) from integers in units of 2^-58 of the largest number's power of two, rounded
+// once (one FP64 operation, the conversion, for five); not finite or beyond 2^977: in FP64
+__device__ __forceinline__ double sum_differences(double a1, double a0, double b1, double b0, double c1, double c0) {
+    int top = 64;
+    auto widest = [&](double x) { top = max(top, (__double2hiint(x) >> 20) & 0x7FF); };
+    widest(a1); widest(a0); widest(b1); widest(b0); widest(c1); widest(c0);
+    if (top > 2000) return sum_differences_fp64(a1, a0, b1, b0, c1, c0);
+    auto fx = [&](double x) { return to_fixed<6>(bits_of(x), top); };
+    return from_fixed(((fx(a1) - fx(a0)) + (fx(b1) - fx(b0))) + (fx(c1) - fx(c0)), top);
+}
+
+// (a + b) + (c + d), and 2^-shift of it, in the same way
+static __device__ __noinline__ double sum4_fp64(double a, double b, double c, double d, int shift) {
+    return ldexp((a + b) + (c + d), -shift);
+}
+__device__ __forceinline__ double sum4(double a, double b, double c, double d, int shift) {
+    int top = 128;
+    auto widest = [&](double x) { top = max(top, (__double2hiint(x) >> 20) & 0x7FF); };
+    widest(a); widest(b); widest(c); widest(d);
+    if (top > 2000) return sum4_fp64(a, b, c, d, shift);
+    auto fx = [&](double x) { return to_fixed<6>(bits_of(x), top); };
+    return from_fixed((fx(a) + fx(b)) + (fx(c) + fx(d)), top - shift);
 }
 
 }  // namespace euler

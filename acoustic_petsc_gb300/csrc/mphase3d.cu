@@ -593,7 +593,7 @@ __device__ __forceinline__ void faces(const double* __restrict__ T, double* __re
     __syncthreads();
     for (int c = gp; c < MF; c += 4)
         if (f < nf)
-            F[(long long)c * nf + f] = 0.25 * ((sh[0][c][lane] + sh[1][c][lane]) + (sh[2][c][lane] + sh[3][c][lane]));
+            F[(long long)c * nf + f] = euler::sum4(sh[0][c][lane], sh[1][c][lane], sh[2][c][lane], sh[3][c][lane], 2);
 }
 
 __global__ void __launch_bounds__(128) k_m3_faces(const double* __restrict__ T, double* __restrict__ Fx, double* __restrict__ Fy,
@@ -627,8 +627,8 @@ __global__ void __launch_bounds__(kUpdateThreads) k_m3_update(const double* __re
     const double cdt = st.rhs_only ? 0.0 : st.c * ds->dt;
     // the flux difference of component q over the three directions
     auto div = [&](int q) {
-        return ((Fx[q * nfx + ix + 1] - Fx[q * nfx + ix]) + (Fy[q * nfy + iy + g.nx] - Fy[q * nfy + iy])) +
-               (Fz[q * nfz + iz + sxy] - Fz[q * nfz + iz]);
+        return euler::sum_differences(Fx[q * nfx + ix + 1], Fx[q * nfx + ix], Fy[q * nfy + iy + g.nx], Fy[q * nfy + iy],
+                                      Fz[q * nfz + iz + sxy], Fz[q * nfz + iz]);
     };
     double L = div(c);
     if (c == 5) L = fma(-Win[5 * g.N + cell], div(6), L);
