@@ -101,3 +101,24 @@ def test_instance_completion_times(hype):
     assert t[cls == 0][0] <= t[cls == n - 1][0]
     print(f"{n} classes; completion times {sorted(set(np.round(t * 1e3, 3)))} ms")
     b.close()
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-290, 1e290], ids=["one", "tiny", "huge"])
+def test_update_scales(hype, scale):
+    """the fixed-point update at the ends of its range and its FP64 form beyond it (a field at rest with no source
+    but its initial value), against numpy's 64-bit steps.  Tolerance: the rounding of 12 linear steps with |a| <= 1/4
+    and weights of sum below 4, 12 * 12 * 1.2e-16."""
+    n, h = 33, 0.05
+    rng = np.random.default_rng(2)
+    p0 = scale * rng.standard_normal((n, n))
+    p1 = 0.99 * p0
+    b = hype.BatchLeapfrog([hype.Monopole(nx=n, ny=n, xmin=-1.0, ymin=-1.0, h=h, c0=1.0, dt=0.5 * h, xs=0.0, ys=0.0,
+                                          sigma=0.05, freq=0.0)], tile=(32, 64))
+    b.set(0, p0, p1)
+    b.step(12)
+    _, p = b.get(0)
+    o, c = p0 / scale, p1 / scale
+    for _ in range(12):
+        e = np.pad(c, 1)
+        o, c = c, 2 * c - o + 0.25 * (e[2:, 1:-1] + e[:-2, 1:-1] + e[1:-1, 2:] + e[1:-1, :-2] - 4 * c)
+    assert np.abs(p / scale - c).max() <= 1.8e-14 * np.abs(p0 / scale).max()
