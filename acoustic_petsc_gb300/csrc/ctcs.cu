@@ -63,6 +63,96 @@ __global__ void __launch_bounds__(256) k_plane2d(const double* __restrict__ pold
     pnew[o] = g.a2 * s + 2.0 * c - pold[o];
 }
 
+// x 2^k as the product rounds it; a normal number's exponent moves on the integer pipe
+static __device__ __noinline__ double scale_any(double x, double f) { return x * f; }
+template <int K>
+__device__ __forceinline__ double scale2(double x) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const unsigned ex = ((unsigned)hi >> 20) & 0x7FFu;
+    if (ex - 1u < 2040u) return __hiloint2double(hi + (K << 20), lo);
+    if (((hi << 1) | lo) == 0) return x;
+    return scale_any(x, (double)(1 << K));
+}
+
+// kSteps (or fewer) plane-wave steps in one launch: a block holds its BX x by tile of both levels in shared memory
+// with a frame of kSteps nodes, updates a region that shrinks by one node a step, every node in the operation order
+// of k_plane2d, and writes the tile's two newest levels.  po, pc and no, nc are different arrays.
+// A launch per step took 6.3 us at 512^2 (9 FP64 operations a node need 4.0 of it) and 2.0 at 48 x 40; here it is 7
+// operations (the products by 2 and 4 are exponent additions), the frame's share and a quarter of the launches:
+// 5.3 and 1.05 us a step; 1200 x 1100 25.0 -> 22.4.  512 threads: 256 leave the FP64 pipe waiting (6.0 us).
+constexpr int kSteps = 4, kTileRows = 32, kPlaneThreads = 512;
+
+template <int BX>
+__global__ void __launch_bounds__(kPlaneThreads) k_plane2d_steps(const double* __restrict__ po, const double* __restrict__ pc,
+                                                                 double* __restrict__ no, double* __restrict__ nc, Grid g,
+                                                                 int by, int steps) {
+    constexpr int W = BX + 2 * kSteps;
+    __shared__ double sh[2][W * (kTileRows + 2 * kSteps)];
+    const int i0 = blockIdx.x * BX - kSteps, j0 = blockIdx.y * by - kSteps, H = by + 2 * kSteps;
+    for (int q = threadIdx.x; q < W * H; q += kPlaneThreads) {
+        int i = i0 + q % W, j = j0 + q / W;
+        double o = 0.0, c = 0.0;
+        if (g.bc == HYPE_BC_PERIODIC) {
+            i = (i % g.nx + g.nx) % g.nx;
+            j = (j % g.ny + g.ny) % g.ny;
+        }
+        if (i >= 0 && i < g.nx && j >= 0 && j < g.ny) {
+            o = __ldg(po + (long long)j * g.nx + i);
+            c = __ldg(pc + (long long)j * g.nx + i);
+        }
+        sh[0][q] = o;
+        sh[1][q] = c;
+    }
+    __syncthreads();
+    double *a = sh[0], *b = sh[1];
+    for (int s = 0; s < steps; ++s) {
+        const int m = kSteps - (steps - 1 - s), w = W - 2 * m, n = w * (H - 2 * m);  // the nodes that later steps need
+#pragma unroll 1
+        for (int q = threadIdx.x; q < n; q += kPlaneThreads) {
+            const int y = q / w, x = q - y * w + m, o = (y + m) * W + x;
+            const int i = i0 + x, j = j0 + y + m;
+            if (g.bc != HYPE_BC_PERIODIC && (i < 0 || i >= g.nx || j < 0 || j >= g.ny)) continue;  // stays zero
+            const double c = b[o];
+            const double l = b[o + W] + b[o - W] + b[o + 1] + b[o - 1] - scale2<2>(c);
+            a[o] = g.a2 * l + scale2<1>(c) - a[o];
+        }
+        __syncthreads();
+        double* t = a;
+        a = b;
+        b = t;
+    }
+    for (int q = threadIdx.x; q < BX * by; q += kPlaneThreads) {
+        const int x = q % BX, y = q / BX, i = i0 + kSteps + x, j = j0 + kSteps + y;
+        if (i >= g.nx || j >= g.ny) continue;
+        const int o = (y + kSteps) * W + x + kSteps;
+        no[(long long)j * g.nx + i] = a[o];
+        nc[(long long)j * g.nx + i] = b[o];
+    }
+}
+
+// The tile of k_plane2d_steps: FP64 issue bounds an SM's blocks together, so the time goes as the fullest SM's
+// blocks times the node updates of one with its frame.  Narrow tiles serve small grids (48^2 is two tiles of
+// 64 x 32, which would leave 150 SMs idle), and the row count is chosen so that the last wave is full.
+struct PlaneTile {
+    int bx, by;
+};
+inline PlaneTile plane_tile(int nx, int ny, int nsm) {
+    PlaneTile best{64, kTileRows};
+    double least = -1.0;
+    for (int bx : {64, 32, 16})
+        for (int by = 4; by <= kTileRows; ++by) {
+            const double blocks = (double)cdiv(nx, bx) * cdiv(ny, by);
+            double updates = 600.0;  // what a block's loads, barriers and stores cost beside them
+            for (int r = 0; r < kSteps; ++r) updates += (double)(bx + 2 * r) * (by + 2 * r);
+            const double time = ceil(blocks / nsm) * updates;
+            if (least < 0.0 || time < least) {
+                least = time;
+                best = PlaneTile{bx, by};
+            }
+        }
+    return best;
+}
+
 __device__ __forceinline__ double d2o2(double m1, double c, double p1, double inv) { return (p1 - 2.0 * c + m1) * inv; }
 __device__ __forceinline__ double d2o4(double m2, double m1, double c, double p1, double p2, double inv) {
     return (-1.0 / 12 * p2 + 4.0 / 3.0 * p1 - 5.0 / 2.0 * c + 4.0 / 3.0 * m1 - 1.0 / 12.0 * m2) * inv;
@@ -152,17 +242,38 @@ struct hype_ctcs {
     hype_ctcs_params p;
     Grid g;
     cudaStream_t stream = nullptr;
-    double* lv[3] = {nullptr, nullptr, nullptr};  // rotating levels
-    int cur = 1;  // index of p (newest); p_old = cur-1 mod 3
+    // point-source form: three rotating levels, p at cur, p_old at cur - 1 mod 3; plane-wave form: two pairs
+    // (p_old, p) of levels, the current one at 2 * pair
+    double* lv[4] = {nullptr, nullptr, nullptr, nullptr};
+    int cur = 1;
+    int pair = 0;
+    PlaneTile tile{64, kTileRows};
+    double* newest() const { return p.form == 0 ? lv[2 * pair + 1] : lv[cur]; }
+    double* older() const { return p.form == 0 ? lv[2 * pair] : lv[(cur + 2) % 3]; }
     double* srcv = nullptr;
     double* recv = nullptr;
     int cap = 0;  // capacity of srcv/recv
     DevStep* st = nullptr;
     long long n = 0;
-    // graph of a chunk of steps for each rotation phase
+    // graph of a chunk of steps for each rotation phase or pair
     cudaGraphExec_t chunk[3] = {nullptr, nullptr, nullptr};
     int chunk_len = 0;
 };
+
+// up to kSteps steps of the plane-wave form from one pair of levels into the other
+static int plane_launch(hype_ctcs* c, int pair, int steps) {
+    const Grid& g = c->g;
+    const dim3 gr(cdiv(g.nx, c->tile.bx), cdiv(g.ny, c->tile.by));
+    double** l = c->lv;
+    auto go = [&](auto kern) {
+        kern<<<gr, kPlaneThreads, 0, c->stream>>>(l[2 * pair], l[2 * pair + 1], l[2 - 2 * pair], l[3 - 2 * pair], g, c->tile.by, steps);
+    };
+    if (c->tile.bx == 64) go(k_plane2d_steps<64>);
+    else if (c->tile.bx == 32) go(k_plane2d_steps<32>);
+    else go(k_plane2d_steps<16>);
+    HYPE_LAUNCHED(1);
+    return HYPE_OK;
+}
 
 static int ctcs_launch(hype_ctcs* c, int phase) {
     const Grid& g = c->g;
@@ -171,11 +282,6 @@ static int ctcs_launch(hype_ctcs* c, int phase) {
     double* pn = c->lv[(phase + 1) % 3];
     const dim3 b(32, 8);
     const dim3 gr(cdiv(g.nx, 32), cdiv(g.ny, 8), g.dim == 3 ? g.nz : 1);
-    if (c->p.form == 0) {
-        k_plane2d<<<gr, b, 0, c->stream>>>(po, pc, pn, g);
-        HYPE_LAUNCHED(1);
-        return HYPE_OK;
-    }
     const bool tick = (g.src >= 0 || g.rec >= 0);
     double* sv = g.src >= 0 ? c->srcv : nullptr;
     double* rv = g.rec >= 0 ? c->recv : nullptr;
@@ -225,9 +331,14 @@ extern "C" int hype_ctcs_create(const hype_ctcs_params* p, hype_ctcs** out) {
     }
     c->n = (long long)g.nx * g.ny * g.nz;
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-    for (int q = 0; q < 3 && e == cudaSuccess; ++q) e = cudaMalloc((void**)&c->lv[q], sizeof(double) * c->n);
+    const int levels = p->form == 0 ? 4 : 3;
+    for (int q = 0; q < levels && e == cudaSuccess; ++q) e = cudaMalloc((void**)&c->lv[q], sizeof(double) * c->n);
     if (e == cudaSuccess) e = cudaMalloc((void**)&c->st, sizeof(DevStep));
-    for (int q = 0; q < 3 && e == cudaSuccess; ++q) e = cudaMemset(c->lv[q], 0, sizeof(double) * c->n);
+    for (int q = 0; q < levels && e == cudaSuccess; ++q) e = cudaMemset(c->lv[q], 0, sizeof(double) * c->n);
+    int dev = 0, nsm = 1;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    c->tile = plane_tile(g.nx, g.ny, nsm);
     if (e != cudaSuccess) {
         set_last_error("hype_ctcs_create", e);
         hype_ctcs_destroy(c);
@@ -240,10 +351,9 @@ extern "C" int hype_ctcs_create(const hype_ctcs_params* p, hype_ctcs** out) {
 extern "C" void hype_ctcs_destroy(hype_ctcs* c) {
     if (!c) return;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (int q = 0; q < 3; ++q) {
-        cudaFree(c->lv[q]);
+    for (int q = 0; q < 4; ++q) cudaFree(c->lv[q]);
+    for (int q = 0; q < 3; ++q)
         if (c->chunk[q]) cudaGraphExecDestroy(c->chunk[q]);
-    }
     cudaFree(c->srcv);
     cudaFree(c->recv);
     cudaFree(c->st);
@@ -254,6 +364,7 @@ extern "C" void hype_ctcs_destroy(hype_ctcs* c) {
 extern "C" int hype_ctcs_set(hype_ctcs* c, const double* p_old, const double* p) {
     if (!c || !p_old || !p) return HYPE_ERR_ARG;
     c->cur = 1;
+    c->pair = 0;
     HYPE_CK(cudaMemcpyAsync(c->lv[0], p_old, sizeof(double) * c->n, cudaMemcpyHostToDevice, c->stream));
     HYPE_CK(cudaMemcpyAsync(c->lv[1], p, sizeof(double) * c->n, cudaMemcpyHostToDevice, c->stream));
     HYPE_CK(cudaStreamSynchronize(c->stream));
@@ -262,15 +373,15 @@ extern "C" int hype_ctcs_set(hype_ctcs* c, const double* p_old, const double* p)
 
 extern "C" int hype_ctcs_get(hype_ctcs* c, double* p_old, double* p) {
     if (!c) return HYPE_ERR_ARG;
-    if (p_old) HYPE_CK(cudaMemcpyAsync(p_old, c->lv[(c->cur + 2) % 3], sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream));
-    if (p) HYPE_CK(cudaMemcpyAsync(p, c->lv[c->cur], sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream));
+    if (p_old) HYPE_CK(cudaMemcpyAsync(p_old, c->older(), sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream));
+    if (p) HYPE_CK(cudaMemcpyAsync(p, c->newest(), sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream));
     HYPE_CK(cudaStreamSynchronize(c->stream));
     return HYPE_OK;
 }
 
 extern "C" double* hype_ctcs_level_device(hype_ctcs* c, int which) {
     if (!c) return nullptr;
-    return which == 0 ? c->lv[c->cur] : c->lv[(c->cur + 2) % 3];
+    return which == 0 ? c->newest() : c->older();
 }
 
 extern "C" int hype_ctcs_sync(hype_ctcs* c) {
@@ -287,11 +398,16 @@ static double ricker(double t, double f0) {
 
 static const int kChunk = 30;  // steps per captured graph (a multiple of the 3-level rotation)
 
+static const int kPlaneChunk = 8;  // launches per captured graph of the plane-wave form (an even number)
+
 static int build_chunk(hype_ctcs* c, int phase) {
     cudaGraph_t graph;
     HYPE_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int rc = HYPE_OK;
-    for (int s = 0; s < kChunk && rc == HYPE_OK; ++s) rc = ctcs_launch(c, (phase + s) % 3);
+    if (c->p.form == 0)
+        for (int s = 0; s < kPlaneChunk && rc == HYPE_OK; ++s) rc = plane_launch(c, (phase + s) % 2, kSteps);
+    else
+        for (int s = 0; s < kChunk && rc == HYPE_OK; ++s) rc = ctcs_launch(c, (phase + s) % 3);
     cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
     if (rc) return rc;
     if (e != cudaSuccess) {
@@ -338,6 +454,18 @@ extern "C" int hype_ctcs_step(hype_ctcs* c, int nsteps, int it0, double* receive
     }
     int s = 0;
     int rc;
+    if (c->p.form == 0) {
+        for (; nsteps - s >= kPlaneChunk * kSteps; s += kPlaneChunk * kSteps) {
+            if (!c->chunk[c->pair] && (rc = build_chunk(c, c->pair))) return rc;
+            HYPE_CK(cudaGraphLaunch(c->chunk[c->pair], c->stream));
+            count_launch(kPlaneChunk);
+        }
+        for (; s < nsteps; s += kSteps) {
+            if ((rc = plane_launch(c, c->pair, nsteps - s < kSteps ? nsteps - s : kSteps))) return rc;
+            c->pair ^= 1;
+        }
+        return HYPE_OK;
+    }
     // whole chunks replay a captured graph; the remainder launches directly
     while (nsteps - s >= kChunk) {
         const int phase = c->cur;

@@ -112,3 +112,23 @@ def test_line_source_2d_program_matches_greens_function(hype):
     misfit = analytic.relative_l2_misfit(rec, analytic.line_source_receiver_2d(t, 80 * np.sqrt(2.0), 580.0, 65.0))
     print(f"CTCS line source 500^2: receiver misfit {misfit:.3e}")
     assert misfit < 0.03
+
+
+@pytest.mark.parametrize("bc", [0, 3])
+@pytest.mark.parametrize("shape", [(3, 3), (5, 17), (33, 64), (65, 130), (200, 31)], ids=str)
+@pytest.mark.parametrize("steps", [1, 3, 4, 6, 35])
+def test_plane_form_tiles_bitwise(hype, oracle, shape, bc, steps):
+    """steps fused in a launch: grids smaller than a tile's frame, ragged tiles, remainders of the fused count, and
+    zeros and subnormal numbers (whose doubling leaves the exponent path), against the checker bit for bit"""
+    rng = np.random.default_rng(shape[0] + steps)
+    p0 = rng.standard_normal(shape)
+    p1 = 0.99 * p0
+    p0[:, : shape[1] // 2] = p1[:, : shape[1] // 2] = 0.0
+    p0[0, 0], p1[0, 0] = 3e-310, 5e-324
+    h, dt = 0.1, 0.04
+    lf = hype.Leapfrog(p0.shape, dx=h, dt=dt, c0=1.0, form=0, bc=bc)
+    lf.set(p0, p1)
+    lf.UpdatePressure(steps)
+    a, b = lf.get()
+    ao, bo = oracle.ctcs2d_plane(p0, p1, 1.0 * dt / h, bc, steps)
+    assert np.array_equal(a, ao) and np.array_equal(b, bo)
