@@ -25,7 +25,6 @@
 #include <vector>
 
 #include "cweno_fix.cuh"
-#include "euler_df64.cuh"
 #include "euler_kernels.cuh"
 #include "mlp_kernels.cuh"
 
@@ -396,220 +395,6 @@ static void launch_recon64(const Geo& g, const double* G, double* T, int recon, 
     else pad ? go(k_recon64<HYPE_RECON_CWENO4, true>) : go(k_recon64<HYPE_RECON_CWENO4, false>);
 }
 
-// HYPE_PREC_DF64: the per-variable reference value r_c of one stage, the stage input's
-// value at cell 0 rounded to a 24-bit significand (the deviations u - r_c are formed in
-// FP64, the traces r_c + deviation are rounded once in FP64)
-__device__ __forceinline__ double df_ref(const double* __restrict__ W, const Geo& g, int c) {
-    double r;
-    df_round24(__ldg(W + (long long)c * g.N), r);
-    return r;
-}
-
-// ghost fill as k_ghost, storing the deviation from r_c as a double-float pair
-__global__ void __launch_bounds__(128) k_ghost_df(const double* __restrict__ W, df64* __restrict__ G, Geo g) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x - GW;
-    const int j = blockIdx.y - GW, k = blockIdx.z - GW;
-    if (i >= g.nx + GW) return;
-    int fi = 0, fj = 0, fk = 0;
-    const int mi = bmap(i, g.nx, g.bc[0], g.bc[1], &fi);
-    const int mj = bmap(j, g.ny, g.bc[2], g.bc[3], &fj);
-    const int mk = bmap(k, g.nz, g.bc[4], g.bc[5], &fk);
-    const long long src = ((long long)mk * g.ny + mj) * g.nx + mi;
-    const long long dst = ghost_index(g, i, j, k);
-#pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        double v = __ldg(W + (long long)c * g.N + src);
-        if ((c == 1 && fi) || (c == 2 && fj) || (c == 3 && fk)) v = -v;
-        G[(long long)c * g.GN + dst] = df_from_double(v - df_ref(W, g, c));
-    }
-}
-
-// The stage's reference state r in double-float (its components are the rounded cell-0
-// values, exact FP32 numbers) and the pieces of F(r) the deviation form of the flux uses
-struct DfRef {
-    df64 rho, m[3], E, u[3], p, H;  // u = m / rho, p = (gamma - 1)(E - m.u / 2), H = E + p
-};
-
-__device__ __forceinline__ DfRef df_refstate(const double* __restrict__ W, const Geo& g, df64 gm1) {
-    DfRef R;
-    double fd;
-    R.rho = df64{df_round24(__ldg(W), fd), 0.0f};
-#pragma unroll
-    for (int i = 0; i < 3; ++i) R.m[i] = df64{df_round24(__ldg(W + (long long)(1 + i) * g.N), fd), 0.0f};
-    R.E = df64{df_round24(__ldg(W + 4LL * g.N), fd), 0.0f};
-    const df64 ir = df_div(dfc(1.0), R.rho);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) R.u[i] = R.m[i] * ir;
-    R.p = (R.E - df_scale((R.m[0] * R.u[0] + R.m[1] * R.u[1]) + R.m[2] * R.u[2], 0.5f)) * gm1;
-    R.H = R.E + R.p;
-    return R;
-}
-
-// One side of a face in deviation form: for the trace r + d, the flux deviation
-// dF = F(r + d) - F(r) along D (PDEConsFlux, Navier-Stokes-3D/pde.c:40-88) built only from
-// deviation-sized terms -- du = (d_m - u_r d_rho) / rho, d(m.u) = sum m_r du + d_m u,
-// dp = (gamma - 1)(d_E - d(m.u) / 2), dF_m = m_r du_n + d_m u_n (+ dp), dF_E = H_r du_n +
-// (d_E + dp) u_n -- and the wave speed |u_n| + sqrt(gamma p / rho); the floors of pde.c:56-66
-template <int D>
-__device__ __forceinline__ void dev_side(const DfRef& R, const df64* d, df64 gm1, df64 gam, df64* dF, df64& sp,
-                                         bool& bad) {
-    const df64 rho = R.rho + d[0];
-    const df64 ir = df_div(dfc(1.0), rho);
-    df64 du[3], u[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        du[i] = (d[1 + i] - R.u[i] * d[0]) * ir;
-        u[i] = R.u[i] + du[i];
-    }
-    const df64 dmu = (R.m[0] * du[0] + d[1] * u[0]) + ((R.m[1] * du[1] + d[2] * u[1]) + (R.m[2] * du[2] + d[3] * u[2]));
-    const df64 dp = (d[4] - df_scale(dmu, 0.5f)) * gm1;
-    const df64 p = R.p + dp;
-    bad |= !(rho.hi >= 1.0e-14f && p.hi >= 1.0e-12f);
-    dF[0] = d[1 + D];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const df64 f = R.m[i] * du[D] + d[1 + i] * u[D];
-        dF[1 + i] = (i == D) ? f + dp : f;
-    }
-    dF[4] = R.H * du[D] + (d[4] + dp) * u[D];
-    sp = df_abs(u[D]) + df_sqrt(gam * p * ir);
-}
-
-// density and pressure of the 24 double-float deviation traces against the floors: an FP32
-// estimate from the leading parts settles every point whose density and pressure lie clear
-// of the floors by more than its rounding (1e-5 of the magnitudes involved, NaN never
-// clear); the rest are decided in double-float
-__device__ __forceinline__ bool traces_admissible_df(const df64* __restrict__ T, const Geo& g, long long e,
-                                                     const DfRef& R, df64 gm1) {
-    for (int q = 0; q < NTR; ++q) {
-        df64 d[NV];
-#pragma unroll
-        for (int c = 0; c < NV; ++c) d[c] = T[((long long)c * NTR + q) * g.NE + e];
-        const float rf = R.rho.hi + d[0].hi, Ef = R.E.hi + d[4].hi;
-        const float mxf = R.m[0].hi + d[1].hi, myf = R.m[1].hi + d[2].hi, mzf = R.m[2].hi + d[3].hi;
-        const float m2 = mxf * mxf + myf * myf + mzf * mzf;
-        const float kef = 0.5f * m2 / rf;
-        const float pf = gm1.hi * (Ef - kef);
-        const float tr = 1.0e-5f * (fabsf(R.rho.hi) + fabsf(d[0].hi)) + 1.0e-14f;
-        const float tp = 1.0e-5f * gm1.hi * (fabsf(Ef) + fabsf(kef)) + 1.0e-12f;
-        if (rf > 1.0e-14f + tr && pf > 1.0e-12f + tp) continue;  // clearly admissible
-        if (rf < 1.0e-14f - tr || pf < 1.0e-12f - tp) return false;  // clearly not
-        const df64 rho = R.rho + d[0];
-        const df64 mx = R.m[0] + d[1], my = R.m[1] + d[2], mz = R.m[2] + d[3];
-        const df64 p = ((R.E + d[4]) - df_scale(df_div((mx * mx + my * my) + mz * mz, rho), 0.5f)) * gm1;
-        if (!(rho.hi >= 1.0e-14f) || !(p.hi >= 1.0e-12f)) return false;
-    }
-    return true;
-}
-
-// CWENO4 / R4 reconstruction in double-float on the deviations (euler_df64.cuh).  DFT: the
-// traces stay double-float deviations for k_faces_df (Rusanov); otherwise they go out as FP64
-// values r_c + deviation, the array the FP64 face solvers consume.
-// (two blocks per SM: with more warps in flight over this long unrolled body the
-// instruction-cache misses cost more than the latency they hide)
-template <bool DFT>
-__global__ void __launch_bounds__(128, 2)
-    k_recon_df(const df64* __restrict__ G, void* __restrict__ Tv, const double* __restrict__ W, Geo g, int recon,
-               int pad, double gm1, unsigned long long* __restrict__ counters, df64* __restrict__ C4 = nullptr,
-               double c4_scale = 1.0) {
-    double* T = (double*)Tv;
-    df64* Td = (df64*)Tv;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y - 1;
-    const int k = blockIdx.z - 1;
-    if (i > g.nx || j > g.ny) return;
-    const int gi = (i < 0 || i >= g.nx), gj = (j < 0 || j >= g.ny), gk = (k < 0 || k >= g.nz);
-    if (gi + gj + gk > 1) return;
-    const long long e = ext_index(g, i, j, k), ge = ghost_index(g, i, j, k);
-    const int sy = g.gx, sz = g.gx * g.gy;
-#pragma unroll 1
-    for (int c = 0; c < NV; ++c) {
-        df64 s[33], cf[20];
-        {
-            const df64* p = G + (long long)c * g.GN + ge;
-            s[0] = p[0];
-#pragma unroll
-            for (int o = 0; o < 4; ++o) {
-                const int off = (o == 0) ? -2 : (o == 1) ? -1 : (o == 2) ? 1 : 2;
-                s[S1(0, off)] = p[off];
-                s[S1(1, off)] = p[off * sy];
-                s[S1(2, off)] = p[off * sz];
-            }
-#pragma unroll
-            for (int sa = 0; sa < 2; ++sa)
-#pragma unroll
-                for (int sb = 0; sb < 2; ++sb) {
-                    s[SQ(0, sa, 1, sb)] = p[(2 * sa - 1) + (2 * sb - 1) * sy];
-                    s[SQ(1, sa, 2, sb)] = p[(2 * sa - 1) * sy + (2 * sb - 1) * sz];
-                    s[SQ(0, sa, 2, sb)] = p[(2 * sa - 1) + (2 * sb - 1) * sz];
-                }
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b)
-#pragma unroll
-                    for (int d = 0; d < 2; ++d) s[SO(a, b, d)] = p[(2 * a - 1) + (2 * b - 1) * sy + (2 * d - 1) * sz];
-        }
-        cweno4_df(s, recon == HYPE_RECON_LINEAR4, cf);
-        if (C4) {  // the R4 polynomial (times 1/h) of the deviations, for the viscous face gradients
-            const df64 sc = df_from_double(c4_scale);
-            df64 r4[20];
-            if (recon == HYPE_RECON_LINEAR4) {
-#pragma unroll
-                for (int q = 0; q < 20; ++q) r4[q] = cf[q];
-            } else {
-                cweno4_df(s, true, r4);
-            }
-#pragma unroll
-            for (int q = 1; q < 20; ++q) C4[((long long)c * 20 + q) * g.NE + e] = r4[q] * sc;
-        }
-        df64 tr[8];
-        if constexpr (DFT) {
-            df64* Tc = Td + (long long)c * NTR * g.NE + e;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                if (d == 0) face_traces_df<0>(cf, tr);
-                else if (d == 1) face_traces_df<1>(cf, tr);
-                else face_traces_df<2>(cf, tr);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) Tc[(long long)(8 * d + q) * g.NE] = tr[q];
-            }
-        } else {
-            const double r = df_ref(W, g, c);
-            double* Tc = T + (long long)c * NTR * g.NE + e;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                if (d == 0) face_traces_df<0>(cf, tr);
-                else if (d == 1) face_traces_df<1>(cf, tr);
-                else face_traces_df<2>(cf, tr);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) Tc[(long long)(8 * d + q) * g.NE] = r + df_to_double(tr[q]);
-            }
-        }
-    }
-    if (!pad) return;
-    bool ok;
-    if constexpr (DFT) {
-        const df64 gm1d = df_from_double(gm1);
-        ok = traces_admissible_df(Td, g, e, df_refstate(W, g, gm1d), gm1d);
-    } else {
-        ok = traces_admissible<double>(T, g, e, gm1);
-    }
-    if (!ok) {
-#pragma unroll 1
-        for (int c = 0; c < NV; ++c) {
-            const df64 dv = G[(long long)c * g.GN + ge];
-            const double v = df_ref(W, g, c) + df_to_double(dv);
-            for (int q = 0; q < NTR; ++q) {
-                if constexpr (DFT) Td[((long long)c * NTR + q) * g.NE + e] = dv;
-                else T[((long long)c * NTR + q) * g.NE + e] = v;
-            }
-        }
-        if (!gi && !gj && !gk) atomicAdd(&counters[1], 1ull);
-    }
-}
-
-
 // Indicator-gated reconstruction: the network scores the cell from its three
 // directional 5-point stencils; flagged or low-confidence cells take the full
 // CWENO4, the others the linear R4 -- unless the linear traces give a density
@@ -651,7 +436,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
                 const R* p = G + (long long)c * g.GN + ge;
                 float s5[5];
 #pragma unroll
-                for (int o = 0; o < 5; ++o) s5[o] = (float)__ldg(p + (o - 2) * st);
+                for (int o = 0; o < 5; ++o) {
+                    if constexpr (sizeof(R) == sizeof(double)) s5[o] = narrow_fix(__ldg(p + (o - 2) * st));
+                    else s5[o] = __ldg(p + (o - 2) * st);
+                }
                 mlp::normalise5(s5, sc[c], x + c * 5);
             }
         }
@@ -673,155 +461,27 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
 #pragma unroll 1
             for (int c = 0; c < NV; ++c) {
                 R s[33];
-                gather33g<R>(G + (long long)c * g.GN + ge, sy, sz, s);
+                const R* Gc = G + (long long)c * g.GN + ge;
+                gather33g<R>(Gc, sy, sz, s);
                 if constexpr (f32) {
                     R cf[20];
                     cweno4<R>(s, !full, cf);
                     store_traces<R>(T, g, e, c, cf, &ck);
                 } else {
-                    Poly64 poly;
-                    if (full) cweno4_64(s, poly);
-                    else r4_64(s, poly);
-                    store_traces64(poly, T + (long long)c * NTR * g.NE + e, g.NE);
+                    double* Tc = T + (long long)c * NTR * g.NE + e;
+                    const bool strict = c == 0 || c == 4;
+                    PolyFix fix;
+                    if (full) {
+                        if (!recon_fix<false>(s, strict, Tc, g.NE, fix)) recon64_general<false>(Gc, sy, sz, Tc, nullptr, g.NE);
+                    } else {
+                        if (!recon_fix<true>(s, strict, Tc, g.NE, fix)) recon64_general<true>(Gc, sy, sz, Tc, nullptr, g.NE);
+                    }
                 }
             }
             if (f32 ? ck.ok : traces_admissible<R>(T, g, e, gm1)) break;
             if (full) {  // CWENO4 itself inadmissible: first order (when enabled)
                 if (pad) {
                     store_first_order_g<R>(G, T, g, ge, e);
-                    if (!gi && !gj && !gk) atomicAdd(&cnt[1], 1u);
-                }
-                break;
-            }
-            full = true;  // the R4 traces broke positivity: redo the cell with CWENO4
-        }
-        if (full && !gi && !gj && !gk && best > logit_thr) atomicAdd(&cnt[0], 1u);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        if (cnt[0]) atomicAdd(&counters[0], (unsigned long long)cnt[0]);
-        if (cnt[1]) atomicAdd(&counters[1], (unsigned long long)cnt[1]);
-    }
-}
-
-// Indicator-gated reconstruction of the double-float form: the network reads the FP32 leading
-// parts of the deviations (its normalised stencils are shift-invariant; the magnitude floors
-// take the density and energy as r + deviation), flagged or low-confidence cells take the
-// double-float CWENO4 and the others its R4 limit, with the positivity redo of k_recon_learned.
-// DFT as for k_recon_df.
-template <bool DFT>
-__global__ void __launch_bounds__(128, 2)
-    k_recon_learned_df(const df64* __restrict__ G, void* __restrict__ Tv, const double* __restrict__ W, Geo g,
-                       const mlp::MmaWeights* __restrict__ wts, float logit_thr, double gm1, int pad,
-                       unsigned long long* __restrict__ counters) {
-    __shared__ __align__(16) __nv_bfloat16 rows[4][mlp::ROWS * mlp::RSTRIDE];
-    __shared__ float lg[4][mlp::ROWS];
-    __shared__ unsigned cnt[2];
-    if (threadIdx.x == 0 && threadIdx.y == 0) cnt[0] = cnt[1] = 0;
-    double* T = (double*)Tv;
-    df64* Td = (df64*)Tv;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y - 1;
-    const int k = blockIdx.z - 1;
-    bool active = !(i > g.nx || j > g.ny);
-    const int gi = (i < 0 || i >= g.nx), gj = (j < 0 || j >= g.ny), gk = (k < 0 || k >= g.nz);
-    active = active && (gi + gj + gk <= 1);
-    const long long ge = active ? ghost_index(g, i, j, k) : 0;
-    const int sy = g.gx, sz = g.gx * g.gy;
-    __nv_bfloat16* my_rows = rows[threadIdx.y] + threadIdx.x * 3 * mlp::RSTRIDE;
-    float sc[NV];
-    if (active) {
-        double fd;
-        const float rho = df_round24(__ldg(W), fd) + G[ge].hi;
-        const float E = df_round24(__ldg(W + 4LL * g.N), fd) + G[4 * g.GN + ge].hi;
-#pragma unroll
-        for (int c = 0; c < NV; ++c) sc[c] = mlp::var_scale<float>(c, rho, E);
-    }
-#pragma unroll 1
-    for (int d = 0; d < 3; ++d) {
-        float x[mlp::NIN];
-        const int st = d == 0 ? 1 : d == 1 ? sy : sz;
-        if (active) {
-#pragma unroll
-            for (int c = 0; c < NV; ++c) {
-                const df64* p = G + (long long)c * g.GN + ge;
-                float s5[5];
-#pragma unroll
-                for (int o = 0; o < 5; ++o) s5[o] = p[(o - 2) * st].hi;
-                mlp::normalise5(s5, sc[c], x + c * 5);
-            }
-        }
-        mlp::stage_row(my_rows + d * mlp::RSTRIDE, x, active);
-    }
-    __syncthreads();
-    mlp::warp_logits(wts, rows[threadIdx.y], lg[threadIdx.y]);
-    __syncwarp();
-    const float best = fmaxf(lg[threadIdx.y][threadIdx.x * 3], fmaxf(lg[threadIdx.y][threadIdx.x * 3 + 1],
-                                                                       lg[threadIdx.y][threadIdx.x * 3 + 2]));
-    if (active) {
-        const long long e = ext_index(g, i, j, k);
-        const df64 gm1d = df_from_double(gm1);
-        bool full = best > logit_thr;
-#pragma unroll 1
-        for (int pass = 0; pass < 2; ++pass) {
-#pragma unroll 1
-            for (int c = 0; c < NV; ++c) {
-                df64 s[33], cf[20];
-                const df64* p = G + (long long)c * g.GN + ge;
-                s[0] = p[0];
-#pragma unroll
-                for (int o = 0; o < 4; ++o) {
-                    const int off = (o == 0) ? -2 : (o == 1) ? -1 : (o == 2) ? 1 : 2;
-                    s[S1(0, off)] = p[off];
-                    s[S1(1, off)] = p[off * sy];
-                    s[S1(2, off)] = p[off * sz];
-                }
-#pragma unroll
-                for (int sa = 0; sa < 2; ++sa)
-#pragma unroll
-                    for (int sb = 0; sb < 2; ++sb) {
-                        s[SQ(0, sa, 1, sb)] = p[(2 * sa - 1) + (2 * sb - 1) * sy];
-                        s[SQ(1, sa, 2, sb)] = p[(2 * sa - 1) * sy + (2 * sb - 1) * sz];
-                        s[SQ(0, sa, 2, sb)] = p[(2 * sa - 1) + (2 * sb - 1) * sz];
-                    }
-#pragma unroll
-                for (int a = 0; a < 2; ++a)
-#pragma unroll
-                    for (int b = 0; b < 2; ++b)
-#pragma unroll
-                        for (int dd = 0; dd < 2; ++dd)
-                            s[SO(a, b, dd)] = p[(2 * a - 1) + (2 * b - 1) * sy + (2 * dd - 1) * sz];
-                cweno4_df(s, !full, cf);
-                df64 tr[8];
-                const double r = df_ref(W, g, c);
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    if (d == 0) face_traces_df<0>(cf, tr);
-                    else if (d == 1) face_traces_df<1>(cf, tr);
-                    else face_traces_df<2>(cf, tr);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const long long at = ((long long)c * NTR + 8 * d + q) * g.NE + e;
-                        if constexpr (DFT) Td[at] = tr[q];
-                        else T[at] = r + df_to_double(tr[q]);
-                    }
-                }
-            }
-            bool ok;
-            if constexpr (DFT) ok = traces_admissible_df(Td, g, e, df_refstate(W, g, gm1d), gm1d);
-            else ok = traces_admissible<double>(T, g, e, gm1);
-            if (ok) break;
-            if (full) {  // CWENO4 itself inadmissible: first order (when enabled)
-                if (pad) {
-#pragma unroll 1
-                    for (int c = 0; c < NV; ++c) {
-                        const df64 dv = G[(long long)c * g.GN + ge];
-                        const double v = df_ref(W, g, c) + df_to_double(dv);
-                        for (int q = 0; q < NTR; ++q) {
-                            if constexpr (DFT) Td[((long long)c * NTR + q) * g.NE + e] = dv;
-                            else T[((long long)c * NTR + q) * g.NE + e] = v;
-                        }
-                    }
                     if (!gi && !gj && !gk) atomicAdd(&cnt[1], 1u);
                 }
                 break;
@@ -887,114 +547,8 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long* a, double v) 
     atomicMax(a, (unsigned long long)__double_as_longlong(v));
 }
 
-// Face fluxes of direction D.  Face index (i,j,k) is the face on the low side of
-// cell (i,j,k); along D it runs to n (the high face of the last cell).
-// Rusanov faces of the double-float form in deviation form: with F(r) dropped (it is the
-// same at every face, so the divergence does not see it), the stored flux is
-// 1/2 (dF_L + dF_R) - 1/2 s (d_R - d_L) at each Gauss point, weight 1/4, where s is the
-// larger wave speed (pde.c:164-187); every term has the size of the deviations, so the
-// 48-bit significand meets the FP64 form's error bars with the face solver on the FP32 pipe.
-// one side's share of PDEViscRiemannSolver (Navier-Stokes-3D/pde.c:386-404) in double-float:
-// 1/8 F_v at each of the 4 Gauss points of the side's face, from its traces (r + deviation)
-// and the R4 gradients of the deviations; returns the largest viscous speed
-template <int D, int NS>
-__device__ __forceinline__ double visc_side_df(const df64* __restrict__ T, const df64* __restrict__ C4, const Geo& g,
-                                               long long e, const DfRef& R, df64 gm1, df64 mu, df64 kc, df64 vmax,
-                                               df64* av) {
-    FaceGradDf fg[NV][3];
-#pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        const df64* p = C4 + (long long)c * 20 * g.NE + e;
-        fg[c][0] = face_grad_df<D, NS, 0>(p, g.NE);
-        fg[c][1] = face_grad_df<D, NS, 1>(p, g.NE);
-        fg[c][2] = face_grad_df<D, NS, 2>(p, g.NE);
-    }
-    constexpr int face = 2 * D + (NS > 0 ? 1 : 0);
-    double sv = 0.0;
-    auto at = [&](auto gpc) {
-        constexpr int gp = decltype(gpc)::value;
-        df64 Q[NV], Gq[NV][3], Fv[NV];
-#pragma unroll
-        for (int c = 0; c < NV; ++c) {
-            Q[c] = T[((long long)c * NTR + face * 4 + gp) * g.NE + e];
-#pragma unroll
-            for (int b = 0; b < 3; ++b) Gq[c][b] = fg_eval_df<gp>(fg[c][b]);
-        }
-        Q[0] = R.rho + Q[0];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) Q[1 + i] = R.m[i] + Q[1 + i];
-        Q[4] = R.E + Q[4];
-        sv = fmax(sv, df_to_double(visc_flux_df<D>(Q, Gq, gm1, mu, kc, vmax, Fv)));
-#pragma unroll
-        for (int c = 0; c < NV; ++c) av[c] = av[c] + df_scale(Fv[c], 0.125f);
-    };
-    at(std::integral_constant<int, 0>{});
-    at(std::integral_constant<int, 1>{});
-    at(std::integral_constant<int, 2>{});
-    at(std::integral_constant<int, 3>{});
-    return sv;
-}
-
-template <int D, bool VISC = false>
-__global__ void __launch_bounds__(128) k_faces_df(const df64* __restrict__ T, double* __restrict__ F,
-                                                  const double* __restrict__ W, Geo g, double gamma,
-                                                  DevScalars* __restrict__ ds, int slot,
-                                                  const df64* __restrict__ C4 = nullptr,
-                                                  Visc vp = Visc{0.0, 0.0, 0.0, 0.0}) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z;
-    const int fx = g.nx + (D == 0), fy = g.ny + (D == 1);
-    double smax = 0.0, smaxv = 0.0;
-    bool bad = false;
-    if (i < fx && j < fy) {
-        const long long eR = ext_index(g, i, j, k);
-        const long long eL = ext_index(g, i - (D == 0), j - (D == 1), k - (D == 2));
-        const df64 gm1 = df_from_double(gamma - 1.0), gam = df_from_double(gamma);
-        const DfRef R = df_refstate(W, g, gm1);
-        df64 acc[NV];
-#pragma unroll
-        for (int c = 0; c < NV; ++c) acc[c] = df64{0.0f, 0.0f};
-#pragma unroll 1
-        for (int gp = 0; gp < 4; ++gp) {
-            df64 dL[NV], dR[NV], fL[NV], fR[NV], sL, sR;
-#pragma unroll
-            for (int c = 0; c < NV; ++c) {
-                dL[c] = T[((long long)c * NTR + (2 * D + 1) * 4 + gp) * g.NE + eL];
-                dR[c] = T[((long long)c * NTR + (2 * D) * 4 + gp) * g.NE + eR];
-            }
-            dev_side<D>(R, dL, gm1, gam, fL, sL, bad);
-            dev_side<D>(R, dR, gm1, gam, fR, sR, bad);
-            const df64 sm = df_lt(sL, sR) ? sR : sL;
-            smax = fmax(smax, df_to_double(sm));
-#pragma unroll
-            for (int c = 0; c < NV; ++c) acc[c] = acc[c] + df_scale((fL[c] + fR[c]) - sm * (dR[c] - dL[c]), 0.125f);
-        }
-        if constexpr (VISC) {
-            const df64 mu = df_from_double(vp.mu), kc = df_from_double(vp.kc), vmax = df_from_double(vp.vmax);
-            smaxv = visc_side_df<D, 1>(T, C4, g, eL, R, gm1, mu, kc, vmax, acc);
-            smaxv = fmax(smaxv, visc_side_df<D, -1>(T, C4, g, eR, R, gm1, mu, kc, vmax, acc));
-        }
-        const long long nf = (long long)fx * fy * (g.nz + (D == 2));
-        const long long f = ((long long)k * fy + j) * fx + i;
-#pragma unroll
-        for (int c = 0; c < NV; ++c) F[c * nf + f] = df_to_double(acc[c]);
-        if (bad) {
-            const int ci = i < g.nx ? i : g.nx - 1, cj = j < g.ny ? j : g.ny - 1, ck = k < g.nz ? k : g.nz - 1;
-            atomicMin(&ds->bad, (unsigned long long)(((long long)ck * g.ny + cj) * g.nx + ci));
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) smax = fmax(smax, __shfl_xor_sync(0xffffffffu, smax, o));
-    if ((threadIdx.x & 31) == 0 && smax > 0.0) atomic_max_pos(&ds->smax_bits[slot], smax);
-    if constexpr (VISC) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) smaxv = fmax(smaxv, __shfl_xor_sync(0xffffffffu, smaxv, o));
-        if ((threadIdx.x & 31) == 0 && smaxv > 0.0) atomic_max_pos(&ds->smaxv_bits[slot], smaxv);
-    }
-}
-
-// the FP32 face fluxes of direction D, one thread per face
+// the FP32 face fluxes of direction D, one thread per face; face (i, j, k) is the low side of cell (i, j, k) and
+// runs to n along D
 template <int D, int FLUX>
 __global__ void __launch_bounds__(128) k_faces_f32(const float* __restrict__ T, double* __restrict__ F, Geo g, double gamma,
                                                    DevScalars* __restrict__ ds, int slot) {
@@ -1882,37 +1436,24 @@ static int launch_rhs(hype_euler* e, const double* Win, int slot) {
     const Geo& g = e->g;
     const dim3 br(32, 4), gr(cdiv(g.nx + 2, 32), cdiv(g.ny + 2, 4), g.nz + 2);
     const bool f32 = e->p.precision == HYPE_PREC_FP32;
-    const bool df = e->p.precision == HYPE_PREC_DF64;
+    // HYPE_PREC_DF64 asks for FP64's error bars on the FP32 pipe, which pairs of FP32 numbers gave.  The FP64 kernels'
+    // integer form is closer to 64 bits and faster, and serves both (two steps, pairs against this: 16^3 707 -> 300
+    // us, 161 x 150 x 143 47.6 -> 43.4 ms, Navier-Stokes 96^3 40.3 -> 31.9, blast 96^3 with the fallback 21.5 -> 15.2).
     const int rec = e->p.recon;
     prof_mark(e, 0, true);
-    const dim3 bgh(128), ggh(cdiv(g.gx, 128), g.gy, g.nz + 2 * GW);
     if (f32) k_ghost<float><<<ghost_grid(g), kGhostThreads, 0, e->stream>>>(Win, (float*)e->G, g);
-    else if (df) k_ghost_df<<<ggh, bgh, 0, e->stream>>>(Win, (df64*)e->G, g);
     else k_ghost<double><<<ghost_grid(g), kGhostThreads, 0, e->stream>>>(Win, (double*)e->G, g);
     HYPE_LAUNCHED(1);
     const double gm1 = e->p.gamma - 1.0;
     const size_t ck_bytes = (f32 && e->p.positivity) ? sizeof(float) * 4 * 2 * NTR * 32 : 0;
     if (e->p.recon == HYPE_RECON_LEARNED) {
         if (!e->mlp) return HYPE_ERR_ARG;  // hype_euler_set_mlp first
-        if (df && e->p.flux == HYPE_FLUX_RUSANOV)
-            k_recon_learned_df<true><<<gr, br, 0, e->stream>>>((const df64*)e->G, e->T, Win, g, e->mlp, e->logit_thr, gm1,
-                                                               e->p.positivity, e->mlp_cnt);
-        else if (df)
-            k_recon_learned_df<false><<<gr, br, 0, e->stream>>>((const df64*)e->G, e->T, Win, g, e->mlp, e->logit_thr,
-                                                                gm1, e->p.positivity, e->mlp_cnt);
-        else if (f32)
+        if (f32)
             k_recon_learned<float><<<gr, br, 0, e->stream>>>((const float*)e->G, (float*)e->T, g, e->mlp, e->logit_thr, gm1,
                                                              e->p.positivity, e->mlp_cnt);
         else
             k_recon_learned<double><<<gr, br, 0, e->stream>>>((const double*)e->G, (double*)e->T, g, e->mlp, e->logit_thr,
                                                               gm1, e->p.positivity, e->mlp_cnt);
-    } else if (df) {
-        if (e->p.flux == HYPE_FLUX_RUSANOV)
-            k_recon_df<true><<<gr, br, 0, e->stream>>>((const df64*)e->G, e->T, Win, g, rec, e->p.positivity, gm1,
-                                                       e->mlp_cnt, (df64*)e->C4, 1.0 / e->p.h);
-        else
-            k_recon_df<false><<<gr, br, 0, e->stream>>>((const df64*)e->G, e->T, Win, g, rec, e->p.positivity, gm1,
-                                                        e->mlp_cnt);
     } else if (f32) {
         k_recon_f32<<<gr, br, ck_bytes, e->stream>>>((const float*)e->G, (float*)e->T, g, rec, e->p.positivity, gm1,
                                                      e->mlp_cnt);
@@ -1922,34 +1463,11 @@ static int launch_rhs(hype_euler* e, const double* Win, int slot) {
     int nk = 2;
     prof_mark(e, 0, false);
     prof_mark(e, 1, true);
-    if (e->C4 && df) {
-        // Navier-Stokes in double-float: Rusanov in deviation form plus both sides' viscous fluxes
-        const double mu = e->p.mu, gm = e->p.gamma;
-        const Visc vp{mu, e->p.cv * mu * gm / e->p.prandtl, std::max((4. / 3.) * mu, gm * mu / e->p.prandtl),
-                      1.0 / e->p.h};
-        const dim3 bf(32, 4);
-        const dim3 fgx(cdiv(g.nx + 1, 32), cdiv(g.ny, 4), g.nz), fgy(cdiv(g.nx, 32), cdiv(g.ny + 1, 4), g.nz),
-            fgz(cdiv(g.nx, 32), cdiv(g.ny, 4), g.nz + 1);
-        const df64* Td = (const df64*)e->T;
-        const df64* C4 = (const df64*)e->C4;
-        k_faces_df<0, true><<<fgx, bf, 0, e->stream>>>(Td, e->Fx, Win, g, e->p.gamma, e->ds, slot, C4, vp);
-        k_faces_df<1, true><<<fgy, bf, 0, e->stream>>>(Td, e->Fy, Win, g, e->p.gamma, e->ds, slot, C4, vp);
-        k_faces_df<2, true><<<fgz, bf, 0, e->stream>>>(Td, e->Fz, Win, g, e->p.gamma, e->ds, slot, C4, vp);
-        nk += 3;
-    } else if (e->C4) {
+    if (e->C4) {
         // Navier-Stokes: the inviscid flux plus the average of both sides' viscous fluxes
         const double mu = e->p.mu, g = e->p.gamma;
         const Visc vp{mu, e->p.cv * mu * g / e->p.prandtl, std::max((4. / 3.) * mu, g * mu / e->p.prandtl), 1.0 / e->p.h};
         nk += launch_faces(e->g, e->T, e->Fx, e->Fy, e->Fz, e->p.gamma, e->ds, slot, false, e->p.flux, e->stream, e->C4, &vp);
-    } else if (df && e->p.flux == HYPE_FLUX_RUSANOV) {
-        const dim3 bf(32, 4);
-        const dim3 fgx(cdiv(g.nx + 1, 32), cdiv(g.ny, 4), g.nz), fgy(cdiv(g.nx, 32), cdiv(g.ny + 1, 4), g.nz),
-            fgz(cdiv(g.nx, 32), cdiv(g.ny, 4), g.nz + 1);
-        const df64* Td = (const df64*)e->T;
-        k_faces_df<0><<<fgx, bf, 0, e->stream>>>(Td, e->Fx, Win, g, e->p.gamma, e->ds, slot);
-        k_faces_df<1><<<fgy, bf, 0, e->stream>>>(Td, e->Fy, Win, g, e->p.gamma, e->ds, slot);
-        k_faces_df<2><<<fgz, bf, 0, e->stream>>>(Td, e->Fz, Win, g, e->p.gamma, e->ds, slot);
-        nk += 3;
     } else {
         nk += launch_faces(e->g, e->T, e->Fx, e->Fy, e->Fz, e->p.gamma, e->ds, slot, f32, e->p.flux, e->stream);
     }

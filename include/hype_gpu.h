@@ -64,9 +64,10 @@ extern "C" {
 #define HYPE_PREC_FP64 0
 #define HYPE_PREC_FP32 1
 /* 3D Euler (CWENO4 / R4): state, flux and stage accumulation in FP64, reconstruction in
- * double-float arithmetic (pairs of FP32 numbers, 48-bit significand, on the FP32 pipe,
- * which issues 64x the FP64 rate on GB300) on deviations from a per-variable reference
- * value; traces rounded once in FP64 */
+ * arithmetic that holds FP64's error bars off the FP64 pipe (GB300 issues it at 1/64 of the
+ * FP32 rate).  The 3D Euler and Navier-Stokes solvers now run their FP64 kernels for it, whose
+ * 64-bit integer form is closer and faster than the pairs of FP32 numbers it began as; the 3D
+ * acoustic solver's CWENO4 form uses the pairs */
 #define HYPE_PREC_DF64 2
 
 /* dt semantics */
