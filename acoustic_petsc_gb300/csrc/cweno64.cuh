@@ -290,12 +290,12 @@ __device__ __forceinline__ void store_grad_coeffs(const Poly64& p, double* __res
     C[19 * st] = __longlong_as_double(top);
 }
 
-// Twice the derivative along axis B (times h) of the R4 polynomial at Gauss point gp = 2 (t1 > 0) + (t2 > 0) of
-// the face x_D = NS/2: the gradient of evaluate_grad (Navier-Stokes-3D/reconstruction.c:24-35) is bilinear
-// there, P + Q t1 + R t2 + S t1 t2, with the squares t1^2 = t2^2 = 1/12 folded in.  On the integer pipe, the
-// conversion included: the 22 forms of a face at its four points were 340 of its 810 FP64 operations.
+// Twice the derivative along axis B (times h) of the R4 polynomial on the face x_D = NS/2, at the 2x2 Gauss points:
+// the gradient of evaluate_grad (Navier-Stokes-3D/reconstruction.c:24-35) is bilinear there,
+// P + Q t1 + R t2 + S t1 t2, with the squares t1^2 = t2^2 = 1/12 and |t1| = |t2| = GPT folded in.  Integers, in the
+// coefficients' units: the 22 forms of a face at its four points were 340 of its 810 FP64 operations.
 template <int D, int NS, int B>
-__device__ __forceinline__ double face_grad64(const double* __restrict__ C, long long st, int gp) {
+__device__ __forceinline__ void face_form64(const double* __restrict__ C, long long st, i64& P, i64& Q, i64& R, i64& S) {
     constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
     constexpr i64 kG2 = 2662558164157085696ll, kG8 = 665639541039271424ll;                // 2^64 times GPT/2 and GPT/8
     constexpr i64 k6 = 3074457345618258603ll, k12 = 1537228672809129301ll, k48 = 384307168202282325ll;  // 1/6, 1/12, 1/48
@@ -306,8 +306,6 @@ __device__ __forceinline__ double face_grad64(const double* __restrict__ C, long
     auto cube = [&](int a) { return ld(9 + a); };
     auto sqlin = [&](int a, int b) { return ld((a < b ? 12 : 13) + 2 * pair_of(a, b)); };  // of x_a^2 x_b
     auto toward = [&](i64 a, i64 b) { return NS > 0 ? a + b : a - b; };
-    const int top = (int)ld(19);
-    i64 P, Q, R, S;
     if constexpr (B == D) {
         P = toward(lin(D), sq(D)) - scaled(cube(D), split(k12));
         Q = scaled(toward(cr2(D, T1), sqlin(D, T1)), split(kG2));
@@ -323,39 +321,40 @@ __device__ __forceinline__ double face_grad64(const double* __restrict__ C, long
         R = B == T1 ? r : q;
         S = scaled(sqlin(B, O), split(k12));
     }
-    const i64 n1 = (gp & 2) ? 0 : -1, n2 = (gp & 1) ? 0 : -1;  // all ones where the coordinate is negative
-    const i64 RS = R + ((S ^ n1) - n1);
-    return double_of(P + ((Q ^ n1) - n1) + ((RS ^ n2) - n2), top);
+}
+
+// form k of a side, in the order visc_point64 takes them: rho along D, T1, T2; m_D likewise; m_T1 along D and T1;
+// m_T2 along D and T2; E along D
+constexpr int NFORM = 11;
+template <int D, int NS, int K>
+__device__ __forceinline__ void side_form64(const double* __restrict__ C4, long long NE, i64& P, i64& Q, i64& R, i64& S) {
+    constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
+    constexpr int var = K < 3 ? 0 : K < 6 ? 1 + D : K < 8 ? 1 + T1 : K < 10 ? 1 + T2 : 4;
+    constexpr int along = K == 1 || K == 4 || K == 7 ? T1 : K == 2 || K == 5 || K == 9 ? T2 : D;
+    face_form64<D, NS, along>(C4 + var * 20 * NE, NE, P, Q, R, S);
 }
 
 // The viscous fluxes (PDEViscFlux, Navier-Stokes-3D/pde.c:90-162) of one face side at Gauss point gp, divided by
 // mu/(2 h): Newtonian stress with Stokes' hypothesis and Fourier heat flux, with the program's velocity
 // gradients u_x = (rho u)_x - u rho_x / rho (:118-130).  Adds the momentum components along D, T1, T2 and the
-// energy's to av; Q is the side's trace, kmu = k / mu; returns 1 / rho.  Only the 11 gradient components that
-// enter the flux along D are formed.
-template <int D, int NS>
-__device__ __forceinline__ double visc_point64(const double* __restrict__ Q, const double* __restrict__ C4, long long NE,
-                                               int gp, double gm1, double kmu, double* av) {
+// energy's to av; Q is the side's trace, grad(k) the value of its form k, kmu = k / mu; returns 1 / rho.  Only the
+// 11 gradient components that enter the flux along D are formed.
+template <int D, class Grad>
+__device__ __forceinline__ double visc_point64(const double* __restrict__ Q, Grad grad, double gm1, double kmu, double* av) {
     constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
-    const long long cs = 20 * NE;
-    const double* Cd = C4 + (1 + D) * cs;
-    const double* C1 = C4 + (1 + T1) * cs;
-    const double* C2 = C4 + (1 + T2) * cs;
     const double rho = Q[0], md = Q[1 + D], m1 = Q[1 + T1], m2 = Q[1 + T2], E = Q[4];
     const double ir = recip_fix(rho);
     const double u = md * ir, v = m1 * ir, w = m2 * ir;
     const double em = fma(-w, m2, fma(-v, m1, fma(-u, md, E)));  // E - |m|^2 / rho
-    const double rd = face_grad64<D, NS, D>(C4, NE, gp) * ir, r1 = face_grad64<D, NS, T1>(C4, NE, gp) * ir,
-                 r2 = face_grad64<D, NS, T2>(C4, NE, gp) * ir;
-    const double gd = face_grad64<D, NS, D>(Cd, NE, gp), g1 = face_grad64<D, NS, D>(C1, NE, gp), g2 = face_grad64<D, NS, D>(C2, NE, gp);
-    const double ud = fma(-u, rd, gd), u1 = fma(-u, r1, face_grad64<D, NS, T1>(Cd, NE, gp)),
-                 u2 = fma(-u, r2, face_grad64<D, NS, T2>(Cd, NE, gp));
-    const double vd = fma(-v, rd, g1), v1 = fma(-v, r1, face_grad64<D, NS, T1>(C1, NE, gp));
-    const double wd = fma(-w, rd, g2), w2 = fma(-w, r2, face_grad64<D, NS, T2>(C2, NE, gp));
+    const double rd = grad(0) * ir, r1 = grad(1) * ir, r2 = grad(2) * ir;
+    const double gd = grad(3), g1 = grad(6), g2 = grad(8);
+    const double ud = fma(-u, rd, gd), u1 = fma(-u, r1, grad(4)), u2 = fma(-u, r2, grad(5));
+    const double vd = fma(-v, rd, g1), v1 = fma(-v, r1, grad(7));
+    const double wd = fma(-w, rd, g2), w2 = fma(-w, r2, grad(9));
     // the temperature gradient (times c_v) of pde.c:118-130, regrouped:
     // (gamma - 1)/rho (E_D - u.m_D - rho_D/rho (E - |m|^2 / rho))
     const double um = fma(w, g2, fma(v, g1, u * gd));
-    const double td = fma(-rd, em, face_grad64<D, NS, D>(C4 + 4 * cs, NE, gp) - um) * (gm1 * ir);
+    const double td = fma(-rd, em, grad(10) - um) * (gm1 * ir);
     const double tn = fma(-2. / 3., (ud + v1) + w2, 2.0 * ud), t1 = u1 + vd, t2 = u2 + wd;
     av[0] += tn;
     av[1] += t1;

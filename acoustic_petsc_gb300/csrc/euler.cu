@@ -686,18 +686,47 @@ __global__ void __launch_bounds__(128) k_faces64(const double* __restrict__ T, d
 // (PDEViscRiemannSolver, Navier-Stokes-3D/pde.c:386-404; rhs_function.c:310-316), laid out as faces64: a Gauss
 // point per warp.  Bound: FP64 issue (120 operations a warp) and the integer pipe's 5000 instructions beside it.
 // 96^3, an RHS: 3.71 ms as a thread per face all in FP64 (203 operations a point), 4.01 with the gradients as
-// integers (180 registers, 8 warps per SM, which fill neither pipe), 3.59 a point per warp at 80 registers.
+// integers (180 registers, 8 warps per SM, which fill neither pipe), 3.59 a point per warp at 80 registers, 2.58
+// with the 22 gradient forms of a face shared out among the four warps.
+struct ViscShared {
+    double flux[4][NV][32];
+    i64 form[2 * NFORM][4][32];
+    int top[2][NV][32];
+};
 template <int D, int FLUX>
 __device__ __forceinline__ void faces_visc64(const double* __restrict__ T, double* __restrict__ F, const Geo& g,
                                              double gamma, DevScalars* __restrict__ ds, int slot,
-                                             const double* __restrict__ C4, const Visc& vp, double (*sh)[NV][32]) {
+                                             const double* __restrict__ C4, const Visc& vp, ViscShared& sh) {
     constexpr int T1 = D == 0 ? 1 : 0, T2 = D == 2 ? 1 : 2;
     const int lane = threadIdx.x & 31, gp = threadIdx.x >> 5;
     const FaceAt<D> at(g, blockIdx.x * 32u + lane);
     if (blockIdx.x * 32u >= at.nf) return;  // the grid is as wide as the direction with the most faces
     double smax = 0.0, smaxv = 0.0;
-    if (at.f < at.nf) {
-        const long long eR = at.hi(g), eL = at.lo(g);
+    const bool in = at.f < at.nf;
+    const long long eR = in ? at.hi(g) : 0, eL = in ? at.lo(g) : 0;
+    if (in) {
+        auto form = [&](auto k) {
+            constexpr int K = decltype(k)::value, side = K / NFORM;
+            i64 P, Q, R, S;
+            side_form64<D, side ? -1 : 1, K % NFORM>(C4 + (side ? eR : eL), g.NE, P, Q, R, S);
+            sh.form[K][0][lane] = P;
+            sh.form[K][1][lane] = Q;
+            sh.form[K][2][lane] = R;
+            sh.form[K][3][lane] = S;
+        };
+        auto forms = [&](auto... k) { (form(k), ...); };
+#define FORM(k) std::integral_constant<int, k>{}
+        if (gp == 0) forms(FORM(0), FORM(4), FORM(8), FORM(12), FORM(16), FORM(20));
+        else if (gp == 1) forms(FORM(1), FORM(5), FORM(9), FORM(13), FORM(17), FORM(21));
+        else if (gp == 2) forms(FORM(2), FORM(6), FORM(10), FORM(14), FORM(18));
+        else forms(FORM(3), FORM(7), FORM(11), FORM(15), FORM(19));
+#undef FORM
+        for (int q = gp; q < 2 * NV; q += 4)
+            sh.top[q / NV][q % NV][lane] =
+                (int)__double_as_longlong(__ldg(C4 + ((q % NV) * 20 + 19) * g.NE + (q < NV ? eL : eR)));
+    }
+    __syncthreads();
+    if (in) {
         const double* TL = T + ((2 * D + 1) * 4 + gp) * g.NE + eL;
         const double* TR = T + (2 * D * 4 + gp) * g.NE + eR;
         double QL[NV], QR[NV], fl[NV], av[4] = {0.0, 0.0, 0.0, 0.0};
@@ -710,8 +739,17 @@ __device__ __forceinline__ void faces_visc64(const double* __restrict__ T, doubl
         if constexpr (FLUX == HYPE_FLUX_RUSANOV) smax = rusanov_fix<D>(QL, QR, gamma, gamma - 1.0, fl, bad);
         else smax = face_solver<double, D, FLUX>(QL, QR, gamma, gamma - 1.0, fl, bad);
         const double kmu = vp.kc / vp.mu;
-        smaxv = visc_point64<D, 1>(QL, C4 + eL, g.NE, gp, gamma - 1.0, kmu, av);
-        smaxv = vp.vmax * max_pos(smaxv, visc_point64<D, -1>(QR, C4 + eR, g.NE, gp, gamma - 1.0, kmu, av));
+        const i64 n1 = (gp & 2) ? 0 : -1, n2 = (gp & 1) ? 0 : -1;  // all ones where the point's coordinate is negative
+        auto grads = [&](int side) {
+            return [&, side](int k) {
+                const i64(*f)[32] = sh.form[side * NFORM + k];
+                const i64 RS = f[2][lane] + ((f[3][lane] ^ n1) - n1);
+                const int var = k < 3 ? 0 : k < 6 ? 1 + D : k < 8 ? 1 + T1 : k < 10 ? 1 + T2 : 4;
+                return double_of(f[0][lane] + ((f[1][lane] ^ n1) - n1) + ((RS ^ n2) - n2), sh.top[side][var][lane]);
+            };
+        };
+        smaxv = visc_point64<D>(QL, grads(0), gamma - 1.0, kmu, av);
+        smaxv = vp.vmax * max_pos(smaxv, visc_point64<D>(QR, grads(1), gamma - 1.0, kmu, av));
         // weight 1/4, both sides' mean, twice the gradients times h: mu / (16 h), in units of the inviscid weight
         constexpr double wq = FLUX == HYPE_FLUX_RUSANOV ? 0.125 : 0.25;
         const double wv = -(1. / 16.) / wq * vp.mu * vp.r1_h;
@@ -720,7 +758,7 @@ __device__ __forceinline__ void faces_visc64(const double* __restrict__ T, doubl
         fl[1 + T2] = fma(wv, av[2], fl[1 + T2]);
         fl[4] = fma(wv, av[3], fl[4]);
 #pragma unroll
-        for (int c = 0; c < NV; ++c) sh[gp][c][lane] = fl[c];
+        for (int c = 0; c < NV; ++c) sh.flux[gp][c][lane] = fl[c];
         if (bad) at.report(g, ds);
     }
     smax = warp_max_pos(smax);
@@ -732,15 +770,16 @@ __device__ __forceinline__ void faces_visc64(const double* __restrict__ T, doubl
     __syncthreads();
     constexpr int shift = FLUX == HYPE_FLUX_RUSANOV ? 3 : 2;
     for (int c = gp; c < NV; c += 4)
-        if (at.f < at.nf) F[(long long)c * at.nf + at.f] = sum4(sh[0][c][lane], sh[1][c][lane], sh[2][c][lane], sh[3][c][lane], shift);
+        if (at.f < at.nf) F[(long long)c * at.nf + at.f] = sum4(sh.flux[0][c][lane], sh.flux[1][c][lane], sh.flux[2][c][lane],
+                                                                   sh.flux[3][c][lane], shift);
 }
 
 template <int FLUX>
-__global__ void __launch_bounds__(128, 6) k_faces_visc64(const double* __restrict__ T, double* __restrict__ Fx,
+__global__ void __launch_bounds__(128, 5) k_faces_visc64(const double* __restrict__ T, double* __restrict__ Fx,
                                                       double* __restrict__ Fy, double* __restrict__ Fz, Geo g, double gamma,
                                                       DevScalars* __restrict__ ds, int slot, const double* __restrict__ C4,
                                                       Visc vp) {
-    __shared__ double sh[4][NV][32];
+    __shared__ ViscShared sh;
     if (blockIdx.y == 0) faces_visc64<0, FLUX>(T, Fx, g, gamma, ds, slot, C4, vp, sh);
     else if (blockIdx.y == 1) faces_visc64<1, FLUX>(T, Fy, g, gamma, ds, slot, C4, vp, sh);
     else faces_visc64<2, FLUX>(T, Fz, g, gamma, ds, slot, C4, vp, sh);
