@@ -297,15 +297,19 @@ __host__ __device__ __forceinline__ double sqrt_rn(double x) {
     return from_bits(((u64)((X + odd) / 2 - 21 + 52 + 1023 - 1) << 52) + n);
 }
 
-// the exact conversion float -> double and the rounded one back, which the FP64 pipe would do at its rate
+// the exact conversion float -> double and the rounded one back, which the FP64 pipe would do at its rate; its
+// instructions in calls, since predicated they would be issued for nothing
+static __device__ __noinline__ double widen_any(float x) { return (double)x; }
+static __device__ __noinline__ float narrow_any(double x) { return (float)x; }
 __device__ __forceinline__ double widen_fix(float x) {
     const unsigned b = __float_as_uint(x), ex = (b >> 23) & 0xFFu;
-    if (ex - 1u > 253u && (b << 1)) return (double)x;  // subnormal, infinite or NaN
+    if (ex - 1u > 253u && (b << 1)) return widen_any(x);  // subnormal, infinite or NaN
     return __hiloint2double((int)((b & 0x80000000u) | (ex ? (((b & 0x7FFFFFFFu) >> 3) + (896u << 20)) : 0u)), (int)(b << 29));
 }
 __device__ __forceinline__ float narrow_fix(double x) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), ex = (hi >> 20) & 0x7FFu;
-    if (ex - 897u > 253u) return (float)x;  // the result is not a normal float
+    if (ex == 0u) return __uint_as_float(hi & 0x80000000u);  // zero, or far below the smallest float
+    if (ex - 897u > 253u) return narrow_any(x);  // the result is zero or not a normal float
     const unsigned f = (hi & 0x80000000u) | ((((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29));
     const unsigned r = lo & 0x1FFFFFFFu;
     return __uint_as_float(f + (r > 0x10000000u || (r == 0x10000000u && (f & 1u)) ? 1u : 0u));
