@@ -97,6 +97,17 @@ struct Side {
     double rho, u, v, w, p, phi, H, a;
 };
 
+// x < c for a positive c as the floating comparison decides it (false for NaN), on the bit pattern
+__device__ __forceinline__ bool below(double x, double c) {
+    const long long b = __double_as_longlong(x);
+    return b < __double_as_longlong(c) && (unsigned long long)b <= 0xFFF0000000000000ull;
+}
+// x / 2, x zero, normal or not finite
+__device__ __forceinline__ double half_of(double x) {
+    const int hi = __double2hiint(x);
+    return ((unsigned)(hi >> 20) & 0x7FFu) - 2u < 2045u ? __hiloint2double(hi - (1 << 20), __double2loint(x)) : x;
+}
+
 __device__ __forceinline__ Side make_side(const Eos& e, const double* V, bool& bad) {
     Side s;
     s.rho = V[0]; s.u = V[1]; s.v = V[2]; s.w = V[3]; s.p = V[4]; s.phi = V[5];
@@ -108,12 +119,12 @@ __device__ __forceinline__ Side make_side(const Eos& e, const double* V, bool& b
         const double c = mix_c(e, s.phi);
         gp = fma(gm1, c, gp);
         pe += c;
-        bad |= gp < PRS_FLOOR * (1.0 + gm1);
+        bad |= below(gp, PRS_FLOOR * (1.0 + gm1));
     } else {
-        bad |= s.p < PRS_FLOOR;
+        bad |= below(s.p, PRS_FLOOR);
     }
-    bad |= s.rho < RHO_FLOOR;
-    s.H = fma(0.5 * s.rho, fma(s.w, s.w, fma(s.v, s.v, s.u * s.u)), pe);
+    bad |= below(s.rho, RHO_FLOOR);
+    s.H = fma(half_of(s.rho), fma(s.w, s.w, fma(s.v, s.v, s.u * s.u)), pe);
     s.a = euler::sqrt_fix(gp * euler::recip_fix(s.rho));
     return s;
 }
@@ -161,28 +172,28 @@ __device__ __forceinline__ int hllc_select(double SL, double SR, double Ss) {
 // is orthonormal and c = n.  In the other branch its t2z (pde.c:302) differs from that of n x t1 by
 // nz (ny - nz) il, and with q2 = (ny + nz)^2 + (nz - nx)^2 + (nx + ny)^2 = 1 / il^2 and d = nz (ny - nz),
 // t1 x t2 / det = (q2 n + d (nz - nx, -(ny + nz), 0)) / (q2 + d (nx (nz - nx) - ny (ny + nz))).
-__device__ __forceinline__ void hllc_momentum(double nx, double ny, double nz, double wt, double p, double Y, HllcSum& h) {
-    double pn = p + Y;
-    const double s = ny + nz, d = ny - nz;
-    if (abs_above(s, d)) {
-        const double b = nz - nx;
-        const double q2 = fma(2.0 * nz, ny - nx, fma(2.0 * nx, ny, 2.0));
-        const double dz = nz * d;
-        const double Yr = Y * euler::recip_fix(fma(dz, fma(nx, b, -ny * s), q2));
-        pn = fma(q2, Yr, p);
-        const double g = wt * (dz * Yr);
+// wp = wt p, wY = wt Y; sum, dif, b, q2: ny + nz, ny - nz, nz - nx and, where |sum| > |dif|, q2
+__device__ __forceinline__ void hllc_momentum(double nx, double ny, double nz, double sum, double dif, double b, double q2,
+                                              double wp, double wY, HllcSum& h) {
+    double pn;
+    if (abs_above(sum, dif)) {
+        const double dz = nz * dif;
+        const double Yr = wY * euler::recip_fix(fma(dz, fma(nx, b, -ny * sum), q2));
+        pn = fma(q2, Yr, wp);
+        const double g = dz * Yr;
         h.px = fma(g, b, h.px);
-        h.py = fma(-g, s, h.py);
+        h.py = fma(-g, sum, h.py);
+    } else {
+        pn = wp + wY;
     }
-    pn *= wt;
     h.px = fma(pn, nx, h.px);
     h.py = fma(pn, ny, h.py);
     h.pz = fma(pn, nz, h.pz);
 }
 
 // One solve of weight wt along a normal of any direction: adds to h, returns the wave speed
-__device__ __forceinline__ double hllc_general(const Side& L, const Side& R, double nx, double ny, double nz, double wt,
-                                               HllcSum& h) {
+__device__ __forceinline__ double hllc_general(const Side& L, const Side& R, double nx, double ny, double nz, double sum,
+                                               double dif, double b, double q2, double wt, HllcSum& h) {
     const double unL = fma(L.w, nz, fma(L.v, ny, L.u * nx)), unR = fma(R.w, nz, fma(R.v, ny, R.u * nx));
     const double SL = fmin(unR - R.a, unL - L.a), SR = fmax(unL + L.a, unR + R.a);
     const double rL = L.rho * (SL - unL), rR = R.rho * (SR - unR);
@@ -191,17 +202,17 @@ __device__ __forceinline__ double hllc_general(const Side& L, const Side& R, dou
     if (sel != 4) {
         const bool left = sel <= 1;
         const double un = left ? unL : unR, p = left ? L.p : R.p;
-        double m = un, Y = 0.0;
+        double m = un, wY = 0.0;
         if (sel == 1 || sel == 2) {
             const double S = left ? SL : SR, e = Ss - un;
             const double z = e * euler::recip_fix(S - Ss);
             m = fma(S, z, un);
-            Y = (S * e) * fma(left ? L.rho : R.rho, z, left ? L.rho : R.rho);
-            h.en = fma(wt * Y, Ss, h.en);
+            wY = wt * ((S * e) * fma(left ? L.rho : R.rho, z, left ? L.rho : R.rho));
+            h.en = fma(wY, Ss, h.en);
         }
         if (left) h.mL = fma(wt, m, h.mL);
         else h.mR = fma(wt, m, h.mR);
-        hllc_momentum(nx, ny, nz, wt, p, Y, h);
+        hllc_momentum(nx, ny, nz, sum, dif, b, q2, wt * p, wY, h);
     }
     return euler::max_pos(fabs(unL) + L.a, fabs(unR) + R.a);
 }
@@ -211,12 +222,12 @@ __device__ __forceinline__ double hllc_general(const Side& L, const Side& R, dou
 // tangents are perpendicular to the jump, so both sides have one normal velocity un there: the acoustic
 // speeds are un -+ amax and S_star - un, and with it z and rho (1 + z), is the same for both tangents.
 // Without a jump n1 is the face normal, the tangents' weights are exactly zero and only their wave
-// speeds count.  About 260 FP64 operations (three general solves: about 800).
+// speeds count.  About 210 FP64 operations (three general solves: about 800).
 template <int D>
 __device__ __forceinline__ double rot_hllc7(const Side& L, const Side& R, double* Flux) {
     const double du = R.u - L.u, dv = R.v - L.v, dw = R.w - L.w;
     const double dq2 = fma(dw, dw, fma(dv, dv, du * du));
-    const bool still = dq2 < 1.0E-20;  // |du| < 1e-10 (pde.c:391)
+    const bool still = below(dq2, 1.0E-20);  // |du| < 1e-10 (pde.c:391)
     double nx = D == 0 ? 1.0 : 0.0, ny = D == 1 ? 1.0 : 0.0, nz = D == 2 ? 1.0 : 0.0, a1 = 1.0;
     if (!still) {
         const double idq = euler::rsqrt_fix(dq2);
@@ -226,18 +237,17 @@ __device__ __forceinline__ double rot_hllc7(const Side& L, const Side& R, double
         a1 = D == 0 ? nx : D == 1 ? ny : nz;
     }
     // t1 and t2 = n1 x t1 of pde.c:402-424
-    double t1x = ny + nz, t1y = nz - nx, t1z = -(nx + ny);
-    if (const double d = ny - nz; !abs_above(t1x, d)) {
-        t1x = d;
-        t1z = nx - ny;
-    }
-    const double il = euler::rsqrt_fix(fma(t1z, t1z, fma(t1y, t1y, t1x * t1x)));
+    const double sum = ny + nz, dif = ny - nz, b = nz - nx;
+    const bool first = abs_above(sum, dif);
+    double t1x = first ? sum : dif, t1y = b, t1z = first ? -(nx + ny) : nx - ny;
+    const double q2 = fma(t1z, t1z, fma(t1y, t1y, t1x * t1x));
+    const double il = euler::rsqrt_fix(q2);
     t1x *= il;
     t1y *= il;
     t1z *= il;
     double t2x = fma(ny, t1z, -nz * t1y), t2y = fma(nz, t1x, -nx * t1z), t2z = fma(nx, t1y, -ny * t1x);
     HllcSum h{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    double smax = hllc_general(L, R, nx, ny, nz, a1, h);
+    double smax = hllc_general(L, R, nx, ny, nz, sum, dif, b, q2, a1, h);
     if (still) {
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -263,16 +273,17 @@ __device__ __forceinline__ double rot_hllc7(const Side& L, const Side& R, double
             smax = euler::max_pos(smax, fabs(un) + am);
             if (sel == 4) continue;
             const bool left = sel <= 1;
-            double m = un, Y = 0.0;
+            double m = un, wY = 0.0;
             if (sel == 1 || sel == 2) {
                 const double S = left ? SL : SR;
                 m = fma(S, left ? zL : zR, un);
-                Y = S * (left ? yL : yR);
-                h.en = fma(wt * Y, Ss, h.en);
+                wY = wt * (S * (left ? yL : yR));
+                h.en = fma(wY, Ss, h.en);
             }
             if (left) h.mL = fma(wt, m, h.mL);
             else h.mR = fma(wt, m, h.mR);
-            hllc_momentum(tx, ty, tz, wt, left ? L.p : R.p, Y, h);
+            const double ts = ty + tz, tb = tz - tx, tf = tx + ty;
+            hllc_momentum(tx, ty, tz, ts, ty - tz, tb, fma(tf, tf, fma(tb, tb, ts * ts)), wt * (left ? L.p : R.p), wY, h);
         }
     }
     const double qL = L.rho * h.mL, qR = R.rho * h.mR;
@@ -546,7 +557,7 @@ __device__ __forceinline__ void raise_max(unsigned long long* a, double v) {
 // through shared memory.  Bound: FP64 issue.  With one thread per face, its four points in turn, and three
 // general solves per point the three face launches of a 40 x 40 x 100 RHS took 3.9 ms of 5.6; a whole RHS
 // and stage then took 1.9 ms (22.5 -> 7.5 ms per step); with reciprocals and roots on the integer pipe the
-// faces are 0.83 ms (4.4 ms per step).
+// faces are 0.77 ms (4.1 ms per step).
 template <int D>
 __device__ __forceinline__ void faces(const double* __restrict__ T, double* __restrict__ F, const Geo& g, const Eos& e,
                                       DevScalars* __restrict__ ds, int slot, double (*sh)[MF][32]) {
