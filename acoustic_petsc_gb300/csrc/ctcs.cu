@@ -334,7 +334,8 @@ extern "C" int hype_ctcs_create(const hype_ctcs_params* p, hype_ctcs** out) {
     const int levels = p->form == 0 ? 4 : 3;
     for (int q = 0; q < levels && e == cudaSuccess; ++q) e = cudaMalloc((void**)&c->lv[q], sizeof(double) * c->n);
     if (e == cudaSuccess) e = cudaMalloc((void**)&c->st, sizeof(DevStep));
-    for (int q = 0; q < levels && e == cudaSuccess; ++q) e = cudaMemset(c->lv[q], 0, sizeof(double) * c->n);
+    // the second pair is written whole before it is read
+    for (int q = 0; q < (p->form == 0 ? 2 : 3) && e == cudaSuccess; ++q) e = cudaMemset(c->lv[q], 0, sizeof(double) * c->n);
     int dev = 0, nsm = 1;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

@@ -9,8 +9,8 @@ cell-updates/s (cells x steps / s).
   python bench.py [--gpus N] [--steps K] [--warmup W] [--workload NAME] [--impl reference]
 
 Other workloads (--workload): euler256_fp32 (FP32 reconstruction/flux, FP64
-state), euler256_df64 (double-float reconstruction on the FP32 pipe, FP64 state and
-flux, held to the FP64 error bars), euler256_linear (optimal-weight linear reconstruction), euler256_weno3,
+state), euler256_df64 (HYPE_PREC_DF64, which runs the FP64 kernels,
+held to the FP64 error bars), euler256_linear (optimal-weight linear reconstruction), euler256_weno3,
 euler256_hllc, ns256_tgv (viscous Taylor-Green), acoustic256 (3D acoustic FV),
 sw2d4096 (2D standing wave, RK104), mp3d256 (3D primitive multiphase), pc2d2048 (2d/HyPE-2D path-conservative
 Kapila, order 3), kapila1024[_fp32|_learned], blast256/512,
@@ -215,8 +215,7 @@ FLUX_NAME = {0: "Rusanov", 1: "HLLC", 2: "rotated HLLC"}
 
 
 EULER_DTYPE = {0: "f64", 1: "f64 state / f32 recon+flux",
-               2: "f64 state and stage accumulation / df64 recon+Rusanov flux (FP32 pairs, 48-bit significand, "
-                  "on deviations from a reference state)"}
+               2: "f64 (HYPE_PREC_DF64 runs the f64 kernels)"}
 
 
 def run_euler(args, ws, rank, local, precision=0, recon=0, n=256, flux=0, viscous=False):
@@ -271,14 +270,16 @@ def run_euler(args, ws, rank, local, precision=0, recon=0, n=256, flux=0, viscou
     bytes_stage = EULER_BYTES_PER_CELL_STAGE + (NS_COEF_BYTES_PER_CELL_STAGE if viscous else 0.0)
     achieved_gbs = bytes_stage * cells / t_stage / 1e9
     peak, peak_kind = _peaks()
-    tag = {0: "fp64", 1: "fp32", 2: "df64"}[precision] + ("_linear" if recon else "") + ("_ns" if viscous else "")
-    prof_file = ("ns3d_tgv_stage_fp64.txt" if precision == 0 else f"ns3d_tgv_stage_{tag}.txt") if viscous else \
-        f"euler_stage_{tag}.txt"
+    # HYPE_PREC_DF64 runs the FP64 kernels
+    tag = ("fp32" if precision == 1 else "fp64") + ("_linear" if recon else "") + ("_ns" if viscous else "")
+    prof_file = "ns3d_tgv_stage_fp64.txt" if viscous and precision != 1 else f"euler_stage_{tag}.txt"
     traffic = _profile_figure(prof_file, "dram_bytes_per_cell_stage")
     flops_cell = _profile_figure(prof_file, "fp_flops_per_cell_stage")
     fpeak = C.c_double()
-    # the double-float form runs its reconstruction on the FP32 pipe
-    H._lib.check(H._lib.probes().hype_probe_fma_peak(1 if precision == 2 else precision, C.byref(fpeak)), "probe")
+    # the FP32 FMA probe issues one instruction a lane and cycle: the issue ceiling of every form; FP64's own peak
+    # beside it
+    issued = _profile_figure(prof_file, "issued_thread_instructions_per_cell_stage")
+    H._lib.check(H._lib.probes().hype_probe_fma_peak(1 if issued else precision % 2, C.byref(fpeak)), "probe")
     # the FP32 Rusanov form runs the fused stage kernel (ghost fill + one pass per stage)
     fused = precision == 1 and flux == 0 and not viscous
     per_kernel = ({"ghost": prof_ms[0] / stages, "stage_fused": prof_ms[1] / stages,
@@ -291,12 +292,11 @@ def run_euler(args, ws, rank, local, precision=0, recon=0, n=256, flux=0, viscou
             "traffic": traffic * cells if traffic else None, "algorithmic_bytes": bytes_stage * cells,
             "per_kernel_ms": per_kernel}
     alu = None
-    instr32 = _profile_figure(prof_file, "issued_thread_instructions_per_cell_stage") if precision == 1 else None
-    if instr32:
-        # the fused FP32 stage: every issued thread instruction against the FP32 pipe's issue ceiling
-        # (the FMA probe's rate / 2: an FMA is two flops, one instruction)
-        ach_i = instr32 * cells / t_stage
-        alu = {"bound": "fp32 issue", "issued_thread_instructions_per_cell_stage": instr32,
+    if issued:
+        # every issued thread instruction against the issue ceiling (the FP32 FMA probe's rate / 2: an FMA is two
+        # flops, one instruction); the FP64 forms run mostly on the integer pipe
+        ach_i = issued * cells / t_stage
+        alu = {"bound": "fp32 issue" if precision == 1 else "integer issue", "issued_thread_instructions_per_cell_stage": issued,
                "achieved_instr_per_s": ach_i, "peak_instr_per_s": fpeak.value * 1e12 / 2,
                "frac": ach_i / (fpeak.value * 1e12 / 2),
                "peak_kind": "measured FMA issue ceiling (hype_probe_fma_peak)"}
@@ -306,9 +306,15 @@ def run_euler(args, ws, rank, local, precision=0, recon=0, n=256, flux=0, viscou
             alu["algorithmic_flops_per_cell_stage"] = alg
             alu["algorithmic_achieved_tflops"] = alg * cells / t_stage / 1e12
             alu["algorithmic_frac"] = alu["algorithmic_achieved_tflops"] / fpeak.value
+        instr_cell = _profile_figure(prof_file, "fp64_instructions_per_cell_stage") if precision != 1 else None
+        if instr_cell:
+            p64 = C.c_double()
+            H._lib.check(H._lib.probes().hype_probe_fma_peak(0, C.byref(p64)), "probe")
+            alu["fp64_instructions_per_cell_stage"] = instr_cell
+            alu["fp64_issue_frac"] = instr_cell * cells / t_stage / (p64.value * 1e12 / 2)
     elif flops_cell:
         ach = flops_cell * cells / t_stage / 1e12
-        alu = {"bound": "fp64" if precision == 0 else "fp32", "achieved": ach, "peak": fpeak.value, "unit": "TFLOP/s",
+        alu = {"bound": "fp32" if precision == 1 else "fp64", "achieved": ach, "peak": fpeak.value, "unit": "TFLOP/s",
                "frac": ach / fpeak.value, "flops_per_cell_stage": flops_cell,
                "peak_kind": "measured FMA issue ceiling (hype_probe_fma_peak)"}
         # the reference algorithm's own operation count (oracle/flopcount.py on its expression trees):
@@ -320,7 +326,7 @@ def run_euler(args, ws, rank, local, precision=0, recon=0, n=256, flux=0, viscou
             alu["algorithmic_achieved"] = alg * cells / t_stage / 1e12
             alu["algorithmic_frac"] = alu["algorithmic_achieved"] / fpeak.value
             alu["algorithmic_source"] = "profiles/flops_euler_cweno4_rusanov.txt (reference expression trees)"
-        instr_cell = _profile_figure(prof_file, "fp64_instructions_per_cell_stage") if precision == 0 else None
+        instr_cell = _profile_figure(prof_file, "fp64_instructions_per_cell_stage") if precision != 1 else None
         if instr_cell:
             # an FMA counts two flops, an add or multiply one: against the issue ceiling
             # (peak / 2 instructions per second) the FP64 pipe's occupancy shows directly
@@ -426,7 +432,7 @@ def _euler_df64_beside(args, ws, n, U0, U_fp64, stream_of, precision=2):
                   "per_kernel_ms": per,
                   "state_rel_linf_diff_vs_fp64": diff,
                   "steps_compared": max(args.warmup, 3) + args.steps,
-                  "profile": f"profiles/euler_stage_{tag}.txt"}}
+                  "profile": "profiles/euler_stage_fp64.txt" if precision == 2 else "profiles/euler_stage_fp32.txt"}}
 
 
 def run_ctcs(args, ws, rank, local, n=512):
