@@ -93,7 +93,8 @@ __global__ void __launch_bounds__(kCellThreads) k_mp_pad(const double* __restric
 
 // FP64 face fluxes, both directions in one launch (blockIdx.y): a block is 32 faces, indexed flat, x the two
 // Gauss points, one per warp, summed through shared memory in the reference's order.  Bound: FP64 issue; 301 x 122:
-// 241 us as a thread per face and a launch per direction with FP64 divisions, here 122.
+// 241 us as a thread per face and a launch per direction with FP64 divisions, 122 with them on the integer pipe, 108
+// with the comparisons there too and only the selected side's flux formed.
 template <int MODEL, int D>
 __device__ __forceinline__ void faces64(const double* __restrict__ T, double* __restrict__ F, const Geo& g, const Eos& e,
                                         DevScalars* __restrict__ ds, int slot, double (*sh)[32]) {
@@ -113,7 +114,7 @@ __device__ __forceinline__ void faces64(const double* __restrict__ T, double* __
             VR[c] = __ldg(T + ((long long)c * 8 + (2 * D) * 2 + q) * g.NE + eR);
         }
         bool bad = false;
-        smax = fmax(0.0, rot_hllc2<double, MODEL>(e, VL, VR, D == 0, D == 1, fl, bad));
+        smax = fmax(0.0, rot_hllc2_64<MODEL>(e, VL, VR, D == 0, D == 1, fl, bad));
         if (bad) atomicMin(&ds->bad, (unsigned long long)((long long)(j < g.ny ? j : g.ny - 1) * g.nx + (i < g.nx ? i : g.nx - 1)));
         if (q == 1) {
 #pragma unroll

@@ -72,6 +72,17 @@ __device__ __forceinline__ R root(R a) {
     else return sqrt(a);
 }
 
+// comparisons of doubles as the floating ones decide them (false for NaN), on the bit patterns: a comparison is an
+// FP64 instruction on GB300, and a face point has about twenty
+__device__ __forceinline__ bool a_number(double a) { return (__double_as_longlong(a) & 0x7FFFFFFFFFFFFFFFll) <= 0x7FF0000000000000ll; }
+__device__ __forceinline__ bool less(double a, double b) {
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    const long long mx = x & 0x7FFFFFFFFFFFFFFFll, my = y & 0x7FFFFFFFFFFFFFFFll;
+    const long long kx = x < 0 ? -mx : mx, ky = y < 0 ? -my : my;  // ordered as the numbers, zeros alike
+    return kx < ky && a_number(a) && a_number(b);
+}
+__device__ __forceinline__ bool at_least(double a, double b) { return !less(a, b) && a_number(a) && a_number(b); }
+
 template <typename R>
 __device__ __forceinline__ R pow4(R a) {
     const R a2 = a * a;
@@ -293,14 +304,14 @@ __device__ __forceinline__ bool pad_ok(const Eos& e, const R* V) {
     }
     if (e.model == HYPE_MP_DI4) {
         const double phi = (double)V[4], p = (double)V[3];
-        if ((double)V[0] < 1.0e-14 || phi < 0.0 || phi > 1.0) return false;
-        if (stiff_nonneg && !(p < 1.0e-12)) return true;
+        if (less((double)V[0], 1.0e-14) || less(phi, 0.0) || less(1.0, phi)) return false;
+        if (stiff_nonneg && !less(p, 1.0e-12)) return true;
         mix(e, phi, g, pi);
         return !((p + pi) < 1.0e-12);
     }
     const double a1 = (double)V[5], p = (double)V[4];
-    if ((double)V[0] < 1.0e-14 || (double)V[1] < 1.0e-14 || a1 < 0.0 || a1 > 1.0) return false;
-    if (stiff_nonneg && !(p < 1.0e-12)) return true;
+    if (less((double)V[0], 1.0e-14) || less((double)V[1], 1.0e-14) || less(a1, 0.0) || less(1.0, a1)) return false;
+    if (stiff_nonneg && !less(p, 1.0e-12)) return true;
     mix(e, a1, g, pi);
     return !((p + pi) < 1.0e-12);
 }
@@ -343,7 +354,8 @@ __device__ __forceinline__ void make_side2(const R* V, R g, R pi, Side2<R>& s, b
         s.rho = V[5] * V[0] + (R(1.0) - V[5]) * V[1];  // a1 r1 + a2 r2
         u = V[2]; v = V[3]; p = V[4];
     }
-    bad |= (s.rho < R(1.0e-14)) || ((p + pi) < R(1.0e-12)) || !(s.rho == s.rho);
+    if constexpr (sizeof(R) == sizeof(double)) bad |= less(s.rho, 1.0e-14) || less(p + pi, 1.0e-12) || !a_number(s.rho);
+    else bad |= (s.rho < R(1.0e-14)) || ((p + pi) < R(1.0e-12)) || !(s.rho == s.rho);
     s.c = root(quot(g * (p + pi), s.rho));
     s.Eh = quot(p + g * pi, g - R(1.0)) + R(0.5) * s.rho * u * u + R(0.5) * s.rho * v * v;
 }
@@ -478,6 +490,116 @@ __device__ __forceinline__ R rot_hllc2(const Eos& e, const R* VL, const R* VR, R
 #pragma unroll
     for (int k = 0; k <= NV; ++k) Flux[k] = a1 * f1[k] + a2 * f2[k];
     return (s1 < s2) ? s2 : s1;
+}
+
+// hllc2 in FP64, the same values: comparisons on bit patterns, and the flux of the selected side alone
+template <int MODEL>
+__device__ __forceinline__ double hllc2_64(const double* VL, const double* VR, const Side2<double>& sL, const Side2<double>& sR,
+                                           double nx, double ny, double* Flux) {
+    constexpr int NV = MODEL == HYPE_MP_DI4 ? 5 : 6;
+    double F[MAXV + 1];
+    const double* QL = sL.Q;
+    const double* QR = sR.Q;
+    double uL, uR, vL, vR, PL, PR;
+    if (MODEL == HYPE_MP_DI4) {
+        uL = VL[1]; vL = VL[2]; PL = VL[3];
+        uR = VR[1]; vR = VR[2]; PR = VR[3];
+    } else {
+        uL = VL[2]; vL = VL[3]; PL = VL[4];
+        uR = VR[2]; vR = VR[3]; PR = VR[4];
+    }
+    const double rL = sL.rho, rR = sR.rho;
+    const double unL = uL * nx + vL * ny, utL = -uL * ny + vL * nx;
+    const double unR = uR * nx + vR * ny, utR = -uR * ny + vR * nx;
+    const double cL = sL.c, cR = sR.c;
+    const double EL = sL.Eh, ER = sR.Eh;
+    const double a1 = unR - cR, b1 = unL - cL;
+    const double SL = less(a1, b1) ? a1 : b1;
+    const double a2 = unL + cL, b2 = unR + cR;
+    const double SR = less(a2, b2) ? b2 : a2;
+    const double Ss = quot(PR - PL + rL * unL * (SL - unL) - rR * unR * (SR - unR), rL * (SL - unL) - rR * (SR - unR));
+    // only the star state of the selected side is needed
+    const int sel = less(0.0, SL) ? 0 : at_least(Ss, 0.0) ? 1 : at_least(SR, 0.0) ? 2 : 3;
+    const bool left = sel <= 1;
+    double V[NV];
+    Side2<double> s;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        V[i] = left ? VL[i] : VR[i];
+        s.Q[i] = left ? QL[i] : QR[i];
+    }
+    s.rho = left ? rL : rR;
+    s.c = left ? cL : cR;
+    flux_prim<double, MODEL>(V, s, nx, ny, F);
+    F[NV] = left ? unL : unR;
+    if (sel == 0 || sel == 3) {
+#pragma unroll
+        for (int i = 0; i <= NV; ++i) Flux[i] = F[i];
+    } else {
+        const double Sk = left ? SL : SR, rk = left ? rL : rR, unk = left ? unL : unR, utk = left ? utL : utR;
+        const double Pk = left ? PL : PR, Ek = left ? EL : ER;
+        double Us[MAXV];
+        if (MODEL == HYPE_MP_DI4) {
+            Us[0] = quot(rk * (Sk - unk), Sk - Ss);
+            Us[1] = Us[0] * (Ss * nx - utk * ny);
+            Us[2] = Us[0] * (Ss * ny + utk * nx);
+            Us[3] = Us[0] * (quot(Ek, rk) + (Ss - unk) * (Ss + quot(Pk, rk * (Sk - unk))));
+            Us[4] = quot(V[4] * (Sk - unk), Sk - Ss);
+        } else {
+            const double f = quot(Sk - unk, Sk - Ss);
+            const double rs = rk * f;
+            Us[0] = s.Q[0] * f;
+            Us[1] = s.Q[1] * f;
+            Us[2] = rs * (Ss * nx - utk * ny);
+            Us[3] = rs * (Ss * ny + utk * nx);
+            Us[4] = rs * (quot(Ek, rk) + (Ss - unk) * (Ss + quot(Pk, rk * (Sk - unk))));
+            Us[5] = V[5] * f;
+        }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) Flux[i] = F[i] + Sk * (Us[i] - s.Q[i]);
+        Flux[NV] = unk + Sk * (quot(Sk - unk, Sk - Ss) - 1.0);
+    }
+    const double sl = fabs(unL) + cL, sr = fabs(unR) + cR;
+    return less(sl, sr) ? sr : sl;
+}
+
+// rot_hllc2 in FP64, the same values
+template <int MODEL>
+__device__ __forceinline__ double rot_hllc2_64(const Eos& e, const double* VL, const double* VR, double nx, double ny,
+                                               double* Flux, bool& bad) {
+    constexpr int NV = MODEL == HYPE_MP_DI4 ? 5 : 6;
+    constexpr int IU = MODEL == HYPE_MP_DI4 ? 1 : 2;
+    const double du = VR[IU] - VL[IU], dv = VR[IU + 1] - VL[IU + 1];
+    const double dq = root(du * du + dv * dv);
+    double n1x, n1y;
+    if (less(dq, 1.0e-10)) {
+        n1x = nx;
+        n1y = ny;
+    } else {
+        n1x = quot(du, dq);
+        n1y = quot(dv, dq);
+    }
+    double a1 = n1x * nx + n1y * ny;
+    if (less(a1, 0.0)) {
+        n1x = -n1x; n1y = -n1y; a1 = -a1;
+    }
+    double n2x = -n1y, n2y = n1x;
+    double a2 = n2x * nx + n2y * ny;
+    if (less(a2, 0.0)) {
+        n2x = -n2x; n2y = -n2y; a2 = -a2;
+    }
+    double gL, piL, gR, piR;  // each side's mixture and EOS quantities, once for both solves
+    mix_r<double>(e, VL[NV - 1], gL, piL);
+    mix_r<double>(e, VR[NV - 1], gR, piR);
+    Side2<double> sL, sR;
+    make_side2<double, MODEL>(VL, gL, piL, sL, bad);
+    make_side2<double, MODEL>(VR, gR, piR, sR, bad);
+    double f1[MAXV + 1], f2[MAXV + 1];
+    const double s1 = hllc2_64<MODEL>(VL, VR, sL, sR, n1x, n1y, f1);
+    const double s2 = hllc2_64<MODEL>(VL, VR, sL, sR, n2x, n2y, f2);
+#pragma unroll
+    for (int k = 0; k <= NV; ++k) Flux[k] = a1 * f1[k] + a2 * f2[k];
+    return less(s1, s2) ? s2 : s1;
 }
 
 }  // namespace mp2d
