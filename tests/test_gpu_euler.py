@@ -330,12 +330,13 @@ def test_graph_replayed_steps_equal_launched_steps(hype, precision, flux):
     assert lg == le > 0
 
 
-@pytest.mark.parametrize("kind", ["exact", "shock", "zeros", "wide", "huge"])
+@pytest.mark.parametrize("kind", ["exact", "shock", "zeros", "wide", "huge", "hypersonic", "thin"])
 @pytest.mark.parametrize("recon", ["cweno4", "linear4"])
 def test_fixed_point_reconstruction_edges(hype, oracle, kind, recon):
     """the integer form of the FP64 reconstruction where its scaling matters: a uniform state (its RHS is zero up to
     the fluxes' rounding), density jumps beyond the factor 8 that sends a cell to the FP64 form, momenta that are
-    zero, 250 orders of magnitude below the density, and a state scaled by 1e30.  Tolerance: the RHS differs from the
+    zero, 250 orders of magnitude below the density, and a state scaled by 1e30; and of the face states' integer form:
+    Mach 40, and a density and pressure just above the floors, which take its FP64 form.  Tolerance: the RHS differs from the
     checker's by rounding, a few 1e-16 of the fluxes' size times 6 faces / h, below 1e-12 of F / h."""
     n, h = 9, 0.1
     rng = np.random.default_rng(11)
@@ -354,6 +355,14 @@ def test_fixed_point_reconstruction_edges(hype, oracle, kind, recon):
             U *= 1e30
     elif kind == "zeros":
         U[..., 0] += 0.2 * rng.random((n, n, n))
+    elif kind == "hypersonic":
+        U[..., 0] += 0.1 * rng.random((n, n, n))
+        u = np.array([47.0, -3.0, 11.0]) * (1 + 0.01 * rng.random((n, n, n, 1)))
+        U[..., 1:4] = U[..., :1] * u
+        U[..., 4] += 0.5 * (U[..., 1:4] * u).sum(axis=-1) + 0.3 * rng.random((n, n, n))
+    elif kind == "thin":
+        U[..., 0] = 1e-13 * (1 + 0.2 * rng.random((n, n, n)))
+        U[..., 4] = 2.5e-11 * (1 + 0.2 * rng.random((n, n, n)))
     code = L.RECON_CWENO4 if recon == "cweno4" else L.RECON_LINEAR4
     cfg = oracle.euler_cfg(n, h, cfl=0.4, recon=code)
     R, _, rc = oracle.euler_rhs(cfg, U)[:3]
