@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(kReconThreads, 8)
     for (int c = c0; c < c1; ++c) {
         double s[33];
         const double* Gc = G + (long long)c * g.GN + ge;
-        double* Cc = C4 + (long long)c * 20 * g.NE + e;
+        double* Cc = C4 ? C4 + (long long)c * 20 * g.NE + e : nullptr;  // null without viscosity: nothing stored
         gather33g<double>(Gc, sy, sz, s);
         double* Tc = T + (long long)c * NTR * g.NE + e;
         if constexpr (RECON == HYPE_RECON_WENO3) {
@@ -375,10 +375,10 @@ __global__ void __launch_bounds__(kReconThreads, 8)
             constexpr bool linear = RECON == HYPE_RECON_LINEAR4;
             PolyFix fix;
             if (!recon_fix<linear>(s, c == 0 || c == 4, Tc, g.NE, fix)) recon64_general<linear>(Gc, sy, sz, Tc, linear ? Cc : nullptr, g.NE);
-            else if (linear && C4) store_grad_coeffs(fix, Cc, g.NE);
+            else if (linear && Cc) store_grad_coeffs(fix, Cc, g.NE);
         }
         // the viscous fluxes take the gradients of R4
-        if (RECON != HYPE_RECON_LINEAR4 && C4) recon64_general<true>(Gc, sy, sz, nullptr, Cc, g.NE);
+        if (RECON != HYPE_RECON_LINEAR4 && Cc) recon64_general<true>(Gc, sy, sz, nullptr, Cc, g.NE);
     }
     if (PAD && !traces_admissible<double>(T, g, e, gm1)) {
         store_first_order_g<double>(G, T, g, ge, e);

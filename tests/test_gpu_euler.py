@@ -374,3 +374,63 @@ def test_fixed_point_reconstruction_edges(hype, oracle, kind, recon):
     R_g = s.RHSFunction(0.0, U)
     size = np.abs(U).max() * 10.0 / h
     assert np.abs(R_g - R).max() <= 1e-12 * size
+
+
+def _outside_fixed_point(U):
+    """the cells whose density or energy lies four or more binary exponents below the largest within two cells along
+    an axis (part of the reconstruction's stencil): the FP64 form takes these"""
+    count = 0
+    for c in (0, 4):
+        e = np.frexp(U[..., c])[1]
+        top = e.copy()
+        for ax in range(3):
+            p = np.pad(e, [(2, 2) if a == ax else (0, 0) for a in range(3)], mode="edge")
+            for s in range(5):
+                top = np.maximum(top, np.take(p, range(s, s + e.shape[ax]), axis=ax))
+        count += int((top - e >= 4).sum())
+    return count
+
+
+def _jump_state(kind, n=13):
+    from acoustic_petsc_gb300 import workloads
+
+    if kind == "blast":  # energy 1.79 against 17.9: exponents 0 and 4
+        return workloads.euler_blast(n, r0=0.25)
+    U = np.zeros((n, n, n, 5))
+    x = np.arange(n)
+    if kind == "ramp":  # 4.2 times per cell, 17.6 over two: the R4 traces of an exponential stay positive
+        U[..., 0] = 1.1 * 4.2 ** x
+        U[..., 4] = 2.5 * 4.2 ** x
+        U[..., 1] = 0.1 * U[..., 0]
+    else:
+        U[..., 0] = np.where(x >= 4, 17.0 if kind == "density" else 1.0, 1.0)
+        U[..., 4] = np.where(x >= 4, 50.0 if kind == "energy" else 2.5, 2.5)
+    return U
+
+
+@pytest.mark.parametrize("precision", [L.PREC_FP64, L.PREC_DF64])
+@pytest.mark.parametrize("recon", [L.RECON_CWENO4, L.RECON_LINEAR4])
+@pytest.mark.parametrize("kind,positivity", [("blast", 1), ("ramp", 0), ("ramp", 1), ("density", 1), ("energy", 1),
+                                             ("density", 0), ("energy", 0), ("nan", 0), ("nan", 1)])
+def test_reconstruction_outside_the_fixed_point_form(hype, oracle, precision, recon, kind, positivity):
+    """states that send cells to the FP64 form of the reconstruction, without viscosity (no gradient array to write to):
+    the right-hand side against the checker's, to the FP64 path's bar of 1e-12 of its largest; where the checker
+    refuses the state (traces below the floors, with no fallback), and for a state that is not finite, the status says
+    so and is no CUDA error"""
+    n = 13
+    U = _jump_state("ramp" if kind == "nan" else kind)
+    assert _outside_fixed_point(U) > 0
+    bc = (2,) * 6
+    cfg = oracle.euler_cfg(n, 1.0 / n, cfl=0.4, bc=bc, recon=recon, positivity=positivity)
+    s = solver(hype, n, bc, recon=recon, precision=precision, positivity=positivity)
+    R, _, rc = oracle.euler_rhs(cfg, U)[:3]
+    if kind == "nan":
+        U[5, 6, 7, 4] = np.nan
+        rc = 1
+    if rc != 0:
+        with pytest.raises(hype.HypeError) as err:
+            s.RHSFunction(0.0, U)
+        assert err.value.code == L.HYPE_ERR_STATE
+        U = _jump_state("ramp")  # the context goes on working
+        R = oracle.euler_rhs(cfg, U)[0]
+    assert rel(s.RHSFunction(0.0, U), R) <= TOL_STEP

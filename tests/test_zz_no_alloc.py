@@ -158,3 +158,21 @@ def test_noalloc_positivity_fallback(hype, prec):
     assert np.isfinite(got).all()
     assert np.abs(got - want).max() <= TOL * np.abs(want).max()
     assert abs(dt_got - dt_want) <= TOL * dt_want
+
+
+@pytest.mark.parametrize("recon", [0, 1])
+def test_noalloc_outside_the_fixed_point_form(hype, oracle, recon):
+    """the pressure-ratio-10 blast, whose energy jump of four binary exponents takes the reconstruction's FP64 form,
+    against the CPU checker's right-hand side"""
+    torch = pytest.importorskip("torch")
+    from acoustic_petsc_gb300 import workloads
+
+    n, bc = 13, (2,) * 6
+    U = workloads.euler_blast(n, r0=0.25)
+    assert np.ptp(np.frexp(U[..., 4])[1]) >= 4
+    _, params = _params(hype, (n, n, n), bc, recon=recon, positivity=1)
+    got, _ = _noalloc(hype, torch, params, _soa(torch, U))
+    Ro, _, rc, _ = oracle.euler_rhs(oracle.euler_cfg(n, 1.0 / n, cfl=0.4, bc=bc, recon=recon, positivity=1), U)
+    assert rc == 0
+    want = np.ascontiguousarray(Ro.transpose(3, 0, 1, 2)).reshape(-1)
+    assert np.abs(got - want).max() <= TOL * np.abs(want).max()
