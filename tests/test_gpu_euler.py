@@ -434,3 +434,18 @@ def test_reconstruction_outside_the_fixed_point_form(hype, oracle, precision, re
         U = _jump_state("ramp")  # the context goes on working
         R = oracle.euler_rhs(cfg, U)[0]
     assert rel(s.RHSFunction(0.0, U), R) <= TOL_STEP
+
+
+@pytest.mark.parametrize("precision", [L.PREC_FP64, L.PREC_DF64])
+def test_vanishing_momenta_in_a_dense_gas(hype, oracle, precision):
+    """momenta at the end of FP64's range over densities of 1000: the velocities are below the smallest normal number.
+    The right-hand side stays what the checker gives, to 1e-12 of its largest; its momenta carry the pressure alone"""
+    n = 12
+    rng = np.random.default_rng(5)
+    U = np.zeros((n, n, n, 5))
+    U[..., 0] = 1e3 * (1.0 + 0.2 * rng.random((n, n, n)))
+    U[..., 1:4] = rng.choice([1e-305, -1e-306, 2e-306, 0.0], (n, n, n, 3))
+    U[..., 4] = 2.5 + 0.3 * rng.random((n, n, n))
+    R, _, rc = oracle.euler_rhs(oracle.euler_cfg(n, 1.0 / n, cfl=0.4), U)[:3]
+    assert rc == 0
+    assert rel(solver(hype, n, precision=precision).RHSFunction(0.0, U), R) <= TOL_STEP
