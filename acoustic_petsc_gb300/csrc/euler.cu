@@ -622,10 +622,10 @@ struct FaceAt {
     }
 };
 
-// the warp's maximum of a non-negative number, decided on the bit pattern
+// the warp's maximum of a non-negative number, decided on the bit pattern; a lane with a NaN does not count
 __device__ __forceinline__ double warp_max_pos(double v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max_pos(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = max_num(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
 // The maximum only grows while a kernel runs: a warp whose value does not exceed what it reads leaves it
@@ -749,7 +749,7 @@ __device__ __forceinline__ void faces_visc64(const double* __restrict__ T, doubl
             };
         };
         smaxv = visc_point64<D>(QL, grads(0), gamma - 1.0, kmu, av);
-        smaxv = vp.vmax * max_pos(smaxv, visc_point64<D>(QR, grads(1), gamma - 1.0, kmu, av));
+        smaxv = vp.vmax * max_num(smaxv, visc_point64<D>(QR, grads(1), gamma - 1.0, kmu, av));
         // weight 1/4, both sides' mean, twice the gradients times h: mu / (16 h), in units of the inviscid weight
         constexpr double wq = FLUX == HYPE_FLUX_RUSANOV ? 0.125 : 0.25;
         const double wv = -(1. / 16.) / wq * vp.mu * vp.r1_h;

@@ -98,11 +98,16 @@ __device__ __forceinline__ bool at_least(double x, double lo) {
     const long long b = __double_as_longlong(x);
     return b >= __double_as_longlong(lo) && b <= 0x7FF0000000000000ll;
 }
-// the larger of two non-negative numbers as fmax and (a < b) ? b : a decide it, on the bit patterns: a NaN
-// in b leaves a
+// the larger of two non-negative numbers as (a < b) ? b : a decides it, on the bit patterns: a NaN in either
+// gives a
 __device__ __forceinline__ double max_pos(double a, double b) {
     const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
     return (y > x && y <= 0x7FF0000000000000ll) ? b : a;
+}
+// as fmax decides it: a NaN in one gives the other
+__device__ __forceinline__ double max_num(double a, double b) {
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return ((y > x && y <= 0x7FF0000000000000ll) || x > 0x7FF0000000000000ll) ? b : a;
 }
 
 // 1/x in the working precision of a face solver

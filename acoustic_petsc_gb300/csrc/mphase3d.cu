@@ -214,7 +214,7 @@ __device__ __forceinline__ double hllc_general(const Side& L, const Side& R, dou
         else h.mR = fma(wt, m, h.mR);
         hllc_momentum(nx, ny, nz, sum, dif, b, q2, wt * p, wY, h);
     }
-    return euler::max_pos(fabs(unL) + L.a, fabs(unR) + R.a);
+    return euler::max_num(fabs(unL) + L.a, fabs(unR) + R.a);
 }
 
 // PDErotHLLCRiemannSolver (pde.c:383-440) across an axis face of normal D: HLLC along the velocity-jump
@@ -253,7 +253,7 @@ __device__ __forceinline__ double rot_hllc7(const Side& L, const Side& R, double
         for (int q = 0; q < 2; ++q) {
             const double tx = q ? t2x : t1x, ty = q ? t2y : t1y, tz = q ? t2z : t1z;
             const double unL = fma(L.w, tz, fma(L.v, ty, L.u * tx)), unR = fma(R.w, tz, fma(R.v, ty, R.u * tx));
-            smax = euler::max_pos(smax, euler::max_pos(fabs(unL) + L.a, fabs(unR) + R.a));
+            smax = euler::max_num(smax, euler::max_num(fabs(unL) + L.a, fabs(unR) + R.a));
         }
     } else {
         const double am = euler::max_pos(L.a, R.a);
@@ -270,7 +270,7 @@ __device__ __forceinline__ double rot_hllc7(const Side& L, const Side& R, double
             const double un = fma(L.w, tz, fma(L.v, ty, L.u * tx));
             const double SL = un - am, SR = un + am, Ss = un + e;
             const int sel = hllc_select(SL, SR, Ss);
-            smax = euler::max_pos(smax, fabs(un) + am);
+            smax = euler::max_num(smax, fabs(un) + am);
             if (sel == 4) continue;
             const bool left = sel <= 1;
             double m = un, wY = 0.0;
@@ -594,8 +594,8 @@ __device__ __forceinline__ void faces(const double* __restrict__ T, double* __re
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        smax = euler::max_pos(smax, __shfl_xor_sync(0xffffffffu, smax, o));
-        smaxv = euler::max_pos(smaxv, __shfl_xor_sync(0xffffffffu, smaxv, o));
+        smax = euler::max_num(smax, __shfl_xor_sync(0xffffffffu, smax, o));
+        smaxv = euler::max_num(smaxv, __shfl_xor_sync(0xffffffffu, smaxv, o));
     }
     if (lane == 0) {
         raise_max(&ds->smax_bits[slot], smax);

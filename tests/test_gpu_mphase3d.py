@@ -138,3 +138,23 @@ def test_mp3d_rejects_bad_parameters(hype):
     for kw in (dict(boundaries=(0, 2, 2, 2, 2, 2)), dict(eos=(1.0, 0.0, 1.6, 0.0)), dict(mu=(-1.0, 0.0))):
         with pytest.raises(hype.HypeError):
             hype.Multiphase3D(8, 8, 8, 0.1, **kw)
+
+
+def test_mp3d_wave_speeds_beside_nan(hype, oracle):
+    """a plane of NaN at i = 0, the first lane of every warp that runs along x, leaves the speed maximum to the finite
+    faces, the fast cells of row j = k = 0 among them: dt is the checker's to its rounding (no comparison with a NaN
+    holds there)"""
+    n = (32, 4, 4)
+    V = np.zeros((n[2], n[1], n[0], 6))
+    V[..., 0] = V[..., 4] = 1.0
+    V[..., 5] = 0.5
+    V[0, 0, 15:27, 1] = 2.0 * np.sin(np.pi * (np.arange(12) + 0.5) / 12)
+    cfg = oracle.mp3d_cfg(n, 0.1, cfl=0.9, mu=(0.0, 0.0))
+    U = oracle.mp3d_prim2cons(cfg, V)
+    U[:, :, 0] = np.nan
+    dt = oracle.mp3d_rhs(cfg, U)[1]
+    V[..., 1] = 0.0
+    assert dt < 0.8 * oracle.mp3d_rhs(cfg, oracle.mp3d_prim2cons(cfg, V))[1]
+    s = hype.Multiphase3D(*n, 0.1, CFL=0.9, mu=(0.0, 0.0))
+    s.RHSFunctionPrimitive(0.0, U)
+    assert abs(s.dt - dt) <= 1e-13 * dt
