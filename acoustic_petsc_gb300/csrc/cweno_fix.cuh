@@ -262,9 +262,9 @@ __device__ __forceinline__ bool recon_fix(const double* __restrict__ s, bool str
 // trace (rho, normal, two tangential momenta, E), each to 2^-59 before its rounding to FP64.  Numbers are
 // 64-bit significands with an exponent; only sums align.  18 FP64 operations (a reciprocal, a root, 9 products
 // and sums) become about 290 integer ones, a third of their issue time.  False (the caller takes the FP64
-// form, which also decides on the floors) for a density below 2^-45, a pressure below 2^-38 or not positive, a
-// normal momentum or velocity that is subnormal (its exponent would not fit), and anything not finite or beyond
-// 2^200 (gamma: 2^100).
+// form, which also decides on the floors) for a density below 2^-45, a pressure below 2^-38 or not positive,
+// and anything not finite or beyond 2^200 (gamma: 2^100).  A normal momentum or velocity that is not a normal number
+// (2^-1021 and less, whose exponent has no place in the result) counts as zero.
 __host__ __device__ __forceinline__ bool side_fix(double rho, double mn, double m1, double m2, double E, double gamma, double gm1,
                                                   double& un, double& p, double& sp) {
     constexpr u64 FRAC = 0xFFFFFFFFFFFFFull, ONE = 0x10000000000000ull;
@@ -273,7 +273,7 @@ __host__ __device__ __forceinline__ bool side_fix(double rho, double mn, double 
     const int x0 = (int)(b0 >> 52) & 0x7FF, x1 = (int)(b1 >> 52) & 0x7FF, x2 = (int)(b2 >> 52) & 0x7FF;
     const int xm = x0 > x1 ? (x0 > x2 ? x0 : x2) : (x1 > x2 ? x1 : x2);
     if ((unsigned)(xr - (1023 - 45)) > 245u || (unsigned)(xe - (1023 - 100)) > 300u || xm > 1223 ||
-        (int)((u64)bits_of(gamma) >> 52) > 1123 || ((b0 << 1) != 0 && (x0 == 0 || x0 - xr < -1021)))
+        (int)((u64)bits_of(gamma) >> 52) > 1123)
         return false;
     const int er = xr - 1023, ee = xe - 1023, em = xm - 1023;
     const u64 y = recip64(((br & FRAC) | ONE) << 11);  // 1/rho = y 2^(-64 - er)
@@ -306,7 +306,8 @@ __host__ __device__ __forceinline__ bool side_fix(double rho, double mn, double 
     // |u_n| = U 2^(e0 - er - 63)
     const u64 U = x0 ? umulhi(((b0 & FRAC) | ONE) << 11, y) : 0;
     const int u1 = (int)((U >> 63) ^ 1), e0 = x0 - 1023;
-    un = from_bits((x0 ? (u64)bits_of(pack(U << u1, e0 - er - 63 - u1)) : 0ull) | (b0 & 0x8000000000000000ull));
+    const int least = xr - 1022 > 0 ? xr - 1022 : 0;
+    un = from_bits((x0 > least ? (u64)bits_of(pack(U << u1, e0 - er - 63 - u1)) : 0ull) | (b0 & 0x8000000000000000ull));
     const int xu = e0 - er - 62, xc = x / 2 - 31, xs = xu > xc ? xu : xc;
     const u64 S = shift_by(U >> 1, xs - xu) + shift_by(C, xs - xc);
     const int c2 = clz64(S);

@@ -108,16 +108,17 @@ def test_face_states(host):
 
 @pytest.mark.parametrize("rho", [8.0, 1e3, 1e6, 2.0 ** 199, 0.7, 1.5])
 def test_face_states_of_vanishing_momenta(host, rho):
-    """velocities down to the smallest numbers: where side_fix takes the state, m / rho as the division gives it; the
-    others it leaves to the FP64 form"""
+    """velocities down to the smallest numbers: m / rho to 2^-52, or, where it or the momentum is not a normal number,
+    zero with the momentum's sign"""
     mn = np.concatenate([10.0 ** np.arange(-300.0, -307.5, -0.25), [5e-308, 3e-308, 2.3e-308, 2.2250738585072014e-308,
                                                                       1e-308, 1e-310, 5e-324, 0.0]])
     mn = np.concatenate([mn, -mn])
     q = np.zeros((mn.size, 5))
     q[:, 0], q[:, 1], q[:, 4] = rho, mn, 2.5 * rho
     out = _sides(host, q, 1.4)
-    taken = out[:, 0] != 0
     want = mn / rho
-    assert (np.abs(out[taken, 1] - want[taken]) <= 2.0 ** -52 * np.abs(want[taken])).all()
-    assert (np.abs(out[taken, 2] - 0.4 * 2.5 * rho) <= 1e-15 * rho).all()
-    assert taken[mn == 0.0].all() and taken[np.abs(mn) / rho > 1e-307].all()
+    assert out[:, 0].all() and (np.signbit(out[:, 1]) == np.signbit(mn)).all()
+    normal = (np.abs(want) >= 2.0 ** -1020) & (np.abs(mn) >= 2.0 ** -1022)
+    assert (np.abs(out[normal, 1] - want[normal]) <= 2.0 ** -52 * np.abs(want[normal])).all()
+    assert (np.abs(out[~normal, 1]) <= np.abs(want[~normal]) * (1 + 2.0 ** -52)).all()
+    assert (np.abs(out[:, 2] - 0.4 * 2.5 * rho) <= 1e-15 * rho).all()
