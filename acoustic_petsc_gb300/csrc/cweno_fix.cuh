@@ -17,9 +17,12 @@
 // About 4300 instructions a warp and variable against 361 FP64 ones of 64 cycles.  At 256^3, four stages: all in
 // FP64 237.7 ms; integers with the weights in FP64 (67 operations) 80.3; that with products of 32-bit halves
 // 76.7; integer weights 73; conversions by instruction 66.4; eps added once 63.0.
-// Errors: 2^-57 of the stencil's largest magnitude, where the FP64 form has a few 2^-53.  A cell whose own
-// value is more than 8 times below the largest of its stencil (a strong shock in density, energy or
-// pressure) or whose stencil is not finite keeps the FP64 form, whose error there is relative to the cell.
+// Errors against 128-bit arithmetic, for stencils of a jump with noise beside it: 0.9e-16 of the stencil's largest
+// magnitude, where the FP64 form has 2 to 4e-16; and of the traces themselves 5e-16, as the FP64 form's, however quiet
+// the cell.  For that the FP64 form keeps the cells whose density, energy or pressure lies four or more binary
+// exponents below its stencil's largest (from a factor 8 to 16 on) or whose polynomial, of any variable, the nonlinear
+// weights leave below 2^-4 of it (faint); and stencils that are not finite.  With R4 alone a trace holds 1/64 of the
+// largest at least, and 3e-15 of itself.
 #pragma once
 
 #include "cweno64.cuh"
@@ -35,9 +38,9 @@ struct PolyFix {
     int top;
 };
 
-// the largest biased exponent of the stencil, not below 2^-959 (so that every result is a normal number)
+// the largest biased exponent of the stencil
 __host__ __device__ __forceinline__ int stencil_top(const double* __restrict__ s) {
-    int top = 64;
+    int top = 0;
 #pragma unroll
     for (int i = 0; i < 33; ++i) {
         const int e = (int)(bits_of(s[i]) >> 52) & 0x7FF;
@@ -45,15 +48,25 @@ __host__ __device__ __forceinline__ int stencil_top(const double* __restrict__ s
     }
     return top;
 }
-// whether the fixed-point form applies: finite, results in range, and (strict) the cell's own
-// value within a factor 8 of the largest
+// whether the fixed-point form applies: finite, all zero or with every result a normal number (not below 2^-959), and
+// (strict) the cell's own value at most three binary exponents below the largest, a factor of 8 to 16
 __host__ __device__ __forceinline__ bool fix_applies(double u0, int top, bool strict) {
-    return top <= 2000 && !(strict && (((int)(bits_of(u0) >> 52) & 0x7FF) < top - 3));
+    return (top == 0 || top >= 64) && top <= 2000 && !(strict && (((int)(bits_of(u0) >> 52) & 0x7FF) < top - 3));
+}
+// whether the polynomial is so much smaller than its stencil (a quiet cell beside a jump: the weights far from linear,
+// cell value and limited derivatives below 2^-4 of the largest's power of two) that the stencil's units do not resolve
+// it as FP64 does; on the upper words
+__host__ __device__ __forceinline__ bool faint(const PolyFix& p) {
+    auto mag = [](i64 x) { return (unsigned)((int)(x >> 32) ^ (int)(x >> 63)); };
+    const unsigned l = mag(p.lin[0]) | mag(p.lin[1]) | mag(p.lin[2]), q = mag(p.sq[0]) | mag(p.sq[1]) | mag(p.sq[2]),
+                   x = mag(p.cr2[0]) | mag(p.cr2[1]) | mag(p.cr2[2]);
+    return p.wr < 1ull << 60 && (mag(p.u0) | (l >> 2) | (q >> 3) | (x >> 4)) < 1u << (58 - 4 - 32);
 }
 
 template <bool LINEAR>
 __host__ __device__ __forceinline__ void poly_fix(const double* __restrict__ s, int top, PolyFix& p) {
     i64 A[3], D[3], dp[3], dm[3];
+    top = top > 64 ? top : 64;
     auto v = [&](int i) { return to_fixed<6>(bits_of(s[i]), top); };
     p.top = top;
     const i64 u0 = v(0);
@@ -159,6 +172,23 @@ __host__ __device__ __forceinline__ void poly_fix(const double* __restrict__ s, 
     i64 o[6];  // w_k - wr g_k of the one-sided stencils, 2^62 for one
 #pragma unroll
     for (int k = 0; k < 6; ++k) o[k] = (i64)(shift_by(umulhi(y4[2 + k], rs), 4 * (x[2 + k] - xm) + 9 - z) - sub);
+    {
+        // The weights are off by 2^-57 of each and of their common factor, so their sum by up to 2^-50.  The combination
+        // below gives the centred stencil one minus the six; where a jump has suppressed that stencil, the largest of
+        // the six takes the difference instead.  o0: the centred stencil's share of w4 / gammaHi and its own weight.
+        const i64 o0 = (i64)(2 * umulhi(p.wr, 16094784204311583785ull) +
+                             shift_by(umulhi(umulhi(y4[1], rt), 9407839477591871324ull), 4 * (x[1] - xm) + 3 - z));
+        i64 rest = (1ll << 62) - o0, most = o0;
+        int at = -1;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            rest -= o[k];
+            at = o[k] > most ? k : at;
+            most = o[k] > most ? o[k] : most;
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) o[k] += at == k ? rest : 0;
+    }
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const i64 f = times62(split(dp[a]), split(o[2 * a])), g = times62(split(dm[a]), split(o[2 * a + 1]));
@@ -245,13 +275,14 @@ __device__ __forceinline__ void store_grad_coeffs(const PolyFix& p, double* __re
 }
 
 // the 24 traces of one variable's stencil, trace q at T[q * st], and with the fixed-point form not applying
-// (fix_applies) false and nothing stored
+// (fix_applies; faint, where nothing bounds the cell's own value) false and nothing stored
 template <bool LINEAR>
-__device__ __forceinline__ bool recon_fix(const double* __restrict__ s, bool strict, double* __restrict__ T, long long st,
+__host__ __device__ __forceinline__ bool recon_fix(const double* __restrict__ s, bool strict, double* __restrict__ T, long long st,
                                           PolyFix& p) {
     const int top = stencil_top(s);
     if (!fix_applies(s[0], top, strict)) return false;
     poly_fix<LINEAR>(s, top, p);
+    if (!LINEAR && !strict && faint(p)) return false;
     traces_fix(p, [&](int q, double v) { T[q * st] = v; });
     return true;
 }
