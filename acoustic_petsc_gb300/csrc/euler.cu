@@ -347,10 +347,35 @@ __device__ __noinline__ void recon64_general(const double* __restrict__ p, int s
     if (C) store_grad_coeffs(poly, C, NE);
 }
 
+// What a fixed-point polynomial stays above in its cell, and what its magnitude stays below: FP32 numbers on the
+// safe side, from the upper words; values outside 2^-100 to 2^117 give none
+__device__ __forceinline__ float above_all(const PolyFix& p) {
+    if ((unsigned)(p.top - 923) > 217u) return -INFINITY;
+    return __int2float_rd((int)((p.u0 - (i64)spread_fix(p)) >> 32)) * __int_as_float((p.top - 1049 + 127) << 23);
+}
+__device__ __forceinline__ float below_all(const PolyFix& p) {
+    if ((unsigned)(p.top - 923) > 217u) return p.top > 923 ? INFINITY : 7.9e-31f;  // 2^-100
+    const u64 u = (u64)(p.u0 < 0 ? -p.u0 : p.u0);
+    return __uint2float_ru((unsigned)((u + spread_fix(p)) >> 32) + 1u) * __int_as_float((p.top - 1049 + 127) << 23);
+}
+
+// The CWENO4 traces of one variable in one cell that the gate sends there; returns the bound (ends: density and
+// energy, above_all; the momenta, below_all).  A call, so that k_recon64's R4 form does not hold its registers.
+__device__ __noinline__ float gated_cweno4(const double* __restrict__ p, int sy, int sz, double* __restrict__ T, long long NE,
+                                           bool ends) {
+    double s[33];
+    gather33g<double>(p, sy, sz, s);
+    PolyFix fix;
+    if (recon_fix<false>(s, ends, T, NE, fix)) return ends ? above_all(fix) : below_all(fix);
+    recon64_general<false>(p, sy, sz, T, nullptr, NE);
+    return ends ? -INFINITY : INFINITY;
+}
+
 template <int RECON, bool PAD>
 __global__ void __launch_bounds__(kReconThreads, 8)
     k_recon64(const double* __restrict__ G, double* __restrict__ T, Geo g, double gm1,
-              unsigned long long* __restrict__ counters, double* __restrict__ C4) {
+              unsigned long long* __restrict__ counters, double* __restrict__ C4, const unsigned char* __restrict__ flag,
+              float* __restrict__ bound) {
     const unsigned e = blockIdx.x * (unsigned)kReconThreads + threadIdx.x;
     if (e >= (unsigned)g.NE) return;
     const unsigned row = e / (unsigned)g.ex, pl = row / (unsigned)g.ey;
@@ -371,6 +396,14 @@ __global__ void __launch_bounds__(kReconThreads, 8)
             double cf[20];
             weno3<double>(s, cf);
             store_traces<double>(T, g, e, c, cf);
+        } else if constexpr (RECON == HYPE_RECON_LEARNED) {
+            const bool ends = c == 0 || c == 4;
+            PolyFix fix;
+            float b = ends ? -INFINITY : INFINITY;
+            if (__ldg(flag + e)) b = gated_cweno4(Gc, sy, sz, Tc, g.NE, ends);
+            else if (recon_fix<true>(s, ends, Tc, g.NE, fix)) b = ends ? above_all(fix) : below_all(fix);
+            else recon64_general<true>(Gc, sy, sz, Tc, nullptr, g.NE);
+            bound[c * g.NE + e] = b;
         } else {
             constexpr bool linear = RECON == HYPE_RECON_LINEAR4;
             PolyFix fix;
@@ -389,10 +422,49 @@ __global__ void __launch_bounds__(kReconThreads, 8)
 static void launch_recon64(const Geo& g, const double* G, double* T, int recon, int pad, double gm1,
                            unsigned long long* counters, double* C4, cudaStream_t st) {
     const dim3 gr(cdiv(g.NE, kReconThreads), pad ? 1 : NV);
-    auto go = [&](auto kern) { kern<<<gr, kReconThreads, 0, st>>>(G, T, g, gm1, counters, C4); };
+    auto go = [&](auto kern) { kern<<<gr, kReconThreads, 0, st>>>(G, T, g, gm1, counters, C4, nullptr, nullptr); };
     if (recon == HYPE_RECON_WENO3) pad ? go(k_recon64<HYPE_RECON_WENO3, true>) : go(k_recon64<HYPE_RECON_WENO3, false>);
     else if (recon == HYPE_RECON_LINEAR4) pad ? go(k_recon64<HYPE_RECON_LINEAR4, true>) : go(k_recon64<HYPE_RECON_LINEAR4, false>);
     else pad ? go(k_recon64<HYPE_RECON_CWENO4, true>) : go(k_recon64<HYPE_RECON_CWENO4, false>);
+}
+
+// The gated FP64 reconstruction's second pass.  k_recon64 took each variable through CWENO4 or R4 by the cell's flag
+// and left a bound of its polynomial; where the bounds keep density and pressure above the floors (all but a few
+// cells), the 24 traces need not be read.  A cell whose R4 traces break them is redone here with CWENO4, then first
+// order with the fallback.
+// 256^3 blast: one kernel for scoring, a cell's variables in turn, and a check that read its 120 traces back, ran at
+// 104.8 M cell-updates/s, below CWENO4 without a gate; a block of 32 cells x 5 variables for all of it at 134.7 M; this, with k_gate's flags, 197.4 M.
+constexpr int kGatedThreads = 128;
+__global__ void __launch_bounds__(kGatedThreads)
+    k_gated_check(const double* __restrict__ G, double* __restrict__ T, Geo g, double gm1, int pad,
+                  const unsigned char* __restrict__ flag, const float* __restrict__ bound,
+                  unsigned long long* __restrict__ counters) {
+    const unsigned e = blockIdx.x * (unsigned)kGatedThreads + threadIdx.x, row = e / (unsigned)g.ex, pl = row / (unsigned)g.ey;
+    const int i = (int)(e - row * (unsigned)g.ex) - 1, j = (int)(row - pl * (unsigned)g.ey) - 1, k = (int)pl - 1;
+    const int gi = (i < 0 || i >= g.nx), gj = (j < 0 || j >= g.ny), gk = (k < 0 || k >= g.nz);
+    const bool active = e < (unsigned)g.NE && gi + gj + gk <= 1, owned = active && !(gi | gj | gk);
+    const bool full = active && __ldg(flag + e);
+    if (active) {
+        const float* b = bound + e;
+        const float rho = __ldg(b), mx = __ldg(b + g.NE), my = __ldg(b + 2 * g.NE), mz = __ldg(b + 3 * g.NE), E = __ldg(b + 4 * g.NE);
+        const float kin = 0.5f * (mx * mx + my * my + mz * mz) / rho;
+        // on the safe side of the FP32 roundings; false for infinities and NaN
+        const bool clear = rho > 1.001e-14f && (E - kin) - 1e-4f * (E + kin) > 1.001e-12f / (float)gm1;
+        bool ok = clear || traces_admissible<double>(T, g, e, gm1);
+        const long long ge = ghost_index(g, i, j, k);
+        if (!ok && !full) {
+#pragma unroll 1
+            for (int c = 0; c < NV; ++c)
+                gated_cweno4(G + (long long)c * g.GN + ge, g.gx, g.gx * g.gy, T + (long long)c * NTR * g.NE + e, g.NE, c == 0 || c == 4);
+            ok = traces_admissible<double>(T, g, e, gm1);
+        }
+        if (!ok && pad) {  // CWENO4 itself inadmissible
+            store_first_order_g<double>(G, T, g, ge, e);
+            if (owned) atomicAdd(&counters[1], 1ull);
+        }
+    }
+    const int flagged = __syncthreads_count(full && owned);
+    if (threadIdx.x == 0 && flagged) atomicAdd(&counters[0], (unsigned long long)flagged);
 }
 
 // Indicator-gated reconstruction: the network scores the cell from its three
@@ -400,11 +472,10 @@ static void launch_recon64(const Geo& g, const double* G, double* T, int recon, 
 // CWENO4, the others the linear R4 -- unless the linear traces give a density
 // or pressure below the floors at any face Gauss point, in which case the cell
 // is redone with CWENO4 (positivity fallback).
-template <typename R>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
-    k_recon_learned(const R* __restrict__ G, R* __restrict__ T, Geo g, const mlp::MmaWeights* __restrict__ wts,
+__global__ void __launch_bounds__(128, 4)
+    k_recon_learned(const float* __restrict__ G, float* __restrict__ T, Geo g, const mlp::MmaWeights* __restrict__ wts,
                     float logit_thr, double gm1, int pad, unsigned long long* __restrict__ counters) {
-    // per warp: the staged network inputs, later the FP32 admissibility scratch
+    // per warp: the staged network inputs, later the admissibility scratch
     static_assert(mlp::ROWS * mlp::RSTRIDE * sizeof(__nv_bfloat16) >= 2 * NTR * 32 * sizeof(float), "scratch");
     __shared__ __align__(16) __nv_bfloat16 rows[4][mlp::ROWS * mlp::RSTRIDE];
     __shared__ float lg[4][mlp::ROWS];
@@ -422,7 +493,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
     __nv_bfloat16* my_rows = rows[threadIdx.y] + threadIdx.x * 3 * mlp::RSTRIDE;
     float sc[NV];
     if (active) {
-        const float rho = (float)__ldg(G + ge), E = (float)__ldg(G + 4 * g.GN + ge);
+        const float rho = __ldg(G + ge), E = __ldg(G + 4 * g.GN + ge);
 #pragma unroll
         for (int c = 0; c < NV; ++c) sc[c] = mlp::var_scale<float>(c, rho, E);
     }
@@ -433,13 +504,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
         if (active) {
 #pragma unroll
             for (int c = 0; c < NV; ++c) {
-                const R* p = G + (long long)c * g.GN + ge;
-                float s5[5];
-#pragma unroll
-                for (int o = 0; o < 5; ++o) {
-                    if constexpr (sizeof(R) == sizeof(double)) s5[o] = narrow_fix(__ldg(p + (o - 2) * st));
-                    else s5[o] = __ldg(p + (o - 2) * st);
-                }
+                const float* p = G + (long long)c * g.GN + ge;
+                const float s5[5] = {__ldg(p - 2 * st), __ldg(p - st), __ldg(p), __ldg(p + st), __ldg(p + 2 * st)};
                 mlp::normalise5(s5, sc[c], x + c * 5);
             }
         }
@@ -452,7 +518,6 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
                                                                        lg[threadIdx.y][threadIdx.x * 3 + 2]));
     if (active) {
         const long long e = ext_index(g, i, j, k);
-        constexpr bool f32 = sizeof(R) == sizeof(float);
         TraceCheck ck{reinterpret_cast<float*>(rows[threadIdx.y]) + threadIdx.x, (float)gm1, true};
         bool full = best > logit_thr;
 #pragma unroll 1
@@ -460,28 +525,15 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 4 : 1)
             ck.ok = true;
 #pragma unroll 1
             for (int c = 0; c < NV; ++c) {
-                R s[33];
-                const R* Gc = G + (long long)c * g.GN + ge;
-                gather33g<R>(Gc, sy, sz, s);
-                if constexpr (f32) {
-                    R cf[20];
-                    cweno4<R>(s, !full, cf);
-                    store_traces<R>(T, g, e, c, cf, &ck);
-                } else {
-                    double* Tc = T + (long long)c * NTR * g.NE + e;
-                    const bool strict = c == 0 || c == 4;
-                    PolyFix fix;
-                    if (full) {
-                        if (!recon_fix<false>(s, strict, Tc, g.NE, fix)) recon64_general<false>(Gc, sy, sz, Tc, nullptr, g.NE);
-                    } else {
-                        if (!recon_fix<true>(s, strict, Tc, g.NE, fix)) recon64_general<true>(Gc, sy, sz, Tc, nullptr, g.NE);
-                    }
-                }
+                float s[33], cf[20];
+                gather33g<float>(G + (long long)c * g.GN + ge, sy, sz, s);
+                cweno4<float>(s, !full, cf);
+                store_traces<float>(T, g, e, c, cf, &ck);
             }
-            if (f32 ? ck.ok : traces_admissible<R>(T, g, e, gm1)) break;
+            if (ck.ok) break;
             if (full) {  // CWENO4 itself inadmissible: first order (when enabled)
                 if (pad) {
-                    store_first_order_g<R>(G, T, g, ge, e);
+                    store_first_order_g<float>(G, T, g, ge, e);
                     if (!gi && !gj && !gk) atomicAdd(&cnt[1], 1u);
                 }
                 break;
@@ -964,14 +1016,19 @@ __device__ __forceinline__ bool fs_admissible(const float* __restrict__ S, int t
     return ok;
 }
 
-// The learned gate of the fused FP32 stage, scored ahead of it from the ghosted FP32 copy: one
+// The learned gate of the fused FP32 stage and of the FP64 reconstruction, scored ahead of them from the ghosted copy: one
 // byte per extended cell, 1 where the network's largest directional logit exceeds the threshold.
 // Scored are the cells the stage reconstructs (the owned cells and the one-cell frame without its
 // edges and corners, which keep the zero the array is created with).  The features, their BF16
 // rounding and the tensor-core scoring are k_recon_learned's, so the flags are that kernel's
 // decisions bit for bit.  Block: 32 x 4 cells of one x-y plane, as k_recon_learned.
-__global__ void __launch_bounds__(128) k_gate_f32(const float* __restrict__ G, unsigned char* __restrict__ flag, Geo g,
-                                                  const mlp::MmaWeights* __restrict__ wts, float logit_thr) {
+template <typename R>
+__global__ void __launch_bounds__(128) k_gate(const R* __restrict__ G, unsigned char* __restrict__ flag, Geo g,
+                                              const mlp::MmaWeights* __restrict__ wts, float logit_thr) {
+    auto ld = [](const R* p) {
+        if constexpr (sizeof(R) == sizeof(double)) return narrow_fix(__ldg(p));
+        else return __ldg(p);
+    };
     __shared__ __align__(16) __nv_bfloat16 rows[4][mlp::ROWS * mlp::RSTRIDE];
     __shared__ float lg[4][mlp::ROWS];
     const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
@@ -981,10 +1038,10 @@ __global__ void __launch_bounds__(128) k_gate_f32(const float* __restrict__ G, u
     const bool active = i <= g.nx && j <= g.ny && gi + gj + gk <= 1;
     const long long ge = active ? ghost_index(g, i, j, k) : 0;
     __nv_bfloat16* my_rows = rows[threadIdx.y] + threadIdx.x * 3 * mlp::RSTRIDE;
-    const float* Gc = G + ge;  // variable c at Gc[c * GN + offset]
+    const R* Gc = G + ge;  // variable c at Gc[c * GN + offset]
     float sc[NV];
     if (active) {
-        const float rho = __ldg(Gc), E = __ldg(Gc + 4 * g.GN);
+        const float rho = ld(Gc), E = ld(Gc + 4 * g.GN);
 #pragma unroll
         for (int c = 0; c < NV; ++c) sc[c] = mlp::var_scale<float>(c, rho, E);
     }
@@ -998,9 +1055,9 @@ __global__ void __launch_bounds__(128) k_gate_f32(const float* __restrict__ G, u
             float s5[NV][5];
 #pragma unroll
             for (int c = 0; c < NV; ++c) {
-                const float* p = Gc + (long long)c * g.GN;
+                const R* p = Gc + (long long)c * g.GN;
 #pragma unroll
-                for (int o = 0; o < 5; ++o) s5[c][o] = __ldg(p + (o - 2) * stp);
+                for (int o = 0; o < 5; ++o) s5[c][o] = ld(p + (o - 2) * stp);
             }
 #pragma unroll
             for (int c = 0; c < NV; ++c) mlp::normalise5(s5[c], sc[c], x + c * 5);
@@ -1043,7 +1100,7 @@ __global__ void __launch_bounds__(128) k_gate_dilate(const unsigned char* __rest
     o[((long long)k * ey + j) * g.ex + i] = (unsigned char)m;
 }
 
-// LEARNED: the indicator gate of k_recon_learned, read from the flags k_gate_f32 wrote for this
+// LEARNED: the indicator gate of k_recon_learned, read from the flags k_gate wrote for this
 // stage's input: flagged cells take CWENO4, the others R4, and a cell whose R4 traces break the
 // floors is redone with CWENO4 (then first order with the positivity fallback)
 template <bool LEARNED>
@@ -1404,6 +1461,9 @@ struct hype_euler {
     // once per step, their one-cell widening that the step's stages read
     unsigned char* gate = nullptr;
     unsigned char* gate_wide = nullptr;
+    // the gated FP64 reconstruction: flags, and a bound of each variable's polynomial, per extended cell
+    unsigned char* flag64 = nullptr;
+    float* bound64 = nullptr;
     int gate_per_step = 0;
     float logit_thr = 0.0f;
     unsigned long long* mlp_cnt = nullptr;
@@ -1488,11 +1548,18 @@ static int launch_rhs(hype_euler* e, const double* Win, int slot) {
     if (e->p.recon == HYPE_RECON_LEARNED) {
         if (!e->mlp) return HYPE_ERR_ARG;  // hype_euler_set_mlp first
         if (f32)
-            k_recon_learned<float><<<gr, br, 0, e->stream>>>((const float*)e->G, (float*)e->T, g, e->mlp, e->logit_thr, gm1,
-                                                             e->p.positivity, e->mlp_cnt);
-        else
-            k_recon_learned<double><<<gr, br, 0, e->stream>>>((const double*)e->G, (double*)e->T, g, e->mlp, e->logit_thr,
-                                                              gm1, e->p.positivity, e->mlp_cnt);
+            k_recon_learned<<<gr, br, 0, e->stream>>>((const float*)e->G, (float*)e->T, g, e->mlp, e->logit_thr, gm1,
+                                                      e->p.positivity, e->mlp_cnt);
+        else {
+            const double* G = (const double*)e->G;
+            double* T = (double*)e->T;
+            k_gate<double><<<gr, br, 0, e->stream>>>(G, e->flag64, g, e->mlp, e->logit_thr);
+            k_recon64<HYPE_RECON_LEARNED, false><<<dim3(cdiv(g.NE, kReconThreads), NV), kReconThreads, 0, e->stream>>>(
+                G, T, g, gm1, e->mlp_cnt, nullptr, e->flag64, e->bound64);
+            k_gated_check<<<cdiv(g.NE, kGatedThreads), kGatedThreads, 0, e->stream>>>(G, T, g, gm1, e->p.positivity, e->flag64,
+                                                                                     e->bound64, e->mlp_cnt);
+            HYPE_LAUNCHED(2);
+        }
     } else if (f32) {
         k_recon_f32<<<gr, br, ck_bytes, e->stream>>>((const float*)e->G, (float*)e->T, g, rec, e->p.positivity, gm1,
                                                      e->mlp_cnt);
@@ -1577,7 +1644,7 @@ static int launch_stage(hype_euler* e, const double* Win, const double* U, const
     const bool score = learned && (!e->gate_per_step || slot == 0 || slot == 4);
     if (score) {
         const dim3 br(32, 4), gr(cdiv(g.nx + 2, 32), cdiv(g.ny + 2, 4), g.nz + 2);
-        k_gate_f32<<<gr, br, 0, e->stream>>>((const float*)e->G, e->gate, g, e->mlp, e->logit_thr);
+        k_gate<float><<<gr, br, 0, e->stream>>>((const float*)e->G, e->gate, g, e->mlp, e->logit_thr);
         if (e->gate_per_step)
             k_gate_dilate<<<dim3(cdiv(g.ex, 128), g.ny + 2, g.nz + 2), 128, 0, e->stream>>>(e->gate, e->gate_wide, g);
     }
@@ -1727,7 +1794,7 @@ extern "C" void hype_euler_destroy(hype_euler* e) {
     if (e->stream) cudaStreamSynchronize(e->stream);
     cudaFree(e->U); cudaFree(e->W); cudaFree(e->L); cudaFree(e->S); cudaFree(e->T);
     cudaFree(e->Fx); cudaFree(e->Fy); cudaFree(e->Fz); cudaFree(e->stage_aos); cudaFree(e->ds); cudaFree(e->G);
-    cudaFree(e->mlp); cudaFree(e->gate); cudaFree(e->gate_wide); cudaFree(e->mlp_cnt); cudaFree(e->C4); cudaFree(e->mon); cudaFree(e->acc);
+    cudaFree(e->mlp); cudaFree(e->gate); cudaFree(e->gate_wide); cudaFree(e->flag64); cudaFree(e->bound64); cudaFree(e->mlp_cnt); cudaFree(e->C4); cudaFree(e->mon); cudaFree(e->acc);
     if (e->hs) cudaFreeHost(e->hs);
     for (auto x : e->ev) cudaEventDestroy(x);
     if (e->step_graph) cudaGraphExecDestroy(e->step_graph);
@@ -1962,6 +2029,11 @@ extern "C" int hype_euler_set_mlp(hype_euler* e, const float* params, float prob
     for (int q = 0; q < mlp::NPARAM; ++q) h[q] = __float2bfloat16_rn(params[q]);
     mlp::MmaWeights hw;  // host staging, copied before the stream synchronisation below
     mlp::pack_weights(h.data(), hw);
+    // before the network, whose presence lets the gated kernels run
+    if (!e->bound64 && e->p.precision != HYPE_PREC_FP32) {
+        if (!e->flag64) HYPE_CK(cudaMalloc((void**)&e->flag64, (size_t)e->g.NE));
+        HYPE_CK(cudaMalloc((void**)&e->bound64, sizeof(float) * NV * (size_t)e->g.NE));
+    }
     if (!e->mlp) HYPE_CK(cudaMalloc((void**)&e->mlp, sizeof(mlp::MmaWeights)));
     if (!e->gate && e->p.precision == HYPE_PREC_FP32) {
         HYPE_CK(cudaMalloc((void**)&e->gate, (size_t)e->g.NE));

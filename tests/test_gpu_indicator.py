@@ -107,3 +107,46 @@ def test_learned_indicator_gain(hype):
           f"positivity fallbacks {fallbacks}; shadow L1 {shadow:.2e}")
     assert e_learn <= 1.05 * e_full
     assert shadow < 1e-3
+
+
+@pytest.mark.parametrize("precision", [0, 2], ids=["fp64", "df64"])
+@pytest.mark.parametrize("shape", [(13, 13, 13), (3, 5, 4), (31, 7, 6)], ids=str)
+def test_gated_fp64_redo(hype, precision, shape):
+    """the gated FP64 reconstruction's second pass.  A network that flags every cell gives plain CWENO4 with the
+    fallback, bit for bit and with its fallback count; one that flags none gives R4 except in the cells whose R4 traces
+    break the floors: equal to R4 with the floors out of reach, and on a blast that plain R4 refuses, equal to the FP32
+    form, whose decisions are the same there, to FP32's accuracy (weights are fourth powers of sums of squares, some 100
+    roundings of 6e-8 that the jump of ten multiplies: below 1e-4 of the largest; a wrong branch differs by a tenth)"""
+    from acoustic_petsc_gb300 import _lib as L, indicator
+
+    nx, ny, nz = shape
+    rng = np.random.default_rng(nx)
+    r2 = sum(((np.arange(m) + 0.5) / m - 0.5).reshape(s) ** 2 for m, s in ((nz, (-1, 1, 1)), (ny, (1, -1, 1)), (nx, (1, 1, -1))))
+    mild = np.zeros((nz, ny, nx, 5))
+    mild[..., 0] = np.where(r2 < 0.06, 1.6, 1.0)
+    mild[..., 4] = 2.5 + 0.1 * rng.random((nz, ny, nx))
+    hard = mild.copy()
+    hard[..., 0] = np.where(r2 < 0.06, 8.0, 1.0)
+    hard[..., 4] = np.where(r2 < 0.06, 17.9, 1.79)
+
+    def rhs(U, recon, prob=None, prec=precision, positivity=1):
+        s = hype.EulerSolver(hype.AppCtx(N_x=nx, N_y=ny, N_z=nz, h=1.0 / nx, CFL=0.4, boundaries=(2,) * 6, precision=prec,
+                                         recon=recon, positivity=positivity))
+        if prob is not None:
+            s.set_mlp(indicator.init_params(3), prob)
+        return s.RHSFunction(0.0, U), s.indicator_stats()
+
+    cells = nx * ny * nz
+    for U in (mild, hard):
+        R, (flagged, fallbacks) = rhs(U, L.RECON_LEARNED, 1e-30)
+        P, (_, plain) = rhs(U, L.RECON_CWENO4)
+        assert np.array_equal(R, P) and flagged == cells and fallbacks == plain
+    R, (flagged, fallbacks) = rhs(mild, L.RECON_LEARNED, 1.0 - 1e-7)
+    assert np.array_equal(R, rhs(mild, L.RECON_LINEAR4)[0]) and (flagged, fallbacks) == (0, 0)
+    with pytest.raises(hype.HypeError) as err:
+        rhs(hard, L.RECON_LINEAR4, positivity=0)
+    assert err.value.code == L.HYPE_ERR_STATE
+    R, st = rhs(hard, L.RECON_LEARNED, 1.0 - 1e-7)
+    F, st32 = rhs(hard, L.RECON_LEARNED, 1.0 - 1e-7, prec=L.PREC_FP32)
+    assert st == st32 and st[0] == 0
+    assert np.abs(R - F).max() <= 1e-4 * np.abs(R).max()
