@@ -190,7 +190,7 @@ __host__ __device__ __forceinline__ i64 to_fixed(i64 b, int top) {
     const u64 m = ((b & 0xFFFFFFFFFFFFFll) | 0x10000000000000ll) << SHIFT;
 #ifdef __CUDA_ARCH__
     i64 v;
-    asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(top - e));  // shifts of 64 and more give 0
+    asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(top - e));  // shifts of 64 and more, and negative ones, give 0
 #else
     const i64 v = (i64)(top - e < 64 ? m >> (top - e) : 0);
 #endif
@@ -320,11 +320,16 @@ static __device__ __noinline__ double sum_differences_fp64(double a1, double a0,
     return ((a1 - a0) + (b1 - b0)) + (c1 - c0);
 }
 // (a1 - a0) + (b1 - b0) + (c1 - c0) from integers in units of 2^-58 of the largest number's power of two, rounded
-// once (one FP64 operation, the conversion, for five); not finite or beyond 2^977: in FP64
+// once (one FP64 operation, the conversion, for five); not finite or beyond 2^977: in FP64.  Two equal numbers
+// cancel exactly and do not count for the units (a uniform pressure would leave a weak shear 2^-58 of itself); their
+// shift is then beyond 63 or negative, and both give 0.
 __device__ __forceinline__ double sum_differences(double a1, double a0, double b1, double b0, double c1, double c0) {
     int top = 64;
-    auto widest = [&](double x) { top = max(top, (__double2hiint(x) >> 20) & 0x7FF); };
-    widest(a1); widest(a0); widest(b1); widest(b0); widest(c1); widest(c0);
+    auto widest = [&](double x, double y) {
+        const int e = max((__double2hiint(x) >> 20) & 0x7FF, (__double2hiint(y) >> 20) & 0x7FF);
+        top = max(top, bits_of(x) == bits_of(y) && e <= 2000 ? 0 : e);
+    };
+    widest(a1, a0); widest(b1, b0); widest(c1, c0);
     if (top > 2000) return sum_differences_fp64(a1, a0, b1, b0, c1, c0);
     auto fx = [&](double x) { return to_fixed<6>(bits_of(x), top); };
     return from_fixed(((fx(a1) - fx(a0)) + (fx(b1) - fx(b0))) + (fx(c1) - fx(c0)), top);
