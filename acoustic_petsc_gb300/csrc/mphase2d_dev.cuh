@@ -176,8 +176,9 @@ __device__ __forceinline__ void mp_cell_fallback(const PT* __restrict__ P, R* __
 }
 
 // PT: the primitives' type (FP64; the FP32 form reads its FP32 copy)
-template <typename R, int MODEL, typename PT = double>
-__global__ void __launch_bounds__(128, 8) k_mp_recon(const PT* __restrict__ P, R* __restrict__ T, Geo g, Eos e,
+// MINB: see k_mp_faces
+template <typename R, int MODEL, typename PT, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_mp_recon(const PT* __restrict__ P, R* __restrict__ T, Geo g, Eos e,
                                                   DevScalars* __restrict__ ds) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y - 1;
@@ -426,9 +427,10 @@ __global__ void __launch_bounds__(128) k_mp_features(const double* __restrict__ 
 }
 
 // face fluxes stored in the solver's type (FP64; the FP32 form keeps them in FP32 for its update)
-// 64 registers, 32 warps per SM where the 103 that the compiler takes leave 16: 1024^2 Kapila, 73 -> 58 us a direction
-template <typename R, int MODEL, int D>
-__global__ void __launch_bounds__(128, 8) k_mp_faces(const R* __restrict__ T, R* __restrict__ F, Geo g, Eos e,
+// MINB 8: 64 registers, 32 warps per SM where the 103 that the compiler takes leave 16: 1024^2 Kapila, 73 -> 58 us a
+// direction.  MINB 1, for grids too small to fill the SMs' registers either way, where spilling only lengthens the chain
+template <typename R, int MODEL, int D, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_mp_faces(const R* __restrict__ T, R* __restrict__ F, Geo g, Eos e,
                                                   DevScalars* __restrict__ ds, int slot) {
     constexpr int NV = MODEL == HYPE_MP_DI4 ? 5 : 6;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

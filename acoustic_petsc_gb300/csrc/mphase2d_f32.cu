@@ -49,6 +49,11 @@ __global__ void __launch_bounds__(256) k_mp_prim_f32(const double* __restrict__ 
     }
 }
 
+// Up to these many cells the latency of one thread's chain counts, not what the SMs issue.  kOneWave: the four blocks
+// of 128 that an SM holds at 103 registers take the grid in one wave, so the reconstruction and the faces are given them.
+// kFewCells: the update then has a thread per variable.
+constexpr long long kOneWave = 152 * 4 * 128, kFewCells = 152 * 256;
+
 // the primitives, the reconstruction (plain or indicator-gated) and the two face-flux launches of one
 // RHS of the FP32 form (Pf: its FP32 primitives)
 int launch_rhs_f32(int model, bool learned, const double* Win, float* Pf, void* T, float* F, float* G, const Geo& g,
@@ -66,10 +71,17 @@ int launch_rhs_f32(int model, bool learned, const double* Win, float* Pf, void* 
         else if (learned)                                                                                      \
             k_mp_recon_learned<float, M, float><<<gr, br, 0, st>>>(P, (float*)T, g, e, ds, mlp, logit_thr,     \
                                                                    flagged);                                   \
+        else if (g.N <= kOneWave)                                                                              \
+            k_mp_recon<float, M, float, 1><<<gr, br, 0, st>>>(P, (float*)T, g, e, ds);                         \
         else                                                                                                   \
-            k_mp_recon<float, M, float><<<gr, br, 0, st>>>(P, (float*)T, g, e, ds);                            \
-        k_mp_faces<float, M, 0><<<gx, br, 0, st>>>((const float*)T, F, g, e, ds, slot);                        \
-        k_mp_faces<float, M, 1><<<gy, br, 0, st>>>((const float*)T, G, g, e, ds, slot);                        \
+            k_mp_recon<float, M, float, 8><<<gr, br, 0, st>>>(P, (float*)T, g, e, ds);                         \
+        if (g.N <= kOneWave) {                                                                                 \
+            k_mp_faces<float, M, 0, 1><<<gx, br, 0, st>>>((const float*)T, F, g, e, ds, slot);                 \
+            k_mp_faces<float, M, 1, 1><<<gy, br, 0, st>>>((const float*)T, G, g, e, ds, slot);                 \
+        } else {                                                                                               \
+            k_mp_faces<float, M, 0, 8><<<gx, br, 0, st>>>((const float*)T, F, g, e, ds, slot);                 \
+            k_mp_faces<float, M, 1, 8><<<gy, br, 0, st>>>((const float*)T, G, g, e, ds, slot);                 \
+        }                                                                                                      \
     } while (0)
     if (model == HYPE_MP_DI4) MP_LAUNCH_F32(HYPE_MP_DI4);
     else MP_LAUNCH_F32(HYPE_MP_KAPILA5);
@@ -83,31 +95,35 @@ int launch_rhs_f32(int model, bool learned, const double* Win, float* Pf, void* 
 // formed in FP64 as k_mp_update does.
 // Bound: FP64 issue; the widenings to FP64 and the stage fraction's division are the integer pipe's.
 // Win, X, Y and out may be one array (in-place stages), so they carry no __restrict__
+// EACH: a thread per variable too (blockIdx.y; the last one alone reads the volume fraction that it writes).  SMALL:
+// conversions and the division by instruction, shorter where the FP64 pipe has room
+template <bool EACH, bool SMALL>
 __global__ void __launch_bounds__(256) k_mp_update_f32(const float* __restrict__ F, const float* __restrict__ G,
                                                        const double* Win, const double* X, const double* Y, double* out,
                                                        Geo g, double r1_h, Stage st, const DevScalars* __restrict__ ds) {
-    const unsigned cell = blockIdx.x * 256u + threadIdx.x;
+    const unsigned cell = blockIdx.x * blockDim.x + threadIdx.x;
     if (cell >= (unsigned)g.N) return;
-    const int nv = g.nv, ia = nv - 1;
+    const int ia = g.nv - 1, c0 = EACH ? blockIdx.y : 0, c1 = EACH ? c0 + 1 : g.nv;
     const long long nfx = (long long)(g.nx + 1) * g.ny, nfy = (long long)g.nx * (g.ny + 1);
-    F += cell + cell / (unsigned)g.nx;  // j (nx + 1) + i
-    G += cell;
-    const double a = Win[ia * g.N + cell];
-    const double cdt = st.rhs_only ? 0.0 : euler::div_rn(st.c * ds->dt, st.d);
+    F += c0 * nfx + cell + cell / (unsigned)g.nx;  // j (nx + 1) + i
+    G += c0 * nfy + cell;
+    const double a = EACH && c0 != ia ? 0.0 : Win[ia * g.N + cell];
+    const double cdt = st.rhs_only ? 0.0 : SMALL ? st.c * ds->dt / st.d : euler::div_rn(st.c * ds->dt, st.d);
+    auto wide = [](float x) { return SMALL ? (double)x : euler::widen_fix(x); };
     const float r1hf = (float)r1_h;
     const bool two = st.b != 0.0;
-    for (int c = 0; c < nv; ++c, F += nfx, G += nfy) {
+    for (int c = c0; c < c1; ++c, F += nfx, G += nfy) {
         double L;
         if (c == ia) {
-            const double fr = euler::widen_fix(F[1]), fl = euler::widen_fix(F[0]);
-            const double ur = euler::widen_fix(F[nfx + 1]), ul = euler::widen_fix(F[nfx]);
-            const double gt = euler::widen_fix(G[g.nx]), gb = euler::widen_fix(G[0]);
-            const double vt = euler::widen_fix(G[nfy + g.nx]), vb = euler::widen_fix(G[nfy]);
+            const double fr = wide(F[1]), fl = wide(F[0]);
+            const double ur = wide(F[nfx + 1]), ul = wide(F[nfx]);
+            const double gt = wide(G[g.nx]), gb = wide(G[0]);
+            const double vt = wide(G[nfy + g.nx]), vb = wide(G[nfy]);
             L = -r1_h * ((fr - a * ur) - (fl - a * ul)) - r1_h * ((gt - a * vt) - (gb - a * vb));
         } else {
             const float dx = F[1] - F[0];
             const float dy = G[g.nx] - G[0];
-            L = euler::widen_fix(-r1hf * (dx + dy));
+            L = wide(-r1hf * (dx + dy));
         }
         double v;
         if (st.rhs_only) {
@@ -122,7 +138,9 @@ __global__ void __launch_bounds__(256) k_mp_update_f32(const float* __restrict__
 
 void launch_update_f32(const float* F, const float* G, const double* Win, const double* X, const double* Y, double* out,
                        const Geo& g, double r1_h, Stage st, const DevScalars* ds, cudaStream_t stream) {
-    k_mp_update_f32<<<cdiv(g.N, 256), 256, 0, stream>>>(F, G, Win, X, Y, out, g, r1_h, st, ds);
+    if (g.N <= kFewCells) k_mp_update_f32<true, true><<<dim3(cdiv(g.N, 64), g.nv), 64, 0, stream>>>(F, G, Win, X, Y, out, g, r1_h, st, ds);
+    else if (g.N <= kOneWave) k_mp_update_f32<false, true><<<cdiv(g.N, 128), 128, 0, stream>>>(F, G, Win, X, Y, out, g, r1_h, st, ds);
+    else k_mp_update_f32<false, false><<<cdiv(g.N, 256), 256, 0, stream>>>(F, G, Win, X, Y, out, g, r1_h, st, ds);
 }
 
 }  // namespace mp2d
