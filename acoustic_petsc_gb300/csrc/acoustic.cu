@@ -193,8 +193,10 @@ __device__ __forceinline__ void face_normal_grads_df(const df64* c, df64* __rest
 }
 
 // k_ac_recon in double-float: the CWENO4 coefficients (euler_df64.cuh) and the 24 face-
-// normal gradients, kept as pairs for k_ac_faces_df
-__global__ void __launch_bounds__(128, 2) k_ac_recon_df(const df64* __restrict__ G, df64* __restrict__ T, Geo g) {
+// normal gradients, kept as pairs for k_ac_faces_df.  linear: R4, which the host takes by the star; it stays an
+// argument because the code that the compiler makes of CWENO4 alone is slower (163 registers and three blocks per SM
+// against 208 and two, whose instruction cache holds the body: 128^3, a launch 474 us against 445)
+__global__ void __launch_bounds__(128, 2) k_ac_recon_df(const df64* __restrict__ G, df64* __restrict__ T, Geo g, int linear) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x - 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y - 1;
     const int k = blockIdx.z - 1;
@@ -226,7 +228,7 @@ __global__ void __launch_bounds__(128, 2) k_ac_recon_df(const df64* __restrict__
         for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int d = 0; d < 2; ++d) s[euler::SO(a, b, d)] = p[(2 * a - 1) + (2 * b - 1) * sy + (2 * d - 1) * sz];
-    euler::cweno4_df(s, false, cf);
+    euler::cweno4_df(s, linear != 0, cf);
     const long long e = ext_index(g, i, j, k);
     face_normal_grads_df<0>(cf, T, g.NE, e);
     face_normal_grads_df<1>(cf, T, g.NE, e);
@@ -471,7 +473,7 @@ static int ac_rhs(hype_acoustic* a, const double* Win) {
     if (a->p.precision == HYPE_PREC_DF64) {
         k_ac_ghost<df64><<<dim3(cdiv(g.gx, 128), g.gy, g.nz + 2 * GW), 128, 0, a->stream>>>(Win, (df64*)a->Gh, g);
         k_ac_recon_df<<<dim3(cdiv(g.nx + 2, 32), cdiv(g.ny + 2, 4), g.nz + 2), dim3(32, 4), 0, a->stream>>>(
-            (const df64*)a->Gh, (df64*)a->T, g);
+            (const df64*)a->Gh, (df64*)a->T, g, a->p.recon == HYPE_RECON_LINEAR4);
         const double c2 = a->p.c * a->p.c;
         const dim3 bf(32, 4);
         const df64* T = (const df64*)a->T;
