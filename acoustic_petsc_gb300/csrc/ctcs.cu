@@ -243,13 +243,14 @@ struct hype_ctcs {
     Grid g;
     cudaStream_t stream = nullptr;
     // point-source form: three rotating levels, p at cur, p_old at cur - 1 mod 3; plane-wave form: two pairs
-    // (p_old, p) of levels, the current one at 2 * pair
+    // (p_old, p) of levels, the current one at 2 * pair, or three rotating levels where a fourth does not fit the memory
     double* lv[4] = {nullptr, nullptr, nullptr, nullptr};
     int cur = 1;
     int pair = 0;
     PlaneTile tile{64, kTileRows};
-    double* newest() const { return p.form == 0 ? lv[2 * pair + 1] : lv[cur]; }
-    double* older() const { return p.form == 0 ? lv[2 * pair] : lv[(cur + 2) % 3]; }
+    bool paired() const { return lv[3] != nullptr; }
+    double* newest() const { return paired() ? lv[2 * pair + 1] : lv[cur]; }
+    double* older() const { return paired() ? lv[2 * pair] : lv[(cur + 2) % 3]; }
     double* srcv = nullptr;
     double* recv = nullptr;
     int cap = 0;  // capacity of srcv/recv
@@ -282,6 +283,11 @@ static int ctcs_launch(hype_ctcs* c, int phase) {
     double* pn = c->lv[(phase + 1) % 3];
     const dim3 b(32, 8);
     const dim3 gr(cdiv(g.nx, 32), cdiv(g.ny, 8), g.dim == 3 ? g.nz : 1);
+    if (c->p.form == 0) {
+        k_plane2d<<<gr, b, 0, c->stream>>>(po, pc, pn, g);
+        HYPE_LAUNCHED(1);
+        return HYPE_OK;
+    }
     const bool tick = (g.src >= 0 || g.rec >= 0);
     double* sv = g.src >= 0 ? c->srcv : nullptr;
     double* rv = g.rec >= 0 ? c->recv : nullptr;
@@ -331,11 +337,14 @@ extern "C" int hype_ctcs_create(const hype_ctcs_params* p, hype_ctcs** out) {
     }
     c->n = (long long)g.nx * g.ny * g.nz;
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-    const int levels = p->form == 0 ? 4 : 3;
-    for (int q = 0; q < levels && e == cudaSuccess; ++q) e = cudaMalloc((void**)&c->lv[q], sizeof(double) * c->n);
+    for (int q = 0; q < 3 && e == cudaSuccess; ++q) e = cudaMalloc((void**)&c->lv[q], sizeof(double) * c->n);
     if (e == cudaSuccess) e = cudaMalloc((void**)&c->st, sizeof(DevStep));
-    // the second pair is written whole before it is read
-    for (int q = 0; q < (p->form == 0 ? 2 : 3) && e == cudaSuccess; ++q) e = cudaMemset(c->lv[q], 0, sizeof(double) * c->n);
+    if (e == cudaSuccess && p->form == 0 && cudaMalloc((void**)&c->lv[3], sizeof(double) * c->n) != cudaSuccess) {
+        c->lv[3] = nullptr;  // a step a launch then
+        cudaGetLastError();
+    }
+    // a level beyond these is written whole before it is read
+    for (int q = 0; q < (c->paired() ? 2 : 3) && e == cudaSuccess; ++q) e = cudaMemset(c->lv[q], 0, sizeof(double) * c->n);
     int dev = 0, nsm = 1;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -405,7 +414,7 @@ static int build_chunk(hype_ctcs* c, int phase) {
     cudaGraph_t graph;
     HYPE_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int rc = HYPE_OK;
-    if (c->p.form == 0)
+    if (c->paired())
         for (int s = 0; s < kPlaneChunk && rc == HYPE_OK; ++s) rc = plane_launch(c, (phase + s) % 2, kSteps);
     else
         for (int s = 0; s < kChunk && rc == HYPE_OK; ++s) rc = ctcs_launch(c, (phase + s) % 3);
@@ -455,7 +464,7 @@ extern "C" int hype_ctcs_step(hype_ctcs* c, int nsteps, int it0, double* receive
     }
     int s = 0;
     int rc;
-    if (c->p.form == 0) {
+    if (c->paired()) {
         for (; nsteps - s >= kPlaneChunk * kSteps; s += kPlaneChunk * kSteps) {
             if (!c->chunk[c->pair] && (rc = build_chunk(c, c->pair))) return rc;
             HYPE_CK(cudaGraphLaunch(c->chunk[c->pair], c->stream));

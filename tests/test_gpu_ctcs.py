@@ -132,3 +132,34 @@ def test_plane_form_tiles_bitwise(hype, oracle, shape, bc, steps):
     a, b = lf.get()
     ao, bo = oracle.ctcs2d_plane(p0, p1, 1.0 * dt / h, bc, steps)
     assert np.array_equal(a, ao) and np.array_equal(b, bo)
+
+
+@pytest.mark.parametrize("bc", [0, 3])
+def test_plane_form_where_a_fourth_level_does_not_fit(hype, bc):
+    """with room for three and a half levels left on the device the plane-wave form is still created; it steps one
+    launch a step, with the fused form's bits"""
+    torch = pytest.importorskip("torch")
+    n = 2896  # a level of 64 MiB
+    rng = np.random.default_rng(3)
+    p0 = rng.standard_normal((n, n))
+    p1 = 0.99 * p0
+
+    def run(steps=(35, 2)):
+        lf = hype.Leapfrog(p0.shape, dx=0.1, dt=0.04, c0=1.0, form=0, bc=bc)
+        lf.set(p0, p1)
+        l0 = hype._lib.launches()
+        for s in steps:
+            lf.UpdatePressure(s)
+        out = lf.get(), hype._lib.launches() - l0
+        lf.close()
+        return out
+
+    (a, b), fused = run()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    held = torch.empty(free - 7 * n * n * 4, dtype=torch.uint8, device="cuda")
+    (c, d), single = run()
+    del held
+    torch.cuda.empty_cache()
+    assert fused < 37 <= single
+    assert np.array_equal(a, c) and np.array_equal(b, d)
