@@ -122,3 +122,24 @@ def test_update_scales(hype, scale):
         e = np.pad(c, 1)
         o, c = c, 2 * c - o + 0.25 * (e[2:, 1:-1] + e[:-2, 1:-1] + e[1:-1, 2:] + e[1:-1, :-2] - 4 * c)
     assert np.abs(p / scale - c).max() <= 1.8e-14 * np.abs(p0 / scale).max()
+
+
+@pytest.mark.parametrize("cfl", [0.7, 0.5, 0.36, 0.35, 0.2, 0.05, 1e-3])
+def test_update_ahead_of_a_wave(hype, cfl):
+    """one step from a single value: its four neighbours are a times it, a = (c0 dt / h)^2, to the rounding of FP64 or,
+    in the fixed-point form (a >= 1/8), two units of 2^-58 of the value: 2^-52 either way, 2^-51 with the product
+    that the comparison forms"""
+    n, h = 33, 0.05
+    rng = np.random.default_rng(4)
+    b = hype.BatchLeapfrog([hype.Monopole(nx=n, ny=n, xmin=-1.0, ymin=-1.0, h=h, c0=1.0, dt=cfl * h, xs=0.0, ys=0.0,
+                                          sigma=0.05, freq=0.0)], tile=(32, 64))
+    a = (cfl * h) * (cfl * h) / (h * h)
+    for _ in range(8):
+        p = np.zeros((n, n))
+        p[16, 9] = 1.0 + rng.random()
+        b.set(0, np.zeros((n, n)), p)
+        b.step(1)
+        q = b.get(0)[1]
+        for j, i in ((15, 9), (17, 9), (16, 8), (16, 10)):
+            assert abs(q[j, i] - a * p[16, 9]) <= 2.0 ** -51 * a * p[16, 9]
+        assert abs(q[16, 9] - (2 - 4 * a) * p[16, 9]) <= 2.0 ** -50 * p[16, 9]
