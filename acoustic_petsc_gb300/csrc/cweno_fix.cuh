@@ -38,9 +38,10 @@ struct PolyFix {
     int top;
 };
 
-// the largest biased exponent of the stencil
+// the largest biased exponent of the stencil, not below 2^-959 (so that every result is a normal number or zero; the
+// first cells that a disturbance reaches hold such values, to 2^-1017)
 __host__ __device__ __forceinline__ int stencil_top(const double* __restrict__ s) {
-    int top = 0;
+    int top = 64;
 #pragma unroll
     for (int i = 0; i < 33; ++i) {
         const int e = (int)(bits_of(s[i]) >> 52) & 0x7FF;
@@ -48,10 +49,10 @@ __host__ __device__ __forceinline__ int stencil_top(const double* __restrict__ s
     }
     return top;
 }
-// whether the fixed-point form applies: finite, all zero or with every result a normal number (not below 2^-959), and
-// (strict) the cell's own value at most three binary exponents below the largest, a factor of 8 to 16
+// whether the fixed-point form applies: finite, results in range, and (strict) the cell's own value at most three
+// binary exponents below the largest, a factor of 8 to 16
 __host__ __device__ __forceinline__ bool fix_applies(double u0, int top, bool strict) {
-    return (top == 0 || top >= 64) && top <= 2000 && !(strict && (((int)(bits_of(u0) >> 52) & 0x7FF) < top - 3));
+    return top <= 2000 && !(strict && (((int)(bits_of(u0) >> 52) & 0x7FF) < top - 3));
 }
 // whether the polynomial is so much smaller than its stencil (a quiet cell beside a jump: the weights far from linear,
 // cell value and limited derivatives below 2^-4 of the largest's power of two) that the stencil's units do not resolve
@@ -66,7 +67,6 @@ __host__ __device__ __forceinline__ bool faint(const PolyFix& p) {
 template <bool LINEAR>
 __host__ __device__ __forceinline__ void poly_fix(const double* __restrict__ s, int top, PolyFix& p) {
     i64 A[3], D[3], dp[3], dm[3];
-    top = top > 64 ? top : 64;
     auto v = [&](int i) { return to_fixed<6>(bits_of(s[i]), top); };
     p.top = top;
     const i64 u0 = v(0);

@@ -228,8 +228,8 @@ def test_reconstruction_of_a_quiet_cell_beside_a_jump(host, offsets, linear, str
 
 @pytest.mark.parametrize("linear", [0, 1])
 def test_reconstruction_of_small_stencils(host, offsets, linear):
-    """a stencil of zeros gives zeros; one whose every value is below 2^-959, and one that is not finite, is left to
-    the FP64 form; and smooth stencils through zero are taken"""
+    """a stencil of zeros gives zeros; one whose every value is below 2^-959 is held in units of 2^-1017 (a few of them
+    off in the traces), one that is not finite is left to the FP64 form; and smooth stencils through zero are taken"""
     rng = np.random.default_rng(8)
     s = np.zeros((6, 33))
     s[1] = 1e-300 * rng.uniform(0.5, 1, 33)
@@ -239,5 +239,7 @@ def test_reconstruction_of_small_stencils(host, offsets, linear):
     s[5] = np.sin(offsets @ [0.3, -0.2, 0.1] + 0.01)
     out = np.zeros((6, 25))
     host.t_recon(C.c_int(6), _p(s), C.c_int(linear), C.c_int(0), _p(out))
-    assert list(out[:, 0]) == [1, 0, 0, 0, 1, 1] and not out[0, 1:].any()
+    assert list(out[:, 0]) == [1, 1, 0, 0, 1, 1] and not out[0, 1:].any()
+    # the differences are far below 1e-12, so the weights are R4's
+    assert np.abs(out[1:2, 1:] - _exact_traces(s[1:2], offsets, 1)).max() <= 2.0 ** -1013
     assert np.abs(out[4:, 1:] - _exact_traces(s[4:], offsets, linear)).max() <= 4e-16
