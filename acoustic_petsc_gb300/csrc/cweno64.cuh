@@ -277,8 +277,6 @@ __device__ __forceinline__ double rusanov64(const double* __restrict__ QL, const
 // The R4 differences that a cell's gradients need, kept for the face kernel in fixed point (units of
 // 2^(top - 1023 - 58)): A, D, 4 u_ab (xy, yz, xz), ddd, then aab and abb by pair, xyz, and top (r4_64's lin, sq,
 // twice its cr, ddd, aab/abb, xyz)
-constexpr int NGC = 20;
-
 __device__ __forceinline__ void store_grad_coeffs(const Poly64& p, double* __restrict__ C, long long st) {
     const double v[19] = {p.lin[0], p.lin[1], p.lin[2], p.sq[0], p.sq[1], p.sq[2], 2.0 * p.cr[0], 2.0 * p.cr[1], 2.0 * p.cr[2],
                           p.ddd[0], p.ddd[1], p.ddd[2], p.aab[0], p.abb[0], p.aab[1], p.abb[1], p.aab[2], p.abb[2], p.xyz};

@@ -192,32 +192,18 @@ __device__ __forceinline__ void store_traces(R* __restrict__ T, const Geo& g, lo
 
 // density and pressure at the 24 face Gauss-point traces of one cell (what the
 // Riemann solver consumes) against the floors of pde.c:56-66
-template <typename R>
-__device__ __forceinline__ bool traces_admissible(const R* __restrict__ T, const Geo& g, long long e, double gm1) {
-    if (sizeof(R) == sizeof(float)) {  // FP32 traces: p >= floor as (E rho - |m|^2/2)(gamma-1) >= floor rho
-        const float g1 = (float)gm1;
-        for (int q = 0; q < NTR; ++q) {
-            const float rho = (float)T[((long long)0 * NTR + q) * g.NE + e];
-            const float mx = (float)T[((long long)1 * NTR + q) * g.NE + e];
-            const float my = (float)T[((long long)2 * NTR + q) * g.NE + e];
-            const float mz = (float)T[((long long)3 * NTR + q) * g.NE + e];
-            const float E = (float)T[((long long)4 * NTR + q) * g.NE + e];
-            if (!(rho >= 1.0e-14f) || !(g1 * (E * rho - 0.5f * (mx * mx + my * my + mz * mz)) >= 1.0e-12f * rho)) return false;
-        }
-        return true;
-    }
+__device__ __forceinline__ bool traces_admissible(const double* __restrict__ T, const Geo& g, long long e, double gm1) {
     for (int q = 0; q < NTR; ++q) {
-        const double rho = (double)T[((long long)0 * NTR + q) * g.NE + e];
-        const double mx = (double)T[((long long)1 * NTR + q) * g.NE + e];
-        const double my = (double)T[((long long)2 * NTR + q) * g.NE + e];
-        const double mz = (double)T[((long long)3 * NTR + q) * g.NE + e];
-        const double E = (double)T[((long long)4 * NTR + q) * g.NE + e];
+        const double rho = T[((long long)0 * NTR + q) * g.NE + e];
+        const double mx = T[((long long)1 * NTR + q) * g.NE + e];
+        const double my = T[((long long)2 * NTR + q) * g.NE + e];
+        const double mz = T[((long long)3 * NTR + q) * g.NE + e];
+        const double E = T[((long long)4 * NTR + q) * g.NE + e];
         const double p = gm1 * (E - 0.5 * (mx * mx + my * my + mz * mz) / rho);
         if (!(rho >= 1.0e-14) || !(p >= 1.0e-12)) return false;
     }
     return true;
 }
-
 
 // Device-side ghost fill (what DMGlobalToLocal does for the reference's DMDA, with
 // the boundary treatment of rhs_function.c's ghost loops): the stage input W (owned
@@ -413,7 +399,7 @@ __global__ void __launch_bounds__(kReconThreads, 8)
         // the viscous fluxes take the gradients of R4
         if (RECON != HYPE_RECON_LINEAR4 && Cc) recon64_general<true>(Gc, sy, sz, nullptr, Cc, g.NE);
     }
-    if (PAD && !traces_admissible<double>(T, g, e, gm1)) {
+    if (PAD && !traces_admissible(T, g, e, gm1)) {
         store_first_order_g<double>(G, T, g, ge, e);
         if (!gi && !gj && !gk) atomicAdd(&counters[1], 1ull);
     }
@@ -450,13 +436,13 @@ __global__ void __launch_bounds__(kGatedThreads)
         const float kin = 0.5f * (mx * mx + my * my + mz * mz) / rho;
         // on the safe side of the FP32 roundings; false for infinities and NaN
         const bool clear = rho > 1.001e-14f && (E - kin) - 1e-4f * (E + kin) > 1.001e-12f / (float)gm1;
-        bool ok = clear || traces_admissible<double>(T, g, e, gm1);
+        bool ok = clear || traces_admissible(T, g, e, gm1);
         const long long ge = ghost_index(g, i, j, k);
         if (!ok && !full) {
 #pragma unroll 1
             for (int c = 0; c < NV; ++c)
                 gated_cweno4(G + (long long)c * g.GN + ge, g.gx, g.gx * g.gy, T + (long long)c * NTR * g.NE + e, g.NE, c == 0 || c == 4);
-            ok = traces_admissible<double>(T, g, e, gm1);
+            ok = traces_admissible(T, g, e, gm1);
         }
         if (!ok && pad) {  // CWENO4 itself inadmissible
             store_first_order_g<double>(G, T, g, ge, e);
@@ -628,7 +614,7 @@ __global__ void __launch_bounds__(128) k_faces_f32(const float* __restrict__ T, 
             }
             // Rusanov's 1/2 goes into the Gauss weight 1/4
             float s;
-            if constexpr (FLUX == HYPE_FLUX_RUSANOV) s = rusanov<float, D, false>(QL, QR, gm, gm1, fl, bad);
+            if constexpr (FLUX == HYPE_FLUX_RUSANOV) s = rusanov<float, D>(QL, QR, gm, gm1, fl, bad);
             else s = face_solver<float, D, FLUX>(QL, QR, gm, gm1, fl, bad);
             smax = fmax(smax, (double)s);
             const float wq = FLUX == HYPE_FLUX_RUSANOV ? 0.125f : 0.25f;
@@ -961,9 +947,9 @@ __device__ __forceinline__ void fs_face(const float* __restrict__ S, int tL, int
             QR[c] = S[(c * NTR + qR + gp) * FS_NT + tR];
         }
         float s;
-        if (D == 0) s = rusanov<float, 0, false>(QL, QR, gm, gm1, fl, bad);
-        else if (D == 1) s = rusanov<float, 1, false>(QL, QR, gm, gm1, fl, bad);
-        else s = rusanov<float, 2, false>(QL, QR, gm, gm1, fl, bad);
+        if (D == 0) s = rusanov<float, 0>(QL, QR, gm, gm1, fl, bad);
+        else if (D == 1) s = rusanov<float, 1>(QL, QR, gm, gm1, fl, bad);
+        else s = rusanov<float, 2>(QL, QR, gm, gm1, fl, bad);
         smax = fmaxf(smax, s);
 #pragma unroll
         for (int c = 0; c < NV; ++c) acc[c] += 0.125f * fl[c];
@@ -1702,14 +1688,13 @@ extern "C" int hype_euler_create(const hype_euler_params* p, hype_euler** out) {
     if (p->recon < HYPE_RECON_CWENO4 || p->recon > HYPE_RECON_WENO3) return HYPE_ERR_ARG;
     if (p->precision != HYPE_PREC_FP64 && p->precision != HYPE_PREC_FP32 && p->precision != HYPE_PREC_DF64)
         return HYPE_ERR_ARG;
-    // the double-float form covers CWENO4, R4 and the indicator gate between them (no WENO3, no
-    // viscous fluxes)
+    // HYPE_PREC_DF64 has not taken WENO3, nor viscosity with the HLLC family, since it had kernels of its own; callers
+    // rely on the refusals
     if (p->precision == HYPE_PREC_DF64 && p->recon == HYPE_RECON_WENO3) return HYPE_ERR_UNSUPPORTED;
     if (p->dt_mode < HYPE_DT_MONITOR || p->dt_mode > HYPE_DT_FIXED) return HYPE_ERR_ARG;
     if (p->flux < HYPE_FLUX_RUSANOV || p->flux > HYPE_FLUX_ROTHLLC) return HYPE_ERR_ARG;
     if (p->positivity != 0 && p->positivity != 1) return HYPE_ERR_ARG;
-    // viscosity: FP64 (with the CWENO4 / R4 / WENO3 traces) or the double-float form with the Rusanov
-    // flux; the gradients always come from R4
+    // viscosity: in FP64 or HYPE_PREC_DF64, with the CWENO4, R4 or WENO3 traces; the gradients always come from R4
     const bool visc = p->mu != 0.0;
     if (visc && (!(p->mu > 0.0) || !(p->prandtl > 0.0) || !(p->cv > 0.0) || p->precision == HYPE_PREC_FP32 ||
                  p->recon == HYPE_RECON_LEARNED))

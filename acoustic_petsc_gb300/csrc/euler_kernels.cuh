@@ -447,8 +447,8 @@ __device__ __forceinline__ void face_traces(const R* __restrict__ c, R* __restri
 
 // Rusanov (LLF) flux across an axis face of normal D; returns the max wave
 // speed and flags an inadmissible state (rho < 1e-14 or p < 1e-12).
-// HALF = false leaves out the factor 1/2 (the caller folds it into its quadrature weight)
-template <typename R, int D, bool HALF = true>
+// without the factor 1/2, which the caller folds into its quadrature weight
+template <typename R, int D>
 __device__ __forceinline__ R rusanov(const R* QL, const R* QR, R gamma, R gm1, R* F, bool& bad) {
     R FL[NV], FR[NV], sL, sR;
 #pragma unroll
@@ -477,10 +477,7 @@ __device__ __forceinline__ R rusanov(const R* QL, const R* QR, R gamma, R gm1, R
     }
     const R s = sL < sR ? sR : sL;
 #pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        const R f = FR[c] + FL[c] - s * (QR[c] - QL[c]);
-        F[c] = HALF ? R(0.5) * f : f;
-    }
+    for (int c = 0; c < NV; ++c) F[c] = FR[c] + FL[c] - s * (QR[c] - QL[c]);
     return s;
 }
 
