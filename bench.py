@@ -254,7 +254,7 @@ def run_euler(args, ws, rank, local, precision=0, recon=0, n=256, flux=0, viscou
     launches = H.launches() - l0
     ms = e0.elapsed_time(e1)
     ms_max = _max_over_ranks(ws, ms)
-    # the state after the timed steps, for the double-float form beside this one (default workload)
+    # the state after the timed steps, for the FP32 form beside this one (default workload)
     with_alt = precision == 0 and recon == 0 and flux == 0 and not viscous and not args.no_alt_forms
     U_fp64 = s.get_state() if with_alt else None
     prof_ms = (C.c_double * 3)()
@@ -359,12 +359,12 @@ def run_euler(args, ws, rank, local, precision=0, recon=0, n=256, flux=0, viscou
         e2e = {"value": ws * cells * ke / (ms_e2e * 1e-3), "unit": "cell-updates/s", "h2d_bytes_per_step": nb,
                "d2h_bytes_per_step": nb, "steps": ke,
                "path": "EulerSolver.set_state -> step(1) -> get_state (hype_euler_upload/step/download)"}
-    # the double-float form (same initial state and steps), timed after the FP64 form's legs
+    # the FP32 form (same initial state and steps), timed after the FP64 form's legs; HYPE_PREC_DF64 runs the FP64
+    # kernels and has no leg of its own
     alt = None
     if with_alt:
         so = lambda h: torch.cuda.ExternalStream(L.hype_euler_stream(h))  # noqa: E731
-        alt = _euler_df64_beside(args, ws, n, U0, U_fp64, stream_of=so)
-        alt.update(_euler_df64_beside(args, ws, n, U0, U_fp64, stream_of=so, precision=1))
+        alt = _euler_fp32_beside(args, ws, n, U0, U_fp64, stream_of=so)
     del U_fp64
     clocks = clk.summary()
     s.close()
@@ -392,17 +392,15 @@ def run_euler(args, ws, rank, local, precision=0, recon=0, n=256, flux=0, viscou
     return out
 
 
-def _euler_df64_beside(args, ws, n, U0, U_fp64, stream_of, precision=2):
-    """another precision form of the same workload (default: HYPE_PREC_DF64, state, face fluxes and
-    stage accumulation in FP64, reconstruction and Rusanov flux in FP32 pairs on deviations; 1: the
-    fused FP32 stage), the same warm-up and timed steps from the same state, and its largest state
-    difference from the FP64 run"""
+def _euler_fp32_beside(args, ws, n, U0, U_fp64, stream_of):
+    """the FP32 form of the same workload (the fused stage), the same warm-up and timed steps from the same state, and
+    its largest state difference from the FP64 run"""
     import torch
 
     import acoustic_petsc_gb300 as H
 
     L = H.lib()
-    ctx = H.AppCtx(N_x=n, N_y=n, N_z=n, h=1.0 / n, CFL=0.4, precision=precision)
+    ctx = H.AppCtx(N_x=n, N_y=n, N_z=n, h=1.0 / n, CFL=0.4, precision=H._lib.PREC_FP32)
     d = H.EulerSolver(ctx)
     d.set_state(U0)
     d.step(max(args.warmup, 3))
@@ -423,16 +421,14 @@ def _euler_df64_beside(args, ws, n, U0, U_fp64, stream_of, precision=2):
     stages = max(prof_n[0], 1)
     diff = float(np.abs(d.get_state() - U_fp64).max() / np.abs(U_fp64).max())
     d.close()
-    tag = "df64" if precision == 2 else "fp32"
-    per = ({"recon": prof_ms[0] / stages, "faces": prof_ms[1] / stages, "update": prof_ms[2] / stages}
-           if precision == 2 else {"ghost": prof_ms[0] / stages, "stage_fused": prof_ms[1] / stages})
-    return {tag: {"value": ws * n**3 * args.steps / (ms * 1e-3), "unit": "cell-updates/s",
-                  "ms_per_step": ms / args.steps,
-                  "dtype": EULER_DTYPE[precision],
-                  "per_kernel_ms": per,
-                  "state_rel_linf_diff_vs_fp64": diff,
-                  "steps_compared": max(args.warmup, 3) + args.steps,
-                  "profile": "profiles/euler_stage_fp64.txt" if precision == 2 else "profiles/euler_stage_fp32.txt"}}
+    per = {"ghost": prof_ms[0] / stages, "stage_fused": prof_ms[1] / stages}
+    return {"fp32": {"value": ws * n**3 * args.steps / (ms * 1e-3), "unit": "cell-updates/s",
+                     "ms_per_step": ms / args.steps,
+                     "dtype": EULER_DTYPE[H._lib.PREC_FP32],
+                     "per_kernel_ms": per,
+                     "state_rel_linf_diff_vs_fp64": diff,
+                     "steps_compared": max(args.warmup, 3) + args.steps,
+                     "profile": "profiles/euler_stage_fp32.txt"}}
 
 
 def run_ctcs(args, ws, rank, local, n=512):
@@ -688,30 +684,8 @@ def run_blast(args, ws, rank, local, n=512, ntrain=64, tau=0.01, prob=0.2):
                      "flagged_per_cell_stage": flagged / (4.0 * cells) if form == "learned_fp64" else None}
         rho64[form] = s64.get_state()[..., 0]
     s64.close()
-    # 4. the same two forms with the double-float reconstruction and flux (FP64 error bars)
-    sdf = H.EulerSolver(H.AppCtx(N_x=n, N_y=n, N_z=n, h=1.0 / n, CFL=0.4, positivity=1,
-                                 precision=H._lib.PREC_DF64))
-    sdf.set_mlp(params, prob)
-    stream = torch.cuda.ExternalStream(L.hype_euler_stream(sdf._h))
-    for form, recon in (("plain_df64", H._lib.RECON_CWENO4), ("learned_df64", H._lib.RECON_LEARNED)):
-        sdf.set_recon(recon)
-        sdf.set_state(U0)
-        sdf.t, sdf.next_dt = 0.0, 0.0
-        sdf.step(1)
-        sdf.indicator_stats(reset=True)
-        e0.record(stream)
-        sdf.step(1)
-        e1.record(stream)
-        e1.synchronize()
-        msdf = _max_over_ranks(ws, e0.elapsed_time(e1))
-        flagged, fb = sdf.indicator_stats(reset=True)
-        res[form] = {"value": ws * cells / (msdf * 1e-3), "ms_per_step": msdf,
-                     "flagged_per_cell_stage": flagged / (4.0 * cells) if form == "learned_df64" else None}
-        rho64[form] = sdf.get_state()[..., 0]
-    sdf.close()
     ref64 = rho64["plain_fp64"]
     l1_64 = float(np.abs(rho64["learned_fp64"] - ref64).mean() / np.abs(ref64).mean())
-    l1_df = {f: float(np.abs(rho64[f] - ref64).mean() / np.abs(ref64).mean()) for f in ("plain_df64", "learned_df64")}
     del rho64, ref64
     v = res["learned_fp32_per_step"]["value"]
     peak, kind = _peaks()
@@ -735,10 +709,6 @@ def run_blast(args, ws, rank, local, n=512, ntrain=64, tau=0.01, prob=0.2):
             "l1_rho_learned_per_step_vs_plain_fp32": l1_step,
             "speedup_learned_fp64_vs_plain_fp64": res["learned_fp64"]["value"] / res["plain_fp64"]["value"],
             "l1_rho_learned_fp64_vs_plain_fp64_after_2_steps": l1_64,
-            "speedup_learned_df64_vs_plain_fp64": res["learned_df64"]["value"] / res["plain_fp64"]["value"],
-            "l1_rho_vs_plain_fp64_after_2_steps": {"plain_df64": l1_df["plain_df64"],
-                                                   "learned_df64": l1_df["learned_df64"],
-                                                   "learned_fp64": l1_64},
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                          "traffic": None},
             "gpu_launches": launches, "clocks": clocks}
@@ -863,14 +833,12 @@ def run_blast_stage_kernels(args, ws, rank, local, n=256, prob=0.2):
 def run_blast_horizon(args, ws, rank, local, n=512, nsteps=500, prob=0.2, smax_bound=3.0, fp32_only=False):
     """The blast workload to its full length: 512^3, 500 SSPRK(4,3) steps at a fixed dt
     (CFL 0.4 against a wave-speed bound of 3), every form timed and compared.
-    (a) distance from the FP64-bar reference at 512^3: L1(rho) of each form against the plain
-        double-float run (the plain FP64 run is too slow to take 500 steps here; the two agree to
-        round-off, shown over the first 50 steps);
+    (a) distance from the FP64 reference at 512^3: L1(rho) of each form against the plain FP64 run;
     (b) accuracy: the same problem at 256^3 (initial state = the 512^3 one averaged over 2^3 cells,
         250 steps of twice the dt) in every form, L1(rho) against the 512^3 reference averaged to
         256^3, and each form's error over plain CWENO4's in the same arithmetic (the 1.05 bar).
     fp32_only: the FP32 forms alone, against the plain FP32 run at 512^3 as the reference (1.2e-8 in
-    L1(rho) from the double-float one after the 500 steps; a few minutes instead of half an hour)."""
+    L1(rho) from the one held to FP64's error bars after the 500 steps; a few minutes instead of half an hour)."""
     import torch
 
     import acoustic_petsc_gb300 as H
@@ -888,21 +856,15 @@ def run_blast_horizon(args, ws, rank, local, n=512, nsteps=500, prob=0.2, smax_b
     if fp32_only:
         return _blast_horizon_fp32(H, n, nsteps, prob, dt, params, meta, U0, l1, ws, local)
     with Clocks(_gpu_index(local)) as clk:
-        ref, forms512["plain_df64"] = _blast_form(H, n, U0, P.PREC_DF64, P.RECON_CWENO4, params, prob, dt, nsteps)
+        ref, forms512["plain_fp64"] = _blast_form(H, n, U0, P.PREC_FP64, P.RECON_CWENO4, params, prob, dt, nsteps)
         for name, prec, recon in (("plain_fp32", P.PREC_FP32, P.RECON_CWENO4),
                                   ("learned_fp32", P.PREC_FP32, P.RECON_LEARNED),
                                   ("learned_fp32_per_step", P.PREC_FP32, P.RECON_LEARNED),
-                                  ("learned_df64", P.PREC_DF64, P.RECON_LEARNED)):
+                                  ("learned_fp64", P.PREC_FP64, P.RECON_LEARNED)):
             rho, forms512[name] = _blast_form(H, n, U0, prec, recon, params, prob, dt, nsteps,
                                               per_step=name.endswith("per_step"))
-            forms512[name]["l1_rho_vs_plain_df64"] = l1(rho, ref)
+            forms512[name]["l1_rho_vs_plain_fp64"] = l1(rho, ref)
             del rho
-        # the double-float reference against plain FP64 over the first 50 steps
-        r64, f64 = _blast_form(H, n, U0, P.PREC_FP64, P.RECON_CWENO4, params, prob, dt, 50)
-        rdf, _ = _blast_form(H, n, U0, P.PREC_DF64, P.RECON_CWENO4, params, prob, dt, 50)
-        f64["l1_rho_vs_plain_df64_after_50_steps"] = l1(rdf, r64)
-        forms512["plain_fp64_50_steps"] = f64
-        del r64, rdf
         # (b) 256^3 from the averaged initial state, against the averaged 512^3 reference
         m = n // 2
         U1 = U0.reshape(m, 2, m, 2, m, 2, 5).mean(axis=(1, 3, 5))
@@ -914,9 +876,7 @@ def run_blast_horizon(args, ws, rank, local, n=512, nsteps=500, prob=0.2, smax_b
                                   ("learned_fp64", P.PREC_FP64, P.RECON_LEARNED),
                                   ("plain_fp32", P.PREC_FP32, P.RECON_CWENO4),
                                   ("learned_fp32", P.PREC_FP32, P.RECON_LEARNED),
-                                  ("learned_fp32_per_step", P.PREC_FP32, P.RECON_LEARNED),
-                                  ("plain_df64", P.PREC_DF64, P.RECON_CWENO4),
-                                  ("learned_df64", P.PREC_DF64, P.RECON_LEARNED)):
+                                  ("learned_fp32_per_step", P.PREC_FP32, P.RECON_LEARNED)):
             rho, forms256[name] = _blast_form(H, m, U1, prec, recon, params, prob, 2.0 * dt, nsteps // 2,
                                               per_step=name.endswith("per_step"))
             forms256[name]["l1_rho_error_vs_512_reference"] = l1(rho, ref_c)
@@ -939,7 +899,7 @@ def run_blast_horizon(args, ws, rank, local, n=512, nsteps=500, prob=0.2, smax_b
             "speedup_learned_fp32_vs_plain_fp32": v / forms512["plain_fp32"]["value"],
             "speedup_learned_fp32_per_step_vs_plain_fp32": (forms512["learned_fp32_per_step"]["value"] /
                                                             forms512["plain_fp32"]["value"]),
-            "speedup_learned_fp32_vs_plain_fp64": v / forms512["plain_fp64_50_steps"]["value"],
+            "speedup_learned_fp32_vs_plain_fp64": v / forms512["plain_fp64"]["value"],
             "gpu_launches": None, "clocks": clk.summary()}
 
 
@@ -1117,7 +1077,7 @@ def run_acoustic(args, ws, rank, local, n=256, precision=0):
     return {"metric": "cell-updates/s", "value": value, "unit": "cell-updates/s", "n_gpus": ws, "steps": args.steps,
             "warmup": max(args.warmup, 3), "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None,
-            "dtype": "f64" if precision == 0 else "f64 state / df64 (FP32 pairs) gradients and fluxes",
+            "dtype": "f64",  # the R4 star, in both precisions
             "data": "synthetic plane wave sin(x+y+z), exact cell-centre values",
             "config": {"workload": f"acoustic_fv_plane_wave_{n}" + ("_df64" if precision else ""), "grid": [n, n, n],
                        "cfl": 0.5,
@@ -1414,7 +1374,7 @@ def main():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--workload", default="euler256", choices=sorted(WORKLOADS))
     ap.add_argument("--no-alt-forms", action="store_true",
-                    help="skip the double-float form measured beside the default FP64 Euler workload")
+                    help="skip the FP32 form measured beside the default FP64 Euler workload")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--grid", type=int, default=0,
                     help="cells per axis of the 3D Euler / Navier-Stokes workloads (default 256; smaller for profiling)")
