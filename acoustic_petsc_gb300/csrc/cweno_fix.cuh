@@ -18,11 +18,13 @@
 // FP64 237.7 ms; integers with the weights in FP64 (67 operations) 80.3; that with products of 32-bit halves
 // 76.7; integer weights 73; conversions by instruction 66.4; eps added once 63.0.
 // Errors against 128-bit arithmetic, for stencils of a jump with noise beside it: 0.9e-16 of the stencil's largest
-// magnitude, where the FP64 form has 2 to 4e-16; and of the traces themselves 5e-16, as the FP64 form's, however quiet
-// the cell.  For that the FP64 form keeps the cells whose density, energy or pressure lies four or more binary
-// exponents below its stencil's largest (from a factor 8 to 16 on) or whose polynomial, of any variable, the nonlinear
-// weights leave below 2^-4 of it (faint); and stencils that are not finite.  With R4 alone a trace holds 1/64 of the
-// largest at least, and 3e-15 of itself.
+// magnitude, where the FP64 form has 2 to 4e-16; and of the traces themselves 5e-16 down to a tenth of it, as the FP64
+// form's.  Cells that are quieter than that beside a jump keep the FP64 form, whose errors stay relative to the cell:
+// where density, energy or pressure lies four or more binary exponents below its stencil's largest (from a factor 8 to
+// 16 on), and where the nonlinear weights leave the polynomial of any variable below 2^-6 of it (faint; up to there
+// 3e-15 of the traces; nearer, a few cells of a smooth pulse would take it too, and on a small grid a few decide: 16^3
+// 0.78 -> 0.94 ms for eight steps at 2^-4).  With R4 alone a trace holds 1/64 of the largest at least.  Stencils that
+// are not finite take the FP64 form too.
 #pragma once
 
 #include "cweno64.cuh"
@@ -55,13 +57,13 @@ __host__ __device__ __forceinline__ bool fix_applies(double u0, int top, bool st
     return top <= 2000 && !(strict && (((int)(bits_of(u0) >> 52) & 0x7FF) < top - 3));
 }
 // whether the polynomial is so much smaller than its stencil (a quiet cell beside a jump: the weights far from linear,
-// cell value and limited derivatives below 2^-4 of the largest's power of two) that the stencil's units do not resolve
+// cell value and limited derivatives below 2^-6 of the largest's power of two) that the stencil's units do not resolve
 // it as FP64 does; on the upper words
 __host__ __device__ __forceinline__ bool faint(const PolyFix& p) {
     auto mag = [](i64 x) { return (unsigned)((int)(x >> 32) ^ (int)(x >> 63)); };
     const unsigned l = mag(p.lin[0]) | mag(p.lin[1]) | mag(p.lin[2]), q = mag(p.sq[0]) | mag(p.sq[1]) | mag(p.sq[2]),
                    x = mag(p.cr2[0]) | mag(p.cr2[1]) | mag(p.cr2[2]);
-    return p.wr < 1ull << 60 && (mag(p.u0) | (l >> 2) | (q >> 3) | (x >> 4)) < 1u << (58 - 4 - 32);
+    return p.wr < 1ull << 60 && (mag(p.u0) | (l >> 2) | (q >> 3) | (x >> 4)) < 1u << (58 - 6 - 32);
 }
 
 template <bool LINEAR>

@@ -201,10 +201,10 @@ def offsets(host):
 def test_reconstruction_of_a_quiet_cell_beside_a_jump(host, offsets, linear, strict, quiet):
     """the traces where the fixed-point form takes the stencil, against extended precision.  The values' units are
     2^-58 of the largest one's power of two and the smoothness indicators' 2^-55, which moves weights between the
-    stencils by 2^-52 or so of it (2.2e-16): 4e-16 of the largest.  A polynomial that the weights leave below 2^-4 of
+    stencils by 2^-52 or so of it (2.2e-16): 4e-16 of the largest.  A polynomial that the weights leave below 2^-6 of
     the largest, and with `strict` (density, energy, pressure) a cell four binary exponents below it, is left to the
-    FP64 form, so that is 16 times as much of the traces or the cell, however small they are.  R4 keeps 1/64 of the
-    largest in its traces"""
+    FP64 form, and R4 keeps 1/64 of the largest in its traces: 64 (`strict`: 16) times as much of the traces or the
+    cell, however small they are"""
     rng = np.random.default_rng(7)
     n = 1500
     normal = rng.standard_normal((n, 3))
@@ -221,7 +221,7 @@ def test_reconstruction_of_a_quiet_cell_beside_a_jump(host, offsets, linear, str
     err = np.abs(out[:, 1:] - _exact_traces(s, offsets, linear)).max(axis=1)[taken]
     size = np.maximum(np.abs(out[:, 1:]).max(axis=1), np.abs(s[:, 0]))[taken]
     assert (err <= 4e-16 * np.abs(s).max(axis=1)[taken]).all()
-    assert (err <= 4e-16 * (64 if linear and not strict else 16) * size).all()
+    assert (err <= 4e-16 * (16 if strict else 64) * size).all()
     if taken.any():
         print(f"linear {linear} strict {strict} quiet {quiet:g}: {taken.mean():.3f} taken, {float((err / size).max()):.2e} of the traces")
 
