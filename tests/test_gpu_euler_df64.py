@@ -222,3 +222,22 @@ def test_smallest_grids_both_forms(hype, oracle, shape, bc):
         s.set_state(U)
         s.step(2)
         assert rel(s.get_state(), Uo) <= TOL_STEP
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(recon=1), dict(flux=1), dict(flux=2, recon=1), dict(mu=0.01, recon=1),
+                                dict(mu=0.01), dict(recon=2, positivity=1)], ids=str)
+def test_df64_is_the_fp64_form(hype, kw):
+    """HYPE_PREC_DF64 runs the FP64 kernels: the same bits, times and counts for every combination that it takes.  What
+    it is held to is checked against the checker and the recorded references, not against the FP64 form"""
+    from acoustic_petsc_gb300 import indicator, workloads
+
+    n = 14
+    out = []
+    for prec in (hype._lib.PREC_FP64, hype._lib.PREC_DF64):
+        s = _solver(hype, n, precision=prec, **kw)
+        if kw.get("recon") == hype._lib.RECON_LEARNED:
+            s.set_mlp(indicator.init_params(5), 0.2)
+        s.set_state(workloads.euler_blast(n, p_ratio=3.0, rho_ratio=2.0, r0=0.25))
+        s.step(3)
+        out.append((s.get_state(), s.t, s.next_dt, s.indicator_stats()))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
