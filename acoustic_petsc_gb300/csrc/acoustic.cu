@@ -318,9 +318,10 @@ __global__ void __launch_bounds__(256) k_ac_update(const double* __restrict__ Fx
 // (R4's derivatives, reconstruction.c:90-108, the central flux pde.c:12-34), so a stage is
 //   out_u = a U_u + b W_u + c dt W_v,   out_v = a U_v + b W_v + c dt c^2 / h^2 (sum over x, y, z).
 // In units of k / 48 the sum is 49 (s1 - 6 w) + 2 s2 - s3 - 6 w over the six, twice six and three directions:
-// integer coefficients, so it is formed exactly on the 19 values in fixed point (fixed.cuh; units of 2^-56 of the
-// largest one's power of two, exact for values within 2^-4 of it) and rounded once.  Stencils that are not
-// finite or beyond 2^877 take the same sum in FP64, differences to w first.
+// integer coefficients, so its two parts, s1 - 6 w and the rest, are formed exactly on the 19 values in fixed point
+// (fixed.cuh; units of 2^-56 of the largest one's power of two, exact for values within 2^-4 of it); each is rounded
+// as it is converted, and their sum once more.  Stencils that are not finite or beyond 2^877 take the same sum in
+// FP64, differences to w first.
 //
 // Bound: what the integer pipe (about 400 instructions a cell) and the FP64 pipe (5 to 9 operations) leave each
 // other; all in FP64 the star was 26 to 30 operations and the polynomial form about 280 with its trace and flux

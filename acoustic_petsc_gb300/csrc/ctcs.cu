@@ -79,7 +79,10 @@ __device__ __forceinline__ double scale2(double x) {
 // of k_plane2d, and writes the tile's two newest levels.  po, pc and no, nc are different arrays.
 // A launch per step took 6.3 us at 512^2 (9 FP64 operations a node need 4.0 of it) and 2.0 at 48 x 40; here it is 7
 // operations (the products by 2 and 4 are exponent additions), the frame's share and a quarter of the launches:
-// 5.3 and 1.05 us a step; 1200 x 1100 25.0 -> 22.4.  512 threads: 256 leave the FP64 pipe waiting (6.0 us).
+// 5.3 and 1.05 us a step; 1200 x 1100 25.0 -> 22.4.  512 threads: 256 leave the FP64 pipe waiting (6.0 us).  The frame
+// makes 1.17 times the updates at 512^2 and up to 1.36 where tiles fit the SMs badly, which takes back what the fewer
+// operations give; what stays is the launches: 300^2 3.5 -> 2.7 us a step, 400^2 4.8 -> 4.3, 600^2 8.2 -> 7.4 (zero
+// exterior 7.7), 800^2 12.9 -> 11.9 (12.2), 2000^2 71 -> 67, 4000^2 277 -> 251.
 constexpr int kSteps = 4, kTileRows = 32, kPlaneThreads = 512;
 
 template <int BX>
