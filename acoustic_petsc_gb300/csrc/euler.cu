@@ -1782,8 +1782,9 @@ extern "C" void hype_euler_destroy(hype_euler* e) {
     if (!e) return;
     if (e->stream) cudaStreamSynchronize(e->stream);
     cudaFree(e->U); cudaFree(e->W); cudaFree(e->L); cudaFree(e->S); cudaFree(e->T);
+    if (e->bound64 != (float*)e->stage_aos) cudaFree(e->bound64);
     cudaFree(e->Fx); cudaFree(e->Fy); cudaFree(e->Fz); cudaFree(e->stage_aos); cudaFree(e->ds); cudaFree(e->G);
-    cudaFree(e->mlp); cudaFree(e->gate); cudaFree(e->gate_wide); cudaFree(e->flag64); cudaFree(e->bound64); cudaFree(e->mlp_cnt); cudaFree(e->C4); cudaFree(e->mon); cudaFree(e->acc);
+    cudaFree(e->mlp); cudaFree(e->gate); cudaFree(e->gate_wide); cudaFree(e->flag64); cudaFree(e->mlp_cnt); cudaFree(e->C4); cudaFree(e->mon); cudaFree(e->acc);
     if (e->hs) cudaFreeHost(e->hs);
     for (auto x : e->ev) cudaEventDestroy(x);
     if (e->step_graph) cudaGraphExecDestroy(e->step_graph);
@@ -2021,7 +2022,11 @@ extern "C" int hype_euler_set_mlp(hype_euler* e, const float* params, float prob
     // before the network, whose presence lets the gated kernels run
     if (!e->bound64 && e->p.precision != HYPE_PREC_FP32) {
         if (!e->flag64) HYPE_CK(cudaMalloc((void**)&e->flag64, (size_t)e->g.NE));
-        HYPE_CK(cudaMalloc((void**)&e->bound64, sizeof(float) * NV * (size_t)e->g.NE));
+        // the bounds lie in the staging array of the host copies, which are in the same stream; grids under 8 cells
+        // a side need one of their own
+        const size_t need = sizeof(float) * NV * (size_t)e->g.NE;
+        if (need <= sizeof(double) * NV * (size_t)e->g.N) e->bound64 = (float*)e->stage_aos;
+        else HYPE_CK(cudaMalloc((void**)&e->bound64, need));
     }
     if (!e->mlp) HYPE_CK(cudaMalloc((void**)&e->mlp, sizeof(mlp::MmaWeights)));
     if (!e->gate && e->p.precision == HYPE_PREC_FP32) {
