@@ -43,8 +43,7 @@ struct Inst {
     double a;        // (c0 dt / h)^2: weight of the neighbours
     double b;        // 2 - 4a: weight of the centre
     double k2;       // c0*c0*dt*dt
-    euler::Split a62;  // a 2^(64 - up), in [2^61, 2^62]
-    int up;            // 0 to 2
+    euler::Split a62;  // a 2^62
     int top_max;       // largest biased exponent the fixed-point update takes
 };
 
@@ -63,7 +62,7 @@ struct Work {
 // and one conversion, 2 FP64 operations and about 150 integer instructions a node (48 instances of 64 to 768
 // nodes a side, a step 36.7 -> 26.6 us).  Values that are not finite or
 // beyond 2^977 take the six operations, and so do a > 1 (unstable) and a < 1/8 (CFL below 0.35): ahead of a wave the
-// new value is a times a neighbour, of which the units are then a larger part than FP64's rounding.
+// new value is a times a neighbour, of which the product's four units of 2^-58 are then more than FP64's rounding.
 // the step index is the class's counter (advanced once per graph chunk) plus s_off
 // a call, so that its operations are not issued where they are not needed
 static __device__ __noinline__ double advance_fp64(double a, double b, double c, double po, double e, double w, double n, double s) {
@@ -78,7 +77,7 @@ __device__ __forceinline__ double advance(const Inst& I, double c, double po, do
     auto fx = [&](double x) { return euler::to_fixed<6>(euler::bits_of(x), top); };
     const i64 ic = fx(c);
     const i64 lap = (fx(e) + fx(w)) + (fx(n) + fx(s)) - 4 * ic;
-    return euler::from_fixed(2 * ic - fx(po) + (euler::scaled(lap, I.a62) << I.up), top);
+    return euler::from_fixed(2 * ic - fx(po) + 4 * euler::scaled(lap, I.a62), top);
 }
 
 template <int TX, int TY, int R>
@@ -486,8 +485,7 @@ extern "C" int hype_batch_create(int ninst, const hype_mono_instance* in, hype_b
         I.a = I.k2 / (m.h * m.h);
         const bool fixed = I.a >= 0.125 && I.a <= 1.0;
         I.top_max = fixed ? 2000 : -1;
-        I.up = I.a >= 0.5 ? 2 : I.a >= 0.25 ? 1 : 0;
-        I.a62 = euler::split(fixed ? (euler::i64)ldexp(I.a, 64 - I.up) : 0);
+        I.a62 = euler::split(fixed ? (euler::i64)ldexp(I.a, 62) : 0);
         I.b = 2.0 - 4.0 * I.a;
         b->inst.push_back(I);
         off += ((long long)m.nx * m.ny + 31) / 32 * 32;  // 256-byte aligned instance starts

@@ -127,7 +127,7 @@ def test_update_scales(hype, scale):
 @pytest.mark.parametrize("cfl", [0.7, 0.5, 0.36, 0.35, 0.2, 0.05, 1e-3])
 def test_update_ahead_of_a_wave(hype, cfl):
     """one step from a single value: its four neighbours are a times it, a = (c0 dt / h)^2, to the rounding of FP64 or,
-    in the fixed-point form (a >= 1/8), two units of 2^-58 of the value: 2^-52 either way, 2^-51 with the product
+    in the fixed-point form (a >= 1/8), four units of 2^-58 of the value: 2^-52 either way, 2^-51 with the product
     that the comparison forms"""
     n, h = 33, 0.05
     rng = np.random.default_rng(4)
