@@ -14,9 +14,10 @@
 //    o_+ dp, o_- dm and (o_+ - o_-) aab;
 //  * the traces are sums of integers with products by fixed-point constants, rounded to FP64 once by the
 //    conversion instruction (the FP64 pipe's only work here).
-// About 4300 instructions a warp and variable against 361 FP64 ones of 64 cycles.  At 256^3, four stages: all in
+// About 4400 instructions a warp and variable against 361 FP64 ones of 64 cycles.  At 256^3, four stages: all in
 // FP64 237.7 ms; integers with the weights in FP64 (67 operations) 80.3; that with products of 32-bit halves
-// 76.7; integer weights 73; conversions by instruction 66.4; eps added once 63.0.
+// 76.7; integer weights 73; conversions by instruction 66.4; eps added once 63.0; the FP64 form as a call 61.1; weights
+// completed to one 62.4.
 // Errors against 128-bit arithmetic, for stencils of a jump with noise beside it: 0.9e-16 of the stencil's largest
 // magnitude, where the FP64 form has 2 to 4e-16; and of the traces themselves 5e-16 down to a tenth of it, as the FP64
 // form's.  Cells that are quieter than that beside a jump keep the FP64 form, whose errors stay relative to the cell:

@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(128, 4)
 // 183 warps of one serial 2300-instruction thread each took 87 us).  kReconThreads is small so that few blocks
 // spread evenly over the SMs.  Bound: integer issue and its latencies (4000 instructions a warp, 60 % of the issue
 // slots taken).  256^3, four stages: 61.1 ms at 128 registers (16 warps per SM), 63.5 at 168, 64 to 66 at 112 and
-// 96; all in FP64 237.7.
+// 96; all in FP64 237.7.  62.4 since the weights are completed to one and faint polynomials looked for.
 constexpr int kReconThreads = 64;
 
 // The FP64 form of one variable in one cell: its traces and, with C, its R4 differences.  A call of its own,
@@ -419,7 +419,8 @@ static void launch_recon64(const Geo& g, const double* G, double* T, int recon, 
 // cells), the 24 traces need not be read.  A cell whose R4 traces break them is redone here with CWENO4, then first
 // order with the fallback.
 // 256^3 blast: one kernel for scoring, a cell's variables in turn, and a check that read its 120 traces back, ran at
-// 104.8 M cell-updates/s, below CWENO4 without a gate; a block of 32 cells x 5 variables for all of it at 134.7 M; this, with k_gate's flags, 197.4 M.
+// 104.8 M cell-updates/s, below CWENO4 without a gate; a block of 32 cells x 5 variables for all of it at 134.7 M; this,
+// with k_gate's flags, 197.8 M.
 constexpr int kGatedThreads = 128;
 __global__ void __launch_bounds__(kGatedThreads)
     k_gated_check(const double* __restrict__ G, double* __restrict__ T, Geo g, double gm1, int pad,

@@ -226,8 +226,8 @@ int hype_euler_shadow_step(hype_euler* e, double* t_inout, double* dt_inout, dou
  *     returns the bound); larger grids return HYPE_ERR_ARG.
  *   - Options: CWENO4, R4 or WENO3; FP64 or FP32 reconstruction and flux; any flux;
  *     the positivity fallback (p->positivity 0 or 1) as in the context path.  No
- *     viscous terms (p->mu != 0 returns HYPE_ERR_UNSUPPORTED), no double-float form
- *     and no learned indicator (both need per-context state).
+ *     viscous terms (p->mu != 0 returns HYPE_ERR_UNSUPPORTED), no HYPE_PREC_DF64
+ *     and no learned indicator (they need a context).
  *   - The first call on a device looks up the array's device address (once per
  *     device, with that device current) and keeps it for the life of the process;
  *     make that first call before any stream capture.  cudaDeviceReset (or any
@@ -321,8 +321,8 @@ typedef struct {
     double dt;  /* fixed time step (hype.c:56: h CFL / (3 c)) */
     int bc[6];  /* HYPE_BC_PERIODIC or HYPE_BC_ADIABATIC */
     int recon;  /* HYPE_RECON_LINEAR4 (the reference's setting) or HYPE_RECON_CWENO4 */
-    int precision; /* HYPE_PREC_FP64, or HYPE_PREC_DF64: reconstruction, gradients and face fluxes in double-float
-                      (FP32 pairs), state and stage accumulation in FP64 */
+    int precision; /* HYPE_PREC_FP64, or HYPE_PREC_DF64: with CWENO4, reconstruction, gradients and face fluxes in
+                      double-float (FP32 pairs), state and stage accumulation in FP64; R4 runs the FP64 star */
 } hype_acoustic_params;
 
 int hype_acoustic_create(const hype_acoustic_params* p, hype_acoustic** out);
