@@ -414,7 +414,7 @@ def _jump_state(kind, n=13):
                                              ("density", 0), ("energy", 0), ("nan", 0), ("nan", 1)])
 def test_reconstruction_outside_the_fixed_point_form(hype, oracle, precision, recon, kind, positivity):
     """states that send cells to the FP64 form of the reconstruction, without viscosity (no gradient array to write to):
-    the right-hand side against the checker's, to the FP64 path's bar of 1e-12 of its largest; where the checker
+    the right-hand side against the oracle's, to the FP64 path's bar of 1e-12 of its largest; where the oracle
     refuses the state (traces below the floors, with no fallback), and for a state that is not finite, the status says
     so and is no CUDA error"""
     n = 13
@@ -439,7 +439,7 @@ def test_reconstruction_outside_the_fixed_point_form(hype, oracle, precision, re
 @pytest.mark.parametrize("precision", [L.PREC_FP64, L.PREC_DF64])
 def test_vanishing_momenta_in_a_dense_gas(hype, oracle, precision):
     """momenta at the end of FP64's range over densities of 1000: the velocities are below the smallest normal number.
-    The right-hand side stays what the checker gives, to 1e-12 of its largest; its momenta carry the pressure alone"""
+    The right-hand side stays what the oracle gives, to 1e-12 of its largest; its momenta carry the pressure alone"""
     n = 12
     rng = np.random.default_rng(5)
     U = np.zeros((n, n, n, 5))
@@ -455,7 +455,7 @@ def test_vanishing_momenta_in_a_dense_gas(hype, oracle, precision):
 def test_weak_shear_under_a_uniform_pressure(hype, oracle, precision):
     """a velocity of 1e-14 that varies along x alone in a uniform stream: the pressure's flux is the same on both sides
     of every cell and cancels exactly, so the shear's own flux differences keep their accuracy: 1e-12 of their
-    largest against the checker, the FP64 path's bar, for that component alone"""
+    largest against the oracle, the FP64 path's bar, for that component alone"""
     n = 16
     x = (np.arange(n) + 0.5) / n
     U = np.zeros((n, n, n, 5))

@@ -228,7 +228,7 @@ def test_smallest_grids_both_forms(hype, oracle, shape, bc):
                                 dict(mu=0.01), dict(recon=2, positivity=1)], ids=str)
 def test_df64_is_the_fp64_form(hype, kw):
     """HYPE_PREC_DF64 runs the FP64 kernels: the same bits, times and counts for every combination that it takes.  What
-    it is held to is checked against the checker and the recorded references, not against the FP64 form"""
+    it is held to is checked against the oracle and the recorded references, not against the FP64 form"""
     from acoustic_petsc_gb300 import indicator, workloads
 
     n = 14

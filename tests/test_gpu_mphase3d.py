@@ -142,7 +142,7 @@ def test_mp3d_rejects_bad_parameters(hype):
 
 def test_mp3d_wave_speeds_beside_nan(hype, oracle):
     """a plane of NaN at i = 0, the first lane of every warp that runs along x, leaves the speed maximum to the finite
-    faces, the fast cells of row j = k = 0 among them: dt is the checker's to its rounding (no comparison with a NaN
+    faces, the fast cells of row j = k = 0 among them: dt is the oracle's to its rounding (no comparison with a NaN
     holds there)"""
     n = (32, 4, 4)
     V = np.zeros((n[2], n[1], n[0], 6))

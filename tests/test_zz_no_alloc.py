@@ -163,7 +163,7 @@ def test_noalloc_positivity_fallback(hype, prec):
 @pytest.mark.parametrize("recon", [0, 1])
 def test_noalloc_outside_the_fixed_point_form(hype, oracle, recon):
     """the pressure-ratio-10 blast, whose energy jump of four binary exponents takes the reconstruction's FP64 form,
-    against the CPU checker's right-hand side"""
+    against the oracle's right-hand side"""
     torch = pytest.importorskip("torch")
     from acoustic_petsc_gb300 import workloads
 
