@@ -347,7 +347,8 @@ extern "C" int hype_ctcs_create(const hype_ctcs_params* p, hype_ctcs** out) {
         cudaGetLastError();
     }
     // a level beyond these is written whole before it is read
-    for (int q = 0; q < (c->paired() ? 2 : 3) && e == cudaSuccess; ++q) e = cudaMemset(c->lv[q], 0, sizeof(double) * c->n);
+    for (int q = 0; q < (c->paired() ? 2 : 3) && e == cudaSuccess; ++q) e = cudaMemsetAsync(c->lv[q], 0, sizeof(double) * c->n, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);  // before the caller's first copy, from whatever stream
     int dev = 0, nsm = 1;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

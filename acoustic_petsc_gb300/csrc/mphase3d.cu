@@ -777,7 +777,7 @@ extern "C" int hype_mp3d_create(const hype_mp3d_params* p, hype_mp3d** out) {
     al(&m->Fy, sizeof(double) * MF * (size_t)g.nx * (g.ny + 1) * g.nz);
     al(&m->Fz, sizeof(double) * MF * (size_t)g.nx * g.ny * (g.nz + 1));
     if (ce == cudaSuccess) ce = cudaMalloc((void**)&m->fail, (size_t)g.NE);
-    if (ce == cudaSuccess) ce = cudaMemset(m->fail, 0, (size_t)g.NE);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(m->fail, 0, (size_t)g.NE, m->stream);
     if (ce == cudaSuccess) ce = cudaMalloc((void**)&m->ds, sizeof(DevScalars));
     if (ce == cudaSuccess) ce = cudaMallocHost((void**)&m->hs, sizeof(DevScalars));
     if (ce == cudaSuccess) {
